@@ -538,7 +538,7 @@ void enqueue_np(cc_ctx *c, const NpArgs &a, uint64_t P_cap, const unsigned long 
 		launch_np_compact(P_cap, P_dev, sc, reinterpret_cast<long long *>(a.pairs), a.norm, a.cpta, a.cptb, a.depth,
 		                  a.bids, &ptr<DevStats>(c->stats)->contacts, P_dev ? hint_P(c) : P_cap, s);
 	}
-	c->launches += 3;  // class grouping, MPR, compaction
+	c->launches += c->np_precision == CC_NP_EXACT ? 2 : 3;  // class grouping (fast modes), MPR, compaction
 }
 
 // The step after the pair test with the narrowphase overlapped (one scene):
@@ -567,7 +567,7 @@ cc_status enqueue_sort_and_np_overlapped(cc_ctx *c, uint64_t n, const NpArgs &a,
 		launch_scan_owner(n, b, s);
 		c->launches += 1;
 	}
-	c->launches += 2;  // class grouping, MPR
+	c->launches += c->np_precision == CC_NP_EXACT ? 1 : 2;  // class grouping (fast modes), MPR
 	enqueue_emit(c, n, reinterpret_cast<unsigned long long *>(a.pairs), pairs_cap, s);
 	CC_CUDA(c, cudaStreamWaitEvent(s, c->ev_join, 0));
 	{

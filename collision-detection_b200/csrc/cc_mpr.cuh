@@ -1,16 +1,18 @@
 // Minkowski portal refinement (the reference's CollideAndFindPoint,
-// src/narrowphase/Narrowphase.cu:122-314, inside function_MPR_Store :316-423)
-// as a per-lane state machine with warp-level work stealing.
+// src/narrowphase/Narrowphase.cu:122-314, inside function_MPR_Store :316-423):
+// shapes, support maps and the contact store of every precision mode, and the
+// fast modes' per-lane state machine with warp-level work stealing. The exact
+// mode's kernel is in cc_mpr_exact.cu.
 //
-// Every loop iteration, each busy lane evaluates exactly ONE support pair
-// (support(A, -d), support(B, d)) and then updates its MPR state; a lane whose
-// pair is finished writes its contact and takes the next pair from a global
-// queue (pairs pre-grouped by shape-type combination). The warp therefore runs
-// the same support code on most of its lanes in every iteration instead of
-// idling while a few pairs refine to the iteration cap.
+// Every loop iteration of run(), each busy lane evaluates exactly ONE support
+// pair (support(A, -d), support(B, d)) and then updates its MPR state; a lane
+// whose pair is finished writes its contact and takes the next pair from a
+// global queue (pairs pre-grouped by shape-type combination). The warp
+// therefore runs the same support code on most of its lanes in every iteration
+// instead of idling while a few pairs refine to the iteration cap.
 //
-// Template parameters:
-//   S       scalar of the support maps (double or float)
+// Template parameters of the support maps:
+//   S       their scalar (double or float)
 //   kExact  true:  the FP64 oracle's arithmetic exactly — world coordinates,
 //                  every direction normalized before the support map,
 //                  normalize = v / sqrt(v.v), the reference's operation order;
@@ -20,7 +22,7 @@
 //           false: pair-local frame (origin = body A's position), one
 //                  reciprocal square root per normalization, fused
 //                  multiply-add allowed.
-// Portal arithmetic is FP64 in every variant.
+// Portal arithmetic is FP64 in every mode.
 #pragma once
 #include "cc_common.cuh"
 #include "cc_internal.h"
@@ -100,35 +102,6 @@ __device__ __forceinline__ vec<T> unit(vec<T> a) {
 		const T il = rsqrt(dotp(a, a));
 		return {a.x * il, a.y * il, a.z * il};
 	}
-}
-
-// a / sqrt(a.a) in double with IEEE results, without the square root and the
-// reciprocal when a.a lies within 2^20 units in the last place of 1 (a vector
-// normalized once already). With s = a.a whose bits are bits(1) + e:
-//  * sqrt(s) has the bits bits(1) + floor(e / 2). For s = 1 + t, sqrt(s) lies
-//    strictly below 1 + t/2 (concavity) and above 1 + t/2 - t^2/8. Above 1
-//    (t = e 2^-52) 1 + t/2 is representable for even e and a midpoint for odd
-//    e; below 1 (t = e 2^-53, spacing 2^-53) the same holds with the halved
-//    spacing. Either way the correctly rounded root is the representable
-//    number at or just below 1 + t/2, t^2/8 being far below half a spacing.
-//  * RN(1 / l) for l with the bits bits(1) + f: for f >= 0, 1/l lies above
-//    1 - f 2^-52 (representable, bits(1) - 2f) by less than f^2 2^-104, under
-//    half the spacing 2^-53 below 1; for f < 0, 1/l lies strictly above
-//    1 - f 2^-53, which is representable (bits(1) - f/2) for even f and a
-//    midpoint for odd f, so RN gives bits(1) + ceil(-f / 2) = bits(1) -
-//    floor(f / 2).
-// The quotients then follow quot_rcp (Markstein) as in div3, so the result is
-// bit for bit unit<double, true>(a).
-__device__ __forceinline__ vec<double> unit_again(vec<double> a) {
-	constexpr long long kOne = 0x3FF0000000000000ll, kNear = 1ll << 20;
-	const long long e = __double_as_longlong(dotp(a, a)) - kOne;
-	if (e >= -kNear && e <= kNear && quot_range(a.x) && quot_range(a.y) && quot_range(a.z)) {
-		const long long f = e >> 1;  // arithmetic shift: floor(e / 2)
-		const double l = __longlong_as_double(kOne + f);
-		const double y = __longlong_as_double(f >= 0 ? kOne - 2 * f : kOne - (f >> 1));
-		return {quot_rcp(a.x, l, y), quot_rcp(a.y, l, y), quot_rcp(a.z, l, y)};
-	}
-	return unit<double, true>(a);
 }
 
 template <class T>
@@ -299,7 +272,7 @@ __device__ __forceinline__ Shape<S> load_shape(uint32_t s, uint32_t id, const in
 // kept, for the warp to finish all such pairs together (run()).
 enum State : int { kIdle = 0, kS1, kS2, kDisc, kRefine, kPost, kParked };
 
-template <class S, bool kExact>
+template <class S>
 struct Lane {
 	uint32_t pair;  // index of the pair being worked on
 	int st;
@@ -330,17 +303,16 @@ __device__ __forceinline__ void st3(float *p, uint64_t i, D3 v) {
 }
 
 // function_MPR_Store :404-422 once the contact normal N and point p0 (or the
-// sphere-sphere p1/p2) are known: envelope, depth, outputs.
-template <class S, bool kExact>
-__device__ __forceinline__ void write_contact(const Lane<S, kExact> &L, D3 N, D3 p1, D3 p2, uint32_t ida, uint32_t idb,
-                                              const NpScratch &sc) {
-	p1 = sub(p1, scl(L.env, N));  // :412-415
-	p2 = add(p2, scl(L.env, N));
+// sphere-sphere p1/p2) of pair i are known, in the frame centred at org:
+// envelope, depth, outputs.
+__device__ __forceinline__ void write_contact(uint64_t i, double env, D3 org, D3 N, D3 p1, D3 p2, uint32_t ida,
+                                              uint32_t idb, const NpScratch &sc) {
+	p1 = sub(p1, scl(env, N));  // :412-415
+	p2 = add(p2, scl(env, N));
 	const double depth = dotp(N, sub(p2, p1));
-	const uint64_t i = L.pair;
 	st3(sc.norm, i, N);
-	st3(sc.pa, i, add(p1, L.org));
-	st3(sc.pb, i, add(p2, L.org));
+	st3(sc.pa, i, add(p1, org));
+	st3(sc.pb, i, add(p2, org));
 	sc.depth[i] = (float)depth;
 	sc.ids[2 * i] = (int32_t)ida;
 	sc.ids[2 * i + 1] = (int32_t)idb;
@@ -364,8 +336,8 @@ __device__ __forceinline__ void write_contact(const Lane<S, kExact> &L, D3 N, D3
 // Starts pair i: the checks and transforms of :338-377; sphere-sphere pairs
 // (:382-397) and skipped pairs finish here. Returns true if the lane now runs
 // the MPR state machine.
-template <class S, bool kExact>
-__device__ __forceinline__ bool start_pair(Lane<S, kExact> &L, uint32_t i, uint64_t n, const int32_t *T,
+template <class S>
+__device__ __forceinline__ bool start_pair(Lane<S> &L, uint32_t i, uint64_t n, const int32_t *T,
                                            const float *A, const float *B, const float *C, const float *R,
                                            const uint32_t *ID, uint64_t nb, const uint8_t *active, const float *pos,
                                            const float *rot, float envelope, const long long *pairs,
@@ -387,12 +359,8 @@ __device__ __forceinline__ bool start_pair(Lane<S, kExact> &L, uint32_t i, uint6
 	}
 	if (!active[ida] && !active[idb]) return false;  // :344-346
 	if (ida == idb) return false;                     // :347-349
-	if constexpr (kExact) {
-		L.org = mk(0.0, 0.0, 0.0);
-	} else {
-		const float3 o = ld3(pos, ida);
-		L.org = mk((double)o.x, (double)o.y, (double)o.z);
-	}
+	const float3 o = ld3(pos, ida);
+	L.org = mk((double)o.x, (double)o.y, (double)o.z);
 	const vec<S> org = cvt<S>(L.org);
 	L.A = load_shape<S>(sa, ida, T, A, B, C, R, pos, rot, org);
 	L.B = load_shape<S>(sb, idb, T, A, B, C, R, pos, rot, org);
@@ -405,8 +373,8 @@ __device__ __forceinline__ bool start_pair(Lane<S, kExact> &L, uint32_t i, uint6
 		const double ra = (double)L.A.Y.x, rb = (double)L.B.Y.x;
 		const double cd = ra + rb;
 		if (!(d2 <= cd * cd)) return false;
-		const D3 N = unit<double, kExact>(rel);
-		write_contact(L, N, add(xa, scl(ra, N)), sub(xb, scl(rb, N)), ida, idb, sc);
+		const D3 N = unit<double, false>(rel);
+		write_contact(L.pair, L.env, L.org, N, add(xa, scl(ra, N)), sub(xb, scl(rb, N)), ida, idb, sc);
 		return false;
 	}
 	// CollideAndFindPoint :137-144
@@ -420,8 +388,8 @@ __device__ __forceinline__ bool start_pair(Lane<S, kExact> &L, uint32_t i, uint6
 
 // Finishes a hit: the contact points of :404-406 need one more support pair
 // along the normal; N, p0 are set here and the post stage evaluates it.
-template <class S, bool kExact>
-__device__ __forceinline__ void to_post(Lane<S, kExact> &L, D3 N, D3 p0) {
+template <class S>
+__device__ __forceinline__ void to_post(Lane<S> &L, D3 N, D3 p0) {
 	L.N = N;
 	L.p0 = p0;
 	L.n = N;
@@ -430,14 +398,14 @@ __device__ __forceinline__ void to_post(Lane<S, kExact> &L, D3 N, D3 p0) {
 
 // Work that happens before a lane's next support evaluation; may finish the
 // pair (returns false) without evaluating a support pair.
-template <class S, bool kExact>
-__device__ __forceinline__ bool pre_step(Lane<S, kExact> &L) {
+template <class S>
+__device__ __forceinline__ bool pre_step(Lane<S> &L) {
 	if (L.st == kDisc) {  // :201-205
 		if (L.phase1 > kMaxIter) return false;
 		L.phase1++;
 	} else if (L.st == kRefine) {  // :240-253
 		L.phase2++;
-		L.n = unit<double, kExact>(crossp(sub(L.v2, L.v1), sub(L.v3, L.v1)));
+		L.n = unit<double, false>(crossp(sub(L.v2, L.v1), sub(L.v3, L.v1)));
 		if (dotp(L.n, L.v1) >= 0.0 && !L.hit) L.hit = true;
 	}
 	return true;
@@ -446,8 +414,8 @@ __device__ __forceinline__ bool pre_step(Lane<S, kExact> &L) {
 // The end of a refinement with a hit (:256-283 once the portal is final): the
 // barycentric contact point and the normal; the post stage then evaluates one
 // more support pair along the normal.
-template <class S, bool kExact>
-__device__ __forceinline__ void finish_refine(Lane<S, kExact> &L) {
+template <class S>
+__device__ __forceinline__ void finish_refine(Lane<S> &L) {
 	const D3 v1 = L.v1, v2 = L.v2, v3v = L.v3, v0 = L.v0, n = L.n;
 	double b0 = dotp(crossp(v1, v2), v3v);
 	double b1 = dotp(crossp(v3v, v2), v0);
@@ -467,14 +435,14 @@ __device__ __forceinline__ void finish_refine(Lane<S, kExact> &L) {
 	const D3 q = add(add(add(scl(b0, v02), scl(b1, dd(L.v12))), scl(b2, dd(L.v22))), scl(b3, dd(L.v32)));
 	const D3 pq = add(p, q);
 	const D3 pt = mk(pq.x * inv * 0.5, pq.y * inv * 0.5, pq.z * inv * 0.5);
-	to_post(L, unit<double, kExact>(n), pt);
+	to_post(L, unit<double, false>(n), pt);
 }
 
 // State update after the support pair (pa = support(A,-n), pb = support(B,n)).
 // Returns false when the pair is finished. park: a refinement that ends with a
 // hit leaves its portal as it is (kParked) instead of finishing it here.
-template <class S, bool kExact>
-__device__ __forceinline__ bool post_step(Lane<S, kExact> &L, vec<S> pa, vec<S> pb, const NpScratch &sc,
+template <class S>
+__device__ __forceinline__ bool post_step(Lane<S> &L, vec<S> pa, vec<S> pb, const NpScratch &sc,
                                           uint32_t ida, uint32_t idb, bool park) {
 	switch (L.st) {
 	case kS1: {  // :146-171
@@ -484,9 +452,9 @@ __device__ __forceinline__ bool post_step(Lane<S, kExact> &L, vec<S> pa, vec<S> 
 		if (dotp(L.v1, L.n) <= 0.0) return false;
 		L.n = crossp(L.v1, L.v0);
 		if (is_zero(L.n)) {
-			const D3 N = unit<double, kExact>(sub(L.v1, L.v0));
+			const D3 N = unit<double, false>(sub(L.v1, L.v0));
 			const D3 s12 = add(dd(L.v11), dd(L.v12));
-			to_post(L, N, kExact ? mk(s12.x * 0.5, s12.y * 0.5, s12.z * 0.5) : scl(0.5, s12));
+			to_post(L, N, scl(0.5, s12));
 			return true;
 		}
 		L.st = kS2;
@@ -557,7 +525,7 @@ __device__ __forceinline__ bool post_step(Lane<S, kExact> &L, vec<S> pa, vec<S> 
 		const D3 N = L.N, p0 = L.p0;
 		const D3 p1 = add(scl(dotp(sub(dd(pa), p0), N), N), p0);
 		const D3 p2 = add(scl(dotp(sub(dd(pb), p0), N), N), p0);
-		write_contact(L, neg(N), p1, p2, ida, idb, sc);
+		write_contact(L.pair, L.env, L.org, neg(N), p1, p2, ida, idb, sc);
 		return false;
 	}
 	}
@@ -572,13 +540,13 @@ __device__ __forceinline__ bool post_step(Lane<S, kExact> &L, vec<S> pa, vec<S> 
 // (barycentric point, normal, one more support pair, the contact) once instead
 // of once for every pair that ends at a different iteration. The finishing
 // arithmetic reads only the parked portal, so the contacts are the same.
-template <class S, bool kExact, int NT>
+template <class S>
 __device__ __forceinline__ void run(uint64_t P_cap, const unsigned long long *P_dev, uint64_t n, const int32_t *T,
                                     const float *A, const float *B, const float *C, const float *R, const uint32_t *ID,
                                     uint64_t nb, const uint8_t *active, const float *pos, const float *rot,
                                     float envelope, const long long *pairs, const NpScratch &sc, uint32_t *queue) {
 	const uint64_t P = P_dev ? min(P_cap, (uint64_t)*P_dev) : P_cap;
-	Lane<S, kExact> L;
+	Lane<S> L;
 	L.st = kIdle;
 	bool done = false;     // the queue is exhausted for this lane
 	bool drained = false;  // the warp has taken the last queue entries (warp-uniform)
@@ -624,11 +592,9 @@ __device__ __forceinline__ void run(uint64_t P_cap, const unsigned long long *P_
 			continue;
 		}
 		// the support pair: support(A, -n), support(B, n)
-		vec<S> d = cvt<S>(L.n);
-		if constexpr (kExact && sizeof(S) == 8) d = unit_again(d);  // n is a unit vector when refining
-		else if constexpr (kExact) d = unit<S, true>(d);
-		const vec<S> pa = support<S, kExact>(L.A, neg(d));
-		const vec<S> pb = support<S, kExact>(L.B, d);
+		const vec<S> d = cvt<S>(L.n);
+		const vec<S> pa = support<S, false>(L.A, neg(d));
+		const vec<S> pb = support<S, false>(L.B, d);
 		if (!post_step(L, pa, pb, sc, ida, idb, drained)) L.st = kIdle;
 	}
 }

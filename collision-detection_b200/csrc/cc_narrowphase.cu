@@ -2,7 +2,8 @@
 // (src/narrowphase/Narrowphase.cu:316-595) as sm_100a kernels.
 //
 // k_mpr: the MPR state machine of cc_mpr.cuh on persistent lanes fed from a
-// queue of pair indices grouped by shape-type combination (k_np_classes).
+// queue of pair indices grouped by shape-type combination (k_np_classes);
+// the exact mode has its own kernel and takes the pairs as they come.
 // Sphere-sphere pairs take the analytic branch (:382-397); every other pair
 // runs Minkowski portal refinement (CollideAndFindPoint :122-314) with the
 // same branch structure, iteration caps (35 discovery, 35 refinement) and
@@ -40,7 +41,7 @@ __global__ void __launch_bounds__(kNT) k_mpr(uint64_t P_cap, const unsigned long
                                               const float *__restrict__ pos, const float *__restrict__ rot,
                                               float envelope, const long long *__restrict__ pairs, NpScratch sc) {
 	pdl_begin();
-	mpr::run<S, false, kNT>(P_cap, P_dev, n, T, A, B, C, R, ID, nb, active, pos, rot, envelope, pairs, sc,
+	mpr::run<S>(P_cap, P_dev, n, T, A, B, C, R, ID, nb, active, pos, rot, envelope, pairs, sc,
 	                        sc.classes + 2 * kNpClasses);
 }
 
@@ -305,10 +306,10 @@ int resident(K kernel) {
 	if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, kernel, kNT, 0) != cudaSuccess || v < 1) v = 1;
 	return v;
 }
-// Blocks of the MPR kernel of a precision mode resident per SM.
+// Blocks of a fast MPR kernel (modes 1 and 2) resident per SM.
 int mpr_resident_blocks(int precision) {
-	static const int b[3] = {mpr_exact_resident_blocks(), resident(k_mpr<double>), resident(k_mpr<float>)};
-	return b[precision == 0 ? 0 : (precision == 2 ? 2 : 1)];
+	static const int b[2] = {resident(k_mpr<double>), resident(k_mpr<float>)};
+	return b[precision == 2 ? 1 : 0];
 }
 
 // Largest co-resident grid of a cooperative kernel of kCoopNT threads.
@@ -340,6 +341,20 @@ void launch_mpr(uint64_t P_cap, const unsigned long long *P_dev, uint64_t n, con
                 const NpScratch &sc, int precision, uint64_t P_hint, cudaStream_t s) {
 	if (!P_cap) return;
 	const uint64_t Pe = std::min<uint64_t>(P_hint ? P_hint : P_cap, P_cap);
+	if (precision == 0) {
+		// The exact kernel's lanes share one instruction sequence whatever their
+		// types, so its pairs are not grouped by class (grouped: 4 us more at
+		// 1,800 pairs, the same at 27,500 and 195,000). Grid: sixteen pairs a
+		// warp; below two blocks per SM the pairs spread over that many blocks
+		// instead, one warp per scheduler (3,400 pairs: 46 us with two blocks per
+		// SM, 60 us with six), at most what is resident (27,500 pairs: 75 us with
+		// six, 82 with three; 195,000: 239 with six, 373 with three).
+		if (!sc.pre_zeroed) cudaMemsetAsync(sc.classes, 0, (2 * kNpClasses + 1) * sizeof(uint32_t), s);
+		const uint64_t want = std::max<uint64_t>((Pe + kNT / 2 - 1) / (kNT / 2), 2 * kNumSMs);
+		launch_mpr_exact((unsigned)std::min<uint64_t>(want, (uint64_t)kNumSMs * mpr_exact_resident_blocks()), P_cap, P_dev, n,
+		                 T, A, B, C, R, ID, nb, active, pos, rot, envelope, pairs, sc, s);
+		return;
+	}
 	{  // group the pairs by shape-type combination; the last word is the work queue
 		// blocks for the expected pair count (the loops stride over the device count)
 		const unsigned g = (unsigned)std::max<uint64_t>(
@@ -354,9 +369,7 @@ void launch_mpr(uint64_t P_cap, const unsigned long long *P_dev, uint64_t n, con
 	const uint64_t want = (Pe + kNT - 1) / kNT;
 	const unsigned grid = (unsigned)std::min<uint64_t>(std::max<uint64_t>(want, kNumSMs),
 	                                                   (uint64_t)kNumSMs * mpr_resident_blocks(precision));
-	if (precision == 0)
-		launch_mpr_exact(grid, P_cap, P_dev, n, T, A, B, C, R, ID, nb, active, pos, rot, envelope, pairs, sc, s);
-	else if (precision == 2)
+	if (precision == 2)
 		launch_pdl(k_mpr<float>, dim3(grid), dim3(kNT), 0, s, P_cap, P_dev, n, T, A, B, C, R, ID, nb, active, pos, rot, envelope, pairs,
 		                                  sc);
 	else
