@@ -1,10 +1,15 @@
 // Uniform-grid broadphase (the reference's Broadphase::detectPossibleCollisions,
 // src/broadphase/Broadphase.cu:344-545) as sm_100a kernels.
 //
-// Pair path (always):
+// Pair path, scenes without crowded cells (the rule is cc_ctx::chain_state):
 //   k_bounds        scene bounds + extent sums + validation     (Broadphase.cu:368-376)
-//   k_count         in-place shift by fabs(min) (:379-386) + per-cell counts on
-//                   the search grid
+//   k_link          in-place shift by fabs(min) (:379-386), one 32-byte entry per
+//                   (cell, body) linked into its cell's chain
+//   k_walk          closed AABB overlap (:237) of every entry with the entries
+//                   behind it in the chain, emitted from the home cell (below)
+// Pair path, crowded scenes:
+//   k_bounds, then k_count  in-place shift by fabs(min) (:379-386) + per-cell
+//                   counts on the search grid
 //   scan            cell offsets (decoupled look-back)
 //   k_scatter       cell-ordered (AABB, body) entries
 //   k_pair_test     closed AABB overlap (:237) of every entry with the later
@@ -13,6 +18,7 @@
 //                   every axis, a point of both boxes and so of both cell
 //                   ranges), so each overlapping pair appears exactly once and no
 //                   unique pass is needed (replaces :484-533)
+// Both:
 //   scan            per-owner offsets (owner = smaller index)
 //   k_owner_scatter bucket pairs by owner; k_segsort sorts each bucket
 //                   -> the sorted, duplicate-free int64 list of :522-535
@@ -166,19 +172,39 @@ __device__ __forceinline__ uint32_t cell_index(const Plan &p, uint32_t base, int
 	return base + (uint32_t)x + (uint32_t)p.dim[0] * ((uint32_t)y + (uint32_t)p.dim[1] * z);
 }
 
+// The plan of the block's shapes [i0, i0 + kNT) into shared memory (sp, base),
+// with a barrier. A batch's tile may span scenes: returns false then, and each
+// shape takes its own (plan_of).
 template <bool kBatch>
-__global__ void __launch_bounds__(kNT) k_count(uint64_t n, float *__restrict__ aabb, const DevStats *stats,
-                                                uint32_t *__restrict__ cell_count, uint32_t *__restrict__ owner_count,
-                                                SceneMap sm, int oshift, uint32_t *__restrict__ owner_cursor) {
-	pdl_begin();
-	__shared__ Plan sp;
-	__shared__ __align__(16) float stage[6 * kNT];  // read and written as float4
-	if (threadIdx.x < sizeof(Plan) / 4)
-		reinterpret_cast<uint32_t *>(&sp)[threadIdx.x] = reinterpret_cast<const uint32_t *>(&stats->plan)[threadIdx.x];
+__device__ __forceinline__ bool tile_plan(uint64_t n, uint64_t i0, const DevStats *stats, const SceneMap &sm, Plan &sp,
+                                          uint32_t &base) {
+	const Plan *from = &stats->plan;
+	bool one = true;
+	base = 0;
+	if constexpr (kBatch) {
+		const uint32_t s0 = __ldg(sm.scene_of + i0), s1 = __ldg(sm.scene_of + min(i0 + kNT, n) - 1);
+		one = s0 == s1;
+		from = sm.plans + s0;
+		base = __ldg(sm.cell_base + s0);
+	}
+	if (one && threadIdx.x < sizeof(Plan) / 4)
+		reinterpret_cast<uint32_t *>(&sp)[threadIdx.x] = reinterpret_cast<const uint32_t *>(from)[threadIdx.x];
 	__syncthreads();
-	if (!kBatch && !sp.valid) return;  // invalid input: nothing is modified
-	const uint64_t i0 = (uint64_t)blockIdx.x * kNT;
-	if (!kBatch && tile_vec_ok32(aabb, n, i0)) {
+	return one;
+}
+
+// The block's boxes [i0, i0 + kNT) shifted in place by fabs(min) (:382-386), in
+// `stage` on return (after a barrier). one: they share the plan sp. shift 0:
+// they are shifted already.
+template <bool kBatch>
+__device__ __forceinline__ void load_shifted_tile(uint64_t n, float *__restrict__ aabb, uint64_t i0, const Plan &sp,
+                                                  const SceneMap &sm, float *stage, int shift, bool one) {
+	if (!shift || (one && !sp.valid)) {
+		load_tile_aabb(aabb, n, i0, stage);
+		__syncthreads();
+		return;
+	}
+	if (one && tile_vec_ok32(aabb, n, i0)) {
 		// in-place shift by fabs(min) (:382-386) on 32-byte vectors, in
 		// registers on the way to shared memory: thread k < 96 takes floats
 		// [8k, 8k + 8) of the min-corner run, thread 96 + k those of the
@@ -202,8 +228,8 @@ __global__ void __launch_bounds__(kNT) k_count(uint64_t n, float *__restrict__ a
 	} else {
 		load_tile_aabb(aabb, n, i0, stage);
 		__syncthreads();
-		// in-place shift by fabs(min) (:382-386), element by element
-		if constexpr (kBatch) {
+		// element by element
+		if (kBatch && !one) {
 			for (int k = threadIdx.x; k < 6 * kNT; k += kNT) {
 				const uint64_t shape = i0 + (uint64_t)((k % (3 * kNT)) / 3);
 				if (shape < n) {
@@ -217,6 +243,20 @@ __global__ void __launch_bounds__(kNT) k_count(uint64_t n, float *__restrict__ a
 		__syncthreads();
 		store_tile_aabb(aabb, n, i0, stage);
 	}
+}
+
+template <bool kBatch>
+__global__ void __launch_bounds__(kNT) k_count(uint64_t n, float *__restrict__ aabb, const DevStats *stats,
+                                                uint32_t *__restrict__ cell_count, uint32_t *__restrict__ owner_count,
+                                                SceneMap sm, int oshift, uint32_t *__restrict__ owner_cursor, int shift) {
+	pdl_begin();
+	__shared__ Plan sp;
+	__shared__ __align__(16) float stage[6 * kNT];  // read and written as float4
+	const uint64_t i0 = (uint64_t)blockIdx.x * kNT;
+	uint32_t base0;
+	const bool one = tile_plan<kBatch>(n, i0, stats, sm, sp, base0);
+	if (!kBatch && !sp.valid) return;  // invalid input: nothing is modified
+	load_shifted_tile<kBatch>(n, aabb, i0, sp, sm, stage, shift, one);
 	const uint64_t i = i0 + threadIdx.x;
 	if (i >= n) return;
 	const float3 mn = f3(stage[3 * threadIdx.x], stage[3 * threadIdx.x + 1], stage[3 * threadIdx.x + 2]);
@@ -226,15 +266,14 @@ __global__ void __launch_bounds__(kNT) k_count(uint64_t n, float *__restrict__ a
 		owner_count[i >> oshift] = 0u;
 		if (owner_cursor) owner_cursor[i >> oshift] = 0u;
 	}
-	uint32_t base;
-	const Plan &p = plan_of<kBatch>(sp, sm, i, base);
+	uint32_t base = base0;
+	const Plan &p = one ? sp : plan_of<kBatch>(sp, sm, i, base);
 	if (kBatch && !p.valid) return;
 	const CellRange r = cell_range(p, mn, mx);
 	for (int z = r.c0[2]; z <= r.c1[2]; z++)
 		for (int y = r.c0[1]; y <= r.c1[1]; y++)
 			for (int x = r.c0[0]; x <= r.c1[0]; x++) atomicAdd(&cell_count[cell_index(p, base, x, y, z)], 1u);
 }
-
 // Cell-ordered entries: one thread per body, a cursor atomic per covered cell.
 template <bool kBatch>
 __global__ void __launch_bounds__(kNT) k_scatter(uint64_t n, const float *__restrict__ aabb, const DevStats *stats,
@@ -490,6 +529,234 @@ __global__ void __launch_bounds__(kNT, 5) k_pair_test(const DevStats *stats, con
 		if (owned) atomicAdd(&owner_count[ida >> oshift], owned);
 	}
 	if (ocnt) flush_pairs(obuf, ocnt, lane, pair_counter, pairs, pair_cap);
+}
+
+// ---------------------------------------------------------------- chained search
+// For scenes without crowded cells: the entries of a cell form a linked list
+// through the entry array instead of a sorted run, which takes the cell counts,
+// their scan and the scatter out of the search. A body's first entry is its
+// own slot i (written in order); the entries for further cells go to slots from
+// n up, taken per block, with their body in extra_body. An entry is one 32-byte
+// record: (min.xyz, next), (max.xyz, packed cell), next = 1 + the slot that
+// headed the cell's chain before it, 0 at the end.
+// Stage times (us), sorted cells (count + scan + scatter + pair test) -> chains
+// (link + walk): 16,384 spheres 39 -> 20, 130K mixed shapes 49 -> 24, 1M 109 ->
+// 64, a batch of 1.4M shapes 160 -> 97, a heap of 50K (20 entries a cell) 60 ->
+// 49. Crowded cells are the other way round (a chain is one lane's serial walk,
+// a sorted cell full warps' work), hence kChainLong.
+//
+// Bound by barriers and the chain heads' atomics (ncu at 1M: 40 % issue, 8 MB of
+// sectors each way are the boxes' shift): the first cell's exchange is under way
+// while the block collects the further ones as work items, so that lanes with
+// one cell (60 % of the boxes) do not wait for those with eight (38 -> 34 us).
+template <bool kBatch>
+__global__ void __launch_bounds__(kNT) k_link(uint64_t n, float *__restrict__ aabb, DevStats *stats,
+                                               uint32_t *__restrict__ head, float4 *__restrict__ entries, uint64_t cap,
+                                               uint32_t *__restrict__ extra_body, uint32_t *__restrict__ owner_count,
+                                               SceneMap sm, int oshift, uint32_t *__restrict__ owner_cursor, int shift) {
+	pdl_begin();
+	__shared__ Plan sp;
+	__shared__ __align__(16) float stage[6 * kNT];  // read and written as float4
+	__shared__ uint32_t s_first[kNT], s_cell[kNT], s_items, s_wide;
+	__shared__ uint16_t s_item[7 * kNT];
+	__shared__ unsigned long long s_base;
+	if (threadIdx.x == 0) s_items = s_wide = 0;
+	const uint64_t i0 = (uint64_t)blockIdx.x * kNT;
+	uint32_t base0;
+	const bool one = tile_plan<kBatch>(n, i0, stats, sm, sp, base0);
+	if (!kBatch && !sp.valid) return;  // invalid input: nothing is modified
+	load_shifted_tile<kBatch>(n, aabb, i0, sp, sm, stage, shift, one);
+	const uint64_t i = i0 + threadIdx.x;
+	const bool have = i < n;
+	const float3 mn = f3(stage[3 * threadIdx.x], stage[3 * threadIdx.x + 1], stage[3 * threadIdx.x + 2]);
+	const float *hs = stage + 3 * kNT;
+	const float3 mx = f3(hs[3 * threadIdx.x], hs[3 * threadIdx.x + 1], hs[3 * threadIdx.x + 2]);
+	if (have && (i & ((1ull << oshift) - 1)) == 0) {  // the first body of its owner bucket
+		owner_count[i >> oshift] = 0u;
+		if (owner_cursor) owner_cursor[i >> oshift] = 0u;
+	}
+	uint32_t base = base0;
+	const Plan &p = one ? sp : plan_of<kBatch>(sp, sm, have ? i : n - 1, base);
+	CellRange r;
+	int nx = 1, ny = 1, nz = 1;
+	bool live = have && (!kBatch || p.valid);
+	if (live) {
+		r = cell_range(p, mn, mx);
+		nx = r.c1[0] - r.c0[0] + 1;
+		ny = r.c1[1] - r.c0[1] + 1;
+		nz = r.c1[2] - r.c0[2] + 1;
+		if ((uint64_t)nx * ny * nz > kChainCells) {  // the search is redone on sorted cells
+			atomicOr(&stats->err, (uint32_t)kErrLongChain);
+			live = false;
+		}
+	}
+	const auto put = [&](uint64_t slot, float3 lo, float3 hi, uint32_t next, uint32_t packed) {
+		st_global_v8(reinterpret_cast<float *>(entries + 2 * slot), make_float4(lo.x, lo.y, lo.z, __uint_as_float(next)),
+		             make_float4(hi.x, hi.y, hi.z, __uint_as_float(packed)));
+	};
+	uint32_t next = 0, first = 0, cell = 0;
+	if (live) {
+		first = pack_cell(r.c0[0], r.c0[1], r.c0[2]);
+		cell = cell_index(p, base, r.c0[0], r.c0[1], r.c0[2]);
+		if (i < cap) next = atomicExch(head + cell, (uint32_t)i + 1u);
+	}
+	// the further cells of boxes within 2x2x2 (nearly all) become work items of
+	// the block, (thread, cell offset), so that they too are written by full warps
+	const bool small = live && nx <= 2 && ny <= 2 && nz <= 2;
+	const uint32_t more = live ? (uint32_t)(nx * ny * nz) - 1u : 0u;
+	const uint32_t incl = warp_incl_scan(small ? more : 0u);
+	uint32_t at = 0;
+	if ((threadIdx.x & 31) == 31 && incl) at = atomicAdd(&s_items, incl);
+	at = __shfl_sync(0xffffffffu, at, 31) + incl - (small ? more : 0u);
+	s_first[threadIdx.x] = first;
+	s_cell[threadIdx.x] = cell;
+	uint32_t wide = 0;
+	if (small) {
+		for (int q = 1; q < 8; q++)
+			if ((q & 1) < nx && ((q >> 1) & 1) < ny && (q >> 2) < nz) s_item[at++] = (uint16_t)(threadIdx.x | (q << 8));
+	} else if (more) {
+		wide = atomicAdd(&s_wide, more);
+	}
+	if (have && i < cap) put(i, mn, mx, next, first);  // not live: an entry in no chain
+	__syncthreads();
+	const uint32_t items = s_items;
+	if (threadIdx.x == 0) s_base = items + s_wide ? n + atomicAdd(&stats->extra, (unsigned long long)items + s_wide) : n;
+	__syncthreads();
+	const uint64_t slot0 = s_base;
+	for (uint32_t k = threadIdx.x; k < items; k += kNT) {
+		const uint32_t w = s_item[k], t = w & 255u, dx = (w >> 8) & 1u, dy = (w >> 9) & 1u, dz = w >> 10;
+		uint32_t b2;
+		const Plan &pt = one ? sp : plan_of<kBatch>(sp, sm, i0 + t, b2);
+		const uint64_t slot = slot0 + k;
+		if (slot < cap) {
+			const uint32_t c = s_cell[t] + dx + (uint32_t)pt.dim[0] * (dy + (uint32_t)pt.dim[1] * dz);
+			const uint32_t prev = atomicExch(head + c, (uint32_t)slot + 1u);
+			put(slot, f3(stage[3 * t], stage[3 * t + 1], stage[3 * t + 2]), f3(hs[3 * t], hs[3 * t + 1], hs[3 * t + 2]), prev,
+			    s_first[t] + (dx | (dy << 10) | (dz << 20)));
+			extra_body[slot - n] = (uint32_t)(i0 + t);
+		}
+	}
+	if (more && !small) {
+		uint64_t slot = slot0 + items + wide;
+		for (int z = r.c0[2]; z <= r.c1[2]; z++)
+			for (int y = r.c0[1]; y <= r.c1[1]; y++)
+				for (int x = r.c0[0]; x <= r.c1[0]; x++) {
+					if (x == r.c0[0] && y == r.c0[1] && z == r.c0[2]) continue;
+					if (slot < cap) {
+						put(slot, mn, mx, atomicExch(head + cell_index(p, base, x, y, z), (uint32_t)slot + 1u), pack_cell(x, y, z));
+						extra_body[slot - n] = (uint32_t)i;
+					}
+					slot++;
+				}
+	}
+}
+
+// Before the walk on a context that knows nothing of its scenes: does any cell
+// hold more than kChainLong entries? (The walk then returns at once.)
+__global__ void __launch_bounds__(kNT) k_chain_check(DevStats *stats, uint64_t g_max, const uint32_t *__restrict__ head,
+                                                      const float4 *__restrict__ entries, uint64_t cap) {
+	pdl_begin();
+	const uint64_t G = min(g_max, (uint64_t)stats->cells);
+	for (uint64_t c = (uint64_t)blockIdx.x * kNT + threadIdx.x; c < G; c += (uint64_t)gridDim.x * kNT) {
+		uint32_t at = head[c], len = 0;
+		while (at && at <= cap && len <= kChainLong) {
+			at = __float_as_uint(entries[2 * (uint64_t)(at - 1)].w);
+			len++;
+		}
+		if (len > kChainLong) {
+			atomicAdd(&stats->dense_items, 1ull);
+			atomicOr(&stats->err, (uint32_t)kErrLongChain);
+		}
+	}
+}
+
+// Every entry is tested against the entries behind it in its cell's chain: each
+// pair of a cell once, whichever of the two was linked later. Bound by the
+// chain's dependent loads (an L2 round trip each; the records of 1M bodies fit
+// the L2): the warp's next entries are loaded while the present ones walk (five
+// blocks per SM: 30 us at 1M; six, which spill, 32; four 31.5). Pairs are
+// emitted as in k_pair_test: from the home cell, through a per-warp buffer.
+constexpr uint32_t kChainMost = 4096;
+template <bool kBatch>
+__global__ void __launch_bounds__(kNT, 5) k_walk(uint64_t n, DevStats *stats, const float4 *__restrict__ entries,
+                                                  uint64_t cap, const uint32_t *__restrict__ extra_body,
+                                                  uint32_t *__restrict__ owner_count,
+                                                  unsigned long long *__restrict__ pairs, uint64_t pair_cap, SceneMap sm,
+                                                  int oshift) {
+	pdl_begin();
+	__shared__ Plan sp;
+	__shared__ unsigned long long out_all[kNT / 32][kOutBuf];
+	__shared__ uint32_t s_stop;
+	if (threadIdx.x < sizeof(Plan) / 4)
+		reinterpret_cast<uint32_t *>(&sp)[threadIdx.x] = reinterpret_cast<const uint32_t *>(&stats->plan)[threadIdx.x];
+	const uint64_t total = n + stats->extra;
+	if (threadIdx.x == 0) s_stop = __ldcg(&stats->err) & kErrLongChain;  // only the check sets it before this kernel's walk
+	if (blockIdx.x == 0 && threadIdx.x == 0) stats->entries = total;
+	__syncthreads();
+	if ((!kBatch && !sp.valid) || s_stop) return;
+	unsigned long long *obuf = out_all[threadIdx.x >> 5];
+	uint32_t ocnt = 0;  // pairs in obuf (warp-uniform)
+	const uint64_t E = min(total, cap);
+	const uint32_t lane = threadIdx.x & 31, lt = (1u << lane) - 1u;
+	const auto body_of = [&](uint64_t slot) { return slot < n ? (uint32_t)slot : __ldg(extra_body + (slot - n)); };
+	const uint64_t warps = (uint64_t)gridDim.x * (kNT / 32);
+	const auto load = [&](uint64_t e, float4 &lo, float4 &hi) {
+		lo.w = 0.f;  // no entry: nothing follows
+		if (e < E) ld_global_v8(reinterpret_cast<const float *>(entries + 2 * e), lo, hi);
+	};
+	uint64_t e = ((uint64_t)blockIdx.x * (kNT / 32) + (threadIdx.x >> 5)) * 32 + lane;
+	float4 nlo = make_float4(0.f, 0.f, 0.f, 0.f), nhi = nlo;
+	load(e, nlo, nhi);
+	for (; e - lane < E; e += warps * 32) {
+		const float4 alo = nlo, ahi = nhi;
+		load(e + warps * 32, nlo, nhi);  // the warp's next entries arrive while these walk
+		uint32_t next = __float_as_uint(alo.w), hops = 0, owned = 0;
+		while (__any_sync(0xffffffffu, next != 0u)) {
+			bool emit = false;
+			unsigned long long key = 0;
+			if (next) {
+				const uint64_t at = next - 1u;
+				float4 blo, bhi;
+				ld_global_v8(reinterpret_cast<const float *>(entries + 2 * at), blo, bhi);
+				next = __float_as_uint(blo.w);
+				if (++hops >= kChainLong && next) {
+					if (hops == kChainLong) atomicAdd(&stats->dense_items, 1ull);
+					if (hops >= kChainMost) {
+						atomicOr(&stats->err, (uint32_t)kErrLongChain);
+						next = 0u;
+					}
+				}
+				if (alo.x <= bhi.x && blo.x <= ahi.x && alo.y <= bhi.y && blo.y <= ahi.y && alo.z <= bhi.z && blo.z <= ahi.z) {
+					const uint32_t pc = __float_as_uint(ahi.w), ia = body_of(e);
+					uint32_t cbase;
+					const Plan &p = plan_of<kBatch>(sp, sm, ia, cbase);
+					if (cell_of(fmaxf(alo.x, blo.x), p.lo[0], p.inv[0], p.dim[0]) == (int)(pc & 1023) &&
+					    cell_of(fmaxf(alo.y, blo.y), p.lo[1], p.inv[1], p.dim[1]) == (int)((pc >> 10) & 1023) &&
+					    cell_of(fmaxf(alo.z, blo.z), p.lo[2], p.inv[2], p.dim[2]) == (int)((pc >> 20) & 1023)) {
+						const uint32_t ib = body_of(at);
+						const uint32_t lo = min(ia, ib), hi = max(ia, ib);
+						key = ((unsigned long long)lo << 32) | hi;
+						emit = true;
+						if (lo == ia) owned++;
+						else atomicAdd(&owner_count[lo >> oshift], 1u);
+					}
+				}
+			}
+			const uint32_t b = __ballot_sync(0xffffffffu, emit);
+			if (b) {
+				const uint32_t nb = __popc(b);
+				if (ocnt + nb > kOutBuf) {
+					flush_pairs(obuf, ocnt, lane, &stats->pairs, pairs, pair_cap);
+					ocnt = 0;
+				}
+				if (emit) obuf[ocnt + __popc(b & lt)] = key;
+				ocnt += nb;
+				__syncwarp();
+			}
+		}
+		if (owned) atomicAdd(&owner_count[body_of(e) >> oshift], owned);
+	}
+	if (ocnt) flush_pairs(obuf, ocnt, lane, &stats->pairs, pairs, pair_cap);
 }
 
 // Dense cells: one block per (cell, chunk of 256 rows). Thread t takes row
@@ -1135,14 +1402,36 @@ void launch_bounds(uint64_t n, const float *aabb, DevStats *stats, const GridPar
 	if (n) k_bounds<<<blocks_for(n), kNT, 0, s>>>(n, aabb, stats, pa, zero);
 }
 
-void launch_count(uint64_t n, float *aabb, const BpBuffers &b, cudaStream_t s) {
+void launch_count(uint64_t n, float *aabb, const BpBuffers &b, cudaStream_t s, bool shift) {
 	if (!n) return;
-	if (b.sm.plans)
-		launch_pdl(k_count<true>, dim3(blocks_for(n)), dim3(kNT), 0, s, n, aabb, b.stats, b.cell_count, b.owner_count, b.sm, 0,
-		           (uint32_t *)nullptr);
-	else
-		launch_pdl(k_count<false>, dim3(blocks_for(n)), dim3(kNT), 0, s, n, aabb, b.stats, b.cell_count, b.owner_count, b.sm,
-		           b.owner_shift, b.owner_cursor);
+	const auto k = b.sm.plans ? k_count<true> : k_count<false>;
+	launch_pdl(k, dim3(blocks_for(n)), dim3(kNT), 0, s, n, aabb, b.stats, b.cell_count, b.owner_count, b.sm, b.owner_shift,
+	           b.owner_cursor, shift ? 1 : 0);
+}
+
+void launch_link(uint64_t n, float *aabb, const BpBuffers &b, cudaStream_t s, bool shift) {
+	if (!n) return;
+	const auto k = b.sm.plans ? k_link<true> : k_link<false>;
+	launch_pdl(k, dim3(blocks_for(n)), dim3(kNT), 0, s, n, aabb, b.stats, b.cell_count, b.entries, b.entry_cap, b.extra_body,
+	           b.owner_count, b.sm, b.owner_shift, b.owner_cursor, shift ? 1 : 0);
+}
+
+void launch_chain_check(const BpBuffers &b, uint32_t g_max, cudaStream_t s) {
+	launch_pdl(k_chain_check, dim3((unsigned)std::min<uint64_t>(blocks_for(g_max), kNumSMs * 8)), dim3(kNT), 0, s, b.stats,
+	           (uint64_t)g_max, b.cell_count, b.entries, b.entry_cap);
+}
+
+void launch_walk(uint64_t n, const BpBuffers &b, uint64_t entries_hint, cudaStream_t s) {
+	if (!n) return;
+	const auto k = b.sm.plans ? k_walk<true> : k_walk<false>;
+	static const int per_sm = [] {
+		int v = 0;
+		if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, k_walk<false>, kNT, 0) != cudaSuccess || v < 1) v = 1;
+		return v;
+	}();
+	const unsigned grid = (unsigned)std::min<uint64_t>(std::max<uint64_t>(blocks_for(entries_hint), 1), (uint64_t)kNumSMs * per_sm);
+	launch_pdl(k, dim3(grid), dim3(kNT), 0, s, n, b.stats, b.entries, b.entry_cap, b.extra_body, b.owner_count, b.pairs_tmp,
+	           b.pair_cap, b.sm, b.owner_shift);
 }
 
 // ---------------------------------------------------------------- cell offsets

@@ -41,6 +41,13 @@ const char *kStageNames[ST_COUNT_] = {"aabb", "bounds", "count", "scan_cells", "
 // back to back as they do unprofiled).
 constexpr int kProfStages = 1, kProfSpans = 2;
 constexpr int kMaxMarks = 64;
+// Boxes per cell of the chained search relative to cc_set_tuning's target: a
+// chain costs a dependent load per entry where a sorted cell costs a share of a
+// coalesced window, so its best cells are smaller (link + walk at 1M mixed
+// shapes: 72 us at 4 boxes a cell, 67 at 2 and at 1; 130K 28, 27, 25; 16,384
+// spheres 22, 20, 19; crowded scenes are bound by the extent floor instead).
+constexpr float kChainCellTarget = 0.25f;
+constexpr int kChainWait = 32;  // calls (cc_ctx::chain_wait)
 
 // A CUDA graph of one kind of call, replayed while the call's configuration
 // (its key: everything its launches depend on) repeats.
@@ -72,6 +79,7 @@ struct cc_ctx {
 	Buf np_norm, np_pa, np_pb, np_depth, np_ids, np_pairs, np_flag, np_pos, np_order, np_classes, np_bsum;
 	Buf bp_bsum;  // block sums of the cooperative cell scan
 	Buf cell_cs;  // packed (start, cursor) words of the cells
+	Buf extra;    // bodies of the chained search's entries past the first n
 	Buf in_T, in_A, in_B, in_C, in_R, in_ID, in_pos, in_rot, in_act, out_aabb, out_pairs, out_norm, out_pa, out_pb,
 	    out_depth, out_bids;
 	// batch scratch: offsets, scene of each shape, global body ids, per-scene
@@ -103,6 +111,13 @@ struct cc_ctx {
 	// not launched (the sparse one tests every cell and counts dense ones)
 	bool dense_skip = false;
 	uint64_t last_dense = 1;  // dense cells of the last call (1: none seen yet)
+	// the search of this call: on chained entries (launch_link, launch_walk) or
+	// on sorted cells; kChainUnknown looks for crowded cells before the walk
+	enum ChainState { kChainUnknown, kChainOk, kChainNo };
+	ChainState chain_state = kChainUnknown;
+	bool chain = false, chain_check = false;
+	GridParams call_gp{};  // gp as this call's search uses it (set by prepare)
+	int chain_wait = 0;  // calls on sorted cells left before the chains are tried again
 	uint64_t last_E = 0, last_P = 0;
 	int last_dim[3] = {0, 0, 0};
 	// owner buckets of the pair sort (BpBuffers::owner_shift / key_bits), chosen
@@ -326,6 +341,7 @@ BpBuffers bp_buffers(cc_ctx *c) {
 	                ? ptr<unsigned long long>(c->cell_cs)
 	                : nullptr;
 	b.sm = c->sm;
+	b.extra_body = ptr<uint32_t>(c->extra);
 	b.dense = c->dense_skip ? nullptr : ptr<uint2>(c->dense);
 	b.dense_cap = c->dense.bytes / sizeof(uint2);
 	b.dense_cell = c->gp.dense_cell;
@@ -383,6 +399,15 @@ cc_status np_prepare(cc_ctx *c, uint64_t P) {
 	return CC_OK;
 }
 
+// Environment CC_CHAIN=0 searches on sorted cells only.
+bool chain_enabled() {
+	static const bool on = [] {
+		const char *v = getenv("CC_CHAIN");
+		return !(v && v[0] == '0');
+	}();
+	return on;
+}
+
 // Allocates the n-dependent broadphase scratch and, if np_cap > 0, the
 // narrowphase scratch for np_cap pairs. Buffers only grow; every public call
 // ends with a synchronize, so nothing in flight uses a buffer replaced here.
@@ -396,6 +421,10 @@ cc_status prepare(cc_ctx *c, uint64_t n, uint64_t np_cap, uint64_t g_override = 
 	}
 	c->fused_now = !g_override && fused_sort_enabled() && fused_sort_fits(owner_buckets(n, c->owner_shift));
 	c->dense_skip = !g_override && c->last_dense == 0;
+	c->chain = chain_enabled() && c->chain_state != cc_ctx::kChainNo && n < ((uint64_t)1 << 31);
+	c->chain_check = c->chain && c->chain_state == cc_ctx::kChainUnknown;
+	c->call_gp = c->gp;
+	if (c->chain) c->call_gp.k_target *= kChainCellTarget;
 	CC_TRY(ensure(c, c->stats, sizeof(DevStats)));
 	CC_TRY(ensure(c, c->bp_bsum, sizeof(unsigned long long) * kScanCoopBlocks));
 	CC_TRY(ensure(c, c->cell_cs, sizeof(unsigned long long) * c->gp.g_max));
@@ -405,6 +434,7 @@ cc_status prepare(cc_ctx *c, uint64_t n, uint64_t np_cap, uint64_t g_override = 
 	CC_TRY(ensure(c, c->owner_off, sizeof(unsigned long long) * (n + 1)));
 	const uint64_t e_guess = std::max<uint64_t>(c->last_E + c->last_E / 4, 2 * n + 1024);
 	CC_TRY(ensure(c, c->entries, 2 * sizeof(float4) * e_guess));
+	CC_TRY(ensure(c, c->extra, sizeof(uint32_t) * (c->entries.bytes / (2 * sizeof(float4)))));
 	const uint64_t p_guess = std::max<uint64_t>(c->last_P + c->last_P / 4, n / 4 + 1024);
 	CC_TRY(ensure(c, c->pairs_tmp, sizeof(unsigned long long) * p_guess));
 	c->st_words[0] = std::max<uint64_t>(c->st_words[0], status_words_for(c->gp.g_max));
@@ -464,14 +494,26 @@ uint64_t pow2ceil(uint64_t v) {
 uint64_t hint_E(const cc_ctx *c, uint64_t n) { return pow2ceil(std::max<uint64_t>(c->last_E, n)); }
 uint64_t hint_P(const cc_ctx *c) { return pow2ceil(std::max<uint64_t>(c->last_P, 1)); }
 
-// count .. owner scan: needs stats zeroed and the plan from the bounds pass.
-void enqueue_search(cc_ctx *c, uint64_t n, float *aabb, cudaStream_t s, bool owner_scan = true) {
+// Shift (unless done) .. pair test: needs stats zeroed and the plan from the
+// bounds pass.
+void enqueue_pairs(cc_ctx *c, uint64_t n, float *aabb, uint64_t entries_hint, cudaStream_t s, bool shift) {
 	BpBuffers b = bp_buffers(c);
 	const uint32_t gmax = c->gp.g_max;
+	if (!b.pre_zeroed) cudaMemsetAsync(b.cell_count, 0, sizeof(uint32_t) * gmax, s);
+	if (c->chain) {
+		{
+			StageMark m(c, ST_COUNT, s);
+			launch_link(n, aabb, b, s, shift);
+		}
+		StageMark m(c, ST_PAIR_TEST, s);
+		if (c->chain_check) launch_chain_check(b, gmax, s);
+		launch_walk(n, b, entries_hint, s);
+		c->launches += c->chain_check ? 3 : 2;
+		return;
+	}
 	{
 		StageMark m(c, ST_COUNT, s);
-		if (!b.pre_zeroed) cudaMemsetAsync(b.cell_count, 0, sizeof(uint32_t) * gmax, s);
-		launch_count(n, aabb, b, s);
+		launch_count(n, aabb, b, s, shift);
 	}
 	{
 		StageMark m(c, ST_SCAN_CELLS, s);
@@ -483,15 +525,19 @@ void enqueue_search(cc_ctx *c, uint64_t n, float *aabb, cudaStream_t s, bool own
 	}
 	{
 		StageMark m(c, ST_PAIR_TEST, s);
-		launch_pair_test(n, b, hint_E(c, n), s);
+		launch_pair_test(n, b, entries_hint, s);
 	}
-	owner_scan = owner_scan && !c->fused_now;  // the fused owner sort scans the buckets itself
-	if (owner_scan) {
+	c->launches += 5 - (c->dense_skip ? 1 : 0);  // count, cell scan, scatter, sparse + dense pair test
+}
+
+// Shift .. owner scan.
+void enqueue_search(cc_ctx *c, uint64_t n, float *aabb, cudaStream_t s, bool owner_scan = true) {
+	enqueue_pairs(c, n, aabb, hint_E(c, n), s, true);
+	if (owner_scan && !c->fused_now) {  // the fused owner sort scans the buckets itself
 		StageMark m(c, ST_SCAN_OWNER, s);
-		launch_scan_owner(n, b, s);
+		launch_scan_owner(n, bp_buffers(c), s);
+		c->launches += 1;
 	}
-	// count, cell scan, scatter, sparse + dense pair test, owner scan
-	c->launches += (owner_scan ? 6 : 5) - (c->dense_skip ? 1 : 0);
 }
 
 // Sorted pair list into `out` (device-driven: writes nothing if the pair
@@ -591,31 +637,43 @@ cc_status reset_pass_counters(cc_ctx *c, uint64_t n, cudaStream_t s) {
 	CC_CUDA(c, cudaMemsetAsync(&d->big_segments, 0, 3 * sizeof(unsigned long long), s));
 	CC_CUDA(c, cudaMemsetAsync(&d->np_n, 0, sizeof(unsigned long long), s));
 	CC_CUDA(c, cudaMemsetAsync(&d->dense_items, 0, sizeof(unsigned long long), s));
+	CC_CUDA(c, cudaMemsetAsync(&d->extra, 0, sizeof(unsigned long long), s));
+	CC_CUDA(c, cudaMemsetAsync(d->bar_scan, 0, sizeof(d->bar_scan), s));
 	return CC_OK;
 }
 
 // After the synchronize: if a scratch guess (entries, unsorted pairs) was too
-// small, grow it and redo the passes after the count (rare: the guesses
-// follow the previous call). h_stats is current on return.
+// small or a chain too long, grow the scratch or turn to sorted cells and redo
+// the search on the shifted boxes (rare: guesses and path follow the previous
+// call). h_stats is current on return.
 cc_status settle(cc_ctx *c, uint64_t n, float *aabb, unsigned long long *out, uint64_t out_cap, const NpArgs *np,
                  cudaStream_t s) {
-	for (int round = 0; round < 3; round++) {
+	for (int round = 0; round < 4; round++) {
 		const uint64_t E = c->h_stats->entries, P = c->h_stats->pairs;
 		BpBuffers b = bp_buffers(c);
-		if (E <= b.entry_cap && P <= b.pair_cap) return CC_OK;
+		const bool crowded = c->chain && (c->h_stats->err & kErrLongChain);
+		if (E <= b.entry_cap && P <= b.pair_cap && !crowded) return CC_OK;
 		if (E >= 0xffffffffull)
 			return set_err(c, CC_ERR_CAPACITY, "search grid needs %llu entries (>= 2^32)", (unsigned long long)E);
 		if (E > b.entry_cap) {
 			CC_TRY(ensure(c, c->entries, 2 * sizeof(float4) * (E + E / 8)));
+			CC_TRY(ensure(c, c->extra, sizeof(uint32_t) * (c->entries.bytes / (2 * sizeof(float4)))));
 			CC_TRY(ensure(c, c->dense, sizeof(uint2) * ((E + E / 8) / kDenseCell + 1024)));
+		}
+		if (crowded) {
+			c->chain = false;
+			c->chain_state = cc_ctx::kChainNo;
+			c->chain_wait = c->h_stats->dense_items && c->gp.dense_cell <= kChainLong ? 0 : kChainWait;
+			c->dense_skip = false;
 		}
 		if (P > b.pair_cap) CC_TRY(ensure(c, c->pairs_tmp, sizeof(unsigned long long) * (P + P / 8)));
 		CC_TRY(reset_pass_counters(c, n, s));
-		b = bp_buffers(c);
-		launch_scatter(n, aabb, b, s);
-		launch_pair_test(n, b, E, s);
-		if (!c->fused_now) launch_scan_owner(n, b, s);
-		c->launches += 4 - (c->fused_now ? 1 : 0) - (c->dense_skip ? 1 : 0);
+		c->chain_check = c->chain_check && c->chain;
+		enqueue_pairs(c, n, aabb, E, s, false);
+		if (!c->fused_now) {
+			launch_scan_owner(n, bp_buffers(c), s);
+			c->launches += 1;
+		}
 		if (out) enqueue_emit(c, n, out, out_cap, s);
 		if (np) enqueue_np(c, *np, out_cap, &ptr<DevStats>(c->stats)->np_n, s);
 		CC_TRY(check_launch(c));
@@ -650,6 +708,15 @@ void remember(cc_ctx *c) {
 	c->last_E = c->h_stats->entries;
 	c->last_P = c->h_stats->pairs;
 	c->last_dense = c->h_stats->dense_items;
+	// chains while no cell is crowded; back to them once sorted cells show none
+	// (which they tell through their dense cells, so a raised threshold makes
+	// them blind) or some calls after a box over too many cells
+	if (c->chain) {
+		c->chain_state = c->last_dense ? cc_ctx::kChainNo : cc_ctx::kChainOk;
+		c->chain_wait = c->gp.dense_cell <= kChainLong ? 0 : kChainWait;
+	} else if (c->last_dense == 0 && --c->chain_wait < 0) {
+		c->chain_state = cc_ctx::kChainUnknown;
+	}
 	for (int d = 0; d < 3; d++) c->last_dim[d] = c->h_stats->plan.dim[d];
 }
 
@@ -792,7 +859,7 @@ cc_status collide_enqueue(cc_ctx *c, const cc_scene &sc, int gx, int gy, int gz,
 			StageMark m(c, ST_AABB, st);
 			CC_CUDA(c, cudaMemsetAsync(d, 0, sizeof(DevStats), st));
 			launch_aabb(n, sc.T, sc.A, sc.B, sc.C, sc.R, sc.ID, sc.nb, sc.body_pos, sc.body_rot, aabb, d, &d->err,
-			            c->gp, grid, st, zero);
+			            c->call_gp, grid, st, zero);
 		}
 		c->launches += 1;
 		c->pass_zeroed = true;
@@ -822,7 +889,7 @@ cc_status collide_enqueue(cc_ctx *c, const cc_scene &sc, int gx, int gy, int gz,
 	struct {
 		uint64_t n, nb, pairs_cap, hE, hP, gen, st[3];
 		const void *p[18];
-		int dims[3], prec, oshift, kbits, ov, fused, dense_skip;
+		int dims[3], prec, oshift, kbits, ov, fused, dense_skip, chain;
 		float env;
 		GridParams gp;
 		uint64_t hslots;
@@ -833,10 +900,11 @@ cc_status collide_enqueue(cc_ctx *c, const cc_scene &sc, int gx, int gy, int gz,
 	const void *ps[18] = {sc.T, sc.A, sc.B, sc.C, sc.R, sc.ID, sc.active, sc.body_pos, sc.body_rot, aabb,
 	                      pairs, norm, cpta, cptb, depth, bids, nullptr, nullptr};
 	memcpy(k.p, ps, sizeof(ps));
-	k.dims[0] = gx; k.dims[1] = gy; k.dims[2] = gz; k.prec = c->np_precision; k.env = envelope; k.gp = c->gp;
+	k.dims[0] = gx; k.dims[1] = gy; k.dims[2] = gz; k.prec = c->np_precision; k.env = envelope; k.gp = c->call_gp;
 	k.oshift = c->owner_shift; k.kbits = c->key_bits; k.ov = ov ? 1 : 0; k.hslots = ov ? c->np_hslots : 0;
 	k.fused = c->fused_now ? 1 : 0;
 	k.dense_skip = c->dense_skip ? 1 : 0;
+	k.chain = (c->chain ? 1 : 0) + (c->chain_check ? 2 : 0);
 	return run_graphed(c, c->g_collide, &k, sizeof(k), enqueue_all, s);
 }
 
@@ -912,7 +980,7 @@ cc_status collide_verlet(cc_ctx *c, const cc_scene &sc, int gx, int gy, int gz, 
 		const auto enqueue_front = [&](cudaStream_t st) -> cc_status {
 			CC_CUDA(c, cudaMemsetAsync(d, 0, sizeof(DevStats), st));
 			launch_aabb(n, sc.T, sc.A, sc.B, sc.C, sc.R, sc.ID, sc.nb, sc.body_pos, sc.body_rot, aabb, d, &d->err,
-			            c->gp, grid, st);
+			            c->call_gp, grid, st);
 			c->launches += 1;
 			return CC_OK;
 		};
@@ -1070,7 +1138,7 @@ void cc_ctx_destroy(cc_ctx *c) {
 	               &c->b_base,   &c->b_status,   &c->b_ticket,   &c->b_res,    &c->g_T,         &c->g_A,
 	               &c->g_B,      &c->g_C,        &c->g_R,        &c->g_ID,     &c->g_pos,       &c->g_rot,
 	               &c->g_act,    &c->g_src,      &c->g_off,      &c->v_ref,    &c->v_backup,   &c->v_scratch, &c->v_cand,   &c->v_status,
-	               &c->np_bsum,  &c->pt_desc,    &c->np_hkeys,   &c->np_hvals,   &c->bp_bsum,    &c->cell_cs};
+	               &c->np_bsum,  &c->pt_desc,    &c->np_hkeys,   &c->np_hvals,   &c->bp_bsum,    &c->cell_cs,  &c->extra};
 	for (Buf *b : bufs)
 		if (b->p) cudaFree(b->p);
 	c->g_collide.drop();
@@ -1158,6 +1226,7 @@ cc_status cc_set_dense_cell(cc_ctx *c, uint32_t entries) {
 	if (!c) return CC_ERR_INVALID_ARGUMENT;
 	c->gp.dense_cell = entries ? std::max<uint32_t>(entries, kDenseCell) : 0xffffffffu;
 	c->last_dense = 1;  // the next call launches the dense-cell kernel and counts again
+	c->chain_state = cc_ctx::kChainUnknown;
 	return CC_OK;
 }
 
@@ -1279,7 +1348,7 @@ cc_status cc_broadphase(cc_ctx *c, uint64_t n, float *aabb, int gx, int gy, int 
 	{
 		StageMark m(c, ST_BOUNDS, s);
 		CC_CUDA(c, cudaMemsetAsync(c->stats.p, 0, sizeof(DevStats), s));
-		launch_bounds(n, aabb, ptr<DevStats>(c->stats), c->gp, grid, s);
+		launch_bounds(n, aabb, ptr<DevStats>(c->stats), c->call_gp, grid, s);
 	}
 	c->launches += 1;
 	enqueue_search(c, n, aabb, s);
@@ -1336,7 +1405,7 @@ cc_status cc_broadphase_bins(cc_ctx *c, uint64_t n, float *aabb, int gx, int gy,
 	BpBuffers b = bp_buffers(c);
 	const int grid[3] = {gx, gy, gz};
 	CC_CUDA(c, cudaMemsetAsync(c->stats.p, 0, sizeof(DevStats), s));
-	launch_bounds(n, aabb, b.stats, c->gp, grid, s);  // + plan
+	launch_bounds(n, aabb, b.stats, c->call_gp, grid, s);  // + plan
 	CC_CUDA(c, cudaMemsetAsync(b.cell_count, 0, sizeof(uint32_t) * c->gp.g_max, s));
 	launch_count(n, aabb, b, s);  // in-place shift
 	// per-body bin counts -> offsets
@@ -1511,12 +1580,12 @@ cc_status batch_impl(cc_ctx *c, const cc_batch *bt, int gx, int gy, int gz, floa
 			CC_CUDA(c, cudaMemsetAsync(sst, 0, sizeof(SceneStats) * S, st));
 			launch_batch_prep(n, (uint32_t)S, d_shape, d_body, sc.ID, scene_of, gid, &d->err, st);
 			launch_aabb(n, sc.T, sc.A, sc.B, sc.C, sc.R, gid, sc.nb, sc.body_pos, sc.body_rot, res->aabb, nullptr,
-			            &d->err, c->gp, grid, st, zero);
+			            &d->err, c->call_gp, grid, st, zero);
 		}
 		{
 			StageMark m(c, ST_BOUNDS, st);
 			launch_batch_bounds(n, res->aabb, scene_of, sst, &d->err, st);
-			launch_batch_plan((uint32_t)S, d_shape, sst, c->gp, grid, plans, G, st);
+			launch_batch_plan((uint32_t)S, d_shape, sst, c->call_gp, grid, plans, G, st);
 			launch_scan_u32_to_u32(G, S, base, ptr<uint64_t>(c->b_status), ptr<uint32_t>(c->b_ticket), &d->err, st,
 			                       nullptr, &d->cells);
 		}
@@ -1539,7 +1608,7 @@ cc_status batch_impl(cc_ctx *c, const cc_batch *bt, int gx, int gy, int gz, floa
 	struct {
 		uint64_t n, nb, S, pairs_cap, hE, hP, gen, st[3];
 		const void *p[16];
-		int dims[3], prec, want;
+		int dims[3], prec, want, chain;
 		float env;
 		GridParams gp;
 	} k;
@@ -1551,7 +1620,8 @@ cc_status batch_impl(cc_ctx *c, const cc_batch *bt, int gx, int gy, int gz, floa
 	                      res->pairs, res->norm, res->cpta, res->cptb, res->depth, res->bids};
 	memcpy(k.p, ps, sizeof(ps));
 	k.dims[0] = gx; k.dims[1] = gy; k.dims[2] = gz; k.prec = c->np_precision; k.want = want_offsets ? 1 : 0;
-	k.env = envelope; k.gp = c->gp;
+	k.chain = (c->chain ? 1 : 0) + (c->chain_check ? 2 : 0);
+	k.env = envelope; k.gp = c->call_gp;
 	CC_TRY(run_graphed(c, c->g_batch, &k, sizeof(k), enqueue_all, s));
 	auto copy_back = [&]() -> cc_status {
 		if (scene_pairs)
@@ -1570,7 +1640,7 @@ cc_status batch_impl(cc_ctx *c, const cc_batch *bt, int gx, int gy, int gz, floa
 	CC_TRY(check_launch(c));
 	CC_TRY(read_stats(c, s));
 	CC_TRY(device_err(c));
-	bool redone = c->h_stats->entries > c->entries.bytes / (2 * sizeof(float4)) ||
+	bool redone = (c->h_stats->err & kErrLongChain) || c->h_stats->entries > c->entries.bytes / (2 * sizeof(float4)) ||
 	              c->h_stats->pairs > c->pairs_tmp.bytes / sizeof(unsigned long long);
 	CC_TRY(settle(c, n, res->aabb, out, pairs_cap, &a, s));
 	remember(c);

@@ -20,6 +20,7 @@ enum DeviceError : uint32_t {
 	kErrSegmentTooLong = 1u << 4,  // a pair segment exceeded the block sort size (host falls back)
 	kErrBinCount = 1u << 5,      // a body covers a negative / overflowing number of reference bins
 	kErrBadIndex = 1u << 6,      // a body id >= nb or a pair index >= n (the access is skipped)
+	kErrLongChain = 1u << 8,     // a cell's chain was too long for the chained search (host redoes it on sorted cells)
 	kErrHashFull = 1u << 7,      // the overlapped narrowphase's contact hash overflowed (host redoes it in order)
 };
 

@@ -39,9 +39,10 @@ struct DevStats {
 	unsigned long long seg_big;       // owner buckets of 1025..16384 pairs (listed from the back)
 	unsigned long long cells;     // plan.G as a 64-bit scan count
 	unsigned long long np_n;      // pairs handed to the narrowphase (0 if an output was too small)
-	unsigned long long dense_items;  // (cell, row chunk) work items of the dense-cell pair test
+	unsigned long long dense_items;  // (cell, row chunk) work items of the dense-cell pair test (chained search: long chains met)
 	uint32_t blocks_done;         // last-block detection of the bounds reduction
 	uint32_t pad_;
+	unsigned long long extra;     // entries of the chained search beyond the first one of every body
 	Plan plan;
 	// grid barriers of the cooperative kernels (GridBarrier: arrived, gen),
 	// zeroed with the rest at the start of a pass
@@ -169,7 +170,15 @@ struct BpBuffers {
 	// cursor 0: the scatter takes a slot with one 64-bit atomic instead of a
 	// start load plus a cursor atomic (launch_scatter with packed = true)
 	unsigned long long *cell_cs = nullptr;
+	// chained search (launch_link, launch_walk): the body of every entry past
+	// the n first ones; cell_count holds the cells' chain heads
+	uint32_t *extra_body = nullptr;
 };
+// Cells with more entries make the next call search on sorted cells: above
+// this the tests of a cell are work for whole warps, not a lane's chain.
+constexpr uint32_t kChainLong = 128;
+// A box over more cells than this also turns the search to sorted cells.
+constexpr uint32_t kChainCells = 65535;
 constexpr uint32_t kScanCoopBlocks = 2048;
 // Owner buckets of n bodies at a shift.
 __host__ __device__ inline uint64_t owner_buckets(uint64_t n, int shift) {
@@ -180,10 +189,21 @@ __host__ __device__ inline uint64_t owner_buckets(uint64_t n, int shift) {
 void launch_bounds(uint64_t n, const float *aabb, DevStats *stats, const GridParams &gp, const int grid[3],
                    cudaStream_t s, const ZeroList &zero = ZeroList());
 // In-place shift + per-cell counts on the plan's search grid.
-void launch_count(uint64_t n, float *aabb, const BpBuffers &b, cudaStream_t s);
+// (shift false: the boxes are shifted already).
+void launch_count(uint64_t n, float *aabb, const BpBuffers &b, cudaStream_t s, bool shift = true);
 void launch_scan_cells(const BpBuffers &b, uint32_t g_max, cudaStream_t s);
 void launch_scatter(uint64_t n, const float *aabb, const BpBuffers &b, cudaStream_t s, bool packed = false);
 void launch_pair_test(uint64_t n, const BpBuffers &b, uint64_t entries_hint, cudaStream_t s);
+// The chained search, for scenes without crowded cells: in-place shift (shift
+// false: done already), entries and the cells' chains in one pass; the pair
+// test along the chains in a second. Entries past entry_cap are counted and
+// dropped (stats->entries tells). check: a pass in between that looks for
+// chains above kChainLong and makes the walk return at once if there are any;
+// without it the walk itself notes them, and gives up (kErrLongChain) only on
+// chains many times as long.
+void launch_link(uint64_t n, float *aabb, const BpBuffers &b, cudaStream_t s, bool shift = true);
+void launch_chain_check(const BpBuffers &b, uint32_t g_max, cudaStream_t s);
+void launch_walk(uint64_t n, const BpBuffers &b, uint64_t entries_hint, cudaStream_t s);
 void launch_scan_owner(uint64_t n, const BpBuffers &b, cudaStream_t s);
 // Cells holding more than b.dense_cell entries are left out of the
 // lane-per-entry pair test and tested here instead, tile by tile (N-body

@@ -82,7 +82,8 @@ CC_API const char *cc_version(void);
  * overlapping boxes share a cell of any grid), so by default (0,0,0) the
  * library picks it from the scene bounds, the body count and the mean box
  * extent: cells hold about `cell_target` boxes and are at least `min_ratio`
- * mean box extents wide. (gx,gy,gz) > 0 pins the grid. */
+ * mean box extents wide (a quarter of cell_target while no cell is crowded:
+ * cells are then chained, not sorted). (gx,gy,gz) > 0 pins the grid. */
 CC_API cc_status cc_set_search_grid(cc_ctx *ctx, int gx, int gy, int gz);
 CC_API cc_status cc_set_tuning(cc_ctx *ctx, float cell_target, float min_ratio);
 /* Incremental broadphase for time-step updates (default off; the reference
