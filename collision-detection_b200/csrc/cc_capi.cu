@@ -83,8 +83,8 @@ struct cc_ctx {
 	Buf in_T, in_A, in_B, in_C, in_R, in_ID, in_pos, in_rot, in_act, out_aabb, out_pairs, out_norm, out_pa, out_pb,
 	    out_depth, out_bids;
 	// batch scratch: offsets, scene of each shape, global body ids, per-scene
-	// stats and plans, scene cell counts and bases, G-scan control, results
-	Buf b_off, b_scene_of, b_gid, b_sst, b_plans, b_G, b_base, b_status, b_ticket, b_res;
+	// stats and plans, cell bases, results
+	Buf b_off, b_scene_of, b_gid, b_sst, b_plans, b_base, b_res;
 	// descriptor table of cc_perturb_scenes
 	Buf pt_desc;
 	// overlapped narrowphase (cc_set_narrowphase_overlap): the MPR on the
@@ -96,7 +96,7 @@ struct cc_ctx {
 	Buf np_hkeys, np_hvals;
 	uint64_t np_hslots = 0;
 	// gather arena of cc_collide_scenes
-	Buf g_T, g_A, g_B, g_C, g_R, g_ID, g_pos, g_rot, g_act, g_src, g_off;
+	Buf g_T, g_A, g_B, g_C, g_R, g_ID, g_pos, g_rot, g_act, g_src;
 	SceneMap sm;  // set while a batch call runs
 	DevStats *h_stats = nullptr;  // pinned
 	uint64_t *h_word = nullptr;   // pinned scratch words
@@ -413,13 +413,8 @@ bool chain_enabled() {
 // ends with a synchronize, so nothing in flight uses a buffer replaced here.
 cc_status prepare(cc_ctx *c, uint64_t n, uint64_t np_cap, uint64_t g_override = 0) {
 	c->gp.g_max = g_override ? (uint32_t)g_override : g_max_for(n);
-	if (g_override) {  // a batch: its per-scene pair counts are read at scene boundaries of the owner offsets
-		c->owner_shift = 0;
-		c->key_bits = 32;
-	} else {
-		choose_owner_shift(c, n);
-	}
-	c->fused_now = !g_override && fused_sort_enabled() && fused_sort_fits(owner_buckets(n, c->owner_shift));
+	choose_owner_shift(c, n);
+	c->fused_now = fused_sort_enabled() && fused_sort_fits(owner_buckets(n, c->owner_shift));
 	c->dense_skip = !g_override && c->last_dense == 0;
 	c->chain = chain_enabled() && c->chain_state != cc_ctx::kChainNo && n < ((uint64_t)1 << 31);
 	c->chain_check = c->chain && c->chain_state == cc_ctx::kChainUnknown;
@@ -625,6 +620,44 @@ cc_status enqueue_sort_and_np_overlapped(cc_ctx *c, uint64_t n, const NpArgs &a,
 	return CC_OK;
 }
 
+// Whether this call's narrowphase is overlapped with the pair sort (outputs of
+// at most 2^24 pairs), with the stream, events and contact hash it needs.
+cc_status overlap_prepare(cc_ctx *c, uint64_t pairs_cap, bool &ov) {
+	ov = c->np_overlap && pairs_cap > 0 && pairs_cap <= ((uint64_t)1 << 24);
+	if (!ov) return CC_OK;
+	if (!c->np_stream) CC_CUDA(c, cudaStreamCreateWithFlags(&c->np_stream, cudaStreamNonBlocking));
+	if (!c->ev_fork) CC_CUDA(c, cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming));
+	if (!c->ev_join) CC_CUDA(c, cudaEventCreateWithFlags(&c->ev_join, cudaEventDisableTiming));
+	c->np_hslots = pow2ceil(std::max<uint64_t>(4 * std::min<uint64_t>(hint_P(c), pairs_cap), 4096));
+	CC_TRY(ensure(c, c->np_hkeys, sizeof(unsigned long long) * c->np_hslots));
+	return ensure(c, c->np_hvals, sizeof(uint32_t) * c->np_hslots);
+}
+
+// What a pass's first kernel zeroes: scan control words, class counters, cell
+// counts and, with the narrowphase overlapped, the contact hash.
+ZeroList pass_zero_list(cc_ctx *c, bool ov) {
+	ZeroList zero;
+	zero.p[0] = ptr<uint32_t>(c->status);
+	zero.words[0] = 2 * (c->st_words[0] + c->st_words[1] + c->st_words[2]);
+	zero.p[1] = ptr<uint32_t>(c->ticket);
+	zero.words[1] = 16;
+	zero.p[2] = ptr<uint32_t>(c->np_classes);
+	zero.words[2] = 2 * kNpClasses + 1;
+	zero.p[3] = ptr<uint32_t>(c->cell_count);
+	zero.words[3] = c->gp.g_max;
+	if (ov) {
+		zero.p[4] = ptr<uint32_t>(c->np_hkeys);
+		zero.words[4] = 2 * c->np_hslots;
+	}
+	for (int r = 0; r < 5; r++)
+		if (!zero.p[r]) zero.words[r] = 0;
+	return zero;
+}
+
+// After a pass's counters were read: runs the narrowphase again, in order, where
+// the sort or the overlapped narrowphase could not finish. *redone tells.
+cc_status finish_np(cc_ctx *c, uint64_t n, const NpArgs &a, uint64_t P, uint64_t pairs_cap, cudaStream_t s, bool *redone);
+
 // Zeroes the per-pass counters before the passes after the count are redone.
 cc_status reset_pass_counters(cc_ctx *c, uint64_t n, cudaStream_t s) {
 	DevStats *d = ptr<DevStats>(c->stats);
@@ -822,38 +855,14 @@ cc_status collide_enqueue(cc_ctx *c, const cc_scene &sc, int gx, int gy, int gz,
 	const uint64_t n = sc.n;
 	PdlScope pdl_(n);
 	CC_TRY(prepare(c, n, pairs_cap));
-	// overlapped narrowphase: one scene, an output of at most 2^24 pairs
-	const bool ov = c->np_overlap && pairs_cap > 0 && pairs_cap <= ((uint64_t)1 << 24);
-	if (ov) {
-		if (!c->np_stream) CC_CUDA(c, cudaStreamCreateWithFlags(&c->np_stream, cudaStreamNonBlocking));
-		if (!c->ev_fork) CC_CUDA(c, cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming));
-		if (!c->ev_join) CC_CUDA(c, cudaEventCreateWithFlags(&c->ev_join, cudaEventDisableTiming));
-		c->np_hslots = pow2ceil(std::max<uint64_t>(4 * std::min<uint64_t>(hint_P(c), pairs_cap), 4096));
-		CC_TRY(ensure(c, c->np_hkeys, sizeof(unsigned long long) * c->np_hslots));
-		CC_TRY(ensure(c, c->np_hvals, sizeof(uint32_t) * c->np_hslots));
-	}
+	bool ov;
+	CC_TRY(overlap_prepare(c, pairs_cap, ov));
 	DevStats *d = ptr<DevStats>(c->stats);
 	const int grid[3] = {gx, gy, gz};
 	unsigned long long *out = reinterpret_cast<unsigned long long *>(pairs);
 	const NpArgs a = {n, sc.nb, sc.T, sc.A, sc.B, sc.C, sc.R, sc.ID, sc.active, sc.body_pos, sc.body_rot, envelope,
 	                  pairs, norm, cpta, cptb, depth, bids};
-	// the AABB kernel also zeroes the pass's scan control words, class
-	// counters and cell counts
-	ZeroList zero;
-	zero.p[0] = ptr<uint32_t>(c->status);
-	zero.words[0] = 2 * (c->st_words[0] + c->st_words[1] + c->st_words[2]);
-	zero.p[1] = ptr<uint32_t>(c->ticket);
-	zero.words[1] = 16;
-	zero.p[2] = ptr<uint32_t>(c->np_classes);
-	zero.words[2] = 2 * kNpClasses + 1;
-	zero.p[3] = ptr<uint32_t>(c->cell_count);
-	zero.words[3] = c->gp.g_max;
-	if (ov) {  // the contact hash starts empty
-		zero.p[4] = ptr<uint32_t>(c->np_hkeys);
-		zero.words[4] = 2 * c->np_hslots;
-	}
-	for (int r = 0; r < 5; r++)
-		if (!zero.p[r]) zero.words[r] = 0;
+	const ZeroList zero = pass_zero_list(c, ov);
 	auto enqueue_all = [&](cudaStream_t st) -> cc_status {
 		{
 			StageMark m(c, ST_AABB, st);
@@ -908,6 +917,25 @@ cc_status collide_enqueue(cc_ctx *c, const cc_scene &sc, int gx, int gy, int gz,
 	return run_graphed(c, c->g_collide, &k, sizeof(k), enqueue_all, s);
 }
 
+cc_status finish_np(cc_ctx *c, uint64_t n, const NpArgs &a, uint64_t P, uint64_t pairs_cap, cudaStream_t s, bool *redone) {
+	DevStats *d = ptr<DevStats>(c->stats);
+	if (c->h_stats->err & kErrSegmentTooLong) {
+		// the list was sorted bucket-wise only up to 4096 per bucket: sort it whole
+		CC_TRY(sort_fallback(c, n, P, reinterpret_cast<unsigned long long *>(a.pairs), s));
+	} else if (c->h_stats->err & kErrHashFull) {
+		// more contacts than the overlapped narrowphase's hash took: run it again on the sorted list,
+		// which its compaction kept in the unsorted-pair scratch before permuting the output
+		CC_CUDA(c, cudaMemcpyAsync(a.pairs, c->pairs_tmp.p, sizeof(unsigned long long) * P, cudaMemcpyDeviceToDevice, s));
+	} else {
+		return CC_OK;
+	}
+	CC_CUDA(c, cudaMemsetAsync(&d->contacts, 0, sizeof(unsigned long long), s));
+	enqueue_np(c, a, pairs_cap, &d->np_n, s);
+	CC_TRY(check_launch(c));
+	if (redone) *redone = true;
+	return read_stats(c, s);
+}
+
 // The second half: with c->h_stats current (the step's DevStats), checks
 // errors, redoes passes whose scratch was too small, and reports the counts.
 cc_status collide_finish(cc_ctx *c, const cc_scene &sc, float envelope, float *aabb, int64_t *pairs,
@@ -928,22 +956,7 @@ cc_status collide_finish(cc_ctx *c, const cc_scene &sc, float envelope, float *a
 		return set_err(c, CC_ERR_CAPACITY, "pair list needs %llu entries, capacity %llu", (unsigned long long)P,
 		               (unsigned long long)pairs_cap);
 	}
-	if (c->h_stats->err & kErrSegmentTooLong) {
-		// the list was sorted bucket-wise only up to 4096 per bucket: sort it whole, redo the narrowphase
-		CC_TRY(sort_fallback(c, n, P, out, s));
-		CC_CUDA(c, cudaMemsetAsync(&d->contacts, 0, sizeof(unsigned long long), s));
-		enqueue_np(c, a, pairs_cap, &d->np_n, s);
-		CC_TRY(check_launch(c));
-		CC_TRY(read_stats(c, s));
-	} else if (c->h_stats->err & kErrHashFull) {
-		// more contacts than the overlapped narrowphase's hash took: run it again on the sorted list,
-		// which its compaction kept in the unsorted-pair scratch before permuting the output
-		CC_CUDA(c, cudaMemcpyAsync(out, c->pairs_tmp.p, sizeof(unsigned long long) * P, cudaMemcpyDeviceToDevice, s));
-		CC_CUDA(c, cudaMemsetAsync(&d->contacts, 0, sizeof(unsigned long long), s));
-		enqueue_np(c, a, pairs_cap, &d->np_n, s);
-		CC_TRY(check_launch(c));
-		CC_TRY(read_stats(c, s));
-	}
+	CC_TRY(finish_np(c, n, a, P, pairs_cap, s, nullptr));
 	if (c->h_stats->err & kErrBadIndex)
 		return set_err(c, CC_ERR_INVALID_INPUT, "a pair index is >= n or a body id is >= nb");
 	*n_contacts = c->h_stats->contacts;
@@ -1134,10 +1147,10 @@ void cc_ctx_destroy(cc_ctx *c) {
 	               &c->np_flag,  &c->np_pos,     &c->np_order, &c->np_classes, &c->in_T,       &c->in_A,     &c->in_B,        &c->in_C,
 	               &c->in_R,     &c->in_ID,      &c->in_pos,     &c->in_rot,   &c->in_act,      &c->out_aabb,
 	               &c->out_pairs, &c->out_norm,  &c->out_pa,     &c->out_pb,   &c->out_depth,   &c->out_bids,
-	               &c->b_off,    &c->b_scene_of, &c->b_gid,      &c->b_sst,    &c->b_plans,     &c->b_G,
-	               &c->b_base,   &c->b_status,   &c->b_ticket,   &c->b_res,    &c->g_T,         &c->g_A,
+	               &c->b_off,    &c->b_scene_of, &c->b_gid,      &c->b_sst,    &c->b_plans,
+	               &c->b_base,   &c->b_res,      &c->g_T,        &c->g_A,
 	               &c->g_B,      &c->g_C,        &c->g_R,        &c->g_ID,     &c->g_pos,       &c->g_rot,
-	               &c->g_act,    &c->g_src,      &c->g_off,      &c->v_ref,    &c->v_backup,   &c->v_scratch, &c->v_cand,   &c->v_status,
+	               &c->g_act,    &c->g_src,      &c->v_ref,    &c->v_backup,   &c->v_scratch, &c->v_cand,   &c->v_status,
 	               &c->np_bsum,  &c->pt_desc,    &c->np_hkeys,   &c->np_hvals,   &c->bp_bsum,    &c->cell_cs,  &c->extra};
 	for (Buf *b : bufs)
 		if (b->p) cudaFree(b->p);
@@ -1496,8 +1509,12 @@ cc_status cc_narrowphase(cc_ctx *c, uint64_t n, const int32_t *T, const float *A
 }  // extern "C"
 
 namespace {
+// src: device table of the scenes' own arrays, gathered into bt->scene's by the
+// pass's first kernel (null: bt->scene holds them); d_off then holds the shape
+// and body offsets already.
 cc_status batch_impl(cc_ctx *c, const cc_batch *bt, int gx, int gy, int gz, float envelope, cc_result *res,
-                     uint64_t *scene_pairs, uint64_t *contact_offsets, void *stream) {
+                     uint64_t *scene_pairs, uint64_t *contact_offsets, void *stream, const SceneSrc *src = nullptr,
+                     unsigned long long *d_off = nullptr) {
 	res->n_pairs = res->n_contacts = 0;
 	c->retained = false;
 	const uint64_t S = bt->num_scenes;
@@ -1526,25 +1543,28 @@ cc_status batch_impl(cc_ctx *c, const cc_batch *bt, int gx, int gy, int gz, floa
 	cudaStream_t s = (cudaStream_t)stream;
 	const uint64_t pairs_cap = res->pairs_cap;
 	CC_TRY(prepare(c, n, pairs_cap, std::max<uint64_t>(g_total, 1)));
-	CC_TRY(ensure(c, c->b_off, sizeof(unsigned long long) * 2 * (S + 1)));
+	bool ov;
+	CC_TRY(overlap_prepare(c, pairs_cap, ov));
 	CC_TRY(ensure(c, c->b_scene_of, sizeof(uint32_t) * n));
 	CC_TRY(ensure(c, c->b_gid, sizeof(uint32_t) * n));
 	CC_TRY(ensure(c, c->b_sst, sizeof(SceneStats) * S));
 	CC_TRY(ensure(c, c->b_plans, sizeof(Plan) * S));
-	CC_TRY(ensure(c, c->b_G, sizeof(uint32_t) * (S + 1)));
 	CC_TRY(ensure(c, c->b_base, sizeof(uint32_t) * (S + 2)));
-	CC_TRY(ensure(c, c->b_status, sizeof(uint64_t) * status_words_for(S + 1)));
-	CC_TRY(ensure(c, c->b_ticket, 64));
 	CC_TRY(ensure(c, c->b_res, sizeof(unsigned long long) * (2 * S + 2)));
-	unsigned long long *d_shape = ptr<unsigned long long>(c->b_off), *d_body = d_shape + (S + 1);
-	CC_CUDA(c, copy_small_h2d(d_shape, bt->shape_offsets, sizeof(uint64_t) * (S + 1), s));
-	CC_CUDA(c, copy_small_h2d(d_body, bt->body_offsets, sizeof(uint64_t) * (S + 1), s));
+	if (!d_off) {
+		CC_TRY(ensure(c, c->b_off, sizeof(unsigned long long) * 2 * (S + 1)));
+		d_off = ptr<unsigned long long>(c->b_off);
+		std::vector<uint64_t> off(bt->shape_offsets, bt->shape_offsets + S + 1);
+		off.insert(off.end(), bt->body_offsets, bt->body_offsets + S + 1);
+		CC_CUDA(c, copy_small_h2d(d_off, off.data(), sizeof(uint64_t) * off.size(), s));
+	}
+	unsigned long long *d_shape = d_off, *d_body = d_off + (S + 1);
 	DevStats *d = ptr<DevStats>(c->stats);
 	const int grid[3] = {gx, gy, gz};
 	uint32_t *scene_of = ptr<uint32_t>(c->b_scene_of), *gid = ptr<uint32_t>(c->b_gid);
 	SceneStats *sst = ptr<SceneStats>(c->b_sst);
 	Plan *plans = ptr<Plan>(c->b_plans);
-	uint32_t *G = ptr<uint32_t>(c->b_G), *base = ptr<uint32_t>(c->b_base);
+	uint32_t *base = ptr<uint32_t>(c->b_base);
 	unsigned long long *d_pairs_s = ptr<unsigned long long>(c->b_res), *d_coff = d_pairs_s + S;
 	unsigned long long *out = reinterpret_cast<unsigned long long *>(res->pairs);
 	// the rest of the pipeline sees one scene of n shapes with global body ids
@@ -1557,17 +1577,7 @@ cc_status batch_impl(cc_ctx *c, const cc_batch *bt, int gx, int gy, int gz, floa
 	} smg_{c};
 	const NpArgs a = {n, sc.nb, sc.T, sc.A, sc.B, sc.C, sc.R, gid, sc.active, sc.body_pos, sc.body_rot, envelope,
 	                  res->pairs, res->norm, res->cpta, res->cptb, res->depth, res->bids};
-	ZeroList zero;
-	zero.p[0] = ptr<uint32_t>(c->status);
-	zero.words[0] = 2 * (c->st_words[0] + c->st_words[1] + c->st_words[2]);
-	zero.p[1] = ptr<uint32_t>(c->ticket);
-	zero.words[1] = 16;
-	zero.p[2] = ptr<uint32_t>(c->np_classes);
-	zero.words[2] = 2 * kNpClasses + 1;
-	zero.p[3] = ptr<uint32_t>(c->cell_count);
-	zero.words[3] = c->gp.g_max;
-	for (int r = 0; r < 4; r++)
-		if (!zero.p[r]) zero.words[r] = 0;
+	const ZeroList zero = pass_zero_list(c, ov);
 	// the rest of the pipeline takes each shape's plan from the scene map
 	c->sm.scene_of = scene_of;
 	c->sm.plans = plans;
@@ -1578,27 +1588,29 @@ cc_status batch_impl(cc_ctx *c, const cc_batch *bt, int gx, int gy, int gz, floa
 			StageMark m(c, ST_AABB, st);
 			CC_CUDA(c, cudaMemsetAsync(d, 0, sizeof(DevStats), st));
 			CC_CUDA(c, cudaMemsetAsync(sst, 0, sizeof(SceneStats) * S, st));
-			launch_batch_prep(n, (uint32_t)S, d_shape, d_body, sc.ID, scene_of, gid, &d->err, st);
-			launch_aabb(n, sc.T, sc.A, sc.B, sc.C, sc.R, gid, sc.nb, sc.body_pos, sc.body_rot, res->aabb, nullptr,
-			            &d->err, c->call_gp, grid, st, zero);
+			const SceneSrc all{sc.T, sc.A, sc.B, sc.C, sc.R, sc.ID, sc.body_pos, sc.body_rot, sc.active};
+			const SceneDst dst = src ? SceneDst{ptr<int32_t>(c->g_T), ptr<float>(c->g_A), ptr<float>(c->g_B),
+			                                    ptr<float>(c->g_C), ptr<float>(c->g_R), ptr<uint32_t>(c->g_ID),
+			                                    ptr<float>(c->g_pos), ptr<float>(c->g_rot), ptr<uint8_t>(c->g_act)}
+			                         : SceneDst{};
+			launch_batch_front(n, sc.nb, (uint32_t)S, d_shape, d_body, all, src, dst, scene_of, gid, res->aabb, d, sst,
+			                   c->call_gp, grid, plans, base, st, zero);
 		}
-		{
-			StageMark m(c, ST_BOUNDS, st);
-			launch_batch_bounds(n, res->aabb, scene_of, sst, &d->err, st);
-			launch_batch_plan((uint32_t)S, d_shape, sst, c->call_gp, grid, plans, G, st);
-			launch_scan_u32_to_u32(G, S, base, ptr<uint64_t>(c->b_status), ptr<uint32_t>(c->b_ticket), &d->err, st,
-			                       nullptr, &d->cells);
-		}
-		c->launches += 6;
+		c->launches += 1;
 		c->pass_zeroed = true;
-		enqueue_search(c, n, res->aabb, st);
-		enqueue_emit(c, n, out, pairs_cap, st);
-		enqueue_np(c, a, pairs_cap, &d->np_n, st);
+		if (ov) {
+			enqueue_search(c, n, res->aabb, st, false);
+			const cc_status r = enqueue_sort_and_np_overlapped(c, n, a, pairs_cap, st);
+			if (r != CC_OK) return r;
+		} else {
+			enqueue_search(c, n, res->aabb, st);
+			enqueue_emit(c, n, out, pairs_cap, st);
+			enqueue_np(c, a, pairs_cap, &d->np_n, st);
+		}
 		c->pass_zeroed = false;
 		// per-scene pair counts and contact offsets, read back behind the pass
 		if (want_offsets) {
-			launch_batch_offsets((uint32_t)S, d_shape, ptr<unsigned long long>(c->owner_off),
-			                     ptr<unsigned long long>(c->np_pos), d, d_pairs_s, d_coff, st);
+			launch_batch_offsets((uint32_t)S, d_shape, out, d, d_pairs_s, d_coff, st);
 			c->launches += 1;
 		}
 		return CC_OK;
@@ -1607,18 +1619,21 @@ cc_status batch_impl(cc_ctx *c, const cc_batch *bt, int gx, int gy, int gz, floa
 	// copied in before every pass, outside the graph)
 	struct {
 		uint64_t n, nb, S, pairs_cap, hE, hP, gen, st[3];
-		const void *p[16];
-		int dims[3], prec, want, chain;
+		const void *p[18];
+		int dims[3], prec, want, chain, oshift, kbits, ov, fused, dense_skip;
 		float env;
 		GridParams gp;
+		uint64_t hslots;
 	} k;
 	memset(&k, 0, sizeof(k));
 	k.n = n; k.nb = sc.nb; k.S = S; k.pairs_cap = pairs_cap; k.hE = hint_E(c, n); k.hP = hint_P(c);
 	k.gen = c->buf_gen;
 	for (int r = 0; r < 3; r++) k.st[r] = c->st_words[r];
-	const void *ps[16] = {sc.T, sc.A, sc.B, sc.C, sc.R, sc.ID, sc.active, sc.body_pos, sc.body_rot, res->aabb,
-	                      res->pairs, res->norm, res->cpta, res->cptb, res->depth, res->bids};
+	const void *ps[18] = {sc.T, sc.A, sc.B, sc.C, sc.R, sc.ID, sc.active, sc.body_pos, sc.body_rot, res->aabb,
+	                      res->pairs, res->norm, res->cpta, res->cptb, res->depth, res->bids, src, d_off};
 	memcpy(k.p, ps, sizeof(ps));
+	k.oshift = c->owner_shift; k.kbits = c->key_bits; k.ov = ov ? 1 : 0; k.hslots = ov ? c->np_hslots : 0;
+	k.fused = c->fused_now ? 1 : 0; k.dense_skip = c->dense_skip ? 1 : 0;
 	k.dims[0] = gx; k.dims[1] = gy; k.dims[2] = gz; k.prec = c->np_precision; k.want = want_offsets ? 1 : 0;
 	k.chain = (c->chain ? 1 : 0) + (c->chain_check ? 2 : 0);
 	k.env = envelope; k.gp = c->call_gp;
@@ -1631,8 +1646,7 @@ cc_status batch_impl(cc_ctx *c, const cc_batch *bt, int gx, int gy, int gz, floa
 		return CC_OK;
 	};
 	auto copy_offsets = [&]() -> cc_status {
-		launch_batch_offsets((uint32_t)S, d_shape, ptr<unsigned long long>(c->owner_off),
-		                     ptr<unsigned long long>(c->np_pos), d, d_pairs_s, d_coff, s);
+		launch_batch_offsets((uint32_t)S, d_shape, out, d, d_pairs_s, d_coff, s);
 		CC_TRY(check_launch(c));
 		return copy_back();
 	};
@@ -1646,17 +1660,17 @@ cc_status batch_impl(cc_ctx *c, const cc_batch *bt, int gx, int gy, int gz, floa
 	remember(c);
 	const uint64_t P = c->h_stats->pairs;
 	res->n_pairs = P;
-	if (P > pairs_cap)
+	if (P > pairs_cap) {
+		if (scene_pairs) {  // no sorted list to count them in
+			CC_CUDA(c, cudaMemsetAsync(d_pairs_s, 0, sizeof(uint64_t) * S, s));
+			launch_batch_pair_counts(P, ptr<unsigned long long>(c->pairs_tmp), scene_of, d_pairs_s, s);
+			CC_CUDA(c, cudaMemcpyAsync(scene_pairs, d_pairs_s, sizeof(uint64_t) * S, cudaMemcpyDeviceToHost, s));
+			CC_CUDA(c, cudaStreamSynchronize(s));
+		}
 		return set_err(c, CC_ERR_CAPACITY, "pair list needs %llu entries, capacity %llu", (unsigned long long)P,
 		               (unsigned long long)pairs_cap);
-	if (c->h_stats->err & kErrSegmentTooLong) {
-		CC_TRY(sort_fallback(c, n, P, out, s));
-		CC_CUDA(c, cudaMemsetAsync(&d->contacts, 0, sizeof(unsigned long long), s));
-		enqueue_np(c, a, pairs_cap, &d->np_n, s);
-		CC_TRY(check_launch(c));
-		CC_TRY(read_stats(c, s));
-		redone = true;
 	}
+	CC_TRY(finish_np(c, n, a, P, pairs_cap, s, &redone));
 	if (c->h_stats->err & kErrBadIndex)
 		return set_err(c, CC_ERR_INVALID_INPUT, "a pair index is >= n or a body id is outside its scene");
 	res->n_contacts = c->h_stats->contacts;
@@ -1710,25 +1724,24 @@ cc_status cc_collide_scenes(cc_ctx *c, uint64_t num_scenes, const cc_scene *scen
 	CC_TRY(ensure(c, c->g_pos, 12 * std::max<uint64_t>(nb, 1)));
 	CC_TRY(ensure(c, c->g_rot, 16 * std::max<uint64_t>(nb, 1)));
 	CC_TRY(ensure(c, c->g_act, std::max<uint64_t>(nb, 1)));
-	CC_TRY(ensure(c, c->g_src, sizeof(SceneSrc) * num_scenes));
-	CC_TRY(ensure(c, c->g_off, sizeof(unsigned long long) * 2 * (num_scenes + 1)));
-	unsigned long long *d_so = ptr<unsigned long long>(c->g_off), *d_bo = d_so + (num_scenes + 1);
-	CC_CUDA(c, copy_small_h2d(c->g_src.p, src.data(), sizeof(SceneSrc) * num_scenes, s));
-	CC_CUDA(c, copy_small_h2d(d_so, so.data(), sizeof(uint64_t) * (num_scenes + 1), s));
-	CC_CUDA(c, copy_small_h2d(d_bo, bo.data(), sizeof(uint64_t) * (num_scenes + 1), s));
-	SceneDst dst{ptr<int32_t>(c->g_T), ptr<float>(c->g_A), ptr<float>(c->g_B), ptr<float>(c->g_C), ptr<float>(c->g_R),
-	             ptr<uint32_t>(c->g_ID), ptr<float>(c->g_pos), ptr<float>(c->g_rot), ptr<uint8_t>(c->g_act)};
-	{
-		StageMark m(c, ST_COPY_IN, s);
-		launch_gather(n, nb, (uint32_t)num_scenes, d_so, d_bo, ptr<SceneSrc>(c->g_src), dst, s);
-	}
-	c->launches += 2;
+	// the scenes' arrays and the offsets as one table: (SceneSrc per scene), shape offsets, body offsets
+	const size_t src_bytes = sizeof(SceneSrc) * num_scenes, off_bytes = sizeof(uint64_t) * (num_scenes + 1);
+	static_assert(sizeof(SceneSrc) % 8 == 0, "the offsets behind the table are 8-byte words");
+	CC_TRY(ensure(c, c->g_src, src_bytes + 2 * off_bytes));
+	std::vector<unsigned char> tab(src_bytes + 2 * off_bytes);
+	memcpy(tab.data(), src.data(), src_bytes);
+	memcpy(tab.data() + src_bytes, so.data(), off_bytes);
+	memcpy(tab.data() + src_bytes + off_bytes, bo.data(), off_bytes);
+	CC_CUDA(c, copy_small_h2d(c->g_src.p, tab.data(), tab.size(), s));
+	unsigned long long *d_off = reinterpret_cast<unsigned long long *>(ptr<unsigned char>(c->g_src) + src_bytes);
 	cc_batch bt;
 	bt.num_scenes = num_scenes;
 	bt.shape_offsets = so.data();
 	bt.body_offsets = bo.data();
-	bt.scene = cc_scene{n, dst.T, dst.A, dst.B, dst.C, dst.R, dst.ID, nb, dst.pos, dst.rot, dst.active};
-	return batch_impl(c, &bt, gx, gy, gz, envelope, res, scene_pairs, contact_offsets, stream);
+	bt.scene = cc_scene{n, ptr<int32_t>(c->g_T), ptr<float>(c->g_A), ptr<float>(c->g_B), ptr<float>(c->g_C),
+	                    ptr<float>(c->g_R), ptr<uint32_t>(c->g_ID), nb, ptr<float>(c->g_pos), ptr<float>(c->g_rot),
+	                    ptr<uint8_t>(c->g_act)};
+	return batch_impl(c, &bt, gx, gy, gz, envelope, res, scene_pairs, contact_offsets, stream, ptr<SceneSrc>(c->g_src), d_off);
 }
 
 cc_status cc_perturb_bodies(cc_ctx *c, uint64_t nb, float *body_pos, float *body_rot, uint64_t seed, float sigma,

@@ -294,21 +294,24 @@ void launch_perturb_scenes(uint32_t count, uint64_t total, const PerturbScene *d
 constexpr size_t kParamChunkBytes = 8192;
 constexpr size_t kParamCopyMax = 64 * 1024;
 cudaError_t copy_small_h2d(void *dst, const void *src, size_t bytes, cudaStream_t s);
-void launch_gather(uint64_t n, uint64_t nb, uint32_t S, const unsigned long long *shape_off,
-                   const unsigned long long *body_off, const SceneSrc *src, const SceneDst &dst, cudaStream_t s);
 // dst[i] = src[i] (3 floats) for the shapes of type CONE or TRIANGLEMESH, the
 // only ones whose C is read; T is on the device, src a device-accessible
 // (pinned, mapped) host array.
 void launch_gather_c(uint64_t n, const int32_t *T, const float *src, float *dst, cudaStream_t s);
-void launch_batch_prep(uint64_t n, uint32_t S, const unsigned long long *shape_off, const unsigned long long *body_off,
-                       const uint32_t *ID, uint32_t *scene_of, uint32_t *gid, uint32_t *err, cudaStream_t s);
-void launch_batch_bounds(uint64_t n, const float *aabb, const uint32_t *scene_of, SceneStats *sst, uint32_t *err,
-                         cudaStream_t s);
-void launch_batch_plan(uint32_t S, const unsigned long long *shape_off, const SceneStats *sst, const GridParams &gp,
-                       const int grid[3], Plan *plans, uint32_t *G, cudaStream_t s);
-void launch_batch_offsets(uint32_t S, const unsigned long long *shape_off, const unsigned long long *owner_off,
-                          const unsigned long long *np_pos, const DevStats *stats, unsigned long long *scene_pairs,
-                          unsigned long long *contact_off, cudaStream_t s);
+// The front of a batch pass (cc_aabb.cu): scene_of, global ids, boxes, bounds,
+// plans, cell_base[0..S] and stats->cells; with src the scenes are gathered into
+// dst on the way (`all` unused), else `all` holds the concatenated arrays.
+void launch_batch_front(uint64_t n, uint64_t nb, uint32_t S, const unsigned long long *shape_off,
+                        const unsigned long long *body_off, const SceneSrc &all, const SceneSrc *src, const SceneDst &dst,
+                        uint32_t *scene_of, uint32_t *gid, float *aabb, DevStats *stats, SceneStats *sst,
+                        const GridParams &gp, const int grid[3], Plan *plans, uint32_t *cell_base, cudaStream_t s,
+                        const ZeroList &zero);
+void launch_batch_pair_counts(uint64_t P, const unsigned long long *pairs, const uint32_t *scene_of,
+                              unsigned long long *scene_pairs, cudaStream_t s);
+// From the final pair list (stats->np_n keys, the stats->contacts contacts' first).
+void launch_batch_offsets(uint32_t S, const unsigned long long *shape_off, const unsigned long long *pairs,
+                          const DevStats *stats, unsigned long long *scene_pairs, unsigned long long *contact_off,
+                          cudaStream_t s);
 
 // Reference-grid bin list (the reference's internal sorted (bin, body) list).
 void launch_ref_count(uint64_t n, const float *aabb_shifted, const DevStats *stats, uint32_t *cnt, cudaStream_t s);

@@ -252,7 +252,8 @@ __device__ __forceinline__ Shape<S> load_shape(uint32_t s, uint32_t id, const in
 	rows_of<S>(qw, qx, qy, qz, sh.r0, sh.r1, sh.r2);
 	sh.X = cvt3<S>(ld3(A, s));
 	sh.Y = cvt3<S>(ld3(B, s));
-	sh.Z = cvt3<S>(ld3(C, s));
+	sh.Z = mk<S>(S(0), S(0), S(0));
+	if (sh.type == TRIANGLEMESH) sh.Z = cvt3<S>(ld3(C, s));  // no other support or centre reads it
 	const vec<S> po = sub(cvt3<S>(p), org);
 	if (sh.type == SPHERE || sh.type == ELLIPSOID || sh.type == BOX || sh.type == CYLINDER) {
 		vec<S> b0, b1, b2;
