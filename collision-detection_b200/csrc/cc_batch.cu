@@ -70,6 +70,14 @@ __global__ void __launch_bounds__(kNT) k_batch_pair_counts(uint64_t P, const uns
 		atomicAdd(scene_pairs + scene_of[pairs[i] >> 32], 1ull);
 }
 
+// The same from the owners' offsets (one owner per bucket).
+__global__ void __launch_bounds__(kNT) k_batch_owner_counts(uint32_t S, const unsigned long long *__restrict__ shape_off,
+                                                             const unsigned long long *__restrict__ owner_off,
+                                                             unsigned long long *__restrict__ scene_pairs) {
+	const uint32_t s = blockIdx.x * kNT + threadIdx.x;
+	if (s < S) scene_pairs[s] = owner_off[shape_off[s + 1]] - owner_off[shape_off[s]];
+}
+
 // The third shape array (C) of the shapes that read it: CONE, which GenerateAABB
 // bounds as a triangle (AABBGenerator.cu:103-107), and TRIANGLEMESH, whose
 // third vertex the support map and centre use (Narrowphase.cu:11-17, 44-47).
@@ -215,6 +223,11 @@ void launch_batch_pair_counts(uint64_t P, const unsigned long long *pairs, const
 	if (!P) return;
 	const unsigned g = (unsigned)std::min<uint64_t>((P + kNT - 1) / kNT, (uint64_t)kNumSMs * 8);
 	k_batch_pair_counts<<<g, kNT, 0, s>>>(P, pairs, scene_of, scene_pairs);
+}
+
+void launch_batch_owner_counts(uint32_t S, const unsigned long long *shape_off, const unsigned long long *owner_off,
+                               unsigned long long *scene_pairs, cudaStream_t s) {
+	k_batch_owner_counts<<<(S + kNT - 1) / kNT, kNT, 0, s>>>(S, shape_off, owner_off, scene_pairs);
 }
 
 void launch_batch_offsets(uint32_t S, const unsigned long long *shape_off, const unsigned long long *pairs,

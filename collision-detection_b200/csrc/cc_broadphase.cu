@@ -12,7 +12,8 @@
 //                   counts on the search grid
 //   scan            cell offsets (decoupled look-back)
 //   k_scatter       cell-ordered (AABB, body) entries
-//   k_pair_test     closed AABB overlap (:237) of every entry with the later
+//   k_pair_test     (cells of many entries: k_dense_order, k_dense_test)
+//                   closed AABB overlap (:237) of every entry with the later
 //                   entries of its cell; a pair is emitted only from its home
 //                   cell (the cell holding the larger of the two min corners on
 //                   every axis, a point of both boxes and so of both cell
@@ -122,26 +123,6 @@ __device__ __forceinline__ CellRange cell_range(const Plan &p, float3 mn, float3
 __device__ __forceinline__ uint32_t pack_cell(int x, int y, int z) {
 	return (uint32_t)x | ((uint32_t)y << 10) | ((uint32_t)z << 20);
 }
-// Home-cell test by per-entry codes. cell_of is monotone, so the cell of the
-// larger min corner of two boxes is, per axis, the larger of the two min
-// corners' cells; it equals the cell (cx, cy, cz) both entries were entered in
-// exactly when one min corner's cell equals it and the other's does not
-// exceed it. home_code: bits 0-2 = min-corner cell == the cell's coordinate
-// on x/y/z, bits 3-5 = min-corner cell <= it; computed once per entry (the
-// dense-cell kernel, where most tested boxes overlap).
-__device__ __forceinline__ uint32_t home_code(const Plan &p, float4 lo, uint32_t packed_cell) {
-	const int cx = packed_cell & 1023, cy = (packed_cell >> 10) & 1023, cz = (packed_cell >> 20) & 1023;
-	const int x = cell_of(lo.x, p.lo[0], p.inv[0], p.dim[0]);
-	const int y = cell_of(lo.y, p.lo[1], p.inv[1], p.dim[1]);
-	const int z = cell_of(lo.z, p.lo[2], p.inv[2], p.dim[2]);
-	return (uint32_t)(x == cx) | ((uint32_t)(y == cy) << 1) | ((uint32_t)(z == cz) << 2) | ((uint32_t)(x <= cx) << 3) |
-	       ((uint32_t)(y <= cy) << 4) | ((uint32_t)(z <= cz) << 5);
-}
-// cell_of(max(a.min, b.min)) == cell on every axis
-__device__ __forceinline__ bool home_pair(uint32_t a, uint32_t b) {
-	return (((a & (b >> 3)) | (b & (a >> 3))) & 7u) == 7u;
-}
-
 __global__ void __launch_bounds__(kNT) k_bounds(uint64_t n, const float *__restrict__ aabb, DevStats *stats,
                                                  PlanArgs pa, ZeroList zero) {
 	zero_ranges(zero);
@@ -376,8 +357,9 @@ __global__ void __launch_bounds__(kNT, 5) k_pair_test(const DevStats *stats, con
                                                     const float4 *__restrict__ entries,
                                                     uint64_t entry_cap, uint32_t *__restrict__ owner_count,
                                                     unsigned long long *__restrict__ pairs, uint64_t pair_cap,
-                                                    unsigned long long *pair_counter, SceneMap sm, uint2 *dense,
+                                                    unsigned long long *pair_counter, SceneMap sm, DenseItem *dense,
                                                     uint64_t dense_cap, unsigned long long *dense_count,
+                                                    unsigned long long *mask_words,
                                                     uint32_t *err, uint32_t dense_cell, int oshift) {
 	pdl_begin();
 	__shared__ Plan sp;
@@ -425,11 +407,16 @@ __global__ void __launch_bounds__(kNT, 5) k_pair_test(const DevStats *stats, con
 				if (dense) {  // left to k_pair_test_dense
 					my_n = 0;
 					if (e == beg) {
-						const uint32_t chunks = (uint32_t)((end - beg + kNT - 1) / kNT);
+						const uint32_t k = (uint32_t)(end - beg), chunks = (k + kNT - 1) / kNT;
 						const unsigned long long at = atomicAdd(dense_count, (unsigned long long)chunks);
-						for (uint32_t q = 0; q < chunks; q++)
-							if (at + q < dense_cap) dense[at + q] = make_uint2(c, q * kNT);
+						unsigned long long words = 0;
+						for (uint32_t q = 0; q < chunks; q++) words += dense_mask_words(k, q * kNT);
+						words = atomicAdd(mask_words, words);
+						for (uint32_t q = 0; q < chunks; q++) {
+							if (at + q < dense_cap) dense[at + q] = DenseItem{c, q * kNT, words};
 							else atomicOr(err, (uint32_t)kErrCapacity);
+							words += dense_mask_words(k, q * kNT);
+						}
 					}
 				} else if (e == beg) {
 					// no dense-cell kernel this call (the last found no dense
@@ -759,121 +746,302 @@ __global__ void __launch_bounds__(kNT, 5) k_walk(uint64_t n, DevStats *stats, co
 	if (ocnt) flush_pairs(obuf, ocnt, lane, &stats->pairs, pairs, pair_cap);
 }
 
-// Dense cells: one block per (cell, chunk of 256 rows). Thread t takes row
-// i = r0 + t and tests it against every later entry j > i of the cell, the
-// columns staged 256 at a time in shared memory and read by all lanes at once
-// (a broadcast), so one warp instruction carries 32 tests. Pairs owned by the
-// row (smaller index) are counted in a register, pairs owned by the column in
-// a shared counter per column; both reach owner_count once per tile.
-constexpr int kDenseOut = 512;
+// In-place bitonic sort of m (a power of two) keys in shared memory by
+// `nt` cooperating threads (thread t of them); sync() separates the steps.
+template <class K, class Sync>
+__device__ __forceinline__ void bitonic_shared(K *s, int m, int t, int nt, Sync sync) {
+	for (int k = 2; k <= m; k <<= 1) {
+		for (int j = k >> 1; j > 0; j >>= 1) {
+			// compare-exchange q pairs (i, i + j), i with bit j clear: every thread busy
+			for (int q = t; q < (m >> 1); q += nt) {
+				const int i = ((q & ~(j - 1)) << 1) | (q & (j - 1));
+				const int p = i + j;
+				const bool up = (i & k) == 0;
+				const K x = s[i], y = s[p];
+				if ((x > y) == up) {
+					s[i] = y;
+					s[p] = x;
+				}
+			}
+			sync();
+		}
+	}
+}
+
+// ---------------------------------------------------------------- dense cells
+// Cells of more than dense_cell entries are listed as (cell, chunk of 256 rows)
+// and tested here, every row against the later entries of its cell:
+//   k_dense_order  the entries of a dense cell in ascending body order, so that
+//                  a pair's owner is always its row and a row meets its
+//                  partners in ascending order;
+//   k_dense_test   (kEmit false) counts the pairs of every row, which gives the
+//                  owner buckets' sizes;
+//   k_dense_test   (kEmit true), once the buckets have their offsets, writes
+//                  each row's pairs as one ascending run into its owner's bucket.
+// A test is some fifteen instructions (tests of 32 columns become one mask per
+// row, by sign bits, kept for the write where there is room), far cheaper than
+// an unsorted list of all pairs and its scatter: at 4.2M clustered spheres (246M pairs) the test
+// that emitted through warp votes took 9.7 ms and the scatter 3.3.
+struct DenseTile {
+	float4 lo[kNT], hi[kNT];  // (min, body), (max, not-home bits)
+};
+// Columns [c0, c0 + kNT) of the cell's entries at s0; those past k fit nothing.
+__device__ __forceinline__ void load_columns(DenseTile &t, const float4 *__restrict__ entries, uint64_t s0, uint32_t c0,
+                                             uint32_t k) {
+	float4 l = make_float4(INFINITY, INFINITY, INFINITY, 0.f), h = make_float4(-INFINITY, -INFINITY, -INFINITY, 0.f);
+	if (c0 + threadIdx.x < k) {
+		l = entries[2 * (s0 + c0 + threadIdx.x)];
+		h = entries[2 * (s0 + c0 + threadIdx.x) + 1];
+	}
+	t.lo[threadIdx.x] = l;
+	t.hi[threadIdx.x] = h;
+}
+// Bit 31 - q: the row (alo, ahi) and column g + q overlap (closed, :237) and this
+// cell is their home cell. All six differences max - min have clear sign bits
+// exactly if the boxes overlap (x - x is +0, differences of floats never round
+// to zero); an axis is at home if either box's min corner is in this cell, so
+// the pair is not at home where both not-home bits are set.
+__device__ __forceinline__ uint32_t test_columns(const DenseTile &t, uint32_t g, float4 alo, float4 ahi) {
+	const uint32_t na = __float_as_uint(ahi.w);
+	uint32_t miss = 0;
+#pragma unroll
+	for (int q = 0; q < 32; q++) {
+		const float4 blo = t.lo[g + q], bhi = t.hi[g + q];
+		const uint32_t s = __float_as_uint(bhi.x - alo.x) | __float_as_uint(ahi.x - blo.x) | __float_as_uint(bhi.y - alo.y) |
+		                   __float_as_uint(ahi.y - blo.y) | __float_as_uint(bhi.z - alo.z) | __float_as_uint(ahi.z - blo.z) |
+		                   (0u - (na & __float_as_uint(bhi.w)));
+		miss = __funnelshift_l(s, miss, 1);
+	}
+	return ~miss;
+}
+
+// Entries of the dense cells in ascending body order, the cell code replaced by
+// the row's not-home bits (an axis whose min corner lies in a lower cell). A
+// cell of up to kOrderSeg entries is one block's bitonic sort of (body, place)
+// in shared memory; larger cells rank each entry by counting smaller bodies,
+// k / 14 instructions an entry (all cells that way: 1.1 ms at 4.2M spheres).
+constexpr uint32_t kOrderSeg = 4096;
 template <bool kBatch>
-__global__ void __launch_bounds__(kNT) k_pair_test_dense(const DevStats *stats, const uint32_t *__restrict__ cell_start,
-                                                          const float4 *__restrict__ entries, uint64_t entry_cap,
-                                                          uint32_t *__restrict__ owner_count,
-                                                          unsigned long long *__restrict__ pairs, uint64_t pair_cap,
-                                                          unsigned long long *pair_counter, SceneMap sm,
-                                                          const uint2 *__restrict__ dense, uint64_t dense_cap,
-                                                          int oshift) {
+__global__ void __launch_bounds__(kNT) k_dense_order(const DevStats *stats, const uint32_t *__restrict__ cell_start,
+                                                      const float4 *__restrict__ entries, uint64_t entry_cap,
+                                                      float4 *__restrict__ sorted, uint32_t *__restrict__ sorted_body,
+                                                      SceneMap sm, const DenseItem *__restrict__ dense, uint64_t dense_cap) {
 	pdl_begin();
 	__shared__ Plan sp;
-	__shared__ float4 tlo[kNT], thi[kNT];
-	__shared__ uint32_t colown[kNT], tcode[kNT];
-	__shared__ unsigned long long out_all[kNT / 32][kDenseOut];
+	__shared__ __align__(16) unsigned long long keys[kOrderSeg];
 	if (threadIdx.x < sizeof(Plan) / 4)
 		reinterpret_cast<uint32_t *>(&sp)[threadIdx.x] = reinterpret_cast<const uint32_t *>(&stats->plan)[threadIdx.x];
 	__syncthreads();
-	if (!kBatch && !sp.valid) return;
-	const uint64_t items = min((uint64_t)stats->dense_items, dense_cap);
-	unsigned long long *obuf = out_all[threadIdx.x >> 5];
-	uint32_t ocnt = 0;
-	const uint32_t lane = threadIdx.x & 31, lt = (1u << lane) - 1u;
-	for (uint64_t it = blockIdx.x; it < items; it += gridDim.x) {
-		const uint2 w = dense[it];
-		const uint64_t s0 = cell_start[w.x];
-		const uint64_t s1 = min((uint64_t)cell_start[w.x + 1], entry_cap);
-		const uint32_t k = (uint32_t)(s1 - s0), r0 = w.y;
-		const uint32_t i = r0 + threadIdx.x;
-		const bool row = i < k;
-		float4 alo = make_float4(0.f, 0.f, 0.f, 0.f), ahi = alo;
-		if (row) {
-			alo = entries[2 * (s0 + i)];
-			ahi = entries[2 * (s0 + i) + 1];
-		}
-		const uint32_t ida = __float_as_uint(alo.w);
-		const uint32_t pc = __float_as_uint(ahi.w);
+	const auto put = [&](uint64_t from, uint64_t to) {
+		float4 lo, hi;
+		ld_global_v8(reinterpret_cast<const float *>(entries + 2 * from), lo, hi);
+		const uint32_t id = __float_as_uint(lo.w), pc = __float_as_uint(hi.w);
 		uint32_t cb;
-		const Plan &pl = plan_of<kBatch>(sp, sm, row ? ida : __float_as_uint(entries[2 * s0].w), cb);
-		const uint32_t rcode = home_code(pl, alo, pc);
-		uint32_t owned = 0;
-		for (uint32_t c0 = r0; c0 < k; c0 += kNT) {
-			const uint32_t nt = min((uint32_t)kNT, k - c0);
-			__syncthreads();  // the previous tile is no longer read
-			if (threadIdx.x < nt) {
-				const float4 l = entries[2 * (s0 + c0 + threadIdx.x)], h = entries[2 * (s0 + c0 + threadIdx.x) + 1];
-				tlo[threadIdx.x] = l;
-				thi[threadIdx.x] = h;
-				tcode[threadIdx.x] = home_code(pl, l, __float_as_uint(h.w));  // the rows' cell
-			}
-			colown[threadIdx.x] = 0;
+		const Plan &p = plan_of<kBatch>(sp, sm, id, cb);
+		const uint32_t not_home = (uint32_t)(cell_of(lo.x, p.lo[0], p.inv[0], p.dim[0]) != (int)(pc & 1023)) |
+		                          ((uint32_t)(cell_of(lo.y, p.lo[1], p.inv[1], p.dim[1]) != (int)((pc >> 10) & 1023)) << 1) |
+		                          ((uint32_t)(cell_of(lo.z, p.lo[2], p.inv[2], p.dim[2]) != (int)((pc >> 20) & 1023)) << 2);
+		hi.w = __uint_as_float(not_home);
+		st_global_v8(reinterpret_cast<float *>(sorted + 2 * to), lo, hi);
+		sorted_body[to] = id;
+	};
+	const uint64_t items = min((uint64_t)stats->dense_items, dense_cap);
+	for (uint64_t it = blockIdx.x; it < items; it += gridDim.x) {
+		const DenseItem w = dense[it];
+		const uint64_t s0 = cell_start[w.cell], s1 = min((uint64_t)cell_start[w.cell + 1], entry_cap);
+		const uint32_t k = (uint32_t)(s1 - s0);
+		if (k <= kOrderSeg) {
+			if (w.row) continue;  // the cell's first item takes it whole
+			uint32_t m = 2;
+			while (m < k) m <<= 1;
 			__syncthreads();
-			// only j > i is tested: on the diagonal tile (c0 == r0) that needs a
-			// check per column, every later tile lies wholly past this block's rows
-			const auto column = [&](uint32_t jj, bool test) {
-				bool emit = false;
-				unsigned long long key = 0;
-				if (test) {
-					const float4 blo = tlo[jj], bhi = thi[jj];
-					if (alo.x <= bhi.x && blo.x <= ahi.x && alo.y <= bhi.y && blo.y <= ahi.y && alo.z <= bhi.z &&
-					    blo.z <= ahi.z) {
-						if (home_pair(rcode, tcode[jj])) {
-							const uint32_t idb = __float_as_uint(blo.w);
-							const uint32_t lo = min(ida, idb), hi = max(ida, idb);
-							key = ((unsigned long long)lo << 32) | hi;
-							emit = true;
-							if (lo == ida) owned++;
-							else atomicAdd(&colown[jj], 1u);
-						}
-					}
-				}
-				const uint32_t bal = __ballot_sync(0xffffffffu, emit);
-				if (bal) {
-					const uint32_t nb = __popc(bal);
-					if (ocnt + nb > kDenseOut) {
-						flush_pairs(obuf, ocnt, lane, pair_counter, pairs, pair_cap);
-						ocnt = 0;
-					}
-					if (emit) obuf[ocnt + __popc(bal & lt)] = key;
-					ocnt += nb;
-					__syncwarp();
-				}
-			};
-			if (c0 == r0) {
-				for (uint32_t jj = 0; jj < nt; jj++) column(jj, row && c0 + jj > i);
-			} else {
-#pragma unroll 4
-				for (uint32_t jj = 0; jj < nt; jj++) column(jj, row);
-			}
-			__syncthreads();  // column counts complete
-			if (threadIdx.x < nt && colown[threadIdx.x])
-				atomicAdd(&owner_count[__float_as_uint(tlo[threadIdx.x].w) >> oshift], colown[threadIdx.x]);
+			for (uint32_t i = threadIdx.x; i < m; i += kNT)
+				keys[i] = i < k ? ((unsigned long long)__float_as_uint(entries[2 * (s0 + i)].w) << 32) | i : ~0ull;
+			__syncthreads();
+			bitonic_shared(keys, (int)m, threadIdx.x, kNT, [] { __syncthreads(); });
+			for (uint32_t i = threadIdx.x; i < k; i += kNT) put(s0 + (uint32_t)keys[i], s0 + i);
+			continue;
 		}
-		if (owned) atomicAdd(&owner_count[ida >> oshift], owned);
+		const uint32_t i = w.row + threadIdx.x;
+		const uint32_t id = i < k ? __float_as_uint(entries[2 * (s0 + i)].w) : 0u;
+		uint32_t *ids = reinterpret_cast<uint32_t *>(keys);
+		uint32_t rank = 0;
+		for (uint32_t c0 = 0; c0 < k; c0 += kNT) {
+			__syncthreads();
+			ids[threadIdx.x] = c0 + threadIdx.x < k ? __float_as_uint(entries[2 * (s0 + c0 + threadIdx.x)].w) : 0xffffffffu;
+			__syncthreads();
+			const uint4 *v = reinterpret_cast<const uint4 *>(ids);
+#pragma unroll 8
+			for (int q = 0; q < kNT / 4; q++) {
+				const uint4 x = v[q];
+				rank += (x.x < id) + (x.y < id) + (x.z < id) + (x.w < id);
+			}
+		}
+		if (i < k) put(s0 + i, s0 + rank);
 	}
-	if (ocnt) flush_pairs(obuf, ocnt, lane, pair_counter, pairs, pair_cap);
 }
 
-// Bucket the unsorted pairs by owner bucket (the smaller index >> oshift). P
-// comes from the device; if it exceeds the scratch or the output nothing is
-// written.
-__global__ void __launch_bounds__(kNT) k_owner_scatter(DevStats *stats, uint64_t pair_cap, uint64_t out_cap,
-                                                        const unsigned long long *__restrict__ tmp,
+// Where there is room the masks of the count are kept for the write (row by row,
+// eight words a column tile); then k_dense_emit writes the item's pairs, else
+// this kernel tests it again.
+template <bool kEmit>
+__global__ void __launch_bounds__(kNT) k_dense_test(DevStats *stats, const uint32_t *__restrict__ cell_start,
+                                                     const float4 *__restrict__ sorted, uint64_t entry_cap,
+                                                     uint32_t *__restrict__ owner_count, uint32_t *__restrict__ row_count,
+                                                     const DenseItem *__restrict__ dense, uint64_t dense_cap, int oshift,
+                                                     uint32_t *__restrict__ masks, uint64_t mask_cap,
+                                                     const unsigned long long *__restrict__ owner_off,
+                                                     unsigned long long *__restrict__ out) {
+	pdl_begin();
+	__shared__ DenseTile tile;
+	__shared__ uint32_t words[kEmit ? 1 : kNT / 32][kNT];  // each thread's masks of the tile
+	__shared__ unsigned long long s_pairs;
+	// the list does not fit the output, or all masks were kept
+	if (kEmit && (stats->np_n != stats->pairs || stats->mask_words <= mask_cap)) return;
+	if (!kEmit) {
+		if (threadIdx.x == 0) s_pairs = blockIdx.x == 0 ? stats->tmp_pairs : 0ull;  // the sparse cells' pairs count too
+		__syncthreads();
+	}
+	const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x / 32;
+	const uint64_t items = min((uint64_t)stats->dense_items, dense_cap);
+	for (uint64_t it = blockIdx.x; it < items; it += gridDim.x) {
+		const DenseItem w = dense[it];
+		const uint64_t s0 = cell_start[w.cell], s1 = min((uint64_t)cell_start[w.cell + 1], entry_cap);
+		const uint32_t k = (uint32_t)(s1 - s0), r0 = w.row, i = r0 + threadIdx.x;
+		const bool kept = w.mask + dense_mask_words(k, r0) <= mask_cap;
+		if (kEmit && kept) continue;
+		uint32_t *mask = masks + w.mask + (uint64_t)threadIdx.x * dense_row_words(k, r0);
+		float4 alo = make_float4(INFINITY, INFINITY, INFINITY, 0.f), ahi = make_float4(-INFINITY, -INFINITY, -INFINITY, 0.f);
+		if (i < k) ld_global_v8(reinterpret_cast<const float *>(sorted + 2 * (s0 + i)), alo, ahi);
+		const uint32_t a = __float_as_uint(alo.w);
+		uint32_t cnt = 0;
+		unsigned long long *to = out;  // of the row's next pair
+		if (kEmit) {
+			cnt = i < k ? row_count[s0 + i] : 0u;
+			if (cnt) to += owner_off[a >> oshift] + atomicSub(&owner_count[a >> oshift], cnt) - cnt;
+		}
+		for (uint32_t c0 = r0; c0 < k; c0 += kNT) {
+			__syncthreads();  // the previous tile is no longer read
+			load_columns(tile, sorted, s0, c0, k);
+			__syncthreads();
+			const uint32_t groups = min((uint32_t)kNT, k - c0 + 31u) / 32u;
+			// in the diagonal tile a warp's rows have no later column before their own group
+			for (uint32_t g = c0 == r0 ? warp : 0u; g < groups; g++) {
+				uint32_t hit = test_columns(tile, 32 * g, alo, ahi);
+				if (c0 == r0 && g == warp) hit &= lane == 31 ? 0u : 0x7fffffffu >> lane;  // later columns only
+				if constexpr (!kEmit) {
+					cnt += __popc(hit);
+					words[g][threadIdx.x] = hit;
+				} else {
+					while (hit) {
+						const uint32_t q = __clz(hit);
+						hit &= ~(0x80000000u >> q);
+						*to++ = ((unsigned long long)a << 32) | __float_as_uint(tile.lo[32 * g + q].w);
+					}
+				}
+			}
+			if (!kEmit && kept && i < k) {  // the tile's eight words of this row (its own: no barrier)
+				float f[8];
+#pragma unroll
+				for (uint32_t g = 0; g < 8; g++)
+					f[g] = __uint_as_float(g < groups && (c0 != r0 || g >= warp) ? words[kEmit ? 0 : g][threadIdx.x] : 0u);
+				st_global_v8(reinterpret_cast<float *>(mask + (c0 - r0) / 32), make_float4(f[0], f[1], f[2], f[3]),
+				             make_float4(f[4], f[5], f[6], f[7]));
+			}
+		}
+		if constexpr (!kEmit) {
+			if (i < k) row_count[s0 + i] = cnt;
+			if (cnt) atomicAdd(&owner_count[a >> oshift], cnt);
+			const uint32_t sum = __reduce_add_sync(0xffffffffu, cnt);
+			if (lane == 0 && sum) atomicAdd(&s_pairs, (unsigned long long)sum);
+		}
+	}
+	if constexpr (!kEmit) {
+		__syncthreads();
+		if (threadIdx.x == 0 && s_pairs) atomicAdd(&stats->pairs, s_pairs);
+	}
+}
+
+// The pairs of the items whose masks were kept: W lanes per row, a lane per mask
+// word, so that a row's pairs are written together (a lane per row kept 300,000
+// partly written lines under way and thrashed the L2: 5.8 ms at 4.2M spheres;
+// 32 lanes for every row 2.4, most of them without a word).
+template <int W>
+__device__ __forceinline__ void emit_rows(unsigned long long *__restrict__ out, const uint32_t *__restrict__ body,
+                                          const uint32_t *__restrict__ masks, uint32_t per, uint32_t cnt, uint32_t a,
+                                          unsigned long long at) {
+	const uint32_t lane = threadIdx.x & 31, sub = lane & (W - 1);
+	const auto word = [&](uint32_t r, uint32_t g) { return g + sub < per ? __ldcs(masks + (uint64_t)r * per + g + sub) : 0u; };
+	uint32_t ahead = word(lane / W, 0);
+	for (uint32_t r0 = 0; r0 < 32; r0 += 32 / W) {
+		const uint32_t r = r0 + lane / W;
+		uint32_t hit = ahead;
+		if (r0 + 32 / W < 32) ahead = word(r + 32 / W, 0);  // the next rows' words arrive meanwhile
+		const uint32_t c = __shfl_sync(0xffffffffu, cnt, r);
+		const unsigned long long key = (unsigned long long)__shfl_sync(0xffffffffu, a, r) << 32;
+		unsigned long long *to = out + __shfl_sync(0xffffffffu, at, r);
+		if (!c) hit = 0u;  // rows past the cell's end: words never written
+		for (uint32_t g = 0; g < per; g += W) {
+			if (g) hit = c ? word(r, g) : 0u;
+			const uint32_t own = __popc(hit);
+			uint32_t incl = own;
+#pragma unroll
+			for (int o = 1; o < W; o <<= 1) {
+				const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o, W);
+				if ((int)sub >= o) incl += t;
+			}
+			unsigned long long *p = to + (incl - own);
+			while (hit) {
+				const uint32_t q = __clz(hit);
+				hit &= ~(0x80000000u >> q);
+				*p++ = key | body[32 * (g + sub) + q];
+			}
+			if (g + W < per) to += __shfl_sync(0xffffffffu, incl, W - 1, W);
+		}
+	}
+}
+__global__ void __launch_bounds__(kNT) k_dense_emit(DevStats *stats, const uint32_t *__restrict__ cell_start,
+                                                     const uint32_t *__restrict__ sorted_body, uint64_t entry_cap,
+                                                     uint32_t *__restrict__ owner_count,
+                                                     const uint32_t *__restrict__ row_count,
+                                                     const DenseItem *__restrict__ dense, uint64_t dense_cap, int oshift,
+                                                     const uint32_t *__restrict__ masks, uint64_t mask_cap,
+                                                     const unsigned long long *__restrict__ owner_off,
+                                                     unsigned long long *__restrict__ out) {
+	pdl_begin();
+	if (stats->np_n != stats->pairs) return;  // the list does not fit the output
+	const uint32_t warp = threadIdx.x / 32;
+	const uint64_t items = min((uint64_t)stats->dense_items, dense_cap);
+	for (uint64_t it = blockIdx.x; it < items; it += gridDim.x) {
+		const DenseItem w = dense[it];
+		const uint64_t s0 = cell_start[w.cell], s1 = min((uint64_t)cell_start[w.cell + 1], entry_cap);
+		const uint32_t k = (uint32_t)(s1 - s0), per = dense_row_words(k, w.row);
+		if (w.mask + dense_mask_words(k, w.row) > mask_cap) continue;
+		const uint32_t *body = sorted_body + s0 + w.row;
+		const uint32_t i = w.row + threadIdx.x;
+		const uint32_t cnt = i < k ? row_count[s0 + i] : 0u, a = i < k ? sorted_body[s0 + i] : 0u;
+		unsigned long long at = 0;
+		if (cnt) at = owner_off[a >> oshift] + atomicSub(&owner_count[a >> oshift], cnt) - cnt;
+		if (!__any_sync(0xffffffffu, cnt != 0u)) continue;
+		const uint32_t *mask = masks + w.mask + (uint64_t)(32 * warp) * per;
+		if (per <= 8) emit_rows<8>(out, body, mask, per, cnt, a, at);
+		else if (per <= 16) emit_rows<16>(out, body, mask, per, cnt, a, at);
+		else emit_rows<32>(out, body, mask, per, cnt, a, at);
+	}
+}
+
+// Bucket the unsorted pairs by owner bucket (the smaller index >> oshift). Their
+// count comes from the device; if they exceed the scratch, or all pairs the
+// output, nothing is written.
+__global__ void __launch_bounds__(kNT) k_owner_scatter(DevStats *stats, const unsigned long long *tmp_n, uint64_t pair_cap,
+                                                        uint64_t out_cap, const unsigned long long *__restrict__ tmp,
                                                         const unsigned long long *__restrict__ owner_off,
                                                         uint32_t *__restrict__ owner_count,
                                                         unsigned long long *__restrict__ out, int oshift) {
 	pdl_begin();
-	const unsigned long long P = stats->pairs;
-	const bool fits = P <= pair_cap && P <= out_cap;
-	if (blockIdx.x == 0 && threadIdx.x == 0) stats->np_n = fits ? P : 0ull;
+	const unsigned long long all = stats->pairs, P = *tmp_n;  // P < all: the dense cells' pairs are not in tmp
+	const bool fits = P <= pair_cap && all <= out_cap;
+	if (blockIdx.x == 0 && threadIdx.x == 0) stats->np_n = fits ? all : 0ull;
 	if (!fits) return;
 	// lanes of a warp whose pairs share an owner take their slots with one
 	// atomic (pair lists of dense cells arrive grouped by owner)
@@ -1013,28 +1181,6 @@ __global__ void __launch_bounds__(kNT) k_segsort(uint64_t n, const unsigned long
 	}
 }
 
-// In-place bitonic sort of m (a power of two) 32-bit keys in shared memory by
-// `nt` cooperating threads (thread t of them); sync() separates the steps.
-template <class Sync>
-__device__ __forceinline__ void bitonic_u32(uint32_t *s, int m, int t, int nt, Sync sync) {
-	for (int k = 2; k <= m; k <<= 1) {
-		for (int j = k >> 1; j > 0; j >>= 1) {
-			// compare-exchange q pairs (i, i + j), i with bit j clear: every thread busy
-			for (int q = t; q < (m >> 1); q += nt) {
-				const int i = ((q & ~(j - 1)) << 1) | (q & (j - 1));
-				const int p = i + j;
-				const bool up = (i & k) == 0;
-				const uint32_t x = s[i], y = s[p];
-				if ((x > y) == up) {
-					s[i] = y;
-					s[p] = x;
-				}
-			}
-			sync();
-		}
-	}
-}
-
 // Register bitonic sort of 32*K keys held by one warp, striped: key e = 32*r
 // + lane sits in v[r] of that lane. Steps whose partner distance j is below 32
 // exchange across lanes (shuffle), the others pair registers of the same lane
@@ -1141,6 +1287,111 @@ __device__ __forceinline__ void sort_bucket_pair(unsigned long long *__restrict_
 	}
 }
 
+// Buckets that are a few ascending runs (the rows of a body in its dense cells,
+// k_dense_emit) are merged instead of sorted: adjacent runs pairwise, every key
+// placed by a binary search in the partner run, between two halves of shared
+// memory. At 4.2M clustered spheres (246M pairs) the bitonic tiers alone take 3.8
+// ms at 15 warp instructions a key, merges and what is left to them 3.3 ms.
+// Returns false, with the bucket untouched, above kMaxRuns runs. NT threads
+// work together, Sync separates the steps; buf holds 2 * cap keys.
+constexpr uint32_t kMaxRuns = 32;
+struct Runs {
+	uint32_t start[kMaxRuns + 2], count;
+};
+template <int NT, bool kPack, class Sync>
+__device__ __forceinline__ bool merge_runs(unsigned long long *__restrict__ out, uint64_t beg, uint32_t len, uint32_t a,
+                                           uint32_t t, uint32_t *buf, uint32_t cap, Runs &runs, KeyPack kp, Sync sync) {
+	uint32_t *src = buf, *dst = buf + cap;
+	if (t == 0) {
+		runs.count = 1;
+		runs.start[0] = 0;
+	}
+	for (uint32_t e = t; e < len; e += NT) src[e] = pack_key<kPack>(out[beg + e], kp);
+	sync();
+	for (uint32_t e = t; e < len; e += NT)
+		if (e && src[e] < src[e - 1]) {  // a run starts here; their order is restored below
+			const uint32_t at = atomicAdd(&runs.count, 1u);
+			if (at < kMaxRuns) runs.start[at] = e;
+		}
+	sync();
+	uint32_t R = runs.count;
+	if (R > kMaxRuns) return false;
+	if (R == 1) return true;
+	// starts in order (at most 32: one warp, rank by counting)
+	const uint32_t mine = t < R ? runs.start[t] : 0xffffffffu;
+	uint32_t rank = 0;
+	if (t < R)
+		for (uint32_t q = 0; q < R; q++) rank += runs.start[q] < mine;
+	sync();
+	if (t < R) runs.start[rank] = mine;
+	if (t == 0) runs.start[R] = len;
+	sync();
+	while (R > 1) {
+		for (uint32_t r = 0; r < R; r += 2) {
+			const uint32_t s0 = runs.start[r], s1 = runs.start[r + 1], s2 = r + 1 < R ? runs.start[r + 2] : s1;
+			for (uint32_t i = s0 + t; i < s2; i += NT) {
+				const uint32_t key = src[i];
+				const bool first = i < s1;
+				uint32_t lo = first ? s1 : s0, hi = first ? s2 : s1;
+				while (lo < hi) {
+					const uint32_t mid = (lo + hi) >> 1;
+					if (src[mid] < key) lo = mid + 1;
+					else hi = mid;
+				}
+				dst[i + lo - s1] = key;  // place in its own run + smaller keys of the other
+			}
+		}
+		const uint32_t half = (R + 1) / 2;
+		const uint32_t next = t < half ? runs.start[2 * t] : 0u;
+		sync();
+		if (t < half) runs.start[t] = next;
+		if (t == 0) runs.start[half] = len;
+		R = half;
+		uint32_t *x = src;
+		src = dst;
+		dst = x;
+		sync();
+	}
+	for (uint32_t e = t; e < len; e += NT) out[beg + e] = unpack_key<kPack>(src[e], a, kp);
+	return true;
+}
+
+// The buckets of the mid and big lists that merge: warps take buckets of up to
+// kMidSeg keys, then blocks those of up to kMergeSeg. A merged bucket leaves its
+// list (kDoneBucket); k_segsort_mid and k_segsort_big sort what is left.
+constexpr uint32_t kMergeSeg = 8 * kMidSeg;
+constexpr uint32_t kDoneBucket = 0xffffffffu;
+template <bool kPack>
+__global__ void __launch_bounds__(kNT) k_segsort_runs(const DevStats *stats, uint64_t big_cap, uint32_t *__restrict__ big_list,
+                                                       const unsigned long long *__restrict__ owner_off,
+                                                       unsigned long long *__restrict__ out, KeyPack kp) {
+	pdl_begin();
+	extern __shared__ uint32_t merge_buf[];  // 2 * kMergeSeg keys
+	__shared__ Runs runs[kNT / 32];
+	if (stats->np_n != stats->pairs) return;
+	const uint32_t warp = threadIdx.x / 32, lane = threadIdx.x & 31;
+	const uint64_t nmid = min((uint64_t)stats->big_segments, big_cap);
+	for (uint64_t g = (uint64_t)blockIdx.x * (kNT / 32) + warp; g < nmid; g += (uint64_t)gridDim.x * (kNT / 32)) {
+		const uint32_t a = big_list[g];
+		const uint64_t beg = owner_off[a], len = owner_off[a + 1] - beg;
+		const bool done = merge_runs<32, kPack>(out, beg, (uint32_t)len, a, lane, merge_buf + 2 * kMidSeg * warp, kMidSeg,
+		                                        runs[warp], kp, [] { __syncwarp(); });
+		__syncwarp();
+		if (done && lane == 0) big_list[g] = kDoneBucket;
+	}
+	__syncthreads();
+	const uint64_t nbig = min((uint64_t)stats->seg_big, big_cap);
+	for (uint64_t g = blockIdx.x; g < nbig; g += gridDim.x) {
+		const uint32_t a = big_list[big_cap - 1 - g];
+		const uint64_t beg = owner_off[a], len = owner_off[a + 1] - beg;
+		if (len > kMergeSeg) continue;
+		const bool done = merge_runs<kNT, kPack>(out, beg, (uint32_t)len, a, threadIdx.x, merge_buf, kMergeSeg, runs[0], kp,
+		                                         [] { __syncthreads(); });
+		__syncthreads();
+		if (done && threadIdx.x == 0) big_list[big_cap - 1 - g] = kDoneBucket;
+	}
+}
+
 // Buckets of 33..1024 keys: one warp per bucket, sorted in registers
 // (2..32 keys per lane by bucket size); then buckets of 1025..2048 keys
 // (listed for k_segsort_big, which leaves them) on pairs of warps.
@@ -1157,6 +1408,7 @@ __global__ void __launch_bounds__(kMidNT, 2) k_segsort_mid(const DevStats *stats
 	const uint64_t warps = (uint64_t)gridDim.x * (kMidNT / 32);
 	for (uint64_t g = (uint64_t)blockIdx.x * (kMidNT / 32) + (threadIdx.x >> 5); g < nmid; g += warps) {
 		const uint32_t a = big_list[g];
+		if (a == kDoneBucket) continue;
 		const uint64_t beg = owner_off[a], len = owner_off[a + 1] - beg;  // 33..1024, listed by k_segsort
 		if (len <= 64) sort_bucket_reg<2, kPack>(out, beg, len, a, lane, kp);
 		else if (len <= 128) sort_bucket_reg<4, kPack>(out, beg, len, a, lane, kp);
@@ -1170,6 +1422,7 @@ __global__ void __launch_bounds__(kMidNT, 2) k_segsort_mid(const DevStats *stats
 	const uint64_t npairs = (uint64_t)gridDim.x * (kMidNT / 64);
 	for (uint64_t g = (uint64_t)blockIdx.x * (kMidNT / 64) + pair; g < nbig; g += npairs) {
 		const uint32_t a = big_list[big_cap - 1 - g];
+		if (a == kDoneBucket) continue;
 		const uint64_t beg = owner_off[a], len = owner_off[a + 1] - beg;
 		if (len > kPairSeg) continue;  // the block tier's (uniform over the pair)
 		sort_bucket_pair<kPack>(out, beg, len, a, half, lane, xch[pair], 1 + pair, kp);
@@ -1190,13 +1443,14 @@ __global__ void __launch_bounds__(512) k_segsort_big(const DevStats *stats, uint
 	const uint64_t nbig = min((uint64_t)stats->seg_big, big_cap);
 	for (uint64_t g = blockIdx.x; g < nbig; g += gridDim.x) {
 		const uint32_t a = big_list[big_cap - 1 - g];
+		if (a == kDoneBucket) continue;
 		const uint64_t beg = owner_off[a], len = owner_off[a + 1] - beg;
 		if (len <= kPairSeg) continue;  // sorted by warp pairs in k_segsort_mid (uniform over the block)
 		int m = 1;
 		while ((uint64_t)m < len) m <<= 1;
 		for (int i = threadIdx.x; i < m; i += blockDim.x) s[i] = (uint64_t)i < len ? pack_key<kPack>(out[beg + i], kp) : 0xffffffffu;
 		__syncthreads();
-		bitonic_u32(s, m, threadIdx.x, blockDim.x, [] { __syncthreads(); });
+		bitonic_shared(s, m, threadIdx.x, blockDim.x, [] { __syncthreads(); });
 		for (int i = threadIdx.x; (uint64_t)i < len; i += blockDim.x) out[beg + i] = unpack_key<kPack>(s[i], a, kp);
 		__syncthreads();
 	}
@@ -1292,7 +1546,7 @@ __global__ void __launch_bounds__(kFusedNT) k_owner_sort_fused(DevStats *stats, 
 		while ((uint32_t)m < len) m <<= 1;
 		for (int i = threadIdx.x; i < m; i += kFusedNT) keys[i] = (uint32_t)i < len ? pack_key<kPack>(out[beg + i], kp) : 0xffffffffu;
 		__syncthreads();
-		bitonic_u32(keys, m, threadIdx.x, kFusedNT, [] { __syncthreads(); });
+		bitonic_shared(keys, m, threadIdx.x, kFusedNT, [] { __syncthreads(); });
 		for (int i = threadIdx.x; (uint32_t)i < len; i += kFusedNT) out[beg + i] = unpack_key<kPack>(keys[i], (uint32_t)b, kp);
 		__syncthreads();
 	}
@@ -1551,8 +1805,8 @@ void launch_scatter(uint64_t n, const float *aabb, const BpBuffers &b, cudaStrea
 template <bool kBatch, int kWin>
 void pair_test_as(const BpBuffers &b, unsigned grid, cudaStream_t s) {
 	launch_pdl((k_pair_test<kBatch, kWin>), dim3(grid), dim3(kNT), 0, s, b.stats, b.cell_start, b.entries, b.entry_cap, b.owner_count,
-	                                               b.pairs_tmp, b.pair_cap, &b.stats->pairs, b.sm, b.dense,
-	                                               b.dense_cap, &b.stats->dense_items, &b.stats->err, b.dense_cell,
+	                                               b.pairs_tmp, b.pair_cap, b.dense ? &b.stats->tmp_pairs : &b.stats->pairs, b.sm,
+	                                               b.dense, b.dense_cap, &b.stats->dense_items, &b.stats->mask_words, &b.stats->err, b.dense_cell,
 	                                               b.owner_shift);
 }
 template <bool kBatch>
@@ -1564,6 +1818,14 @@ void pair_test_window(const BpBuffers &b, unsigned grid, cudaStream_t s) {
 	}
 }
 
+// Persistent blocks over the device-side work items of the dense cells.
+template <class K>
+unsigned dense_grid(K kernel) {
+	int v = 0;
+	if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, kernel, kNT, 0) != cudaSuccess || v < 1) v = 1;
+	return (unsigned)kNumSMs * v;
+}
+
 void launch_pair_test(uint64_t n, const BpBuffers &b, uint64_t entries_hint, cudaStream_t s) {
 	(void)n;
 	uint64_t want = (entries_hint + kNT - 1) / kNT;
@@ -1573,22 +1835,13 @@ void launch_pair_test(uint64_t n, const BpBuffers &b, uint64_t entries_hint, cud
 		pair_test_window<true>(b, grid, s);
 	else
 		pair_test_window<false>(b, grid, s);
-	launch_pair_test_dense(b, s);
-}
-
-
-void launch_pair_test_dense(const BpBuffers &b, cudaStream_t s) {
-	if (!b.dense || !b.dense_cap) return;
-	// persistent blocks over the device-side item count (41 KB of shared memory each)
-	const unsigned grid = kNumSMs * 4;
-	if (b.sm.plans)
-		launch_pdl(k_pair_test_dense<true>, dim3(grid), dim3(kNT), 0, s, b.stats, b.cell_start, b.entries, b.entry_cap, b.owner_count,
-		                                             b.pairs_tmp, b.pair_cap, &b.stats->pairs, b.sm, b.dense,
-		                                             b.dense_cap, b.owner_shift);
-	else
-		launch_pdl(k_pair_test_dense<false>, dim3(grid), dim3(kNT), 0, s, b.stats, b.cell_start, b.entries, b.entry_cap, b.owner_count,
-		                                              b.pairs_tmp, b.pair_cap, &b.stats->pairs, b.sm, b.dense,
-		                                              b.dense_cap, b.owner_shift);
+	if (!b.dense) return;
+	static const unsigned g_order = dense_grid(k_dense_order<true>), g_test = dense_grid(k_dense_test<false>);
+	launch_pdl(b.sm.plans ? k_dense_order<true> : k_dense_order<false>, dim3(g_order), dim3(kNT), 0, s, b.stats, b.cell_start, b.entries,
+	           b.entry_cap, b.sorted, b.sorted_body, b.sm, b.dense, b.dense_cap);
+	launch_pdl(k_dense_test<false>, dim3(g_test), dim3(kNT), 0, s, b.stats, b.cell_start, b.sorted, b.entry_cap, b.owner_count,
+	           b.row_count, b.dense, b.dense_cap, b.owner_shift, b.masks, b.mask_cap, (const unsigned long long *)nullptr,
+	           (unsigned long long *)nullptr);
 }
 
 void launch_scan_owner(uint64_t n, const BpBuffers &b, cudaStream_t s) {
@@ -1599,8 +1852,14 @@ void launch_scan_owner(uint64_t n, const BpBuffers &b, cudaStream_t s) {
 void launch_owner_scatter(uint64_t out_cap, unsigned long long *out, const BpBuffers &b, cudaStream_t s) {
 	const uint64_t bound = std::min<uint64_t>(b.pair_cap, out_cap);
 	const unsigned grid = (unsigned)std::min<uint64_t>(std::max<uint64_t>(blocks_for(bound), 1), (uint64_t)kNumSMs * 8);
-	launch_pdl(k_owner_scatter, dim3(grid), dim3(kNT), 0, s, b.stats, b.pair_cap, out_cap, b.pairs_tmp, b.owner_off, b.owner_count, out,
-	                                     b.owner_shift);
+	launch_pdl(k_owner_scatter, dim3(grid), dim3(kNT), 0, s, b.stats, b.dense ? &b.stats->tmp_pairs : &b.stats->pairs, b.pair_cap,
+	           out_cap, b.pairs_tmp, b.owner_off, b.owner_count, out, b.owner_shift);
+	if (!b.dense) return;
+	static const unsigned g_emit = dense_grid(k_dense_emit), g_test = dense_grid(k_dense_test<true>);
+	launch_pdl(k_dense_emit, dim3(g_emit), dim3(kNT), 0, s, b.stats, b.cell_start, b.sorted_body, b.entry_cap, b.owner_count,
+	           b.row_count, b.dense, b.dense_cap, b.owner_shift, b.masks, b.mask_cap, b.owner_off, out);
+	launch_pdl(k_dense_test<true>, dim3(g_test), dim3(kNT), 0, s, b.stats, b.cell_start, b.sorted, b.entry_cap, b.owner_count,
+	           b.row_count, b.dense, b.dense_cap, b.owner_shift, b.masks, b.mask_cap, b.owner_off, out);
 }
 
 void launch_segsort(uint64_t n, unsigned long long *out, const BpBuffers &b, cudaStream_t s) {
@@ -1610,6 +1869,15 @@ void launch_segsort(uint64_t n, unsigned long long *out, const BpBuffers &b, cud
 
 void launch_segsort_mid(unsigned long long *out, const BpBuffers &b, cudaStream_t s) {
 	const KeyPack kp{b.owner_shift, b.key_bits};
+	if (b.dense) {  // rows of dense cells arrive as ascending runs
+		constexpr int bytes = 2 * kMergeSeg * (int)sizeof(uint32_t);  // 64 KB: three blocks fit on an SM
+		static const bool attr =
+		    cudaFuncSetAttribute(k_segsort_runs<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess &&
+		    cudaFuncSetAttribute(k_segsort_runs<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess;
+		(void)attr;
+		launch_pdl(kp.shift ? k_segsort_runs<true> : k_segsort_runs<false>, dim3(kNumSMs * 3), dim3(kNT), bytes, s, b.stats,
+		           b.big_cap, b.big_list, b.owner_off, out, kp);
+	}
 	if (kp.shift)
 		launch_pdl(k_segsort_mid<true>, dim3(kNumSMs * 6), dim3(kMidNT), 0, s, b.stats, b.big_cap, b.big_list, b.owner_off,
 		           out, kp);

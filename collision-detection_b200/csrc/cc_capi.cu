@@ -79,6 +79,7 @@ struct cc_ctx {
 	Buf np_norm, np_pa, np_pb, np_depth, np_ids, np_pairs, np_flag, np_pos, np_order, np_classes, np_bsum;
 	Buf bp_bsum;  // block sums of the cooperative cell scan
 	Buf cell_cs;  // packed (start, cursor) words of the cells
+	Buf sorted, sorted_body, row_count, masks;  // entries of dense cells in body order, their pairs as rows, hit masks
 	Buf extra;    // bodies of the chained search's entries past the first n
 	Buf in_T, in_A, in_B, in_C, in_R, in_ID, in_pos, in_rot, in_act, out_aabb, out_pairs, out_norm, out_pa, out_pb,
 	    out_depth, out_bids;
@@ -103,13 +104,16 @@ struct cc_ctx {
 	// retained broadphase result (owner buckets not yet scattered)
 	bool retained = false;
 	uint64_t retained_n = 0, retained_P = 0;
-	bool retained_fused = false;
+	bool retained_fused = false, retained_direct = false;
 	// this call's pairs are emitted by the fused owner sort (one scene, not
 	// incremental, few owner buckets); set by prepare and the call
 	bool fused_now = false;
 	// one scene whose last call found no dense cell: the dense-cell pair test is
 	// not launched (the sparse one tests every cell and counts dense ones)
 	bool dense_skip = false;
+	// sorted cells with the dense-cell test (its pairs go straight to their owners'
+	// buckets, so the narrowphase runs on the sorted list)
+	bool direct = false;
 	uint64_t last_dense = 1;  // dense cells of the last call (1: none seen yet)
 	// the search of this call: on chained entries (launch_link, launch_walk) or
 	// on sorted cells; kChainUnknown looks for crowded cells before the walk
@@ -118,7 +122,7 @@ struct cc_ctx {
 	bool chain = false, chain_check = false;
 	GridParams call_gp{};  // gp as this call's search uses it (set by prepare)
 	int chain_wait = 0;  // calls on sorted cells left before the chains are tried again
-	uint64_t last_E = 0, last_P = 0;
+	uint64_t last_E = 0, last_P = 0, last_tmp = 0, last_mask = 0;  // last_tmp: pairs that went through pairs_tmp
 	int last_dim[3] = {0, 0, 0};
 	// owner buckets of the pair sort (BpBuffers::owner_shift / key_bits), chosen
 	// per call from the last call's pairs per body
@@ -154,6 +158,7 @@ struct cc_ctx {
 		int grid[3] = {0, 0, 0};
 		float env = 0.f;
 		uint64_t cap = 0, entry_cap = 0, pair_cap = 0;
+		bool direct = false;
 	} hs[2];
 	cudaStream_t hs_copy = nullptr, hs_comp = nullptr, hs_out = nullptr;
 	cudaEvent_t hs_user = nullptr, hs_back = nullptr;
@@ -342,8 +347,13 @@ BpBuffers bp_buffers(cc_ctx *c) {
 	                : nullptr;
 	b.sm = c->sm;
 	b.extra_body = ptr<uint32_t>(c->extra);
-	b.dense = c->dense_skip ? nullptr : ptr<uint2>(c->dense);
-	b.dense_cap = c->dense.bytes / sizeof(uint2);
+	b.dense = c->direct ? ptr<DenseItem>(c->dense) : nullptr;
+	b.sorted = ptr<float4>(c->sorted);
+	b.sorted_body = ptr<uint32_t>(c->sorted_body);
+	b.row_count = ptr<uint32_t>(c->row_count);
+	b.masks = ptr<uint32_t>(c->masks);
+	b.mask_cap = c->masks.bytes / sizeof(uint32_t);
+	b.dense_cap = c->dense.bytes / sizeof(DenseItem);
 	b.dense_cell = c->gp.dense_cell;
 	b.owner_shift = c->owner_shift;
 	b.key_bits = c->key_bits;
@@ -408,16 +418,33 @@ bool chain_enabled() {
 	return on;
 }
 
+// Scratch of the dense-cell test for the entries there is room for.
+cc_status direct_prepare(cc_ctx *c) {
+	CC_TRY(ensure(c, c->sorted, c->entries.bytes));
+	CC_TRY(ensure(c, c->sorted_body, sizeof(uint32_t) * (c->entries.bytes / (2 * sizeof(float4)))));
+	// the last call's mask words, up to 16 GB (what does not fit is tested twice)
+	CC_TRY(ensure(c, c->masks, std::min<uint64_t>(sizeof(uint32_t) * (c->last_mask + c->last_mask / 8), (uint64_t)1 << 34)));
+	return ensure(c, c->row_count, sizeof(uint32_t) * (c->entries.bytes / (2 * sizeof(float4))));
+}
+
+// Pairs of a pass that went through the unsorted scratch list.
+uint64_t unsorted_pairs(const DevStats &st, bool direct) { return direct ? st.tmp_pairs : st.pairs; }
+
 // Allocates the n-dependent broadphase scratch and, if np_cap > 0, the
 // narrowphase scratch for np_cap pairs. Buffers only grow; every public call
 // ends with a synchronize, so nothing in flight uses a buffer replaced here.
 cc_status prepare(cc_ctx *c, uint64_t n, uint64_t np_cap, uint64_t g_override = 0) {
 	c->gp.g_max = g_override ? (uint32_t)g_override : g_max_for(n);
-	choose_owner_shift(c, n);
-	c->fused_now = fused_sort_enabled() && fused_sort_fits(owner_buckets(n, c->owner_shift));
-	c->dense_skip = !g_override && c->last_dense == 0;
+	c->dense_skip = c->last_dense == 0;
 	c->chain = chain_enabled() && c->chain_state != cc_ctx::kChainNo && n < ((uint64_t)1 << 31);
 	c->chain_check = c->chain && c->chain_state == cc_ctx::kChainUnknown;
+	c->direct = !c->chain && !c->dense_skip;
+	choose_owner_shift(c, n);
+	if (g_override && c->direct) {  // a batch counts its scenes' pairs by owner if its output is too small
+		c->owner_shift = 0;
+		c->key_bits = 32;
+	}
+	c->fused_now = !c->direct && fused_sort_enabled() && fused_sort_fits(owner_buckets(n, c->owner_shift));
 	c->call_gp = c->gp;
 	if (c->chain) c->call_gp.k_target *= kChainCellTarget;
 	CC_TRY(ensure(c, c->stats, sizeof(DevStats)));
@@ -429,15 +456,16 @@ cc_status prepare(cc_ctx *c, uint64_t n, uint64_t np_cap, uint64_t g_override = 
 	CC_TRY(ensure(c, c->owner_off, sizeof(unsigned long long) * (n + 1)));
 	const uint64_t e_guess = std::max<uint64_t>(c->last_E + c->last_E / 4, 2 * n + 1024);
 	CC_TRY(ensure(c, c->entries, 2 * sizeof(float4) * e_guess));
-	CC_TRY(ensure(c, c->extra, sizeof(uint32_t) * (c->entries.bytes / (2 * sizeof(float4)))));
-	const uint64_t p_guess = std::max<uint64_t>(c->last_P + c->last_P / 4, n / 4 + 1024);
+	if (c->chain) CC_TRY(ensure(c, c->extra, sizeof(uint32_t) * (c->entries.bytes / (2 * sizeof(float4)))));
+	if (c->direct) CC_TRY(direct_prepare(c));
+	const uint64_t p_guess = std::max<uint64_t>(c->last_tmp + c->last_tmp / 4, n / 4 + 1024);
 	CC_TRY(ensure(c, c->pairs_tmp, sizeof(unsigned long long) * p_guess));
 	c->st_words[0] = std::max<uint64_t>(c->st_words[0], status_words_for(c->gp.g_max));
 	c->st_words[1] = std::max<uint64_t>(c->st_words[1], status_words_for(n + 1));
 	CC_TRY(ensure_status(c));
 	CC_TRY(ensure(c, c->ticket, 64));
 	CC_TRY(ensure(c, c->big_list, sizeof(uint32_t) * (n + 1024)));
-	CC_TRY(ensure(c, c->dense, sizeof(uint2) * (c->entries.bytes / (2 * sizeof(float4)) / kDenseCell + 1024)));
+	CC_TRY(ensure(c, c->dense, sizeof(DenseItem) * (c->entries.bytes / (2 * sizeof(float4)) / kDenseCell + 1024)));
 	if (np_cap) CC_TRY(np_prepare(c, np_cap));
 	return CC_OK;
 }
@@ -522,7 +550,7 @@ void enqueue_pairs(cc_ctx *c, uint64_t n, float *aabb, uint64_t entries_hint, cu
 		StageMark m(c, ST_PAIR_TEST, s);
 		launch_pair_test(n, b, entries_hint, s);
 	}
-	c->launches += 5 - (c->dense_skip ? 1 : 0);  // count, cell scan, scatter, sparse + dense pair test
+	c->launches += c->direct ? 6 : 4;  // count, cell scan, scatter, pair test (+ dense cells: ranks, counts)
 }
 
 // Shift .. owner scan.
@@ -548,6 +576,7 @@ void enqueue_emit(cc_ctx *c, uint64_t n, unsigned long long *out, uint64_t out_c
 	{
 		StageMark m(c, ST_OWNER_SCATTER, s);
 		launch_owner_scatter(out_cap, out, b, s);
+		c->launches += c->direct ? 2 : 0;  // the dense cells' pairs
 	}
 	{
 		StageMark m(c, ST_SEGSORT, s);
@@ -556,6 +585,7 @@ void enqueue_emit(cc_ctx *c, uint64_t n, unsigned long long *out, uint64_t out_c
 	{
 		StageMark m(c, ST_SEGSORT_MID, s);
 		launch_segsort_mid(out, b, s);
+		c->launches += c->direct ? 1 : 0;  // the merges
 	}
 	{
 		StageMark m(c, ST_SEGSORT_BIG, s);
@@ -623,7 +653,7 @@ cc_status enqueue_sort_and_np_overlapped(cc_ctx *c, uint64_t n, const NpArgs &a,
 // Whether this call's narrowphase is overlapped with the pair sort (outputs of
 // at most 2^24 pairs), with the stream, events and contact hash it needs.
 cc_status overlap_prepare(cc_ctx *c, uint64_t pairs_cap, bool &ov) {
-	ov = c->np_overlap && pairs_cap > 0 && pairs_cap <= ((uint64_t)1 << 24);
+	ov = c->np_overlap && !c->direct && pairs_cap > 0 && pairs_cap <= ((uint64_t)1 << 24);
 	if (!ov) return CC_OK;
 	if (!c->np_stream) CC_CUDA(c, cudaStreamCreateWithFlags(&c->np_stream, cudaStreamNonBlocking));
 	if (!c->ev_fork) CC_CUDA(c, cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming));
@@ -670,7 +700,7 @@ cc_status reset_pass_counters(cc_ctx *c, uint64_t n, cudaStream_t s) {
 	CC_CUDA(c, cudaMemsetAsync(&d->big_segments, 0, 3 * sizeof(unsigned long long), s));
 	CC_CUDA(c, cudaMemsetAsync(&d->np_n, 0, sizeof(unsigned long long), s));
 	CC_CUDA(c, cudaMemsetAsync(&d->dense_items, 0, sizeof(unsigned long long), s));
-	CC_CUDA(c, cudaMemsetAsync(&d->extra, 0, sizeof(unsigned long long), s));
+	CC_CUDA(c, cudaMemsetAsync(&d->mask_words, 0, 3 * sizeof(unsigned long long), s));
 	CC_CUDA(c, cudaMemsetAsync(d->bar_scan, 0, sizeof(d->bar_scan), s));
 	return CC_OK;
 }
@@ -680,9 +710,9 @@ cc_status reset_pass_counters(cc_ctx *c, uint64_t n, cudaStream_t s) {
 // the search on the shifted boxes (rare: guesses and path follow the previous
 // call). h_stats is current on return.
 cc_status settle(cc_ctx *c, uint64_t n, float *aabb, unsigned long long *out, uint64_t out_cap, const NpArgs *np,
-                 cudaStream_t s) {
+                 cudaStream_t s, bool *redone = nullptr) {
 	for (int round = 0; round < 4; round++) {
-		const uint64_t E = c->h_stats->entries, P = c->h_stats->pairs;
+		const uint64_t E = c->h_stats->entries, P = unsorted_pairs(*c->h_stats, c->direct);
 		BpBuffers b = bp_buffers(c);
 		const bool crowded = c->chain && (c->h_stats->err & kErrLongChain);
 		if (E <= b.entry_cap && P <= b.pair_cap && !crowded) return CC_OK;
@@ -690,15 +720,23 @@ cc_status settle(cc_ctx *c, uint64_t n, float *aabb, unsigned long long *out, ui
 			return set_err(c, CC_ERR_CAPACITY, "search grid needs %llu entries (>= 2^32)", (unsigned long long)E);
 		if (E > b.entry_cap) {
 			CC_TRY(ensure(c, c->entries, 2 * sizeof(float4) * (E + E / 8)));
-			CC_TRY(ensure(c, c->extra, sizeof(uint32_t) * (c->entries.bytes / (2 * sizeof(float4)))));
-			CC_TRY(ensure(c, c->dense, sizeof(uint2) * ((E + E / 8) / kDenseCell + 1024)));
+			if (c->chain) CC_TRY(ensure(c, c->extra, sizeof(uint32_t) * (c->entries.bytes / (2 * sizeof(float4)))));
+			CC_TRY(ensure(c, c->dense, sizeof(DenseItem) * ((E + E / 8) / kDenseCell + 1024)));
 		}
+		if (redone) *redone = true;
 		if (crowded) {
 			c->chain = false;
 			c->chain_state = cc_ctx::kChainNo;
 			c->chain_wait = c->h_stats->dense_items && c->gp.dense_cell <= kChainLong ? 0 : kChainWait;
 			c->dense_skip = false;
+			c->direct = true;
+			c->fused_now = false;
+			if (c->sm.plans) {
+				c->owner_shift = 0;
+				c->key_bits = 32;
+			}
 		}
+		if (c->direct) CC_TRY(direct_prepare(c));
 		if (P > b.pair_cap) CC_TRY(ensure(c, c->pairs_tmp, sizeof(unsigned long long) * (P + P / 8)));
 		CC_TRY(reset_pass_counters(c, n, s));
 		c->chain_check = c->chain_check && c->chain;
@@ -740,6 +778,8 @@ cc_status sort_fallback(cc_ctx *c, uint64_t n, uint64_t P, unsigned long long *o
 void remember(cc_ctx *c) {
 	c->last_E = c->h_stats->entries;
 	c->last_P = c->h_stats->pairs;
+	c->last_tmp = unsorted_pairs(*c->h_stats, c->direct);
+	c->last_mask = c->h_stats->mask_words;
 	c->last_dense = c->h_stats->dense_items;
 	// chains while no cell is crowded; back to them once sorted cells show none
 	// (which they tell through their dense cells, so a raised threshold makes
@@ -758,6 +798,7 @@ void retain(cc_ctx *c, uint64_t n, uint64_t P) {
 	c->retained_n = n;
 	c->retained_P = P;
 	c->retained_fused = c->fused_now;
+	c->retained_direct = c->direct;
 }
 
 // Writes the retained pair list into `out` (cap >= P checked by the caller).
@@ -769,6 +810,7 @@ cc_status emit_retained(cc_ctx *c, unsigned long long *out, uint64_t cap, cudaSt
 	CC_CUDA(c, cudaMemsetAsync(&d->big_segments, 0, 3 * sizeof(unsigned long long), s));
 	CC_CUDA(c, cudaMemsetAsync(&d->err, 0, sizeof(uint32_t), s));
 	c->fused_now = c->retained_fused;
+	c->direct = c->retained_direct;
 	enqueue_emit(c, c->retained_n, out, cap, s);
 	CC_TRY(check_launch(c));
 	CC_TRY(read_stats(c, s));
@@ -1073,7 +1115,7 @@ cc_status collide_verlet(cc_ctx *c, const cc_scene &sc, int gx, int gy, int gz, 
 		c->inc_n = n;
 		c->inc_allocs = c->v_ref.allocs + c->v_cand.allocs;
 		const uint64_t P = c->h_stats->pairs;
-		c->last_P = P;
+		c->last_P = c->last_tmp = P;
 		*n_pairs = P;
 		if (P > pairs_cap)
 			return set_err(c, CC_ERR_CAPACITY, "pair list needs %llu entries, capacity %llu", (unsigned long long)P,
@@ -1151,7 +1193,8 @@ void cc_ctx_destroy(cc_ctx *c) {
 	               &c->b_base,   &c->b_res,      &c->g_T,        &c->g_A,
 	               &c->g_B,      &c->g_C,        &c->g_R,        &c->g_ID,     &c->g_pos,       &c->g_rot,
 	               &c->g_act,    &c->g_src,      &c->v_ref,    &c->v_backup,   &c->v_scratch, &c->v_cand,   &c->v_status,
-	               &c->np_bsum,  &c->pt_desc,    &c->np_hkeys,   &c->np_hvals,   &c->bp_bsum,    &c->cell_cs,  &c->extra};
+	               &c->np_bsum,  &c->pt_desc,    &c->np_hkeys,   &c->np_hvals,   &c->bp_bsum,    &c->cell_cs,  &c->extra,
+	               &c->sorted,   &c->row_count,  &c->masks,    &c->sorted_body};
 	for (Buf *b : bufs)
 		if (b->p) cudaFree(b->p);
 	c->g_collide.drop();
@@ -1654,16 +1697,18 @@ cc_status batch_impl(cc_ctx *c, const cc_batch *bt, int gx, int gy, int gz, floa
 	CC_TRY(check_launch(c));
 	CC_TRY(read_stats(c, s));
 	CC_TRY(device_err(c));
-	bool redone = (c->h_stats->err & kErrLongChain) || c->h_stats->entries > c->entries.bytes / (2 * sizeof(float4)) ||
-	              c->h_stats->pairs > c->pairs_tmp.bytes / sizeof(unsigned long long);
-	CC_TRY(settle(c, n, res->aabb, out, pairs_cap, &a, s));
+	bool redone = false;
+	CC_TRY(settle(c, n, res->aabb, out, pairs_cap, &a, s, &redone));
 	remember(c);
 	const uint64_t P = c->h_stats->pairs;
 	res->n_pairs = P;
 	if (P > pairs_cap) {
 		if (scene_pairs) {  // no sorted list to count them in
 			CC_CUDA(c, cudaMemsetAsync(d_pairs_s, 0, sizeof(uint64_t) * S, s));
-			launch_batch_pair_counts(P, ptr<unsigned long long>(c->pairs_tmp), scene_of, d_pairs_s, s);
+			if (c->direct)  // one owner per bucket, the dense cells' pairs only counted
+				launch_batch_owner_counts((uint32_t)S, d_shape, ptr<unsigned long long>(c->owner_off), d_pairs_s, s);
+			else
+				launch_batch_pair_counts(P, ptr<unsigned long long>(c->pairs_tmp), scene_of, d_pairs_s, s);
 			CC_CUDA(c, cudaMemcpyAsync(scene_pairs, d_pairs_s, sizeof(uint64_t) * S, cudaMemcpyDeviceToHost, s));
 			CC_CUDA(c, cudaStreamSynchronize(s));
 		}
@@ -1967,6 +2012,7 @@ cc_status cc_collide_host_submit(cc_ctx *c, const cc_scene *sc, int gx, int gy, 
 		const BpBuffers b = bp_buffers(c);
 		h.entry_cap = b.entry_cap;
 		h.pair_cap = b.pair_cap;
+		h.direct = c->direct;
 	} else {
 		memset(h.h_stats, 0, sizeof(DevStats));
 	}
@@ -1996,7 +2042,7 @@ cc_status cc_collide_host_wait(cc_ctx *c, cc_result *res, void *stream) {
 	res->n_pairs = res->n_contacts = 0;
 	if (h.dev.n == 0) return CC_OK;
 	const DevStats &st = *h.h_stats;
-	const bool fast = st.err == 0 && st.entries <= h.entry_cap && st.pairs <= h.pair_cap && st.pairs <= h.cap &&
+	const bool fast = st.err == 0 && st.entries <= h.entry_cap && unsorted_pairs(st, h.direct) <= h.pair_cap && st.pairs <= h.cap &&
 	                  st.np_n == st.pairs;
 	uint64_t P = st.pairs, nc = st.contacts;
 	if (fast) {

@@ -42,6 +42,8 @@ struct DevStats {
 	unsigned long long dense_items;  // (cell, row chunk) work items of the dense-cell pair test (chained search: long chains met)
 	uint32_t blocks_done;         // last-block detection of the bounds reduction
 	uint32_t pad_;
+	unsigned long long mask_words;  // hit-mask words of the dense cells' rows
+	unsigned long long tmp_pairs; // pairs of the sparse cells where dense cells have their own test (else `pairs`)
 	unsigned long long extra;     // entries of the chained search beyond the first one of every body
 	Plan plan;
 	// grid barriers of the cooperative kernels (GridBarrier: arrived, gen),
@@ -126,6 +128,17 @@ struct SceneMap {
 	const uint32_t *cell_base = nullptr;  // per scene + 1
 };
 
+// Work item of the dense-cell test: 256 rows of a cell from `row` on, and the
+// place of their hit masks (in words: 256 rows of dense_row_words each).
+struct DenseItem {
+	uint32_t cell, row;
+	unsigned long long mask;
+};
+__host__ __device__ inline uint32_t dense_row_words(uint32_t k, uint32_t row) { return 8 * ((k - row + 255) / 256); }
+__host__ __device__ inline unsigned long long dense_mask_words(uint32_t k, uint32_t row) {
+	return 256ull * dense_row_words(k, row);
+}
+
 struct BpBuffers {
 	DevStats *stats;
 	uint32_t *cell_count;    // g_max
@@ -145,7 +158,12 @@ struct BpBuffers {
 	uint32_t *ticket2 = nullptr;
 	bool pre_zeroed = false;      // status/ticket regions were zeroed by the pass's first kernel
 	SceneMap sm;                  // batch layout (empty: one scene)
-	uint2 *dense = nullptr;       // dense-cell work items (cell, first row)
+	DenseItem *dense = nullptr;   // work items of the dense cells; null: no dense-cell test this call
+	float4 *sorted = nullptr;     // entries of the dense cells in body order (entry_cap records)
+	uint32_t *sorted_body = nullptr;  // their bodies alone
+	uint32_t *row_count = nullptr;  // pairs of each of them as a row
+	uint32_t *masks = nullptr;      // their hit masks (items past mask_cap words are tested twice)
+	uint64_t mask_cap = 0;
 	uint64_t dense_cap = 0;
 	uint32_t dense_cell = 128;    // threshold (entries) of a dense cell
 	// Pairs are bucketed by owner (the smaller index a) coarsened to a >> owner_shift:
@@ -205,12 +223,12 @@ void launch_link(uint64_t n, float *aabb, const BpBuffers &b, cudaStream_t s, bo
 void launch_chain_check(const BpBuffers &b, uint32_t g_max, cudaStream_t s);
 void launch_walk(uint64_t n, const BpBuffers &b, uint64_t entries_hint, cudaStream_t s);
 void launch_scan_owner(uint64_t n, const BpBuffers &b, cudaStream_t s);
-// Cells holding more than b.dense_cell entries are left out of the
-// lane-per-entry pair test and tested here instead, tile by tile (N-body
-// style); kDenseCell is the default threshold and the smallest sizing unit of
-// the work list.
+// With b.dense, cells holding more than b.dense_cell entries are left out of the
+// lane-per-entry pair test; launch_pair_test counts their pairs per owner and
+// launch_owner_scatter writes them, so pairs_tmp (stats->tmp_pairs) holds the
+// others only. kDenseCell is the default threshold and the smallest sizing unit
+// of the work list.
 constexpr uint32_t kDenseCell = 128;
-void launch_pair_test_dense(const BpBuffers &b, cudaStream_t s);
 // Device-driven emission: P is read from stats->pairs. If P exceeds the
 // scratch (pair_cap) or out_cap nothing is written and stats->np_n = 0, else
 // stats->np_n = P.
@@ -308,6 +326,8 @@ void launch_batch_front(uint64_t n, uint64_t nb, uint32_t S, const unsigned long
                         const ZeroList &zero);
 void launch_batch_pair_counts(uint64_t P, const unsigned long long *pairs, const uint32_t *scene_of,
                               unsigned long long *scene_pairs, cudaStream_t s);
+void launch_batch_owner_counts(uint32_t S, const unsigned long long *shape_off, const unsigned long long *owner_off,
+                               unsigned long long *scene_pairs, cudaStream_t s);
 // From the final pair list (stats->np_n keys, the stats->contacts contacts' first).
 void launch_batch_offsets(uint32_t S, const unsigned long long *shape_off, const unsigned long long *pairs,
                           const DevStats *stats, unsigned long long *scene_pairs, unsigned long long *contact_off,
