@@ -116,8 +116,8 @@ __device__ __forceinline__ bool is_zero(vec<T> a) {
 template <class S>
 struct Shape {
 	int type;
-	vec<S> X, Y, Z;  // centre (or triangle vertex 0), B (or vertex 1), C (or vertex 2)
-	vec<S> r0, r1, r2;
+	vec<S> X, Y;        // centre (or triangle vertex 0), B (or vertex 1)
+	vec<S> r0, r1, r2;  // rotation rows (r0: triangle vertex 2)
 };
 
 template <class S>
@@ -209,7 +209,7 @@ __device__ __forceinline__ vec<S> support(const Shape<S> &s, vec<S> d) {
 		S dist = dotp(s.X, d);
 		vec<S> p = s.X;
 		if (dotp(s.Y, d) > dist) { dist = dotp(s.Y, d); p = s.Y; }
-		if (dotp(s.Z, d) > dist) { p = s.Z; }
+		if (dotp(s.r0, d) > dist) { p = s.r0; }
 		return p;
 	}
 	const vec<S> rn = mcol(s.r0, s.r1, s.r2, d);
@@ -221,8 +221,8 @@ typedef vec<double> D3;
 template <class S>
 __device__ __forceinline__ D3 centre(const Shape<S> &s) {  // GetCenter :11-17
 	if (s.type == TRIANGLEMESH)
-		return {((double)s.X.x + s.Y.x + s.Z.x) / 3.0, ((double)s.X.y + s.Y.y + s.Z.y) / 3.0,
-		        ((double)s.X.z + s.Y.z + s.Z.z) / 3.0};
+		return {((double)s.X.x + s.Y.x + s.r0.x) / 3.0, ((double)s.X.y + s.Y.y + s.r0.y) / 3.0,
+		        ((double)s.X.z + s.Y.z + s.r0.z) / 3.0};
 	return {(double)s.X.x + 0.0, (double)s.X.y + 0.0, (double)s.X.z + 0.0};  // R3(0,0,0) + A
 }
 
@@ -252,8 +252,6 @@ __device__ __forceinline__ Shape<S> load_shape(uint32_t s, uint32_t id, const in
 	rows_of<S>(qw, qx, qy, qz, sh.r0, sh.r1, sh.r2);
 	sh.X = cvt3<S>(ld3(A, s));
 	sh.Y = cvt3<S>(ld3(B, s));
-	sh.Z = mk<S>(S(0), S(0), S(0));
-	if (sh.type == TRIANGLEMESH) sh.Z = cvt3<S>(ld3(C, s));  // no other support or centre reads it
 	const vec<S> po = sub(cvt3<S>(p), org);
 	if (sh.type == SPHERE || sh.type == ELLIPSOID || sh.type == BOX || sh.type == CYLINDER) {
 		vec<S> b0, b1, b2;
@@ -261,9 +259,10 @@ __device__ __forceinline__ Shape<S> load_shape(uint32_t s, uint32_t id, const in
 		sh.X = add(mrow(b0, b1, b2, sh.X), po);  // quatRotate(A, body_rot) + pos
 	} else if (sh.type == TRIANGLEMESH) {
 		const vec<S> pw = cvt3<S>(p);  // quatRotate(v + pos, body_rot * local_rot), then into the frame
+		const vec<S> Z = cvt3<S>(ld3(C, s));
 		sh.X = sub(mrow(sh.r0, sh.r1, sh.r2, add(sh.X, pw)), org);
 		sh.Y = sub(mrow(sh.r0, sh.r1, sh.r2, add(sh.Y, pw)), org);
-		sh.Z = sub(mrow(sh.r0, sh.r1, sh.r2, add(sh.Z, pw)), org);
+		sh.r0 = sub(mrow(sh.r0, sh.r1, sh.r2, add(Z, pw)), org);
 	}
 	return sh;
 }
@@ -278,14 +277,28 @@ struct Lane {
 	uint32_t pair;  // index of the pair being worked on
 	int st;
 	int phase1, phase2;
-	bool hit;
+	bool hit, mesh;  // mesh: a shape is a TRIANGLEMESH (no envelope, :378-380)
 	Shape<S> A, B;
 	D3 v0, v1, v2, v3;
-	vec<S> v11, v12, v21, v22, v31, v32;
-	D3 n;      // direction of the next support pair
-	D3 N, p0;  // contact normal and point (post stage)
-	D3 org;    // frame origin
-	double env;
+	D3 n;  // direction of the next support pair (post stage: the normal, with the contact point in v1)
+};
+
+// The support points behind a portal's three vertices (v11, v12, v21, v22, v31,
+// v32), read only when a contact is finished: in shared memory, where they cost
+// no registers and a new one is a few stores instead of selects.
+template <class S, int NT>
+struct Points {
+	S *p;  // this lane's column of [3 vertices][6 coordinates][NT]
+	__device__ __forceinline__ void put(int vertex, vec<S> a, vec<S> b) const {
+		S *q = p + vertex * (6 * NT);
+		q[0] = a.x; q[NT] = a.y; q[2 * NT] = a.z;
+		q[3 * NT] = b.x; q[4 * NT] = b.y; q[5 * NT] = b.z;
+	}
+	__device__ __forceinline__ vec<S> a(int vertex) const {
+		const S *q = p + vertex * (6 * NT);
+		return {q[0], q[NT], q[2 * NT]};
+	}
+	__device__ __forceinline__ vec<S> b(int vertex) const { return Points{p + 3 * NT}.a(vertex); }
 };
 
 template <class S>
@@ -361,12 +374,11 @@ __device__ __forceinline__ bool start_pair(Lane<S> &L, uint32_t i, uint64_t n, c
 	if (!active[ida] && !active[idb]) return false;  // :344-346
 	if (ida == idb) return false;                     // :347-349
 	const float3 o = ld3(pos, ida);
-	L.org = mk((double)o.x, (double)o.y, (double)o.z);
-	const vec<S> org = cvt<S>(L.org);
+	const D3 origin = mk((double)o.x, (double)o.y, (double)o.z);
+	const vec<S> org = cvt<S>(origin);
 	L.A = load_shape<S>(sa, ida, T, A, B, C, R, pos, rot, org);
 	L.B = load_shape<S>(sb, idb, T, A, B, C, R, pos, rot, org);
-	L.env = envelope;
-	if (L.A.type == TRIANGLEMESH || L.B.type == TRIANGLEMESH) L.env = 0.0;
+	L.mesh = L.A.type == TRIANGLEMESH || L.B.type == TRIANGLEMESH;
 	if (L.A.type == SPHERE && L.B.type == SPHERE) {  // :382-397
 		const D3 xa = dd(L.A.X), xb = dd(L.B.X);
 		const D3 rel = sub(xb, xa);
@@ -375,7 +387,7 @@ __device__ __forceinline__ bool start_pair(Lane<S> &L, uint32_t i, uint64_t n, c
 		const double cd = ra + rb;
 		if (!(d2 <= cd * cd)) return false;
 		const D3 N = unit<double, false>(rel);
-		write_contact(L.pair, L.env, L.org, N, add(xa, scl(ra, N)), sub(xb, scl(rb, N)), ida, idb, sc);
+		write_contact(L.pair, (double)envelope, origin, N, add(xa, scl(ra, N)), sub(xb, scl(rb, N)), ida, idb, sc);
 		return false;
 	}
 	// CollideAndFindPoint :137-144
@@ -388,12 +400,11 @@ __device__ __forceinline__ bool start_pair(Lane<S> &L, uint32_t i, uint64_t n, c
 }
 
 // Finishes a hit: the contact points of :404-406 need one more support pair
-// along the normal; N, p0 are set here and the post stage evaluates it.
+// along the normal, which the post stage evaluates.
 template <class S>
 __device__ __forceinline__ void to_post(Lane<S> &L, D3 N, D3 p0) {
-	L.N = N;
-	L.p0 = p0;
 	L.n = N;
+	L.v1 = p0;
 	L.st = kPost;
 }
 
@@ -415,8 +426,8 @@ __device__ __forceinline__ bool pre_step(Lane<S> &L) {
 // The end of a refinement with a hit (:256-283 once the portal is final): the
 // barycentric contact point and the normal; the post stage then evaluates one
 // more support pair along the normal.
-template <class S>
-__device__ __forceinline__ void finish_refine(Lane<S> &L) {
+template <class S, int NT>
+__device__ __forceinline__ void finish_refine(Lane<S> &L, const Points<S, NT> &pts) {
 	const D3 v1 = L.v1, v2 = L.v2, v3v = L.v3, v0 = L.v0, n = L.n;
 	double b0 = dotp(crossp(v1, v2), v3v);
 	double b1 = dotp(crossp(v3v, v2), v0);
@@ -432,46 +443,46 @@ __device__ __forceinline__ void finish_refine(Lane<S> &L) {
 	}
 	const double inv = 1.0 / sum;
 	const D3 v01 = centre(L.A), v02 = centre(L.B);
-	const D3 p = add(add(add(scl(b0, v01), scl(b1, dd(L.v11))), scl(b2, dd(L.v21))), scl(b3, dd(L.v31)));
-	const D3 q = add(add(add(scl(b0, v02), scl(b1, dd(L.v12))), scl(b2, dd(L.v22))), scl(b3, dd(L.v32)));
+	const D3 p = add(add(add(scl(b0, v01), scl(b1, dd(pts.a(0)))), scl(b2, dd(pts.a(1)))), scl(b3, dd(pts.a(2))));
+	const D3 q = add(add(add(scl(b0, v02), scl(b1, dd(pts.b(0)))), scl(b2, dd(pts.b(1)))), scl(b3, dd(pts.b(2))));
 	const D3 pq = add(p, q);
 	const D3 pt = mk(pq.x * inv * 0.5, pq.y * inv * 0.5, pq.z * inv * 0.5);
 	to_post(L, unit<double, false>(n), pt);
 }
 
 // State update after the support pair (pa = support(A,-n), pb = support(B,n)).
-// Returns false when the pair is finished. park: a refinement that ends with a
-// hit leaves its portal as it is (kParked) instead of finishing it here.
-template <class S>
-__device__ __forceinline__ bool post_step(Lane<S> &L, vec<S> pa, vec<S> pb, const NpScratch &sc,
-                                          uint32_t ida, uint32_t idb, bool park) {
+// Returns false when the pair is finished. A refinement that ends with a hit
+// leaves its portal as it is (kParked).
+template <class S, int NT>
+__device__ __forceinline__ bool post_step(Lane<S> &L, const Points<S, NT> &pts, vec<S> pa, vec<S> pb, float envelope,
+                                          const long long *pairs, const uint32_t *ID, const float *pos,
+                                          const NpScratch &sc) {
 	switch (L.st) {
 	case kS1: {  // :146-171
-		L.v11 = pa;
-		L.v12 = pb;
 		L.v1 = vd(pb, pa);
 		if (dotp(L.v1, L.n) <= 0.0) return false;
 		L.n = crossp(L.v1, L.v0);
 		if (is_zero(L.n)) {
 			const D3 N = unit<double, false>(sub(L.v1, L.v0));
-			const D3 s12 = add(dd(L.v11), dd(L.v12));
+			const D3 s12 = add(dd(pa), dd(pb));
 			to_post(L, N, scl(0.5, s12));
 			return true;
 		}
+		pts.put(0, pa, pb);
 		L.st = kS2;
 		return true;
 	}
 	case kS2: {  // :173-191
-		L.v21 = pa;
-		L.v22 = pb;
 		L.v2 = vd(pb, pa);
 		if (dotp(L.v2, L.n) <= 0.0) return false;
 		L.n = crossp(sub(L.v1, L.v0), sub(L.v2, L.v0));
-		if (dotp(L.n, L.v0) > 0.0) {
+		if (dotp(L.n, L.v0) > 0.0) {  // the new vertex becomes the first
 			D3 t = L.v1; L.v1 = L.v2; L.v2 = t;
-			vec<S> u = L.v11; L.v11 = L.v21; L.v21 = u;
-			u = L.v12; L.v12 = L.v22; L.v22 = u;
+			pts.put(1, pts.a(0), pts.b(0));
+			pts.put(0, pa, pb);
 			L.n = neg(L.n);
+		} else {
+			pts.put(1, pa, pb);
 		}
 		L.phase1 = 0;
 		L.phase2 = 0;
@@ -480,22 +491,23 @@ __device__ __forceinline__ bool post_step(Lane<S> &L, vec<S> pa, vec<S> pb, cons
 		return true;
 	}
 	case kDisc: {  // :209-232
-		L.v31 = pa;
-		L.v32 = pb;
 		L.v3 = vd(pb, pa);
 		if (dotp(L.v3, L.n) <= 0.0) return false;
 		// both side tests evaluated up front (independent; same arithmetic)
 		const double s13 = dotp(crossp(L.v1, L.v3), L.v0), s32 = dotp(crossp(L.v3, L.v2), L.v0);
 		if (s13 < 0.0) {
-			L.v2 = L.v3; L.v21 = L.v31; L.v22 = L.v32;
+			L.v2 = L.v3;
+			pts.put(1, pa, pb);
 			L.n = crossp(sub(L.v1, L.v0), sub(L.v3, L.v0));
 			return true;
 		}
 		if (s32 < 0.0) {
-			L.v1 = L.v3; L.v11 = L.v31; L.v12 = L.v32;
+			L.v1 = L.v3;
+			pts.put(0, pa, pb);
 			L.n = crossp(sub(L.v3, L.v0), sub(L.v2, L.v0));
 			return true;
 		}
+		pts.put(2, pa, pb);
 		L.st = kRefine;
 		return true;
 	}
@@ -509,24 +521,25 @@ __device__ __forceinline__ bool post_step(Lane<S> &L, vec<S> pa, vec<S> pb, cons
 		             s43 = dotp(crossp(v4, L.v3), L.v0);
 		if (delta <= 1e-20 || depth <= 0.0 || L.phase2 > kMaxIter) {
 			if (!L.hit) return false;
-			if (park) L.st = kParked;
-			else finish_refine(L);
+			L.st = kParked;
 			return true;
 		}
-		if (s41 < 0.0) {
-			if (s42 < 0.0) { L.v1 = v4; L.v11 = pa; L.v12 = pb; }
-			else { L.v3 = v4; L.v31 = pa; L.v32 = pb; }
-		} else {
-			if (s43 < 0.0) { L.v2 = v4; L.v21 = pa; L.v22 = pb; }
-			else { L.v1 = v4; L.v11 = pa; L.v12 = pb; }
-		}
+		const bool to3 = s41 < 0.0 && !(s42 < 0.0), to2 = !(s41 < 0.0) && s43 < 0.0;
+		pts.put(to3 ? 2 : (to2 ? 1 : 0), pa, pb);
+		if (to3) L.v3 = v4;
+		else if (to2) L.v2 = v4;
+		else L.v1 = v4;
 		return true;
 	}
 	case kPost: {  // :404-406
-		const D3 N = L.N, p0 = L.p0;
+		const D3 N = L.n, p0 = L.v1;
 		const D3 p1 = add(scl(dotp(sub(dd(pa), p0), N), N), p0);
 		const D3 p2 = add(scl(dotp(sub(dd(pb), p0), N), N), p0);
-		write_contact(L.pair, L.env, L.org, neg(N), p1, p2, ida, idb, sc);
+		const uint64_t key = (uint64_t)pairs[L.pair];
+		const uint32_t ida = __ldg(ID + (uint32_t)(key >> 32)), idb = __ldg(ID + (uint32_t)key);
+		const float3 o = ld3(pos, ida);
+		write_contact(L.pair, L.mesh ? 0.0 : (double)envelope, mk((double)o.x, (double)o.y, (double)o.z), neg(N), p1, p2, ida,
+		              idb, sc);
 		return false;
 	}
 	}
@@ -535,59 +548,60 @@ __device__ __forceinline__ bool post_step(Lane<S> &L, vec<S> pa, vec<S> pb, cons
 
 // Persistent kernel: lanes take pairs from the global queue `order`
 // (P = min(P_cap, *P_dev) entries), one support pair per busy lane per
-// iteration. Once the warp has seen the queue drained, a refinement that ends
-// with a hit parks, and the parked pairs of the warp are finished together
-// when none of its lanes runs any more: the warp then runs the finishing code
-// (barycentric point, normal, one more support pair, the contact) once instead
-// of once for every pair that ends at a different iteration. The finishing
-// arithmetic reads only the parked portal, so the contacts are the same.
-template <class S>
+// iteration. Lanes wait for one another at the two costly turns of a pair: a
+// refinement that ends with a hit parks, and once kBatch lanes of the warp have
+// nothing to do (or none runs) the parked pairs are finished (barycentric point,
+// normal, one more support pair, the contact) and the idle lanes take new pairs
+// together; one at a time, every end of a pair cost the whole warp a finish, or
+// a start with its chain of loads. The arithmetic reads only the pair's own
+// state, so the contacts do not depend on it. (A finish ends the iteration: run
+// on into the next support pair, the compiler fused other products and sums, and
+// the contacts of these modes change with their rounding.) With fewer pairs than
+// lanes each warp takes only its share of them.
+// 600,000 pairs, fp64 / mixed mode: 832 / 516 us with 1, 627 / 417 with 6, 548 /
+// 366 with 12, 550 / 363 with 18; with the support points in shared memory and
+// the post stage in the portal's registers (218 -> 166, six blocks per SM for
+// four) 413 / 379.
+constexpr int kBatchLanes = 12;
+template <class S, int NT>
 __device__ __forceinline__ void run(uint64_t P_cap, const unsigned long long *P_dev, uint64_t n, const int32_t *T,
                                     const float *A, const float *B, const float *C, const float *R, const uint32_t *ID,
                                     uint64_t nb, const uint8_t *active, const float *pos, const float *rot,
                                     float envelope, const long long *pairs, const NpScratch &sc, uint32_t *queue) {
 	const uint64_t P = P_dev ? min(P_cap, (uint64_t)*P_dev) : P_cap;
+	const uint64_t warps = (uint64_t)gridDim.x * (blockDim.x / 32);
+	const uint32_t width = (uint32_t)min((P + warps - 1) / warps, (uint64_t)32);
+	const int batch = min(kBatchLanes, (int)width);
 	Lane<S> L;
 	L.st = kIdle;
-	bool done = false;     // the queue is exhausted for this lane
-	bool drained = false;  // the warp has taken the last queue entries (warp-uniform)
-	uint32_t ida = 0, idb = 0;
+	bool drained = false;  // the queue is exhausted (warp-uniform)
+	__shared__ S points[3 * 6 * NT];
+	const Points<S, NT> pts = {points + threadIdx.x};
 	const uint32_t lane = threadIdx.x & 31, lt = (1u << lane) - 1u;
 	while (true) {
-		// lanes without a pair take the next ones from the queue (one atomic per warp)
-		const bool want = L.st == kIdle && !done;
-		const uint32_t m = __ballot_sync(0xffffffffu, want);
-		if (m) {
-			uint32_t base = 0;
-			const int leader = __ffs(m) - 1;
-			if ((int)lane == leader) base = atomicAdd(queue, (uint32_t)__popc(m));
-			base = __shfl_sync(0xffffffffu, base, leader);
-			drained = drained || (uint64_t)base + __popc(m) >= P;
-			if (want) {
-				const uint64_t j = (uint64_t)base + __popc(m & lt);
-				if (j >= P) {
-					done = true;
-				} else {
+		const bool wants = L.st == kIdle && !drained && lane < width;
+		const uint32_t idle = __ballot_sync(0xffffffffu, wants), parked = __ballot_sync(0xffffffffu, L.st == kParked);
+		const uint32_t runs = __ballot_sync(0xffffffffu, L.st != kIdle && L.st != kParked);
+		if (!(idle | parked | runs)) break;
+		if (!runs || __popc(idle | parked) >= batch) {
+			if (idle) {  // new pairs for the idle lanes, one atomic per warp
+				uint32_t base = 0;
+				const int leader = __ffs(idle) - 1;
+				if ((int)lane == leader) base = atomicAdd(queue, (uint32_t)__popc(idle));
+				base = __shfl_sync(0xffffffffu, base, leader);
+				drained = (uint64_t)base + __popc(idle) >= P;
+				const uint64_t j = (uint64_t)base + __popc(idle & lt);
+				if (wants && j < P) {
 					const uint32_t i = sc.order[j];
-					if (start_pair(L, i, n, T, A, B, C, R, ID, nb, active, pos, rot, envelope, pairs, sc)) {
-						const uint64_t key = (uint64_t)pairs[i];
-						ida = __ldg(ID + (uint32_t)(key >> 32));
-						idb = __ldg(ID + (uint32_t)(key & 0xffffffffull));
-					} else {
-						L.st = kIdle;
-					}
+					if (!start_pair(L, i, n, T, A, B, C, R, ID, nb, active, pos, rot, envelope, pairs, sc)) L.st = kIdle;
 				}
 			}
+			if (parked) {
+				if (L.st == kParked) finish_refine(L, pts);  // -> kPost: the next iteration writes the contact
+				continue;
+			}
 		}
-		done = done || drained;
-		const bool running = L.st != kIdle && L.st != kParked;
-		if (!__any_sync(0xffffffffu, running || !done)) {
-			const bool parked = L.st == kParked;
-			if (!__any_sync(0xffffffffu, parked)) break;
-			if (parked) finish_refine(L);  // -> kPost: the next iteration writes the contact
-			continue;
-		}
-		if (!running) continue;
+		if (L.st == kIdle || L.st == kParked) continue;
 		if (!pre_step(L)) {
 			L.st = kIdle;
 			continue;
@@ -596,7 +610,7 @@ __device__ __forceinline__ void run(uint64_t P_cap, const unsigned long long *P_
 		const vec<S> d = cvt<S>(L.n);
 		const vec<S> pa = support<S, false>(L.A, neg(d));
 		const vec<S> pb = support<S, false>(L.B, d);
-		if (!post_step(L, pa, pb, sc, ida, idb, drained)) L.st = kIdle;
+		if (!post_step(L, pts, pa, pb, envelope, pairs, ID, pos, sc)) L.st = kIdle;
 	}
 }
 

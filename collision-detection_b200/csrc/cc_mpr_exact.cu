@@ -114,7 +114,6 @@ __device__ __forceinline__ Side side_of(const Shape<double> &s) {
 		o.fast = usual(s.Y.x) & usual(s.Y.y) & usual(s.Y.z);
 	} else if (s.type != BOX) {
 		o.fast = false;
-		if (s.type == TRIANGLEMESH) o.r0 = s.Z;
 	}
 	return o;
 }
@@ -123,7 +122,7 @@ __device__ __forceinline__ Side side_of(const Shape<double> &s) {
 __device__ __forceinline__ Shape<double> shape_of(const Side &s) {
 	Shape<double> o;
 	o.type = s.type;
-	o.X = s.X; o.Y = s.Y; o.Z = s.r0;
+	o.X = s.X; o.Y = s.Y;
 	o.r0 = s.r0; o.r1 = s.r1; o.r2 = s.r2;
 	return o;
 }
@@ -184,7 +183,7 @@ struct Pair {
 // or v12, v22, v32), read only when a contact is finished: in shared memory,
 // so that an iteration stores the new one with three stores instead of nine
 // selects among 18 registers.
-struct Points {
+struct LanePoints {
 	double *p;  // this lane's column of [3 vertices][3 coordinates][kNT]
 	__device__ __forceinline__ void put(int vertex, D3 a) const {
 		double *q = p + vertex * (3 * kNT);
@@ -223,7 +222,7 @@ __device__ __forceinline__ D3 trip(Pair &L, D3 w, bool refines, bool odd, uint32
 
 // A refinement's portal update (:240-311) with the new normal in L.n and the
 // support points p (this lane's) and p2 (its partner's).
-__device__ __forceinline__ void refine_update(Pair &L, D3 p, D3 p2, bool odd, const Points &pts) {
+__device__ __forceinline__ void refine_update(Pair &L, D3 p, D3 p2, bool odd, const LanePoints &pts) {
 	L.it++;
 	L.hit |= dotp(L.n, L.v1) >= 0.0;
 	const D3 v = sub(pick(odd, p, p2), pick(odd, p2, p));
@@ -245,7 +244,7 @@ __device__ __forceinline__ void refine_update(Pair &L, D3 p, D3 p2, bool odd, co
 
 // finish_refine (cc_mpr.cuh): the contact point; the normal stays in L.n.
 // Called by the lanes of `mask`.
-__device__ __forceinline__ void finish(Pair &L, const Points &pts, uint32_t mask) {
+__device__ __forceinline__ void finish(Pair &L, const LanePoints &pts, uint32_t mask) {
 	const D3 v1 = L.v1, v2 = L.v2, v3 = L.v3, v0 = L.v0, n = L.n;
 	double b0 = dotp(crossp(v1, v2), v3);
 	double b1 = dotp(crossp(v3, v2), v0);
@@ -268,7 +267,7 @@ __device__ __forceinline__ void finish(Pair &L, const Points &pts, uint32_t mask
 }
 
 // State update of the phases before and after the refinement.
-__device__ __forceinline__ void other_update(Pair &L, D3 p, D3 p2, bool odd, const Points &pts, float envelope,
+__device__ __forceinline__ void other_update(Pair &L, D3 p, D3 p2, bool odd, const LanePoints &pts, float envelope,
                                              const long long *pairs, const uint32_t *ID, const NpScratch &sc) {
 	const D3 v = sub(pick(odd, p, p2), pick(odd, p2, p));
 	const bool miss = dotp(v, L.n) <= 0.0;
@@ -355,7 +354,7 @@ __device__ __forceinline__ void start(Pair &L, uint32_t i, bool odd, uint32_t ma
 	const bool live = !bad & (act | act2) & (id != id2);  // :344-349
 	Shape<double> s;
 	s.type = SPHERE;
-	s.X = s.Y = s.Z = s.r0 = s.r1 = s.r2 = mk(0.0, 0.0, 0.0);
+	s.X = s.Y = s.r0 = s.r1 = s.r2 = mk(0.0, 0.0, 0.0);
 	if (live) s = load_shape<double>(sh, id, T, A, B, C, R, pos, rot, mk(0.0, 0.0, 0.0));
 	const int type2 = __shfl_xor_sync(mask, s.type, 1);
 	const D3 c = centre(s), c2 = shfl_partner(mask, c);
@@ -404,7 +403,7 @@ __global__ void __launch_bounds__(kNT, 6) k_mpr_exact(uint64_t P_cap, const unsi
 	uint64_t j = ((uint64_t)blockIdx.x * (kNT / 32) + (threadIdx.x >> 5)) * width + (lane >> 1);
 	const uint32_t batch = min((uint32_t)kBatch, width);
 	__shared__ double points[3 * 3 * kNT];
-	const Points pts = {points + threadIdx.x};
+	const LanePoints pts = {points + threadIdx.x};
 	Pair L;
 	L.st = kIdle;
 	bool fresh = true, drained = false;  // before the first fill; the queue is exhausted (warp-uniform)

@@ -33,7 +33,7 @@ namespace {
 constexpr int kNT = 64;  // MPR: few, long-running threads; small blocks spread them over all SMs
 
 template <class S>
-__global__ void __launch_bounds__(kNT) k_mpr(uint64_t P_cap, const unsigned long long *P_dev, uint64_t n,
+__global__ void __launch_bounds__(kNT, 6) k_mpr(uint64_t P_cap, const unsigned long long *P_dev, uint64_t n,
                                               const int32_t *__restrict__ T, const float *__restrict__ A,
                                               const float *__restrict__ B, const float *__restrict__ C,
                                               const float *__restrict__ R, const uint32_t *__restrict__ ID,
@@ -41,7 +41,7 @@ __global__ void __launch_bounds__(kNT) k_mpr(uint64_t P_cap, const unsigned long
                                               const float *__restrict__ pos, const float *__restrict__ rot,
                                               float envelope, const long long *__restrict__ pairs, NpScratch sc) {
 	pdl_begin();
-	mpr::run<S>(P_cap, P_dev, n, T, A, B, C, R, ID, nb, active, pos, rot, envelope, pairs, sc,
+	mpr::run<S, kNT>(P_cap, P_dev, n, T, A, B, C, R, ID, nb, active, pos, rot, envelope, pairs, sc,
 	                        sc.classes + 2 * kNpClasses);
 }
 
@@ -367,7 +367,7 @@ void launch_mpr(uint64_t P_cap, const unsigned long long *P_dev, uint64_t n, con
 	// pair starts at once (the kernel is latency-bound: its time is the
 	// longest pair's dependency chain); beyond that the queue balances
 	const uint64_t want = (Pe + kNT - 1) / kNT;
-	const unsigned grid = (unsigned)std::min<uint64_t>(std::max<uint64_t>(want, kNumSMs),
+	const unsigned grid = (unsigned)std::min<uint64_t>(std::max<uint64_t>(want, 2 * kNumSMs),
 	                                                   (uint64_t)kNumSMs * mpr_resident_blocks(precision));
 	if (precision == 2)
 		launch_pdl(k_mpr<float>, dim3(grid), dim3(kNT), 0, s, P_cap, P_dev, n, T, A, B, C, R, ID, nb, active, pos, rot, envelope, pairs,
