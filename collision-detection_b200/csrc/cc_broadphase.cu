@@ -1093,34 +1093,36 @@ __device__ __forceinline__ unsigned long long unpack_key(uint32_t v, uint32_t bu
 constexpr int kTinySeg = 8;    // buckets sorted by one thread with a bubble network in registers
 constexpr int kSmallSeg = 32;  // buckets sorted by one thread with a bitonic network in registers
 
-// Compare-exchange of two 64-bit keys held in registers (ascending).
-__device__ __forceinline__ void cx64(unsigned long long &x, unsigned long long &y) {
-	const unsigned long long a = x, b = y;
-	x = a < b ? a : b;
-	y = a < b ? b : a;
+// Compare-exchange of two keys held in registers (ascending).
+__device__ __forceinline__ void cx(uint32_t &x, uint32_t &y) {
+	const uint32_t a = x, b = y;
+	x = min(a, b);
+	y = max(a, b);
 }
 constexpr int kMidSeg = 1024;
 constexpr int kBigSeg = 16384;
 
-// One bucket of at most kSmallSeg 64-bit keys sorted by one thread in
-// registers: a bubble network up to kTinySeg keys, a bitonic network padded
-// to kSmallSeg above (one load and one store round trip either way).
-__device__ __forceinline__ void sort_thread_bucket(unsigned long long *__restrict__ out, uint64_t beg, uint64_t len) {
+// One bucket of at most kSmallSeg keys sorted by one thread in registers, on the
+// packed 32-bit keys: a bubble network up to kTinySeg keys, a bitonic network
+// padded to kSmallSeg above (one load and one store round trip either way).
+template <bool kPack>
+__device__ __forceinline__ void sort_thread_bucket(unsigned long long *__restrict__ out, uint64_t beg, uint64_t len,
+                                                   uint32_t a, KeyPack kp) {
 	if (len > 1 && len <= kTinySeg) {
-		unsigned long long v[kTinySeg];
+		uint32_t v[kTinySeg];
 #pragma unroll
-		for (int q = 0; q < kTinySeg; q++) v[q] = (uint64_t)q < len ? out[beg + q] : ~0ull;
+		for (int q = 0; q < kTinySeg; q++) v[q] = (uint64_t)q < len ? pack_key<kPack>(out[beg + q], kp) : 0xffffffffu;
 #pragma unroll
 		for (int r = 0; r < kTinySeg - 1; r++)
 #pragma unroll
-			for (int q = 0; q < kTinySeg - 1 - r; q++) cx64(v[q], v[q + 1]);
+			for (int q = 0; q < kTinySeg - 1 - r; q++) cx(v[q], v[q + 1]);
 #pragma unroll
 		for (int q = 0; q < kTinySeg; q++)
-			if ((uint64_t)q < len) out[beg + q] = v[q];
+			if ((uint64_t)q < len) out[beg + q] = unpack_key<kPack>(v[q], a, kp);
 	} else if (len > kTinySeg && len <= kSmallSeg) {
-		unsigned long long v[kSmallSeg];
+		uint32_t v[kSmallSeg];
 #pragma unroll
-		for (int q = 0; q < kSmallSeg; q++) v[q] = (uint64_t)q < len ? out[beg + q] : ~0ull;
+		for (int q = 0; q < kSmallSeg; q++) v[q] = (uint64_t)q < len ? pack_key<kPack>(out[beg + q], kp) : 0xffffffffu;
 #pragma unroll
 		for (int k = 2; k <= kSmallSeg; k <<= 1)
 #pragma unroll
@@ -1129,25 +1131,26 @@ __device__ __forceinline__ void sort_thread_bucket(unsigned long long *__restric
 				for (int i = 0; i < kSmallSeg; i++) {
 					const int l = i ^ j;
 					if (l > i) {
-						if ((i & k) == 0) cx64(v[i], v[l]);
-						else cx64(v[l], v[i]);
+						if ((i & k) == 0) cx(v[i], v[l]);
+						else cx(v[l], v[i]);
 					}
 				}
 #pragma unroll
 		for (int q = 0; q < kSmallSeg; q++)
-			if ((uint64_t)q < len) out[beg + q] = v[q];
+			if ((uint64_t)q < len) out[beg + q] = unpack_key<kPack>(v[q], a, kp);
 	}
 }
 
 // Sorts each owner bucket (all keys share the bucket's owners, n here is the
 // bucket count): <= 32 keys by one thread, loaded into registers at once and
-// sorted there by a static network on the 64-bit keys (a bubble network up to
+// sorted there by a static network on the packed keys (a bubble network up to
 // 8 keys, a bitonic network padded to 32 above); longer buckets are listed for
 // k_segsort_mid (<= 1024 keys, from the front of big_list) or k_segsort_big
 // (<= 16384, from the back), which sort the packed 32-bit keys (pack_key).
+template <bool kPack>
 __global__ void __launch_bounds__(kNT) k_segsort(uint64_t n, const unsigned long long *__restrict__ owner_off,
                                                   unsigned long long *__restrict__ out, uint32_t *big_list,
-                                                  uint64_t big_cap, DevStats *stats) {
+                                                  uint64_t big_cap, DevStats *stats, KeyPack kp) {
 	pdl_begin();
 	if (stats->np_n != stats->pairs) return;  // the pairs were not emitted (uniform over the grid)
 	const uint64_t a = (uint64_t)blockIdx.x * kNT + threadIdx.x;
@@ -1155,7 +1158,7 @@ __global__ void __launch_bounds__(kNT) k_segsort(uint64_t n, const unsigned long
 	if (a < n) {
 		const uint64_t beg = owner_off[a], end = owner_off[a + 1];
 		len = end - beg;
-		sort_thread_bucket(out, beg, len);
+		sort_thread_bucket<kPack>(out, beg, len, (uint32_t)a, kp);
 	}
 	const bool longer = len > kSmallSeg;
 	const uint32_t wmax = __reduce_max_sync(0xffffffffu, longer ? (uint32_t)min(len, (uint64_t)0xffffffffu) : 0u);
@@ -1466,18 +1469,22 @@ __global__ void __launch_bounds__(512) k_segsort_big(const DevStats *stats, uint
 // while other blocks still scan them), waits at one grid barrier, and sorts
 // the buckets: <= 32 keys per thread, 33..1024 per warp in registers,
 // 1025..kFusedSeg per block in shared memory. A longer bucket sets
-// kErrSegmentTooLong (the caller then sorts the whole list).
+// kErrSegmentTooLong (the caller then sorts the whole list). The grid is short
+// (128 blocks for 1M bodies) and latency-bound: 21 us there, under the MPR that
+// runs beside it; the bound of 64 registers leaves the MPR's blocks
+// their room.
 constexpr int kFusedNT = 256;
 constexpr int kFusedSeg = 4096;
 constexpr uint32_t kFusedBuckets = 8191;  // offsets + block-tier keys fit the default 48 KB of shared memory
 
 template <bool kPack>
-__global__ void __launch_bounds__(kFusedNT) k_owner_sort_fused(DevStats *stats, uint64_t pair_cap, uint64_t out_cap,
+__global__ void __launch_bounds__(kFusedNT, 4) k_owner_sort_fused(DevStats *stats, uint64_t pair_cap, uint64_t out_cap,
                                                              const unsigned long long *__restrict__ tmp,
                                                              const uint32_t *__restrict__ owner_count,
                                                              uint32_t *__restrict__ cursor, uint32_t nbk,
                                                              unsigned long long *__restrict__ out, int oshift,
                                                              KeyPack kp) {
+	pdl_trigger();  // (every block is resident: a cooperative launch)
 	extern __shared__ uint32_t fsm[];  // off[nbk + 1], then kFusedSeg keys of the block tier
 	__shared__ unsigned long long scan_sm[40];
 	uint32_t *off = fsm, *keys = fsm + nbk + 1;
@@ -1523,7 +1530,7 @@ __global__ void __launch_bounds__(kFusedNT) k_owner_sort_fused(DevStats *stats, 
 	uint32_t longest = 0;
 	for (uint64_t b = gt; b < nbk; b += step) {
 		const uint32_t beg = off[b], len = off[b + 1] - beg;
-		sort_thread_bucket(out, beg, len);
+		sort_thread_bucket<kPack>(out, beg, len, (uint32_t)b, kp);
 		longest = max(longest, len);
 	}
 	longest = __reduce_max_sync(0xffffffffu, longest);
@@ -1864,7 +1871,9 @@ void launch_owner_scatter(uint64_t out_cap, unsigned long long *out, const BpBuf
 
 void launch_segsort(uint64_t n, unsigned long long *out, const BpBuffers &b, cudaStream_t s) {
 	const uint64_t nbk = owner_buckets(n, b.owner_shift);
-	launch_pdl(k_segsort, dim3(blocks_for(nbk)), dim3(kNT), 0, s, nbk, b.owner_off, out, b.big_list, b.big_cap, b.stats);
+	const KeyPack kp{b.owner_shift, b.key_bits};
+	launch_pdl(kp.shift ? k_segsort<true> : k_segsort<false>, dim3(blocks_for(nbk)), dim3(kNT), 0, s, nbk, b.owner_off, out,
+	           b.big_list, b.big_cap, b.stats, kp);
 }
 
 void launch_segsort_mid(unsigned long long *out, const BpBuffers &b, cudaStream_t s) {

@@ -245,6 +245,9 @@ __device__ __forceinline__ void pdl_begin() {
 	asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 inline int pdl_mode() {
 	static const int m = [] {
 		const char *v = getenv("CC_PDL");
@@ -265,9 +268,10 @@ struct PdlScope {
 };
 inline bool pdl_enabled() { return t_pdl_call && pdl_mode() != 0; }
 
-template <class... KArgs, class... Args>
+// `always`: also above kPdlMaxBodies (CC_PDL=0 still turns it off).
+template <bool always = false, class... KArgs, class... Args>
 inline void launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args &&...args) {
-	if (!pdl_enabled()) {
+	if (!(always ? pdl_mode() != 0 : pdl_enabled())) {
 		kernel<<<grid, block, smem, s>>>(std::forward<Args>(args)...);
 		return;
 	}

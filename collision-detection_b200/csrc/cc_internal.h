@@ -377,18 +377,20 @@ constexpr unsigned kNpCoopBlocks = 148 * 8;
 // pair is reported as no contact. precision: 0 exact (the reference's FP64
 // arithmetic), 1 fp64 (pair-local frame), 2 mixed (FP32 support maps).
 // P_cap: host bound on the pair count; with P_dev the count is min(P_cap,
-// *P_dev), read on the device. P_hint sizes the persistent grid.
+// *P_dev), read on the device. P_hint sizes the persistent grid. beside (exact
+// mode): the launch before it on s is the fused owner sort; the two run side by
+// side, and what follows on s follows both.
 void launch_mpr(uint64_t P_cap, const unsigned long long *P_dev, uint64_t n, const int32_t *T, const float *A,
                 const float *B, const float *C, const float *R, const uint32_t *ID, uint64_t nb,
                 const uint8_t *active, const float *pos, const float *rot, float envelope, const long long *pairs,
-                const NpScratch &sc, int precision, uint64_t P_hint, cudaStream_t s);
+                const NpScratch &sc, int precision, uint64_t P_hint, cudaStream_t s, bool beside = false);
 // The exact variant lives in its own -fmad=false translation unit.
 // Blocks of the exact MPR kernel resident per SM.
 int mpr_exact_resident_blocks();
 void launch_mpr_exact(unsigned grid, uint64_t P_cap, const unsigned long long *P_dev, uint64_t n, const int32_t *T,
                       const float *A, const float *B, const float *C, const float *R, const uint32_t *ID, uint64_t nb,
                       const uint8_t *active, const float *pos, const float *rot, float envelope,
-                      const long long *pairs, const NpScratch &sc, cudaStream_t s);
+                      const long long *pairs, const NpScratch &sc, cudaStream_t s, bool beside);
 void launch_np_compact(uint64_t P_cap, const unsigned long long *P_dev, const NpScratch &sc, long long *pairs,
                        float *norm, float *cpta, float *cptb, float *depth, int32_t *bids,
                        unsigned long long *contacts_out, uint64_t P_hint, cudaStream_t s);

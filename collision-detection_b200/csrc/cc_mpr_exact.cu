@@ -389,8 +389,12 @@ __global__ void __launch_bounds__(kNT, 6) k_mpr_exact(uint64_t P_cap, const unsi
                                                     uint64_t nb, const uint8_t *__restrict__ active,
                                                     const float *__restrict__ pos, const float *__restrict__ rot,
                                                     float envelope, const long long *__restrict__ pairs,
-                                                    NpScratch sc) {
-	pdl_begin();
+                                                    NpScratch sc, int beside) {
+	// beside: the kernel before is the pair sort, whose blocks are all resident
+	// once this one starts and which shares no data with it: they run side by
+	// side, and this kernel ends after it (below)
+	if (!beside) pdl_wait();
+	pdl_trigger();
 	const uint64_t P = P_dev ? min(P_cap, (uint64_t)*P_dev) : P_cap;
 	uint32_t *queue = sc.classes + 2 * kNpClasses;
 	const uint32_t lane = threadIdx.x & 31, lt = (1u << lane) - 1u;
@@ -464,6 +468,7 @@ __global__ void __launch_bounds__(kNT, 6) k_mpr_exact(uint64_t P_cap, const unsi
 			}
 		}
 	}
+	if (beside) pdl_wait();
 }
 }  // namespace
 
@@ -479,8 +484,13 @@ int mpr_exact_resident_blocks() {
 void launch_mpr_exact(unsigned grid, uint64_t P_cap, const unsigned long long *P_dev, uint64_t n, const int32_t *T,
                       const float *A, const float *B, const float *C, const float *R, const uint32_t *ID, uint64_t nb,
                       const uint8_t *active, const float *pos, const float *rot, float envelope,
-                      const long long *pairs, const NpScratch &sc, cudaStream_t s) {
-	launch_pdl(k_mpr_exact, dim3(grid), dim3(kNT), 0, s, P_cap, P_dev, n, T, A, B, C, R, ID, nb, active, pos, rot, envelope, pairs, sc);
+                      const long long *pairs, const NpScratch &sc, cudaStream_t s, bool beside) {
+	if (beside)
+		launch_pdl<true>(k_mpr_exact, dim3(grid), dim3(kNT), 0, s, P_cap, P_dev, n, T, A, B, C, R, ID, nb, active, pos, rot,
+		                 envelope, pairs, sc, 1);
+	else
+		launch_pdl(k_mpr_exact, dim3(grid), dim3(kNT), 0, s, P_cap, P_dev, n, T, A, B, C, R, ID, nb, active, pos, rot, envelope,
+		           pairs, sc, 0);
 }
 
 }  // namespace cc

@@ -338,7 +338,7 @@ unsigned np_coop_max_blocks() {
 void launch_mpr(uint64_t P_cap, const unsigned long long *P_dev, uint64_t n, const int32_t *T, const float *A,
                 const float *B, const float *C, const float *R, const uint32_t *ID, uint64_t nb,
                 const uint8_t *active, const float *pos, const float *rot, float envelope, const long long *pairs,
-                const NpScratch &sc, int precision, uint64_t P_hint, cudaStream_t s) {
+                const NpScratch &sc, int precision, uint64_t P_hint, cudaStream_t s, bool beside) {
 	if (!P_cap) return;
 	const uint64_t Pe = std::min<uint64_t>(P_hint ? P_hint : P_cap, P_cap);
 	if (precision == 0) {
@@ -352,7 +352,7 @@ void launch_mpr(uint64_t P_cap, const unsigned long long *P_dev, uint64_t n, con
 		if (!sc.pre_zeroed) cudaMemsetAsync(sc.classes, 0, (2 * kNpClasses + 1) * sizeof(uint32_t), s);
 		const uint64_t want = std::max<uint64_t>((Pe + kNT / 2 - 1) / (kNT / 2), 2 * kNumSMs);
 		launch_mpr_exact((unsigned)std::min<uint64_t>(want, (uint64_t)kNumSMs * mpr_exact_resident_blocks()), P_cap, P_dev, n,
-		                 T, A, B, C, R, ID, nb, active, pos, rot, envelope, pairs, sc, s);
+		                 T, A, B, C, R, ID, nb, active, pos, rot, envelope, pairs, sc, s, beside);
 		return;
 	}
 	{  // group the pairs by shape-type combination; the last word is the work queue
