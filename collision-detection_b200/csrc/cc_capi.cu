@@ -123,6 +123,7 @@ struct cc_ctx {
 	GridParams call_gp{};  // gp as this call's search uses it (set by prepare)
 	int chain_wait = 0;  // calls on sorted cells left before the chains are tried again
 	uint64_t last_E = 0, last_P = 0, last_tmp = 0, last_mask = 0;  // last_tmp: pairs that went through pairs_tmp
+	bool sized = false;  // a pass has set these
 	int last_dim[3] = {0, 0, 0};
 	// owner buckets of the pair sort (BpBuffers::owner_shift / key_bits), chosen
 	// per call from the last call's pairs per body
@@ -430,6 +431,9 @@ cc_status direct_prepare(cc_ctx *c) {
 // Pairs of a pass that went through the unsorted scratch list.
 uint64_t unsorted_pairs(const DevStats &st, bool direct) { return direct ? st.tmp_pairs : st.pairs; }
 
+// Room to ask for where the last call used `used` and there is room for `room`.
+uint64_t with_slack(uint64_t used, uint64_t room) { return used + used / 16 <= room ? room : used + used / 4; }
+
 // Allocates the n-dependent broadphase scratch and, if np_cap > 0, the
 // narrowphase scratch for np_cap pairs. Buffers only grow; every public call
 // ends with a synchronize, so nothing in flight uses a buffer replaced here.
@@ -454,11 +458,13 @@ cc_status prepare(cc_ctx *c, uint64_t n, uint64_t np_cap, uint64_t g_override = 
 	CC_TRY(ensure(c, c->cell_start, sizeof(uint32_t) * (c->gp.g_max + 1)));
 	CC_TRY(ensure(c, c->owner_count, sizeof(uint32_t) * std::max<uint64_t>(n, 1)));
 	CC_TRY(ensure(c, c->owner_off, sizeof(unsigned long long) * (n + 1)));
-	const uint64_t e_guess = std::max<uint64_t>(c->last_E + c->last_E / 4, 2 * n + 1024);
+	// Small cells (chained search) hold a body 2.4 to 2.8 times. Room that is there
+	// is enough while a sixteenth of the last call's count is left.
+	const uint64_t e_guess = std::max<uint64_t>(with_slack(c->last_E, c->entries.bytes / (2 * sizeof(float4))), (c->chain ? 3 : 2) * n + 1024);
 	CC_TRY(ensure(c, c->entries, 2 * sizeof(float4) * e_guess));
 	if (c->chain) CC_TRY(ensure(c, c->extra, sizeof(uint32_t) * (c->entries.bytes / (2 * sizeof(float4)))));
 	if (c->direct) CC_TRY(direct_prepare(c));
-	const uint64_t p_guess = std::max<uint64_t>(c->last_tmp + c->last_tmp / 4, n / 4 + 1024);
+	const uint64_t p_guess = std::max<uint64_t>(with_slack(c->last_tmp, c->pairs_tmp.bytes / sizeof(unsigned long long)), n / 4 + 1024);
 	CC_TRY(ensure(c, c->pairs_tmp, sizeof(unsigned long long) * p_guess));
 	c->st_words[0] = std::max<uint64_t>(c->st_words[0], status_words_for(c->gp.g_max));
 	c->st_words[1] = std::max<uint64_t>(c->st_words[1], status_words_for(n + 1));
@@ -515,7 +521,10 @@ uint64_t pow2ceil(uint64_t v) {
 	return p;
 }
 uint64_t hint_E(const cc_ctx *c, uint64_t n) { return pow2ceil(std::max<uint64_t>(c->last_E, n)); }
-uint64_t hint_P(const cc_ctx *c) { return pow2ceil(std::max<uint64_t>(c->last_P, 1)); }
+// Before the first pass the guess of choose_owner_shift: a grid
+// for one pair would leave all of the first pass's pairs to it (1M bodies: a
+// compaction of 6.7 ms).
+uint64_t hint_P(const cc_ctx *c, uint64_t n) { return pow2ceil(std::max<uint64_t>(c->sized ? c->last_P : n / 4, 1)); }
 
 // Shift (unless done) .. pair test: needs stats zeroed and the plan from the
 // bounds pass.
@@ -569,7 +578,7 @@ void enqueue_emit(cc_ctx *c, uint64_t n, unsigned long long *out, uint64_t out_c
 	BpBuffers b = bp_buffers(c);
 	if (c->fused_now) {
 		StageMark m(c, ST_SEGSORT, s);
-		launch_owner_sort_fused(n, out_cap, out, hint_P(c), b, s);
+		launch_owner_sort_fused(n, out_cap, out, hint_P(c, n), b, s);
 		c->launches += 1;
 		return;
 	}
@@ -602,12 +611,12 @@ void enqueue_np(cc_ctx *c, const NpArgs &a, uint64_t P_cap, const unsigned long 
 		StageMark m(c, ST_MPR, s);
 		launch_mpr(P_cap, P_dev, a.n, a.T, a.A, a.B, a.C, a.R, a.ID, a.nb, a.active, a.pos, a.rot, a.envelope,
 		           reinterpret_cast<const long long *>(a.pairs), sc, c->np_precision,
-		           P_dev ? hint_P(c) : P_cap, s);
+		           P_dev ? hint_P(c, a.n) : P_cap, s);
 	}
 	{
 		StageMark m(c, ST_NP_COMPACT, s);
 		launch_np_compact(P_cap, P_dev, sc, reinterpret_cast<long long *>(a.pairs), a.norm, a.cpta, a.cptb, a.depth,
-		                  a.bids, &ptr<DevStats>(c->stats)->contacts, P_dev ? hint_P(c) : P_cap, s);
+		                  a.bids, &ptr<DevStats>(c->stats)->contacts, P_dev ? hint_P(c, a.n) : P_cap, s);
 	}
 	c->launches += c->np_precision == CC_NP_EXACT ? 2 : 3;  // class grouping (fast modes), MPR, compaction
 }
@@ -642,7 +651,7 @@ cc_status enqueue_sort_and_np_overlapped(cc_ctx *c, uint64_t n, const NpArgs &a,
 		StageMark m(c, ST_MPR, t);
 		launch_mpr(std::min<uint64_t>(pairs_cap, b.pair_cap), &d->pairs, a.n, a.T, a.A, a.B, a.C, a.R, a.ID, a.nb,
 		           a.active, a.pos, a.rot, a.envelope, reinterpret_cast<const long long *>(b.pairs_tmp), sc,
-		           c->np_precision, hint_P(c), t, beside);
+		           c->np_precision, hint_P(c, n), t, beside);
 	}
 	c->launches += c->np_precision == CC_NP_EXACT ? 1 : 2;  // class grouping (fast modes), MPR
 	if (!beside) {
@@ -658,7 +667,7 @@ cc_status enqueue_sort_and_np_overlapped(cc_ctx *c, uint64_t n, const NpArgs &a,
 	{
 		StageMark m(c, ST_NP_COMPACT, s);
 		launch_np_compact_sorted(pairs_cap, &d->np_n, sc, reinterpret_cast<long long *>(a.pairs), b.pairs_tmp,
-		                         a.norm, a.cpta, a.cptb, a.depth, a.bids, &d->contacts, hint_P(c), s);
+		                         a.norm, a.cpta, a.cptb, a.depth, a.bids, &d->contacts, hint_P(c, n), s);
 	}
 	c->launches += 1;
 	return CC_OK;
@@ -666,13 +675,13 @@ cc_status enqueue_sort_and_np_overlapped(cc_ctx *c, uint64_t n, const NpArgs &a,
 
 // Whether this call's narrowphase is overlapped with the pair sort (outputs of
 // at most 2^24 pairs), with the stream, events and contact hash it needs.
-cc_status overlap_prepare(cc_ctx *c, uint64_t pairs_cap, bool &ov) {
+cc_status overlap_prepare(cc_ctx *c, uint64_t n, uint64_t pairs_cap, bool &ov) {
 	ov = c->np_overlap && !c->direct && pairs_cap > 0 && pairs_cap <= ((uint64_t)1 << 24);
 	if (!ov) return CC_OK;
 	if (!c->np_stream) CC_CUDA(c, cudaStreamCreateWithFlags(&c->np_stream, cudaStreamNonBlocking));
 	if (!c->ev_fork) CC_CUDA(c, cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming));
 	if (!c->ev_join) CC_CUDA(c, cudaEventCreateWithFlags(&c->ev_join, cudaEventDisableTiming));
-	c->np_hslots = pow2ceil(std::max<uint64_t>(4 * std::min<uint64_t>(hint_P(c), pairs_cap), 4096));
+	c->np_hslots = pow2ceil(std::max<uint64_t>(4 * std::min<uint64_t>(hint_P(c, n), pairs_cap), 4096));
 	CC_TRY(ensure(c, c->np_hkeys, sizeof(unsigned long long) * c->np_hslots));
 	return ensure(c, c->np_hvals, sizeof(uint32_t) * c->np_hslots);
 }
@@ -792,6 +801,7 @@ cc_status sort_fallback(cc_ctx *c, uint64_t n, uint64_t P, unsigned long long *o
 void remember(cc_ctx *c) {
 	c->last_E = c->h_stats->entries;
 	c->last_P = c->h_stats->pairs;
+	c->sized = true;
 	c->last_tmp = unsorted_pairs(*c->h_stats, c->direct);
 	c->last_mask = c->h_stats->mask_words;
 	c->last_dense = c->h_stats->dense_items;
@@ -912,7 +922,7 @@ cc_status collide_enqueue(cc_ctx *c, const cc_scene &sc, int gx, int gy, int gz,
 	PdlScope pdl_(n);
 	CC_TRY(prepare(c, n, pairs_cap));
 	bool ov;
-	CC_TRY(overlap_prepare(c, pairs_cap, ov));
+	CC_TRY(overlap_prepare(c, n, pairs_cap, ov));
 	DevStats *d = ptr<DevStats>(c->stats);
 	const int grid[3] = {gx, gy, gz};
 	unsigned long long *out = reinterpret_cast<unsigned long long *>(pairs);
@@ -960,7 +970,7 @@ cc_status collide_enqueue(cc_ctx *c, const cc_scene &sc, int gx, int gy, int gz,
 		uint64_t hslots;
 	} k;
 	memset(&k, 0, sizeof(k));
-	k.n = n; k.nb = sc.nb; k.pairs_cap = pairs_cap; k.hE = hint_E(c, n); k.hP = hint_P(c); k.gen = c->buf_gen;
+	k.n = n; k.nb = sc.nb; k.pairs_cap = pairs_cap; k.hE = hint_E(c, n); k.hP = hint_P(c, n); k.gen = c->buf_gen;
 	for (int r = 0; r < 3; r++) k.st[r] = c->st_words[r];
 	const void *ps[18] = {sc.T, sc.A, sc.B, sc.C, sc.R, sc.ID, sc.active, sc.body_pos, sc.body_rot, aabb,
 	                      pairs, norm, cpta, cptb, depth, bids, nullptr, nullptr};
@@ -1130,6 +1140,7 @@ cc_status collide_verlet(cc_ctx *c, const cc_scene &sc, int gx, int gy, int gz, 
 		c->inc_allocs = c->v_ref.allocs + c->v_cand.allocs;
 		const uint64_t P = c->h_stats->pairs;
 		c->last_P = c->last_tmp = P;
+		c->sized = true;
 		*n_pairs = P;
 		if (P > pairs_cap)
 			return set_err(c, CC_ERR_CAPACITY, "pair list needs %llu entries, capacity %llu", (unsigned long long)P,
@@ -1601,7 +1612,7 @@ cc_status batch_impl(cc_ctx *c, const cc_batch *bt, int gx, int gy, int gz, floa
 	const uint64_t pairs_cap = res->pairs_cap;
 	CC_TRY(prepare(c, n, pairs_cap, std::max<uint64_t>(g_total, 1)));
 	bool ov;
-	CC_TRY(overlap_prepare(c, pairs_cap, ov));
+	CC_TRY(overlap_prepare(c, n, pairs_cap, ov));
 	CC_TRY(ensure(c, c->b_scene_of, sizeof(uint32_t) * n));
 	CC_TRY(ensure(c, c->b_gid, sizeof(uint32_t) * n));
 	CC_TRY(ensure(c, c->b_sst, sizeof(SceneStats) * S));
@@ -1683,7 +1694,7 @@ cc_status batch_impl(cc_ctx *c, const cc_batch *bt, int gx, int gy, int gz, floa
 		uint64_t hslots;
 	} k;
 	memset(&k, 0, sizeof(k));
-	k.n = n; k.nb = sc.nb; k.S = S; k.pairs_cap = pairs_cap; k.hE = hint_E(c, n); k.hP = hint_P(c);
+	k.n = n; k.nb = sc.nb; k.S = S; k.pairs_cap = pairs_cap; k.hE = hint_E(c, n); k.hP = hint_P(c, n);
 	k.gen = c->buf_gen;
 	for (int r = 0; r < 3; r++) k.st[r] = c->st_words[r];
 	const void *ps[18] = {sc.T, sc.A, sc.B, sc.C, sc.R, sc.ID, sc.active, sc.body_pos, sc.body_rot, res->aabb,
