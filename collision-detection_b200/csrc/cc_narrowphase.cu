@@ -17,7 +17,7 @@
 //  2 mixed  (k_mpr<float>): as fp64 with FP32 support maps.
 //
 // k_np_classes: the pairs grouped by shape-type class (counting sort), and
-// k_np_compact_coop: the stable hit-first ordering of :580-593
+// k_np_compact: the stable hit-first ordering of :580-593
 // (thrust::sort_by_key on the 0/1 flag) as a scan + scatter, the pair keys
 // permuted the same way; each is one cooperative launch with a grid barrier.
 #include <algorithm>
@@ -126,77 +126,76 @@ __global__ void __launch_bounds__(kCoopNT) k_np_classes(uint64_t P_cap, const un
 	}
 }
 
-// Hit-first stable compaction as one cooperative launch: block b owns the
-// contiguous chunk b of the flags; it counts its hits, a grid barrier, then it
-// adds the counts of the blocks before it and scans its chunk tile by tile,
-// writing the exclusive positions (pos, pos[P] = total) and the outputs.
-__device__ __forceinline__ void compact_one(uint64_t i, uint64_t P, const NpScratch &sc, long long *__restrict__ pairs,
-                                            float *__restrict__ norm, float *__restrict__ cpta,
-                                            float *__restrict__ cptb, float *__restrict__ depth,
-                                            int32_t *__restrict__ bids, uint64_t before, uint64_t nh);
+// ---------------------------------------------------------------- compaction
+// Hit-first stable compaction in one cooperative launch: block b owns the contiguous chunk b
+// of the results; it counts its hits, a barrier over the grid, then it adds the
+// counts of the blocks before it and ranks its chunk's hits tile by tile. A pass's
+// list is short, so all of it is latency: chains of dependent loads, the barrier,
+// the launch. Where a chunk is one tile (the grids below make it so) every thread
+// has its row in registers before the barrier and only writes behind it, and the
+// block's sums take two block barriers. A step of 1M mixed shapes (25K pairs) 191.5
+// -> 181.4 us, 130K 105 -> 97, a batch of 64 285 -> 278, 500K stepping 158 -> 150.
+// (As one cluster of 16 blocks, with its cheaper barrier: up to 1.5 us less below
+// 16K pairs, 9 more at 25K.)
 
-__global__ void __launch_bounds__(kCoopNT) k_np_compact_coop(uint64_t P_cap, const unsigned long long *P_dev,
-                                                              NpScratch sc, long long *__restrict__ pairs,
-                                                              float *__restrict__ norm, float *__restrict__ cpta,
-                                                              float *__restrict__ cptb, float *__restrict__ depth,
-                                                              int32_t *__restrict__ bids,
-                                                              unsigned long long *contacts_out) {
-	__shared__ unsigned long long sm[40];
-	__shared__ unsigned long long s_pre, s_total;
-	const uint64_t P = P_dev ? min(P_cap, (uint64_t)*P_dev) : P_cap;
-	const uint64_t chunk = (P + gridDim.x - 1) / gridDim.x;
-	const uint64_t c0 = min((uint64_t)blockIdx.x * chunk, P), c1 = min(c0 + chunk, P);
-	unsigned long long cnt = 0;
-	for (uint64_t i = c0 + threadIdx.x; i < c1; i += kCoopNT) cnt += sc.flag[i] ? 1ull : 0ull;
-	unsigned long long tot;
-	block_excl_scan<unsigned long long, kCoopNT>(cnt, sm, &tot);
-	if (threadIdx.x == 0) sc.block_sums[blockIdx.x] = tot;
-	grid_barrier(reinterpret_cast<GridBarrier *>(sc.bar_compact), sc.err);
-	// prefix of this block and the grand total, from the per-block counts
-	unsigned long long pre = 0, all = 0;
-	for (uint32_t b = threadIdx.x; b < gridDim.x; b += kCoopNT) {
-		const unsigned long long v = __ldcg(&sc.block_sums[b]);
-		all += v;
-		if (b < blockIdx.x) pre += v;
+// Sums of a and b over the block, in every thread (sm: 64 words).
+__device__ __forceinline__ void block_sum2(unsigned long long &a, unsigned long long &b, unsigned long long *sm) {
+	constexpr int NW = kCoopNT / 32;
+	const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+	for (int d = 16; d; d >>= 1) {
+		a += __shfl_xor_sync(0xffffffffu, a, d);
+		b += __shfl_xor_sync(0xffffffffu, b, d);
 	}
-	{
-		unsigned long long t1, t2;
-		const unsigned long long p0 = block_excl_scan<unsigned long long, kCoopNT>(pre, sm, &t1);
-		const unsigned long long a0 = block_excl_scan<unsigned long long, kCoopNT>(all, sm, &t2);
-		(void)p0;
-		(void)a0;
-		if (threadIdx.x == 0) {
-			s_pre = t1;
-			s_total = t2;
-		}
+	if (l == 0) {
+		sm[w] = a;
+		sm[32 + w] = b;
 	}
 	__syncthreads();
-	unsigned long long run = s_pre;
-	const unsigned long long nh = s_total;
-	if (blockIdx.x == 0 && threadIdx.x == 0) {
-		sc.pos[P] = nh;
-		if (contacts_out) *contacts_out = nh;
+	a = l < NW ? sm[l] : 0ull;
+	b = l < NW ? sm[32 + l] : 0ull;
+	for (int d = 16; d; d >>= 1) {
+		a += __shfl_xor_sync(0xffffffffu, a, d);
+		b += __shfl_xor_sync(0xffffffffu, b, d);
 	}
-	for (uint64_t t0 = c0; t0 < c1; t0 += kCoopNT) {
-		const uint64_t i = t0 + threadIdx.x;
-		const unsigned long long f = (i < c1 && sc.flag[i]) ? 1ull : 0ull;
-		unsigned long long tile_total;
-		const unsigned long long ex = block_excl_scan<unsigned long long, kCoopNT>(f, sm, &tile_total);
-		if (i < c1) {
-			const uint64_t before = run + ex;
-			sc.pos[i] = before;
-			compact_one(i, P, sc, pairs, norm, cpta, cptb, depth, bids, before, nh);
-		}
-		run += tile_total;
-	}
+	__syncthreads();
 }
 
-// The overlapped narrowphase's compaction (one cooperative launch): the MPR
-// ran on the unsorted pairs, so each sorted key finds its result through the
-// contact hash. Phase 1: block b copies its chunk of sorted keys to `tmp`,
-// looks each one up and counts its hits; grid barrier; phase 2: it adds the
-// counts of the blocks before it and writes the hit-first order and the
-// contacts, as k_np_compact_coop does for results in sorted order.
+// Hits of the block's threads before this one, and of the block (sm: 32 words).
+__device__ __forceinline__ uint32_t block_rank(bool f, uint32_t *sm, uint32_t &total) {
+	constexpr int NW = kCoopNT / 32;
+	const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+	const uint32_t m = __ballot_sync(0xffffffffu, f);
+	if (l == 0) sm[w] = __popc(m);
+	__syncthreads();
+	const uint32_t v = l < NW ? sm[l] : 0u;
+	total = __reduce_add_sync(0xffffffffu, v);
+	const uint32_t r = __reduce_add_sync(0xffffffffu, l < w ? v : 0u) + __popc(m & ((1u << l) - 1u));
+	__syncthreads();
+	return r;
+}
+
+// One result row.
+struct ContactRow {
+	float v[10];
+	int32_t ida, idb;
+};
+__device__ __forceinline__ ContactRow load_row(const NpScratch &sc, uint64_t t) {
+	ContactRow r;
+#pragma unroll
+	for (int d = 0; d < 3; d++) {
+		r.v[d] = sc.norm[3 * t + d];
+		r.v[3 + d] = sc.pa[3 * t + d];
+		r.v[6 + d] = sc.pb[3 * t + d];
+	}
+	r.v[9] = sc.depth[t];
+	r.ida = sc.ids[2 * t];
+	r.idb = sc.ids[2 * t + 1];
+	return r;
+}
+
+constexpr uint32_t kNoHit = 0xffffffffu;
+
+// Contact hash: the row of a pair's result, kNoHit where it is no contact.
 __device__ __forceinline__ uint32_t hash_find(const NpScratch &sc, unsigned long long key) {
 	const unsigned long long tag = key + 1ull;
 	uint64_t h = (tag * 0x9E3779B97F4A7C15ull) >> 20;
@@ -205,96 +204,95 @@ __device__ __forceinline__ uint32_t hash_find(const NpScratch &sc, unsigned long
 		if (v == tag) return __ldcg(&sc.hvals[h & sc.hmask]);
 		if (v == 0ull) break;
 	}
-	return 0xffffffffu;
+	return kNoHit;
 }
 
-__global__ void __launch_bounds__(kCoopNT) k_np_compact_sorted(uint64_t P_cap, const unsigned long long *P_dev,
-                                                                NpScratch sc, long long *__restrict__ pairs,
-                                                                unsigned long long *__restrict__ tmp,
-                                                                float *__restrict__ norm, float *__restrict__ cpta,
-                                                                float *__restrict__ cptb, float *__restrict__ depth,
-                                                                int32_t *__restrict__ bids,
-                                                                unsigned long long *contacts_out) {
-	__shared__ unsigned long long sm[40];
-	__shared__ unsigned long long s_pre, s_total;
+// kSorted: the MPR ran on the unsorted pairs (overlapped with their sort) and each
+// sorted key in `pairs` finds its result through the contact hash; else results
+// and sc.pairs are in pair order. tmp: the sorted keys of chunks of several tiles.
+template <bool kSorted>
+__global__ void __launch_bounds__(kCoopNT) k_np_compact(uint64_t P_cap, const unsigned long long *P_dev, NpScratch sc,
+                                                   long long *__restrict__ pairs, unsigned long long *__restrict__ tmp,
+                                                   float *__restrict__ norm, float *__restrict__ cpta,
+                                                   float *__restrict__ cptb, float *__restrict__ depth,
+                                                   int32_t *__restrict__ bids, unsigned long long *contacts_out) {
+	__shared__ unsigned long long sm[64];
 	const uint64_t P = P_dev ? min(P_cap, (uint64_t)*P_dev) : P_cap;
 	const uint64_t chunk = (P + gridDim.x - 1) / gridDim.x;
 	const uint64_t c0 = min((uint64_t)blockIdx.x * chunk, P), c1 = min(c0 + chunk, P);
-	unsigned long long cnt = 0;
+	const bool one = chunk <= kCoopNT;
+	unsigned long long cnt = 0, unused = 0;
+	unsigned long long key = 0;
+	uint64_t t = kNoHit;
+	ContactRow row = {};
 	for (uint64_t i = c0 + threadIdx.x; i < c1; i += kCoopNT) {
-		const unsigned long long key = (unsigned long long)pairs[i];
-		tmp[i] = key;
-		const uint32_t t = hash_find(sc, key);
-		sc.order[i] = t;
-		cnt += t != 0xffffffffu ? 1ull : 0ull;
+		key = kSorted ? (unsigned long long)pairs[i] : sc.pairs[i];
+		bool hit;
+		if constexpr (kSorted) {
+			t = hash_find(sc, key);
+			hit = t != kNoHit;
+			if (!one) {
+				tmp[i] = key;
+				sc.order[i] = (uint32_t)t;
+			}
+		} else {
+			hit = sc.flag[i] != 0;
+			t = hit ? i : (uint64_t)kNoHit;
+		}
+		if (one && hit) row = load_row(sc, t);
+		cnt += hit ? 1ull : 0ull;
 	}
-	unsigned long long tot;
-	block_excl_scan<unsigned long long, kCoopNT>(cnt, sm, &tot);
-	if (threadIdx.x == 0) sc.block_sums[blockIdx.x] = tot;
+	bool hit = kSorted ? t != kNoHit : cnt != 0;  // one tile
+	block_sum2(cnt, unused, sm);
+	if (threadIdx.x == 0) sc.block_sums[blockIdx.x] = cnt;
 	grid_barrier(reinterpret_cast<GridBarrier *>(sc.bar_compact), sc.err);
-	{
-		unsigned long long pre = 0, all = 0, t1, t2;
-		for (uint32_t b = threadIdx.x; b < gridDim.x; b += kCoopNT) {
-			const unsigned long long v = __ldcg(&sc.block_sums[b]);
-			all += v;
-			if (b < blockIdx.x) pre += v;
-		}
-		block_excl_scan<unsigned long long, kCoopNT>(pre, sm, &t1);
-		block_excl_scan<unsigned long long, kCoopNT>(all, sm, &t2);
-		if (threadIdx.x == 0) {
-			s_pre = t1;
-			s_total = t2;
-		}
-		__syncthreads();
+	// hits before this block's, and all, from the per-block counts
+	unsigned long long run = 0, nh = 0;
+	for (uint32_t b = threadIdx.x; b < gridDim.x; b += kCoopNT) {
+		const unsigned long long v = __ldcg(&sc.block_sums[b]);
+		nh += v;
+		if (b < blockIdx.x) run += v;
 	}
-	unsigned long long run = s_pre;
-	const unsigned long long nh = s_total;
-	if (blockIdx.x == 0 && threadIdx.x == 0 && contacts_out) *contacts_out = nh;
+	block_sum2(run, nh, sm);
+	if (blockIdx.x == 0 && threadIdx.x == 0) {
+		if (!kSorted) sc.pos[P] = nh;
+		if (contacts_out) *contacts_out = nh;
+	}
 	for (uint64_t t0 = c0; t0 < c1; t0 += kCoopNT) {
 		const uint64_t i = t0 + threadIdx.x;
-		const uint32_t t = i < c1 ? sc.order[i] : 0xffffffffu;
-		const unsigned long long f = t != 0xffffffffu ? 1ull : 0ull;
-		unsigned long long tile_total;
-		const unsigned long long ex = block_excl_scan<unsigned long long, kCoopNT>(f, sm, &tile_total);
-		if (i < c1) {
-			const uint64_t before = run + ex;
-			if (f) {
-				const uint64_t j = before;
-				pairs[j] = (long long)tmp[i];
-				for (int d = 0; d < 3; d++) {
-					norm[3 * j + d] = sc.norm[3 * (uint64_t)t + d];
-					cpta[3 * j + d] = sc.pa[3 * (uint64_t)t + d];
-					cptb[3 * j + d] = sc.pb[3 * (uint64_t)t + d];
-				}
-				depth[j] = sc.depth[t];
-				bids[2 * j] = sc.ids[2 * (uint64_t)t];
-				bids[2 * j + 1] = sc.ids[2 * (uint64_t)t + 1];
+		if (!one && i < c1) {
+			if constexpr (kSorted) {
+				key = tmp[i];
+				t = sc.order[i];
+				hit = t != kNoHit;
 			} else {
-				pairs[nh + (i - before)] = (long long)tmp[i];
+				key = sc.pairs[i];
+				t = i;
+				hit = sc.flag[i] != 0;
+			}
+			if (hit) row = load_row(sc, t);
+		}
+		uint32_t tile_total;
+		const uint32_t r = block_rank(i < c1 && hit, reinterpret_cast<uint32_t *>(sm), tile_total);
+		if (i < c1) {
+			const uint64_t j = run + r;
+			if (!kSorted) sc.pos[i] = j;
+			if (hit) {
+				pairs[j] = (long long)key;
+#pragma unroll
+				for (int d = 0; d < 3; d++) {
+					norm[3 * j + d] = row.v[d];
+					cpta[3 * j + d] = row.v[3 + d];
+					cptb[3 * j + d] = row.v[6 + d];
+				}
+				depth[j] = row.v[9];
+				bids[2 * j] = row.ida;
+				bids[2 * j + 1] = row.idb;
+			} else {
+				pairs[nh + (i - j)] = (long long)key;
 			}
 		}
 		run += tile_total;
-	}
-}
-
-__device__ __forceinline__ void compact_one(uint64_t i, uint64_t P, const NpScratch &sc, long long *__restrict__ pairs,
-                                            float *__restrict__ norm, float *__restrict__ cpta,
-                                            float *__restrict__ cptb, float *__restrict__ depth,
-                                            int32_t *__restrict__ bids, uint64_t before, uint64_t nh) {
-	(void)P;
-	if (sc.flag[i]) {
-		const uint64_t j = before;
-		pairs[j] = (long long)sc.pairs[i];
-		for (int d = 0; d < 3; d++) {
-			norm[3 * j + d] = sc.norm[3 * i + d];
-			cpta[3 * j + d] = sc.pa[3 * i + d];
-			cptb[3 * j + d] = sc.pb[3 * i + d];
-		}
-		depth[j] = sc.depth[i];
-		bids[2 * j] = sc.ids[2 * i];
-		bids[2 * j + 1] = sc.ids[2 * i + 1];
-	} else {
-		pairs[nh + (i - before)] = (long long)sc.pairs[i];
 	}
 }
 }  // namespace
@@ -330,8 +328,8 @@ void launch_coop(void (*k)(A...), unsigned grid, cudaStream_t s, A... args) {
 }  // namespace
 
 unsigned np_coop_max_blocks() {
-	static const unsigned m = std::min(std::min(coop_blocks(k_np_classes), coop_blocks(k_np_compact_coop)),
-	                                   coop_blocks(k_np_compact_sorted));
+	static const unsigned m = std::min(std::min(coop_blocks(k_np_classes), coop_blocks(k_np_compact<false>)),
+	                                   coop_blocks(k_np_compact<true>));
 	return m;
 }
 
@@ -390,7 +388,8 @@ void launch_np_compact(uint64_t P_cap, const unsigned long long *P_dev, const Np
 	const uint64_t Pe = std::min<uint64_t>(P_hint ? P_hint : P_cap, P_cap);
 	const unsigned grid = (unsigned)std::max<uint64_t>(
 	    1, std::min<uint64_t>((Pe + kCoopNT - 1) / kCoopNT, std::min<uint64_t>(np_coop_max_blocks(), kNpCoopBlocks)));
-	launch_coop(k_np_compact_coop, grid, s, P_cap, P_dev, sc, pairs, norm, cpta, cptb, depth, bids, contacts_out);
+	launch_coop(k_np_compact<false>, grid, s, P_cap, P_dev, sc, pairs, (unsigned long long *)nullptr, norm,
+	            cpta, cptb, depth, bids, contacts_out);
 }
 
 void launch_np_compact_sorted(uint64_t P_cap, const unsigned long long *P_dev, const NpScratch &sc,
@@ -404,7 +403,7 @@ void launch_np_compact_sorted(uint64_t P_cap, const unsigned long long *P_dev, c
 	const uint64_t Pe = std::min<uint64_t>(P_hint ? P_hint : P_cap, P_cap);
 	const unsigned grid = (unsigned)std::max<uint64_t>(
 	    1, std::min<uint64_t>((Pe + kCoopNT - 1) / kCoopNT, std::min<uint64_t>(np_coop_max_blocks(), kNpCoopBlocks)));
-	launch_coop(k_np_compact_sorted, grid, s, P_cap, P_dev, sc, pairs, tmp, norm, cpta, cptb, depth, bids,
+	launch_coop(k_np_compact<true>, grid, s, P_cap, P_dev, sc, pairs, tmp, norm, cpta, cptb, depth, bids,
 	            contacts_out);
 }
 
