@@ -124,6 +124,7 @@ struct cc_ctx {
 	int chain_wait = 0;  // calls on sorted cells left before the chains are tried again
 	uint64_t last_E = 0, last_P = 0, last_tmp = 0, last_mask = 0;  // last_tmp: pairs that went through pairs_tmp
 	bool sized = false;  // a pass has set these
+	bool rank_now = false;  // this call's overlapped pairs are few: ordered by counting
 	int last_dim[3] = {0, 0, 0};
 	// owner buckets of the pair sort (BpBuffers::owner_shift / key_bits), chosen
 	// per call from the last call's pairs per body
@@ -621,7 +622,8 @@ void enqueue_np(cc_ctx *c, const NpArgs &a, uint64_t P_cap, const unsigned long 
 	c->launches += c->np_precision == CC_NP_EXACT ? 2 : 3;  // class grouping (fast modes), MPR, compaction
 }
 
-// The step after the pair test with the narrowphase overlapped (one scene):
+// The step after the pair test with the narrowphase overlapped: a short list
+// (rank_now) is ordered by counting behind the MPR; else
 // the MPR runs on the unsorted pairs on c->np_stream (forked after the pair
 // test) while `s` sorts them into a.pairs; the compaction joins both and
 // finds each sorted key's result through the contact hash.
@@ -630,6 +632,21 @@ cc_status enqueue_sort_and_np_overlapped(cc_ctx *c, uint64_t n, const NpArgs &a,
 	DevStats *d = ptr<DevStats>(c->stats);
 	BpBuffers b = bp_buffers(c);
 	NpScratch sc = np_scratch(c);
+	if (c->rank_now) {
+		{
+			StageMark m(c, ST_MPR, s);
+			launch_mpr(std::min<uint64_t>(pairs_cap, b.pair_cap), &d->pairs, a.n, a.T, a.A, a.B, a.C, a.R, a.ID, a.nb,
+			           a.active, a.pos, a.rot, a.envelope, reinterpret_cast<const long long *>(b.pairs_tmp), sc,
+			           c->np_precision, hint_P(c, n), s);
+		}
+		{
+			StageMark m(c, ST_NP_COMPACT, s);
+			launch_np_rank(d, b.pair_cap, pairs_cap, sc, reinterpret_cast<long long *>(a.pairs), a.norm, a.cpta, a.cptb,
+			               a.depth, a.bids, hint_P(c, n), s);
+		}
+		c->launches += c->np_precision == CC_NP_EXACT ? 2 : 3;  // class grouping (fast modes), MPR, order
+		return CC_OK;
+	}
 	sc.hkeys = ptr<unsigned long long>(c->np_hkeys);
 	sc.hvals = ptr<uint32_t>(c->np_hvals);
 	sc.hmask = c->np_hslots - 1;
@@ -677,7 +694,8 @@ cc_status enqueue_sort_and_np_overlapped(cc_ctx *c, uint64_t n, const NpArgs &a,
 // at most 2^24 pairs), with the stream, events and contact hash it needs.
 cc_status overlap_prepare(cc_ctx *c, uint64_t n, uint64_t pairs_cap, bool &ov) {
 	ov = c->np_overlap && !c->direct && pairs_cap > 0 && pairs_cap <= ((uint64_t)1 << 24);
-	if (!ov) return CC_OK;
+	c->rank_now = ov && hint_P(c, n) <= kRankPairs && n < ((uint64_t)1 << 31);
+	if (!ov || c->rank_now) return CC_OK;
 	if (!c->np_stream) CC_CUDA(c, cudaStreamCreateWithFlags(&c->np_stream, cudaStreamNonBlocking));
 	if (!c->ev_fork) CC_CUDA(c, cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming));
 	if (!c->ev_join) CC_CUDA(c, cudaEventCreateWithFlags(&c->ev_join, cudaEventDisableTiming));
@@ -698,7 +716,7 @@ ZeroList pass_zero_list(cc_ctx *c, bool ov) {
 	zero.words[2] = 2 * kNpClasses + 1;
 	zero.p[3] = ptr<uint32_t>(c->cell_count);
 	zero.words[3] = c->gp.g_max;
-	if (ov) {
+	if (ov && !c->rank_now) {
 		zero.p[4] = ptr<uint32_t>(c->np_hkeys);
 		zero.words[4] = 2 * c->np_hslots;
 	}
@@ -976,7 +994,8 @@ cc_status collide_enqueue(cc_ctx *c, const cc_scene &sc, int gx, int gy, int gz,
 	                      pairs, norm, cpta, cptb, depth, bids, nullptr, nullptr};
 	memcpy(k.p, ps, sizeof(ps));
 	k.dims[0] = gx; k.dims[1] = gy; k.dims[2] = gz; k.prec = c->np_precision; k.env = envelope; k.gp = c->call_gp;
-	k.oshift = c->owner_shift; k.kbits = c->key_bits; k.ov = ov ? 1 : 0; k.hslots = ov ? c->np_hslots : 0;
+	k.oshift = c->owner_shift; k.kbits = c->key_bits; k.ov = ov ? 1 + (c->rank_now ? 1 : 0) : 0;
+	k.hslots = k.ov == 1 ? c->np_hslots : 0;
 	k.fused = c->fused_now ? 1 : 0;
 	k.dense_skip = c->dense_skip ? 1 : 0;
 	k.chain = (c->chain ? 1 : 0) + (c->chain_check ? 2 : 0);
@@ -987,6 +1006,10 @@ cc_status finish_np(cc_ctx *c, uint64_t n, const NpArgs &a, uint64_t P, uint64_t
 	DevStats *d = ptr<DevStats>(c->stats);
 	if (c->h_stats->err & kErrSegmentTooLong) {
 		// the list was sorted bucket-wise only up to 4096 per bucket: sort it whole
+		CC_TRY(sort_fallback(c, n, P, reinterpret_cast<unsigned long long *>(a.pairs), s));
+	} else if (c->h_stats->err & kErrLongList) {
+		// far more pairs than the last call had: sort the list whole
+		CC_CUDA(c, cudaMemcpyAsync(a.pairs, c->pairs_tmp.p, sizeof(unsigned long long) * P, cudaMemcpyDeviceToDevice, s));
 		CC_TRY(sort_fallback(c, n, P, reinterpret_cast<unsigned long long *>(a.pairs), s));
 	} else if (c->h_stats->err & kErrHashFull) {
 		// more contacts than the overlapped narrowphase's hash took: run it again on the sorted list,
@@ -1700,7 +1723,8 @@ cc_status batch_impl(cc_ctx *c, const cc_batch *bt, int gx, int gy, int gz, floa
 	const void *ps[18] = {sc.T, sc.A, sc.B, sc.C, sc.R, sc.ID, sc.active, sc.body_pos, sc.body_rot, res->aabb,
 	                      res->pairs, res->norm, res->cpta, res->cptb, res->depth, res->bids, src, d_off};
 	memcpy(k.p, ps, sizeof(ps));
-	k.oshift = c->owner_shift; k.kbits = c->key_bits; k.ov = ov ? 1 : 0; k.hslots = ov ? c->np_hslots : 0;
+	k.oshift = c->owner_shift; k.kbits = c->key_bits; k.ov = ov ? 1 + (c->rank_now ? 1 : 0) : 0;
+	k.hslots = k.ov == 1 ? c->np_hslots : 0;
 	k.fused = c->fused_now ? 1 : 0; k.dense_skip = c->dense_skip ? 1 : 0;
 	k.dims[0] = gx; k.dims[1] = gy; k.dims[2] = gz; k.prec = c->np_precision; k.want = want_offsets ? 1 : 0;
 	k.chain = (c->chain ? 1 : 0) + (c->chain_check ? 2 : 0);

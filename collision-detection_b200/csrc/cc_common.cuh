@@ -21,6 +21,7 @@ enum DeviceError : uint32_t {
 	kErrBinCount = 1u << 5,      // a body covers a negative / overflowing number of reference bins
 	kErrBadIndex = 1u << 6,      // a body id >= nb or a pair index >= n (the access is skipped)
 	kErrLongChain = 1u << 8,     // a cell's chain was too long for the chained search (host redoes it on sorted cells)
+	kErrLongList = 1u << 9,      // more pairs than the counting order takes (host sorts the list and redoes the narrowphase)
 	kErrHashFull = 1u << 7,      // the overlapped narrowphase's contact hash overflowed (host redoes it in order)
 };
 

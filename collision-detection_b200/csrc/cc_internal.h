@@ -394,6 +394,13 @@ void launch_mpr_exact(unsigned grid, uint64_t P_cap, const unsigned long long *P
 void launch_np_compact(uint64_t P_cap, const unsigned long long *P_dev, const NpScratch &sc, long long *pairs,
                        float *norm, float *cpta, float *cptb, float *depth, int32_t *bids,
                        unsigned long long *contacts_out, uint64_t P_hint, cudaStream_t s);
+// Short lists: the MPR ran on the unsorted pairs and neither sort nor hash
+// follows; every row's place in the hit-first order is counted. Sets
+// stats->np_n (0: the list does not fit pair_cap or out_cap) and
+// stats->contacts; above kRankRoom pairs only kErrLongList.
+constexpr uint64_t kRankPairs = 4096, kRankRoom = 8192;
+void launch_np_rank(DevStats *stats, uint64_t pair_cap, uint64_t out_cap, const NpScratch &sc, long long *pairs,
+                    float *norm, float *cpta, float *cptb, float *depth, int32_t *bids, uint64_t P_hint, cudaStream_t s);
 // The overlapped narrowphase's compaction: the MPR ran on the unsorted pairs
 // (results at their unsorted index, contacts in sc's hash); `pairs` holds the
 // sorted list of *P_dev keys. Writes the hit-first order into `pairs` and the

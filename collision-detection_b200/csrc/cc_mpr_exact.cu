@@ -389,12 +389,7 @@ __global__ void __launch_bounds__(kNT, 6) k_mpr_exact(uint64_t P_cap, const unsi
                                                     uint64_t nb, const uint8_t *__restrict__ active,
                                                     const float *__restrict__ pos, const float *__restrict__ rot,
                                                     float envelope, const long long *__restrict__ pairs,
-                                                    NpScratch sc, int beside) {
-	// beside: the kernel before is the pair sort, whose blocks are all resident
-	// once this one starts and which shares no data with it: they run side by
-	// side, and this kernel ends after it (below)
-	if (!beside) pdl_wait();
-	pdl_trigger();
+                                                    NpScratch sc) {
 	const uint64_t P = P_dev ? min(P_cap, (uint64_t)*P_dev) : P_cap;
 	uint32_t *queue = sc.classes + 2 * kNpClasses;
 	const uint32_t lane = threadIdx.x & 31, lt = (1u << lane) - 1u;
@@ -468,7 +463,7 @@ __global__ void __launch_bounds__(kNT, 6) k_mpr_exact(uint64_t P_cap, const unsi
 			}
 		}
 	}
-	if (beside) pdl_wait();
+	pdl_wait();  // beside the pair sort: this kernel ends after it
 }
 }  // namespace
 
@@ -485,12 +480,18 @@ void launch_mpr_exact(unsigned grid, uint64_t P_cap, const unsigned long long *P
                       const float *A, const float *B, const float *C, const float *R, const uint32_t *ID, uint64_t nb,
                       const uint8_t *active, const float *pos, const float *rot, float envelope,
                       const long long *pairs, const NpScratch &sc, cudaStream_t s, bool beside) {
+	// Beside the pair sort: its blocks, a cooperative launch, are all resident once
+	// this kernel starts, the two share no data, and this one ends after it. Else a
+	// plain launch, and no early start of what follows either: blocks that become
+	// resident among a neighbour's spread unevenly, and few warps of FP64 chains run
+	// as slow as the fullest SM (3.4K pairs of 130K bodies: a step of 99 us with the
+	// MPR's blocks launched early, 86 without; 2K pairs of 1K bodies: 91 us with its
+	// successor's launched early, 85 without).
 	if (beside)
 		launch_pdl<true>(k_mpr_exact, dim3(grid), dim3(kNT), 0, s, P_cap, P_dev, n, T, A, B, C, R, ID, nb, active, pos, rot,
-		                 envelope, pairs, sc, 1);
+		                 envelope, pairs, sc);
 	else
-		launch_pdl(k_mpr_exact, dim3(grid), dim3(kNT), 0, s, P_cap, P_dev, n, T, A, B, C, R, ID, nb, active, pos, rot, envelope,
-		           pairs, sc, 0);
+		k_mpr_exact<<<grid, kNT, 0, s>>>(P_cap, P_dev, n, T, A, B, C, R, ID, nb, active, pos, rot, envelope, pairs, sc);
 }
 
 }  // namespace cc
