@@ -1079,15 +1079,15 @@ cc_status collide_verlet(cc_ctx *c, const cc_scene &sc, int gx, int gy, int gz, 
 		const uint64_t allocs = c->v_ref.allocs + c->v_cand.allocs;
 		const bool rebuild = attempt > 0 || !c->inc_valid || c->inc_n != n || c->inc_allocs != allocs ||
 		                     c->inc_disp > 0.25f * c->inc_m;
-		const auto enqueue_front = [&](cudaStream_t st) -> cc_status {
+		const auto enqueue_front = [&](cudaStream_t st, const ZeroList &zero) -> cc_status {
 			CC_CUDA(c, cudaMemsetAsync(d, 0, sizeof(DevStats), st));
 			launch_aabb(n, sc.T, sc.A, sc.B, sc.C, sc.R, sc.ID, sc.nb, sc.body_pos, sc.body_rot, aabb, d, &d->err,
-			            c->call_gp, grid, st);
+			            c->call_gp, grid, st, zero);
 			c->launches += 1;
 			return CC_OK;
 		};
 		if (rebuild) {
-			CC_TRY(enqueue_front(s));
+			CC_TRY(enqueue_front(s, ZeroList()));
 			c->inc_valid = false;
 			CC_TRY(ensure(c, c->v_scratch, 24 * n));
 			const uint64_t want = std::max<uint64_t>(2 * c->inc_nc, std::max<uint64_t>(c->last_P, n / 4) + 1024);
@@ -1139,13 +1139,24 @@ cc_status collide_verlet(cc_ctx *c, const cc_scene &sc, int gx, int gy, int gz, 
 			{
 				StageMark m(c, ST_PAIR_TEST, st);
 				launch_vcompact(nc, ptr<unsigned long long>(c->v_cand), aabb, n, d, out, pairs_cap,
-				                ptr<uint64_t>(c->v_status), ptr<uint32_t>(c->ticket) + 12, rebuild, c->inc_m, st);
+				                ptr<uint64_t>(c->v_status), ptr<uint32_t>(c->ticket) + 12, rebuild, c->inc_m, !rebuild, st);
 			}
 			c->launches += 2;
+			c->pass_zeroed = !rebuild;
 			enqueue_np(c, a, pairs_cap, &d->np_n, st);
+			c->pass_zeroed = false;
 			return CC_OK;
 		};
-		if (!rebuild) CC_TRY(enqueue_front(s));
+		if (!rebuild) {  // the first kernel zeroes what the others count in
+			ZeroList zero;
+			zero.p[0] = ptr<uint32_t>(c->v_status);
+			zero.words[0] = 2 * vcompact_status_words(nc);
+			zero.p[1] = ptr<uint32_t>(c->ticket);
+			zero.words[1] = 16;
+			zero.p[2] = ptr<uint32_t>(c->np_classes);
+			zero.words[2] = 2 * kNpClasses + 1;
+			CC_TRY(enqueue_front(s, zero));
+		}
 		CC_TRY(enqueue_tail(s));
 		CC_TRY(check_launch(c));
 		CC_TRY(read_stats(c, s));

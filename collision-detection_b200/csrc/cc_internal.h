@@ -258,11 +258,12 @@ void launch_owner_sort_fused(uint64_t n, uint64_t out_cap, unsigned long long *o
 void launch_vinflate(uint64_t n, const float *aabb, float *scratch, DevStats *stats, float factor, cudaStream_t s);
 void launch_vcheck(uint64_t n, float *aabb, const float *ref, float *backup, const int32_t *T, DevStats *stats,
                    cudaStream_t s);
+// zeroed: the pass's first kernel zeroed status and ticket.
 // Words of the status region launch_vcompact needs for nc candidates.
 uint64_t vcompact_status_words(uint64_t nc);
 void launch_vcompact(uint64_t nc, const unsigned long long *cand, const float *aabb, uint64_t n, DevStats *stats,
                      unsigned long long *out, uint64_t out_cap, uint64_t *status, uint32_t *ticket, bool rebuild,
-                     float margin, cudaStream_t s);
+                     float margin, bool zeroed, cudaStream_t s);
 
 // ------------------------------------------------------------------ batches
 // Per-scene accumulators of the batch bounds pass (zeroed per call).
