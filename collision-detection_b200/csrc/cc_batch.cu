@@ -96,6 +96,80 @@ __global__ void __launch_bounds__(kNT) k_gather_c(uint64_t n, const int32_t *__r
 	}
 }
 
+// The arrays of a MoveList, through the host mapping: the link to the host is
+// filled by the loads or stores of all SMs at once, where nine copies one after the
+// other spend most of their time starting (60K shapes, 4.6 MB in: a step of 315 us, by
+// kernel 291, with the results out by kernel too 272; 2K shapes 147, 121, 94). An array
+// is cut into units of 16 bytes, or of 4 or 1 where its addresses ask for that; a
+// thread has four units in flight.
+struct MoveUnits {
+	uint64_t end[MoveList::kMax];  // units of the arrays so far
+	uint64_t bytes[MoveList::kMax];
+	uint32_t size[MoveList::kMax];
+};
+__device__ __forceinline__ void move_bytes(const char *src, char *dst, uint64_t from, uint64_t to) {
+	for (uint64_t b = from; b < to; b++) dst[b] = src[b];
+}
+__global__ void __launch_bounds__(kNT) k_move(MoveList m, const DevStats *stats, uint64_t pair_cap) {
+	__shared__ MoveUnits u;
+	if (threadIdx.x == 0) {
+		uint64_t P = 0, nc = 0, end = 0;
+		bool ok = true;
+		if (stats) {
+			P = stats->np_n;
+			nc = stats->contacts;
+			ok = stats->err == 0 && P == stats->pairs && P <= pair_cap && nc <= P;
+		}
+		for (int k = 0; k < m.count; k++) {
+			const uint64_t at = reinterpret_cast<uint64_t>(m.src[k]) | reinterpret_cast<uint64_t>(m.dst[k]);
+			u.size[k] = at % 16 == 0 ? 16 : at % 4 == 0 ? 4 : 1;
+			u.bytes[k] = ok ? m.fixed[k] + m.per_pair[k] * P + m.per_contact[k] * nc : 0;
+			end += (u.bytes[k] + u.size[k] - 1) / u.size[k];
+			u.end[k] = end;
+		}
+	}
+	__syncthreads();
+	const uint64_t total = m.count ? u.end[m.count - 1] : 0, step = (uint64_t)gridDim.x * kNT;
+	for (uint64_t i0 = (uint64_t)blockIdx.x * kNT + threadIdx.x; i0 < total; i0 += 4 * step) {
+		uint4 v[4];
+		int arr[4];
+		uint64_t at[4];  // first byte of the unit
+#pragma unroll
+		for (int q = 0; q < 4; q++) {
+			const uint64_t i = i0 + q * step;
+			arr[q] = -1;
+			if (i >= total) continue;
+			int k = 0;
+			while (i >= u.end[k]) k++;
+			arr[q] = k;
+			at[q] = (i - (k ? u.end[k - 1] : 0)) * u.size[k];
+			if (at[q] + u.size[k] > u.bytes[k]) continue;  // the last, partial unit
+			const char *src = static_cast<const char *>(m.src[k]) + at[q];
+			if (u.size[k] == 16) v[q] = __ldcs(reinterpret_cast<const uint4 *>(src));
+			else if (u.size[k] == 4) v[q].x = __ldcs(reinterpret_cast<const uint32_t *>(src));
+			else v[q].x = *reinterpret_cast<const uint8_t *>(src);
+		}
+#pragma unroll
+		for (int q = 0; q < 4; q++) {
+			const int k = arr[q];
+			if (k < 0) continue;
+			char *dst = static_cast<char *>(m.dst[k]);
+			if (at[q] + u.size[k] > u.bytes[k]) move_bytes(static_cast<const char *>(m.src[k]), dst, at[q], u.bytes[k]);
+			else if (u.size[k] == 16) *reinterpret_cast<uint4 *>(dst + at[q]) = v[q];
+			else if (u.size[k] == 4) *reinterpret_cast<uint32_t *>(dst + at[q]) = v[q].x;
+			else *reinterpret_cast<uint8_t *>(dst + at[q]) = (uint8_t)v[q].x;
+			if (k == 0 && m.c_src) {  // shape types: this unit's shapes with a third vertex or axis
+				const uint64_t last = min(at[q] + u.size[k], u.bytes[k]) / 4;
+				for (uint64_t s = at[q] / 4; s < last; s++) {
+					const int t = reinterpret_cast<const int32_t *>(dst)[s];
+					if (t == CONE || t == TRIANGLEMESH)
+						for (int d = 0; d < 3; d++) m.c_dst[3 * s + d] = m.c_src[3 * s + d];
+				}
+			}
+		}
+	}
+}
+
 // Counter-based random numbers for the time-step update: SplitMix64's output
 // function (Steele, Lea, Flood 2014) applied to seed + counter, so every body
 // draws the same numbers whatever the launch shape.
@@ -216,6 +290,11 @@ void launch_gather_c(uint64_t n, const int32_t *T, const float *src, float *dst,
 	if (!n) return;
 	const unsigned g = (unsigned)std::min<uint64_t>((n + kNT - 1) / kNT, (uint64_t)kNumSMs * 8);
 	k_gather_c<<<g, kNT, 0, s>>>(n, T, src, dst);
+}
+
+void launch_move(const MoveList &m, uint64_t bytes_hint, const DevStats *stats, uint64_t pair_cap, cudaStream_t s) {
+	const unsigned g = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(bytes_hint / (16 * 4 * kNT) + 1, (uint64_t)kNumSMs * 8));
+	k_move<<<g, kNT, 0, s>>>(m, stats, pair_cap);
 }
 
 void launch_batch_pair_counts(uint64_t P, const unsigned long long *pairs, const uint32_t *scene_of,

@@ -1187,11 +1187,18 @@ cc_status collide_verlet(cc_ctx *c, const cc_scene &sc, int gx, int gy, int gz, 
 	return set_err(c, CC_ERR_INTERNAL, "incremental step did not settle");
 }
 
+// Whether a pass's counters show a result that needs no redo.
+bool complete_pass(const DevStats &st, uint64_t entry_cap, uint64_t pair_cap, bool direct, uint64_t out_cap) {
+	return st.err == 0 && st.entries <= entry_cap && unsorted_pairs(st, direct) <= pair_cap && st.pairs <= out_cap &&
+	       st.np_n == st.pairs;
+}
+
 // GenerateAABB -> broadphase -> narrowphase on device pointers with one
 // synchronize in the common case.
 cc_status collide_dev(cc_ctx *c, const cc_scene &sc, int gx, int gy, int gz, float envelope, float *aabb,
                       int64_t *pairs, uint64_t pairs_cap, float *norm, float *cpta, float *cptb, float *depth,
-                      int32_t *bids, uint64_t *n_pairs, uint64_t *n_contacts, cudaStream_t s) {
+                      int32_t *bids, uint64_t *n_pairs, uint64_t *n_contacts, cudaStream_t s,
+                      const MoveList *push = nullptr, bool *pushed = nullptr) {
 	*n_pairs = 0;
 	*n_contacts = 0;
 	c->retained = false;
@@ -1201,12 +1208,17 @@ cc_status collide_dev(cc_ctx *c, const cc_scene &sc, int gx, int gy, int gz, flo
 		                      n_pairs, n_contacts, s);
 	CC_TRY(collide_enqueue(c, sc, gx, gy, gz, envelope, aabb, pairs, pairs_cap, norm, cpta, cptb, depth, bids, s,
 	                       true));
-	const uint64_t gen = c->buf_gen;
+	if (push) {
+		StageMark m(c, ST_COPY_OUT, s);
+		launch_move(*push, 24 * sc.n + 56 * hint_P(c, sc.n), ptr<DevStats>(c->stats), pairs_cap, s);
+		c->launches += 1;
+		CC_TRY(check_launch(c));
+	}
+	const BpBuffers b = bp_buffers(c);
 	CC_TRY(read_stats(c, s));
-	const cc_status st = collide_finish(c, sc, envelope, aabb, pairs, pairs_cap, norm, cpta, cptb, depth, bids,
-	                                    n_pairs, n_contacts, s);
-	(void)gen;
-	return st;
+	// what went out is the result unless something is redone below
+	if (push) *pushed = complete_pass(*c->h_stats, b.entry_cap, b.pair_cap, c->direct, pairs_cap);
+	return collide_finish(c, sc, envelope, aabb, pairs, pairs_cap, norm, cpta, cptb, depth, bids, n_pairs, n_contacts, s);
 }
 
 }  // namespace
@@ -1955,8 +1967,9 @@ const void *mapped_host(const void *p) {
 // *gather_c receives its device mapping and the caller gathers those shapes'
 // C with launch_gather_c once T is on the device, on its compute stream (a
 // kernel on the copy stream would hold the later copies until the SMs are free).
+// list: the other arrays are mapped too and join it instead of being copied.
 cc_status upload_shapes(cc_ctx *c, cc_ctx::ShapeCopy &sh, Buf *const dst[6], const cc_scene *sc, cudaStream_t t,
-                        const float **gather_c) {
+                        const float **gather_c, MoveList *list = nullptr) {
 	*gather_c = nullptr;
 	const void *src[6] = {sc->T, sc->A, sc->B, sc->C, sc->R, sc->ID};
 	static const uint64_t bytes[6] = {4, 12, 12, 12, 16, 4};
@@ -1969,6 +1982,8 @@ cc_status upload_shapes(cc_ctx *c, cc_ctx::ShapeCopy &sh, Buf *const dst[6], con
 	for (int k = 0; k < 6; k++) {
 		if (k == 3 && c_mapped)
 			*gather_c = c_mapped;
+		else if (list)
+			list->add(mapped_host(src[k]), dst[k]->p, bytes[k] * sc->n);
 		else
 			CC_CUDA(c, cudaMemcpyAsync(dst[k]->p, src[k], bytes[k] * sc->n, cudaMemcpyHostToDevice, t));
 		sh.src[k] = src[k];
@@ -1978,6 +1993,17 @@ cc_status upload_shapes(cc_ctx *c, cc_ctx::ShapeCopy &sh, Buf *const dst[6], con
 	sh.n = sc->n;
 	sh.gen = c->shapes_gen;
 	return CC_OK;
+}
+
+// Scenes of up to kMoveBytes of input whose arrays are all mapped move by kernel.
+// Steps with copies and with kernels, us: 2K shapes 147 and 94, 60K (4.6 MB) 315 and
+// 272, 130K 367 and 337; 400K (31 MB, inputs alone) 813 both ways, 1M 1797 and 1865.
+constexpr uint64_t kMoveBytes = (uint64_t)16 << 20;
+template <size_t K>
+bool all_mapped(const void *const (&p)[K]) {
+	for (const void *q : p)
+		if (!mapped_host(q)) return false;
+	return true;
 }
 
 // Sizes one slot for a scene of n shapes / nb bodies and cap pairs and points
@@ -2102,8 +2128,7 @@ cc_status cc_collide_host_wait(cc_ctx *c, cc_result *res, void *stream) {
 	res->n_pairs = res->n_contacts = 0;
 	if (h.dev.n == 0) return CC_OK;
 	const DevStats &st = *h.h_stats;
-	const bool fast = st.err == 0 && st.entries <= h.entry_cap && unsorted_pairs(st, h.direct) <= h.pair_cap && st.pairs <= h.cap &&
-	                  st.np_n == st.pairs;
+	const bool fast = complete_pass(st, h.entry_cap, h.pair_cap, h.direct, h.cap);
 	uint64_t P = st.pairs, nc = st.contacts;
 	if (fast) {
 		memcpy(c->h_stats, h.h_stats, sizeof(DevStats));
@@ -2164,20 +2189,36 @@ cc_status cc_collide_host(cc_ctx *c, const cc_scene *sc, int gx, int gy, int gz,
 	CC_TRY(ensure(c, c->out_pb, 12 * std::max<uint64_t>(cap, 1)));
 	CC_TRY(ensure(c, c->out_depth, 4 * std::max<uint64_t>(cap, 1)));
 	CC_TRY(ensure(c, c->out_bids, 8 * std::max<uint64_t>(cap, 1)));
+	const void *const in[] = {sc->T, sc->A, sc->B, sc->C, sc->R, sc->ID, sc->body_pos, sc->body_rot, sc->active};
+	const bool pull = 77 * std::max(n, nb) <= kMoveBytes && all_mapped(in) && (!res->aabb || mapped_host(res->aabb));
 	std::unique_ptr<StageMark> cin(new StageMark(c, ST_COPY_IN, s));
 	{
 		Buf *const dst[6] = {&c->in_T, &c->in_A, &c->in_B, &c->in_C, &c->in_R, &c->in_ID};
 		const float *gather_c = nullptr;
-		CC_TRY(upload_shapes(c, c->in_shapes, dst, sc, s, &gather_c));
-		if (gather_c) {
-			launch_gather_c(n, ptr<int32_t>(c->in_T), gather_c, ptr<float>(c->in_C), s);
+		MoveList list;
+		CC_TRY(upload_shapes(c, c->in_shapes, dst, sc, s, &gather_c, pull ? &list : nullptr));
+		if (pull) {
+			if (list.count) {  // (T is the first)
+				list.c_src = gather_c;
+				list.c_dst = ptr<float>(c->in_C);
+			}
+			list.add(mapped_host(sc->body_pos), c->in_pos.p, 12 * nb);
+			list.add(mapped_host(sc->body_rot), c->in_rot.p, 16 * nb);
+			list.add(mapped_host(sc->active), c->in_act.p, nb);
+			if (res->aabb) list.add(mapped_host(res->aabb), c->out_aabb.p, 24 * n);
+			launch_move(list, 77 * std::max(n, nb), nullptr, 0, s);
 			c->launches += 1;
+		} else {
+			if (gather_c) {
+				launch_gather_c(n, ptr<int32_t>(c->in_T), gather_c, ptr<float>(c->in_C), s);
+				c->launches += 1;
+			}
+			CC_CUDA(c, cudaMemcpyAsync(c->in_pos.p, sc->body_pos, 12 * nb, cudaMemcpyHostToDevice, s));
+			CC_CUDA(c, cudaMemcpyAsync(c->in_rot.p, sc->body_rot, 16 * nb, cudaMemcpyHostToDevice, s));
+			CC_CUDA(c, cudaMemcpyAsync(c->in_act.p, sc->active, nb, cudaMemcpyHostToDevice, s));
+			if (res->aabb) CC_CUDA(c, cudaMemcpyAsync(c->out_aabb.p, res->aabb, 24 * n, cudaMemcpyHostToDevice, s));
 		}
 	}
-	CC_CUDA(c, cudaMemcpyAsync(c->in_pos.p, sc->body_pos, 12 * nb, cudaMemcpyHostToDevice, s));
-	CC_CUDA(c, cudaMemcpyAsync(c->in_rot.p, sc->body_rot, 16 * nb, cudaMemcpyHostToDevice, s));
-	CC_CUDA(c, cudaMemcpyAsync(c->in_act.p, sc->active, nb, cudaMemcpyHostToDevice, s));
-	if (res->aabb) CC_CUDA(c, cudaMemcpyAsync(c->out_aabb.p, res->aabb, 24 * n, cudaMemcpyHostToDevice, s));
 	cin.reset();
 	cc_scene d;
 	d.n = n;
@@ -2192,12 +2233,29 @@ cc_status cc_collide_host(cc_ctx *c, const cc_scene *sc, int gx, int gy, int gz,
 	d.body_rot = ptr<float>(c->in_rot);
 	d.active = ptr<uint8_t>(c->in_act);
 	uint64_t P = 0, nc = 0;
+	MoveList push;
+	bool pushed = false;
+	const void *const outs[] = {res->aabb, res->pairs, res->norm, res->cpta, res->cptb, res->depth, res->bids};
+	if (pull && !c->incremental) {
+		const void *const from[] = {c->out_aabb.p, c->out_pairs.p, c->out_norm.p, c->out_pa.p,
+		                            c->out_pb.p,   c->out_depth.p, c->out_bids.p};
+		static const uint32_t per_contact[] = {0, 0, 12, 12, 12, 4, 8};
+		bool ok = true;
+		for (int k = 0; k < 7; k++) {
+			if (!outs[k]) continue;
+			void *to = const_cast<void *>(mapped_host(outs[k]));
+			ok = ok && to;
+			push.add(from[k], to, k == 0 ? 24 * n : 0, k == 1 ? 8 : 0, per_contact[k]);
+		}
+		if (!ok) push.count = 0;
+	}
 	cc_status st = collide_dev(c, d, gx, gy, gz, envelope, ptr<float>(c->out_aabb), ptr<int64_t>(c->out_pairs), cap,
 	                           ptr<float>(c->out_norm), ptr<float>(c->out_pa), ptr<float>(c->out_pb),
-	                           ptr<float>(c->out_depth), ptr<int32_t>(c->out_bids), &P, &nc, s);
+	                           ptr<float>(c->out_depth), ptr<int32_t>(c->out_bids), &P, &nc, s,
+	                           push.count ? &push : nullptr, &pushed);
 	res->n_pairs = P;
 	res->n_contacts = nc;
-	if (st != CC_OK) return st;
+	if (st != CC_OK || pushed) return st;
 	StageMark cout_mark(c, ST_COPY_OUT, s);
 	if (res->aabb) CC_CUDA(c, cudaMemcpyAsync(res->aabb, c->out_aabb.p, 24 * n, cudaMemcpyDeviceToHost, s));
 	if (res->pairs && P) CC_CUDA(c, cudaMemcpyAsync(res->pairs, c->out_pairs.p, 8 * P, cudaMemcpyDeviceToHost, s));

@@ -316,6 +316,29 @@ cudaError_t copy_small_h2d(void *dst, const void *src, size_t bytes, cudaStream_
 // dst[i] = src[i] (3 floats) for the shapes of type CONE or TRIANGLEMESH, the
 // only ones whose C is read; T is on the device, src a device-accessible
 // (pinned, mapped) host array.
+// Moves whole arrays between mapped host memory and the device in one launch.
+// Array k has fixed + per_pair * np_n + per_contact * contacts bytes (counts of
+// `stats`, whose lists must be complete: else nothing moves; null: fixed only).
+// Where array 0 holds the shape types and c_src is set, c_dst also receives C of
+// the CONE and TRIANGLEMESH shapes.
+struct MoveList {
+	static constexpr int kMax = 11;
+	int count = 0;
+	const void *src[kMax];
+	void *dst[kMax];
+	uint64_t fixed[kMax];
+	uint32_t per_pair[kMax], per_contact[kMax];
+	const float *c_src = nullptr;
+	float *c_dst = nullptr;
+	void add(const void *from, void *to, uint64_t bytes, uint32_t pair_bytes = 0, uint32_t contact_bytes = 0) {
+		src[count] = from;
+		dst[count] = to;
+		fixed[count] = bytes;
+		per_pair[count] = pair_bytes;
+		per_contact[count++] = contact_bytes;
+	}
+};
+void launch_move(const MoveList &m, uint64_t bytes_hint, const DevStats *stats, uint64_t pair_cap, cudaStream_t s);
 void launch_gather_c(uint64_t n, const int32_t *T, const float *src, float *dst, cudaStream_t s);
 // The front of a batch pass (cc_aabb.cu): scene_of, global ids, boxes, bounds,
 // plans, cell_base[0..S] and stats->cells; with src the scenes are gathered into
