@@ -495,6 +495,7 @@ NpScratch np_scratch(cc_ctx *c) {
 	sc.err = &ptr<DevStats>(c->stats)->err;
 	sc.order = ptr<uint32_t>(c->np_order);
 	sc.classes = ptr<uint32_t>(c->np_classes);
+	sc.queue = &ptr<DevStats>(c->stats)->np_queue;
 	sc.pre_zeroed = c->pass_zeroed;
 	return sc;
 }
@@ -1442,18 +1443,16 @@ cc_status cc_generate_aabb(cc_ctx *c, uint64_t n, const int32_t *T, const float 
 	CC_CUDA(c, cudaSetDevice(c->device));
 	cudaStream_t s = (cudaStream_t)stream;
 	if (n == 0) return CC_OK;
-	CC_TRY(ensure(c, c->stats, sizeof(DevStats)));
-	uint32_t *err = &ptr<DevStats>(c->stats)->err;
+	c->h_word[0] = 0;
+	uint32_t *err = reinterpret_cast<uint32_t *>(c->h_word);  // mapped: written by the kernel where an id is bad
 	{
 		StageMark m(c, ST_AABB, s);
-		CC_CUDA(c, cudaMemsetAsync(err, 0, sizeof(uint32_t), s));
 		launch_aabb(n, T, A, B, C, R, ID, nb, pos, rot, aabb, nullptr, err, c->gp, nullptr, s);
 	}
 	c->launches += 1;
 	CC_TRY(check_launch(c));
-	CC_CUDA(c, cudaMemcpyAsync(c->h_word, err, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
 	CC_CUDA(c, cudaStreamSynchronize(s));
-	if ((uint32_t)c->h_word[0] & kErrBadIndex) return set_err(c, CC_ERR_INVALID_INPUT, "a body id is >= nb");
+	if (*reinterpret_cast<volatile uint32_t *>(c->h_word) & kErrBadIndex) return set_err(c, CC_ERR_INVALID_INPUT, "a body id is >= nb");
 	return CC_OK;
 }
 
@@ -1475,13 +1474,15 @@ cc_status cc_broadphase(cc_ctx *c, uint64_t n, float *aabb, int gx, int gy, int 
 	{
 		StageMark m(c, ST_BOUNDS, s);
 		CC_CUDA(c, cudaMemsetAsync(c->stats.p, 0, sizeof(DevStats), s));
-		launch_bounds(n, aabb, ptr<DevStats>(c->stats), c->call_gp, grid, s);
+		launch_bounds(n, aabb, ptr<DevStats>(c->stats), c->call_gp, grid, s, pass_zero_list(c, false));
 	}
 	c->launches += 1;
+	c->pass_zeroed = true;
 	enqueue_search(c, n, aabb, s);
 	unsigned long long *out = reinterpret_cast<unsigned long long *>(pairs);
 	const uint64_t cap = pairs ? pairs_cap : 0;
 	if (cap) enqueue_emit(c, n, out, cap, s);
+	c->pass_zeroed = false;
 	CC_TRY(check_launch(c));
 	CC_TRY(read_stats(c, s));
 	CC_TRY(device_err(c));
@@ -1610,7 +1611,9 @@ cc_status cc_narrowphase(cc_ctx *c, uint64_t n, const int32_t *T, const float *A
 	CC_TRY(np_prepare(c, n_pairs));
 	CC_CUDA(c, cudaMemsetAsync(c->stats.p, 0, sizeof(DevStats), s));
 	const NpArgs a = {n, nb, T, A, B, C, R, ID, active, pos, rot, envelope, pairs, norm, cpta, cptb, depth, bids};
+	c->pass_zeroed = c->np_precision == CC_NP_EXACT;  // its queue, with the counters above
 	enqueue_np(c, a, n_pairs, nullptr, s);
+	c->pass_zeroed = false;
 	CC_TRY(check_launch(c));
 	CC_TRY(read_stats(c, s));
 	if (c->h_stats->err & kErrBadIndex)

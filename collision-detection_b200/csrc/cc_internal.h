@@ -41,7 +41,7 @@ struct DevStats {
 	unsigned long long np_n;      // pairs handed to the narrowphase (0 if an output was too small)
 	unsigned long long dense_items;  // (cell, row chunk) work items of the dense-cell pair test (chained search: long chains met)
 	uint32_t blocks_done;         // last-block detection of the bounds reduction
-	uint32_t pad_;
+	uint32_t np_queue;            // work queue of the exact MPR
 	unsigned long long mask_words;  // hit-mask words of the dense cells' rows
 	unsigned long long tmp_pairs; // pairs of the sparse cells where dense cells have their own test (else `pairs`)
 	unsigned long long extra;     // entries of the chained search beyond the first one of every body
@@ -380,7 +380,8 @@ struct NpScratch {
 	uint32_t *err;
 	uint32_t *order;        // P: pair indices grouped by (type A, type B)
 	uint32_t *classes;      // 2 * kNpClasses counters + the work-queue counter (zeroed per call)
-	bool pre_zeroed = false;  // classes, status and ticket already zeroed for this pass
+	uint32_t *queue;        // the exact MPR's work queue (zeroed per call)
+	bool pre_zeroed = false;  // classes, queue, status and ticket already zeroed for this pass
 	void *bar_classes = nullptr;  // grid barriers (GridBarrier) of the cooperative class sort and compaction,
 	void *bar_compact = nullptr;  // zeroed at the start of the call
 	unsigned long long *block_sums = nullptr;  // per-block flag counts of the compaction (>= its grid)

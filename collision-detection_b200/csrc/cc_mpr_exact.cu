@@ -391,7 +391,7 @@ __global__ void __launch_bounds__(kNT, 6) k_mpr_exact(uint64_t P_cap, const unsi
                                                     float envelope, const long long *__restrict__ pairs,
                                                     NpScratch sc) {
 	const uint64_t P = P_dev ? min(P_cap, (uint64_t)*P_dev) : P_cap;
-	uint32_t *queue = sc.classes + 2 * kNpClasses;
+	uint32_t *queue = sc.queue;
 	const uint32_t lane = threadIdx.x & 31, lt = (1u << lane) - 1u;
 	const bool odd = lane & 1;
 	// pairs a warp holds: as few as take all of them at once over the grid's

@@ -434,7 +434,7 @@ void launch_mpr(uint64_t P_cap, const unsigned long long *P_dev, uint64_t n, con
 		// instead, one warp per scheduler (3,400 pairs: 46 us with two blocks per
 		// SM, 60 us with six), at most what is resident (27,500 pairs: 75 us with
 		// six, 82 with three; 195,000: 239 with six, 373 with three).
-		if (!sc.pre_zeroed) cudaMemsetAsync(sc.classes, 0, (2 * kNpClasses + 1) * sizeof(uint32_t), s);
+		if (!sc.pre_zeroed) cudaMemsetAsync(sc.queue, 0, sizeof(uint32_t), s);
 		const uint64_t want = std::max<uint64_t>((Pe + kNT / 2 - 1) / (kNT / 2), 2 * kNumSMs);
 		launch_mpr_exact((unsigned)std::min<uint64_t>(want, (uint64_t)kNumSMs * mpr_exact_resident_blocks()), P_cap, P_dev, n,
 		                 T, A, B, C, R, ID, nb, active, pos, rot, envelope, pairs, sc, s, beside);
