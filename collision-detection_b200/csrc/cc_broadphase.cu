@@ -746,6 +746,74 @@ __global__ void __launch_bounds__(kNT, 5) k_walk(uint64_t n, DevStats *stats, co
 	if (ocnt) flush_pairs(obuf, ocnt, lane, &stats->pairs, pairs, pair_cap);
 }
 
+// ---------------------------------------------------------------- small scenes
+// Up to kAllPairsBodies bodies every box is tested against every later one: a
+// search through cells is a chain of dependent loads (a heap of 1,000 bodies: link
+// 4 us, walk 14), n^2 / 2 tests of boxes in shared memory are not. Steps
+// with cells and with this, us, at 2 pairs a body and at 0.1: 500 bodies 83 and 71, 71
+// and 70; 1,000 87 and 71, 71 and 70; 2,000 101 and 88, 72 and 70; 3,000 107 and 97,
+// but 71 and 81.
+__global__ void __launch_bounds__(kNT) k_shift(uint64_t n, float *__restrict__ aabb, const DevStats *stats,
+                                                uint32_t *__restrict__ owner_count, uint32_t *__restrict__ cursor,
+                                                uint32_t buckets, int shift) {
+	pdl_begin();
+	if (!stats->plan.valid) return;  // invalid input: nothing is modified
+	const uint64_t k = (uint64_t)blockIdx.x * kNT + threadIdx.x;
+	if (k < buckets) {
+		owner_count[k] = 0u;
+		if (cursor) cursor[k] = 0u;
+	}
+	if (shift && k < 6 * n) aabb[k] = aabb[k] + stats->plan.origin[k % 3];
+}
+
+constexpr int kAllCols = 64;
+// Block (x, y): rows [256 x, 256 x + 256), one a thread, against columns
+// [64 y, 64 y + 64).
+__global__ void __launch_bounds__(kNT) k_all_pairs(uint32_t n, DevStats *stats, const float *__restrict__ aabb,
+                                                    uint32_t *__restrict__ owner_count,
+                                                    unsigned long long *__restrict__ pairs, uint64_t pair_cap, int oshift) {
+	pdl_begin();
+	__shared__ float4 lo[kAllCols], hi[kAllCols];
+	if (!stats->plan.valid) return;
+	if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) stats->entries = n;
+	const uint32_t i = blockIdx.x * kNT + threadIdx.x, c0 = blockIdx.y * kAllCols;
+	if (c0 + kAllCols <= blockIdx.x * kNT + 1) return;  // no later column
+	const float *mx = aabb + 3 * (uint64_t)n;
+	if (threadIdx.x < kAllCols) {
+		const uint32_t j = c0 + threadIdx.x;
+		lo[threadIdx.x] = j < n ? make_float4(aabb[3 * j], aabb[3 * j + 1], aabb[3 * j + 2], 0.f)
+		                        : make_float4(INFINITY, INFINITY, INFINITY, 0.f);
+		hi[threadIdx.x] = j < n ? make_float4(mx[3 * j], mx[3 * j + 1], mx[3 * j + 2], 0.f)
+		                        : make_float4(-INFINITY, -INFINITY, -INFINITY, 0.f);
+	}
+	float3 a0 = f3(INFINITY, INFINITY, INFINITY), a1 = f3(-INFINITY, -INFINITY, -INFINITY);
+	if (i < n) {
+		a0 = f3(aabb[3 * i], aabb[3 * i + 1], aabb[3 * i + 2]);
+		a1 = f3(mx[3 * i], mx[3 * i + 1], mx[3 * i + 2]);
+	}
+	__syncthreads();
+	uint32_t m[2] = {0u, 0u};
+#pragma unroll
+	for (int h = 0; h < 2; h++)
+#pragma unroll
+		for (int q = 0; q < 32; q++) {
+			const float4 b0 = lo[32 * h + q], b1 = hi[32 * h + q];
+			const bool over = (a0.x <= b1.x) & (b0.x <= a1.x) & (a0.y <= b1.y) & (b0.y <= a1.y) & (a0.z <= b1.z) & (b0.z <= a1.z);
+			m[h] |= over ? 1u << q : 0u;
+		}
+	unsigned long long hits = (unsigned long long)m[1] << 32 | m[0];
+	if (i >= c0) hits = i - c0 >= kAllCols - 1 ? 0ull : hits & ~0ull << (i - c0 + 1);  // later columns only
+	const uint32_t cnt = __popcll(hits), incl = warp_incl_scan(cnt), lane = threadIdx.x & 31;
+	const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
+	if (!total) return;
+	unsigned long long at = 0;
+	if (lane == 31) at = atomicAdd(&stats->pairs, (unsigned long long)total);
+	at = __shfl_sync(0xffffffffu, at, 31) + incl - cnt;
+	if (cnt) atomicAdd(&owner_count[i >> oshift], cnt);
+	for (; hits; hits &= hits - 1, at++)
+		if (at < pair_cap) pairs[at] = (unsigned long long)i << 32 | (c0 + (uint32_t)__ffsll((long long)hits) - 1u);
+}
+
 // In-place bitonic sort of m (a power of two) keys in shared memory by
 // `nt` cooperating threads (thread t of them); sync() separates the steps.
 template <class K, class Sync>
@@ -1675,6 +1743,16 @@ void launch_link(uint64_t n, float *aabb, const BpBuffers &b, cudaStream_t s, bo
 	const auto k = b.sm.plans ? k_link<true> : k_link<false>;
 	launch_pdl(k, dim3(blocks_for(n)), dim3(kNT), 0, s, n, aabb, b.stats, b.cell_count, b.entries, b.entry_cap, b.extra_body,
 	           b.owner_count, b.sm, b.owner_shift, b.owner_cursor, shift ? 1 : 0);
+}
+
+void launch_shift(uint64_t n, float *aabb, const BpBuffers &b, cudaStream_t s, bool shift) {
+	launch_pdl(k_shift, dim3(blocks_for(6 * n)), dim3(kNT), 0, s, n, aabb, b.stats, b.owner_count, b.owner_cursor,
+	           (uint32_t)owner_buckets(n, b.owner_shift), shift ? 1 : 0);
+}
+
+void launch_all_pairs(uint64_t n, const float *aabb, const BpBuffers &b, cudaStream_t s) {
+	launch_pdl(k_all_pairs, dim3(blocks_for(n), (unsigned)((n + kAllCols - 1) / kAllCols)), dim3(kNT), 0, s, (uint32_t)n,
+	           b.stats, aabb, b.owner_count, b.pairs_tmp, b.pair_cap, b.owner_shift);
 }
 
 void launch_chain_check(const BpBuffers &b, uint32_t g_max, cudaStream_t s) {

@@ -124,6 +124,7 @@ struct cc_ctx {
 	int chain_wait = 0;  // calls on sorted cells left before the chains are tried again
 	uint64_t last_E = 0, last_P = 0, last_tmp = 0, last_mask = 0;  // last_tmp: pairs that went through pairs_tmp
 	bool sized = false;  // a pass has set these
+	bool all_pairs = false;  // this call tests all pairs of boxes
 	bool rank_now = false;  // this call's overlapped pairs are few: ordered by counting
 	int last_dim[3] = {0, 0, 0};
 	// owner buckets of the pair sort (BpBuffers::owner_shift / key_bits), chosen
@@ -442,7 +443,9 @@ cc_status prepare(cc_ctx *c, uint64_t n, uint64_t np_cap, uint64_t g_override = 
 	c->gp.g_max = g_override ? (uint32_t)g_override : g_max_for(n);
 	c->dense_skip = c->last_dense == 0;
 	c->chain = chain_enabled() && c->chain_state != cc_ctx::kChainNo && n < ((uint64_t)1 << 31);
-	c->chain_check = c->chain && c->chain_state == cc_ctx::kChainUnknown;
+	// (a scene of nearly all pairs is left to the dense cells, which write them in order)
+	c->all_pairs = c->chain && !g_override && n <= kAllPairsBodies && c->last_P <= 32 * n;
+	c->chain_check = c->chain && !c->all_pairs && c->chain_state == cc_ctx::kChainUnknown;
 	c->direct = !c->chain && !c->dense_skip;
 	choose_owner_shift(c, n);
 	if (g_override && c->direct) {  // a batch counts its scenes' pairs by owner if its output is too small
@@ -533,6 +536,16 @@ uint64_t hint_P(const cc_ctx *c, uint64_t n) { return pow2ceil(std::max<uint64_t
 void enqueue_pairs(cc_ctx *c, uint64_t n, float *aabb, uint64_t entries_hint, cudaStream_t s, bool shift) {
 	BpBuffers b = bp_buffers(c);
 	const uint32_t gmax = c->gp.g_max;
+	if (c->all_pairs) {
+		{
+			StageMark m(c, ST_COUNT, s);
+			launch_shift(n, aabb, b, s, shift);
+		}
+		StageMark m(c, ST_PAIR_TEST, s);
+		launch_all_pairs(n, aabb, b, s);
+		c->launches += 2;
+		return;
+	}
 	if (!b.pre_zeroed) cudaMemsetAsync(b.cell_count, 0, sizeof(uint32_t) * gmax, s);
 	if (c->chain) {
 		{
@@ -716,7 +729,7 @@ ZeroList pass_zero_list(cc_ctx *c, bool ov) {
 	zero.p[2] = ptr<uint32_t>(c->np_classes);
 	zero.words[2] = 2 * kNpClasses + 1;
 	zero.p[3] = ptr<uint32_t>(c->cell_count);
-	zero.words[3] = c->gp.g_max;
+	zero.words[3] = c->all_pairs ? 0 : c->gp.g_max;
 	if (ov && !c->rank_now) {
 		zero.p[4] = ptr<uint32_t>(c->np_hkeys);
 		zero.words[4] = 2 * c->np_hslots;
@@ -827,7 +840,8 @@ void remember(cc_ctx *c) {
 	// chains while no cell is crowded; back to them once sorted cells show none
 	// (which they tell through their dense cells, so a raised threshold makes
 	// them blind) or some calls after a box over too many cells
-	if (c->chain) {
+	if (c->all_pairs) {  // tells nothing of the cells
+	} else if (c->chain) {
 		c->chain_state = c->last_dense ? cc_ctx::kChainNo : cc_ctx::kChainOk;
 		c->chain_wait = c->gp.dense_cell <= kChainLong ? 0 : kChainWait;
 	} else if (c->last_dense == 0 && --c->chain_wait < 0) {
@@ -999,7 +1013,7 @@ cc_status collide_enqueue(cc_ctx *c, const cc_scene &sc, int gx, int gy, int gz,
 	k.hslots = k.ov == 1 ? c->np_hslots : 0;
 	k.fused = c->fused_now ? 1 : 0;
 	k.dense_skip = c->dense_skip ? 1 : 0;
-	k.chain = (c->chain ? 1 : 0) + (c->chain_check ? 2 : 0);
+	k.chain = (c->chain ? 1 : 0) + (c->chain_check ? 2 : 0) + (c->all_pairs ? 4 : 0);
 	return run_graphed(c, c->g_collide, &k, sizeof(k), enqueue_all, s);
 }
 
@@ -1753,7 +1767,7 @@ cc_status batch_impl(cc_ctx *c, const cc_batch *bt, int gx, int gy, int gz, floa
 	k.hslots = k.ov == 1 ? c->np_hslots : 0;
 	k.fused = c->fused_now ? 1 : 0; k.dense_skip = c->dense_skip ? 1 : 0;
 	k.dims[0] = gx; k.dims[1] = gy; k.dims[2] = gz; k.prec = c->np_precision; k.want = want_offsets ? 1 : 0;
-	k.chain = (c->chain ? 1 : 0) + (c->chain_check ? 2 : 0);
+	k.chain = (c->chain ? 1 : 0) + (c->chain_check ? 2 : 0) + (c->all_pairs ? 4 : 0);
 	k.env = envelope; k.gp = c->call_gp;
 	CC_TRY(run_graphed(c, c->g_batch, &k, sizeof(k), enqueue_all, s));
 	auto copy_back = [&]() -> cc_status {

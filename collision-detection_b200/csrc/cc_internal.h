@@ -219,6 +219,11 @@ void launch_pair_test(uint64_t n, const BpBuffers &b, uint64_t entries_hint, cud
 // chains above kChainLong and makes the walk return at once if there are any;
 // without it the walk itself notes them, and gives up (kErrLongChain) only on
 // chains many times as long.
+// Small scenes: the in-place shift alone (with the owner counts zeroed), then
+// every box against every later one.
+constexpr uint64_t kAllPairsBodies = 2048;
+void launch_shift(uint64_t n, float *aabb, const BpBuffers &b, cudaStream_t s, bool shift);
+void launch_all_pairs(uint64_t n, const float *aabb, const BpBuffers &b, cudaStream_t s);
 void launch_link(uint64_t n, float *aabb, const BpBuffers &b, cudaStream_t s, bool shift = true);
 void launch_chain_check(const BpBuffers &b, uint32_t g_max, cudaStream_t s);
 void launch_walk(uint64_t n, const BpBuffers &b, uint64_t entries_hint, cudaStream_t s);
