@@ -1362,10 +1362,11 @@ __device__ __forceinline__ void sort_bucket_pair(unsigned long long *__restrict_
 // k_dense_emit) are merged instead of sorted: adjacent runs pairwise, every key
 // placed by a binary search in the partner run, between two halves of shared
 // memory. At 4.2M clustered spheres (246M pairs) the bitonic tiers alone take 3.8
-// ms at 15 warp instructions a key, merges and what is left to them 3.3 ms.
+// ms at 15 warp instructions a key, merges and what is left to them 2.9 ms.
 // Returns false, with the bucket untouched, above kMaxRuns runs. NT threads
 // work together, Sync separates the steps; buf holds 2 * cap keys.
 constexpr uint32_t kMaxRuns = 32;
+constexpr int kSearch = 2;  // 4.2M clustered spheres, the mid tier: one 3.34 ms, two 2.89, four 3.06, eight 3.77
 struct Runs {
 	uint32_t start[kMaxRuns + 2], count;
 };
@@ -1377,7 +1378,14 @@ __device__ __forceinline__ bool merge_runs(unsigned long long *__restrict__ out,
 		runs.count = 1;
 		runs.start[0] = 0;
 	}
-	for (uint32_t e = t; e < len; e += NT) src[e] = pack_key<kPack>(out[beg + e], kp);
+	for (uint32_t e0 = t; e0 < len; e0 += 8 * NT) {  // eight loads in flight
+		unsigned long long v[8];
+#pragma unroll
+		for (int q = 0; q < 8; q++) v[q] = e0 + q * NT < len ? out[beg + e0 + q * NT] : 0ull;
+#pragma unroll
+		for (int q = 0; q < 8; q++)
+			if (e0 + q * NT < len) src[e0 + q * NT] = pack_key<kPack>(v[q], kp);
+	}
 	sync();
 	for (uint32_t e = t; e < len; e += NT)
 		if (e && src[e] < src[e - 1]) {  // a run starts here; their order is restored below
@@ -1400,16 +1408,26 @@ __device__ __forceinline__ bool merge_runs(unsigned long long *__restrict__ out,
 	while (R > 1) {
 		for (uint32_t r = 0; r < R; r += 2) {
 			const uint32_t s0 = runs.start[r], s1 = runs.start[r + 1], s2 = r + 1 < R ? runs.start[r + 2] : s1;
-			for (uint32_t i = s0 + t; i < s2; i += NT) {
-				const uint32_t key = src[i];
-				const bool first = i < s1;
-				uint32_t lo = first ? s1 : s0, hi = first ? s2 : s1;
-				while (lo < hi) {
-					const uint32_t mid = (lo + hi) >> 1;
-					if (src[mid] < key) lo = mid + 1;
-					else hi = mid;
+			// branch-free searches of kSearch keys side by side: a search is a chain of
+			// shared loads
+			const uint32_t longer = max(s1 - s0, s2 - s1);
+			const uint32_t top = longer ? 1u << (31 - __clz((int)longer)) : 0u;
+			for (uint32_t i0 = s0 + t; i0 < s2; i0 += kSearch * NT) {
+				uint32_t key[kSearch], lo[kSearch], end[kSearch];
+#pragma unroll
+				for (int q = 0; q < kSearch; q++) {
+					const uint32_t i = i0 + q * NT;
+					key[q] = i < s2 ? src[i] : 0u;
+					lo[q] = i < s1 ? s1 : s0;
+					end[q] = i < s1 ? s2 : s1;
 				}
-				dst[i + lo - s1] = key;  // place in its own run + smaller keys of the other
+				for (uint32_t step = top; step; step >>= 1)
+#pragma unroll
+					for (int q = 0; q < kSearch; q++)
+						if (lo[q] + step <= end[q] && src[lo[q] + step - 1] < key[q]) lo[q] += step;
+#pragma unroll
+				for (int q = 0; q < kSearch; q++)
+					if (i0 + q * NT < s2) dst[i0 + q * NT + lo[q] - s1] = key[q];  // place in its own run + smaller keys of the other
 			}
 		}
 		const uint32_t half = (R + 1) / 2;
