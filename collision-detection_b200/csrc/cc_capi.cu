@@ -640,7 +640,7 @@ void enqueue_np(cc_ctx *c, const NpArgs &a, uint64_t P_cap, const unsigned long 
 		launch_np_compact(P_cap, P_dev, sc, reinterpret_cast<long long *>(a.pairs), a.norm, a.cpta, a.cptb, a.depth,
 		                  a.bids, &ptr<DevStats>(c->stats)->contacts, P_dev ? hint_P(c, a.n) : P_cap, s);
 	}
-	c->launches += c->np_precision == CC_NP_EXACT ? 2 : 3;  // class grouping (fast modes), MPR, compaction
+	c->launches += 1 + mpr_launches(P_cap, c->np_precision, P_dev ? hint_P(c, a.n) : P_cap);  // MPR, compaction
 }
 
 // The step after the pair test with the narrowphase overlapped: a short list
@@ -665,7 +665,7 @@ cc_status enqueue_sort_and_np_overlapped(cc_ctx *c, uint64_t n, const NpArgs &a,
 			launch_np_rank(d, b.pair_cap, pairs_cap, sc, reinterpret_cast<long long *>(a.pairs), a.norm, a.cpta, a.cptb,
 			               a.depth, a.bids, hint_P(c, n), s);
 		}
-		c->launches += c->np_precision == CC_NP_EXACT ? 2 : 3;  // class grouping (fast modes), MPR, order
+		c->launches += 1 + mpr_launches(pairs_cap, c->np_precision, hint_P(c, n));  // MPR, order
 		return CC_OK;
 	}
 	sc.hkeys = ptr<unsigned long long>(c->np_hkeys);
@@ -691,7 +691,7 @@ cc_status enqueue_sort_and_np_overlapped(cc_ctx *c, uint64_t n, const NpArgs &a,
 		           a.active, a.pos, a.rot, a.envelope, reinterpret_cast<const long long *>(b.pairs_tmp), sc,
 		           c->np_precision, hint_P(c, n), t, beside);
 	}
-	c->launches += c->np_precision == CC_NP_EXACT ? 1 : 2;  // class grouping (fast modes), MPR
+	c->launches += mpr_launches(pairs_cap, c->np_precision, hint_P(c, n));
 	if (!beside) {
 		CC_CUDA(c, cudaEventRecord(c->ev_join, t));
 		if (!c->fused_now) {

@@ -383,7 +383,7 @@ struct NpScratch {
 	uint64_t *status;       // look-back tiles of the flag scan
 	uint32_t *ticket;
 	uint32_t *err;
-	uint32_t *order;        // P: pair indices grouped by (type A, type B)
+	uint32_t *order;        // P: pair indices grouped by (type A, type B); null for the MPR: not grouped
 	uint32_t *classes;      // 2 * kNpClasses counters + the work-queue counter (zeroed per call)
 	uint32_t *queue;        // the exact MPR's work queue (zeroed per call)
 	bool pre_zeroed = false;  // classes, queue, status and ticket already zeroed for this pass
@@ -414,6 +414,8 @@ void launch_mpr(uint64_t P_cap, const unsigned long long *P_dev, uint64_t n, con
                 const float *B, const float *C, const float *R, const uint32_t *ID, uint64_t nb,
                 const uint8_t *active, const float *pos, const float *rot, float envelope, const long long *pairs,
                 const NpScratch &sc, int precision, uint64_t P_hint, cudaStream_t s, bool beside = false);
+// Its launches: the MPR and, in the fast modes on longer lists, the class grouping.
+int mpr_launches(uint64_t P_cap, int precision, uint64_t P_hint);
 // The exact variant lives in its own -fmad=false translation unit.
 // Blocks of the exact MPR kernel resident per SM.
 int mpr_exact_resident_blocks();
@@ -428,7 +430,7 @@ void launch_np_compact(uint64_t P_cap, const unsigned long long *P_dev, const Np
 // follows; every row's place in the hit-first order is counted. Sets
 // stats->np_n (0: the list does not fit pair_cap or out_cap) and
 // stats->contacts; above kRankRoom pairs only kErrLongList.
-constexpr uint64_t kRankPairs = 4096, kRankRoom = 8192;
+constexpr uint64_t kRankPairs = 4096, kRankRoom = 6144;
 void launch_np_rank(DevStats *stats, uint64_t pair_cap, uint64_t out_cap, const NpScratch &sc, long long *pairs,
                     float *norm, float *cpta, float *cptb, float *depth, int32_t *bids, uint64_t P_hint, cudaStream_t s);
 // The overlapped narrowphase's compaction: the MPR ran on the unsorted pairs

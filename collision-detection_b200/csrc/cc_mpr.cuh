@@ -592,7 +592,7 @@ __device__ __forceinline__ void run(uint64_t P_cap, const unsigned long long *P_
 				drained = (uint64_t)base + __popc(idle) >= P;
 				const uint64_t j = (uint64_t)base + __popc(idle & lt);
 				if (wants && j < P) {
-					const uint32_t i = sc.order[j];
+					const uint32_t i = sc.order ? sc.order[j] : (uint32_t)j;
 					if (!start_pair(L, i, n, T, A, B, C, R, ID, nb, active, pos, rot, envelope, pairs, sc)) L.st = kIdle;
 				}
 			}

@@ -420,6 +420,15 @@ unsigned np_coop_max_blocks() {
 	return m;
 }
 
+// Up to kUngrouped pairs a warp of the fast modes' grid has one or two, and grouping
+// them costs more than their divergence (steps, us, grouped and not: 16K spheres with
+// 600 pairs in fp64 56 and 44, 600 mixed shapes with 540 in fp64 81 and 77, in mixed
+// 81 and 72; but 130K mixed shapes with 3.4K pairs in fp64 106 and 115).
+constexpr uint64_t kUngrouped = 1024;
+int mpr_launches(uint64_t P_cap, int precision, uint64_t P_hint) {
+	return precision == 0 || std::min<uint64_t>(P_hint ? P_hint : P_cap, P_cap) <= kUngrouped ? 1 : 2;
+}
+
 void launch_mpr(uint64_t P_cap, const unsigned long long *P_dev, uint64_t n, const int32_t *T, const float *A,
                 const float *B, const float *C, const float *R, const uint32_t *ID, uint64_t nb,
                 const uint8_t *active, const float *pos, const float *rot, float envelope, const long long *pairs,
@@ -440,11 +449,14 @@ void launch_mpr(uint64_t P_cap, const unsigned long long *P_dev, uint64_t n, con
 		                 T, A, B, C, R, ID, nb, active, pos, rot, envelope, pairs, sc, s, beside);
 		return;
 	}
-	{  // group the pairs by shape-type combination; the last word is the work queue
+	NpScratch scm = sc;
+	if (!sc.pre_zeroed) cudaMemsetAsync(sc.classes, 0, (2 * kNpClasses + 1) * sizeof(uint32_t), s);
+	if (mpr_launches(P_cap, precision, P_hint) == 1) {
+		scm.order = nullptr;
+	} else {  // group the pairs by shape-type combination; the last word is the work queue
 		// blocks for the expected pair count (the loops stride over the device count)
 		const unsigned g = (unsigned)std::max<uint64_t>(
 		    1, std::min<uint64_t>((Pe + kCoopNT - 1) / kCoopNT, std::min<uint64_t>(np_coop_max_blocks(), kNpCoopBlocks)));
-		if (!sc.pre_zeroed) cudaMemsetAsync(sc.classes, 0, (2 * kNpClasses + 1) * sizeof(uint32_t), s);
 		launch_coop(k_np_classes, g, s, P_cap, P_dev, n, T, pairs, sc.classes, sc.order,
 		            reinterpret_cast<GridBarrier *>(sc.bar_classes), sc.err);
 	}
@@ -456,10 +468,10 @@ void launch_mpr(uint64_t P_cap, const unsigned long long *P_dev, uint64_t n, con
 	                                                   (uint64_t)kNumSMs * mpr_resident_blocks(precision));
 	if (precision == 2)
 		launch_pdl(k_mpr<float>, dim3(grid), dim3(kNT), 0, s, P_cap, P_dev, n, T, A, B, C, R, ID, nb, active, pos, rot, envelope, pairs,
-		                                  sc);
+		           scm);
 	else
 		launch_pdl(k_mpr<double>, dim3(grid), dim3(kNT), 0, s, P_cap, P_dev, n, T, A, B, C, R, ID, nb, active, pos, rot, envelope, pairs,
-		                                   sc);
+		           scm);
 }
 
 void launch_np_compact(uint64_t P_cap, const unsigned long long *P_dev, const NpScratch &sc, long long *pairs,
@@ -496,10 +508,7 @@ void launch_np_compact_sorted(uint64_t P_cap, const unsigned long long *P_dev, c
 
 void launch_np_rank(DevStats *stats, uint64_t pair_cap, uint64_t out_cap, const NpScratch &sc, long long *pairs,
                     float *norm, float *cpta, float *cptb, float *depth, int32_t *bids, uint64_t P_hint, cudaStream_t s) {
-	// keys for twice the expected count
-	static const bool ok = cudaFuncSetAttribute(k_np_rank, cudaFuncAttributeMaxDynamicSharedMemorySize,
-	                                            (int)(kRankRoom * sizeof(unsigned long long))) == cudaSuccess;
-	(void)ok;  // a launch without the room fails and is reported
+	// keys for twice the expected count, within the 48 KB that need no opt-in (which is per device)
 	const uint32_t room = (uint32_t)std::min<uint64_t>(kRankRoom, std::max<uint64_t>(1024, 2 * P_hint));
 	constexpr unsigned rows = (kRankNT / 32) * kRankRows;
 	const unsigned grid = (unsigned)std::max<uint64_t>(1, (std::min(P_hint, kRankRoom) + rows - 1) / rows);
