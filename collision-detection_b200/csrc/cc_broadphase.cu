@@ -1569,7 +1569,7 @@ __global__ void __launch_bounds__(kFusedNT, 4) k_owner_sort_fused(DevStats *stat
                                                              const uint32_t *__restrict__ owner_count,
                                                              uint32_t *__restrict__ cursor, uint32_t nbk,
                                                              unsigned long long *__restrict__ out, int oshift,
-                                                             KeyPack kp) {
+                                                             KeyPack kp, uint32_t *host_stats) {
 	pdl_trigger();  // (every block is resident: a cooperative launch)
 	extern __shared__ uint32_t fsm[];  // off[nbk + 1], then kFusedSeg keys of the block tier
 	__shared__ unsigned long long scan_sm[40];
@@ -1577,7 +1577,7 @@ __global__ void __launch_bounds__(kFusedNT, 4) k_owner_sort_fused(DevStats *stat
 	const unsigned long long P = stats->pairs;
 	const bool fits = P <= pair_cap && P <= out_cap && P < 0xffffffffull;
 	if (blockIdx.x == 0 && threadIdx.x == 0) stats->np_n = fits ? P : 0ull;
-	if (!fits) return;  // uniform over the grid: no block reaches the barrier
+	if (!fits) return report_by_last(stats, host_stats);  // uniform over the grid: no block reaches the barrier
 	// 1. exclusive scan of the bucket counts: coalesced loads into shared
 	// memory (all in flight at once), then one contiguous run per thread
 	copy_words_to_shared<kFusedNT>(off, owner_count, nbk);
@@ -1643,6 +1643,7 @@ __global__ void __launch_bounds__(kFusedNT, 4) k_owner_sort_fused(DevStats *stat
 		for (int i = threadIdx.x; (uint32_t)i < len; i += kFusedNT) out[beg + i] = unpack_key<kPack>(keys[i], (uint32_t)b, kp);
 		__syncthreads();
 	}
+	report_by_last(stats, host_stats);
 }
 
 // ---------------------------------------------------------------- bin list
@@ -2018,7 +2019,7 @@ bool fused_sort_enabled() {
 }
 
 void launch_owner_sort_fused(uint64_t n, uint64_t out_cap, unsigned long long *out, uint64_t P_hint, const BpBuffers &b,
-                             cudaStream_t s) {
+                             uint32_t *host_stats, cudaStream_t s) {
 	const uint32_t nbk = (uint32_t)owner_buckets(n, b.owner_shift);
 	const size_t smem = sizeof(uint32_t) * ((size_t)nbk + 1 + kFusedSeg);
 	static const int per_sm = [] {
@@ -2037,7 +2038,7 @@ void launch_owner_sort_fused(uint64_t n, uint64_t out_cap, unsigned long long *o
 	int oshift = b.owner_shift;
 	KeyPack kp{b.owner_shift, b.key_bits};
 	DevStats *st = b.stats;
-	void *args[] = {&st, &pair_cap, &out_cap, &tmp, &cnt, &cur, (void *)&nbk, &out, &oshift, &kp};
+	void *args[] = {&st, &pair_cap, &out_cap, &tmp, &cnt, &cur, (void *)&nbk, &out, &oshift, &kp, &host_stats};
 	const void *k = kp.shift ? (const void *)k_owner_sort_fused<true> : (const void *)k_owner_sort_fused<false>;
 	cudaLaunchCooperativeKernel(k, dim3(grid), dim3(kFusedNT), args, smem, s);
 }

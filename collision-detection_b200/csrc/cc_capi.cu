@@ -125,6 +125,7 @@ struct cc_ctx {
 	uint64_t last_E = 0, last_P = 0, last_tmp = 0, last_mask = 0;  // last_tmp: pairs that went through pairs_tmp
 	bool sized = false;  // a pass has set these
 	bool all_pairs = false;  // this call tests all pairs of boxes
+	bool report_now = false, report_sort = false;  // this call's last kernel, the contacts' order or the owner sort, writes h_stats
 	bool rank_now = false;  // this call's overlapped pairs are few: ordered by counting
 	int last_dim[3] = {0, 0, 0};
 	// owner buckets of the pair sort (BpBuffers::owner_shift / key_bits), chosen
@@ -309,6 +310,15 @@ cc_status read_stats(cc_ctx *c, cudaStream_t s) {
 	return CC_OK;
 }
 
+// The same where the call's last kernel may have written them itself.
+cc_status await_stats(cc_ctx *c, cudaStream_t s) {
+	const bool reported = c->report_now || c->report_sort;
+	c->report_now = c->report_sort = false;
+	if (!reported) return read_stats(c, s);
+	CC_CUDA(c, cudaStreamSynchronize(s));
+	return CC_OK;
+}
+
 cc_status device_err(cc_ctx *c) {
 	const uint32_t e = c->h_stats->err;
 	if (e & (kErrNonFinite | kErrInverted))
@@ -446,6 +456,7 @@ uint64_t with_slack(uint64_t used, uint64_t room) { return used + used / 16 <= r
 // narrowphase scratch for np_cap pairs. Buffers only grow; every public call
 // ends with a synchronize, so nothing in flight uses a buffer replaced here.
 cc_status prepare(cc_ctx *c, uint64_t n, uint64_t np_cap, uint64_t g_override = 0) {
+	c->report_now = c->report_sort = false;  // (left by a call that failed before its wait)
 	c->gp.g_max = g_override ? (uint32_t)g_override : g_max_for(n);
 	c->dense_skip = c->last_dense == 0;
 	c->chain = chain_enabled() && c->chain_state != cc_ctx::kChainNo && n < ((uint64_t)1 << 31);
@@ -506,6 +517,8 @@ NpScratch np_scratch(cc_ctx *c) {
 	sc.order = ptr<uint32_t>(c->np_order);
 	sc.classes = ptr<uint32_t>(c->np_classes);
 	sc.queue = &ptr<DevStats>(c->stats)->np_queue;
+	sc.stats = ptr<DevStats>(c->stats);
+	sc.host_stats = c->report_now ? reinterpret_cast<uint32_t *>(c->h_stats) : nullptr;
 	sc.pre_zeroed = c->pass_zeroed;
 	return sc;
 }
@@ -600,7 +613,7 @@ void enqueue_emit(cc_ctx *c, uint64_t n, unsigned long long *out, uint64_t out_c
 	BpBuffers b = bp_buffers(c);
 	if (c->fused_now) {
 		StageMark m(c, ST_SEGSORT, s);
-		launch_owner_sort_fused(n, out_cap, out, hint_P(c, n), b, s);
+		launch_owner_sort_fused(n, out_cap, out, hint_P(c, n), b, c->report_sort ? reinterpret_cast<uint32_t *>(c->h_stats) : nullptr, s);
 		c->launches += 1;
 		return;
 	}
@@ -963,6 +976,7 @@ cc_status collide_enqueue(cc_ctx *c, const cc_scene &sc, int gx, int gy, int gz,
 	CC_TRY(prepare(c, n, pairs_cap));
 	bool ov;
 	CC_TRY(overlap_prepare(c, n, pairs_cap, ov));
+	c->report_now = graphs && pairs_cap;  // (a submitted step has a copy of its own)
 	DevStats *d = ptr<DevStats>(c->stats);
 	const int grid[3] = {gx, gy, gz};
 	unsigned long long *out = reinterpret_cast<unsigned long long *>(pairs);
@@ -1179,9 +1193,10 @@ cc_status collide_verlet(cc_ctx *c, const cc_scene &sc, int gx, int gy, int gz, 
 			zero.words[2] = 2 * kNpClasses + 1;
 			CC_TRY(enqueue_front(s, zero));
 		}
+		c->report_now = pairs_cap != 0;
 		CC_TRY(enqueue_tail(s));
 		CC_TRY(check_launch(c));
-		CC_TRY(read_stats(c, s));
+		CC_TRY(await_stats(c, s));
 		CC_TRY(device_err(c));
 		if (c->h_stats->vbad) {
 			// moved too far: redo as a rebuild, from the caller's RECT / TRIANGLEMESH boxes (the
@@ -1237,7 +1252,7 @@ cc_status collide_dev(cc_ctx *c, const cc_scene &sc, int gx, int gy, int gz, flo
 		CC_TRY(check_launch(c));
 	}
 	const BpBuffers b = bp_buffers(c);
-	CC_TRY(read_stats(c, s));
+	CC_TRY(await_stats(c, s));
 	// what went out is the result unless something is redone below
 	if (push) *pushed = complete_pass(*c->h_stats, b.entry_cap, b.pair_cap, c->direct, pairs_cap);
 	return collide_finish(c, sc, envelope, aabb, pairs, pairs_cap, norm, cpta, cptb, depth, bids, n_pairs, n_contacts, s);
@@ -1502,10 +1517,12 @@ cc_status cc_broadphase(cc_ctx *c, uint64_t n, float *aabb, int gx, int gy, int 
 	enqueue_search(c, n, aabb, s);
 	unsigned long long *out = reinterpret_cast<unsigned long long *>(pairs);
 	const uint64_t cap = pairs ? pairs_cap : 0;
+	c->report_now = false;
+	c->report_sort = cap && c->fused_now;
 	if (cap) enqueue_emit(c, n, out, cap, s);
 	c->pass_zeroed = false;
 	CC_TRY(check_launch(c));
-	CC_TRY(read_stats(c, s));
+	CC_TRY(await_stats(c, s));
 	CC_TRY(device_err(c));
 	CC_TRY(settle(c, n, aabb, cap ? out : nullptr, cap, nullptr, s));
 	remember(c);
@@ -1633,10 +1650,12 @@ cc_status cc_narrowphase(cc_ctx *c, uint64_t n, const int32_t *T, const float *A
 	CC_CUDA(c, cudaMemsetAsync(c->stats.p, 0, sizeof(DevStats), s));
 	const NpArgs a = {n, nb, T, A, B, C, R, ID, active, pos, rot, envelope, pairs, norm, cpta, cptb, depth, bids};
 	c->pass_zeroed = c->np_precision == CC_NP_EXACT;  // its queue, with the counters above
+	c->report_sort = false;
+	c->report_now = true;
 	enqueue_np(c, a, n_pairs, nullptr, s);
 	c->pass_zeroed = false;
 	CC_TRY(check_launch(c));
-	CC_TRY(read_stats(c, s));
+	CC_TRY(await_stats(c, s));
 	if (c->h_stats->err & kErrBadIndex)
 		return set_err(c, CC_ERR_INVALID_INPUT, "a pair index is >= n or a body id is >= nb");
 	if (c->h_stats->err & kErrSpinLimit) return set_err(c, CC_ERR_INTERNAL, "device-side look-back wait gave up");

@@ -258,6 +258,7 @@ __global__ void __launch_bounds__(kCoopNT) k_np_compact(uint64_t P_cap, const un
 		if (!kSorted) sc.pos[P] = nh;
 		if (contacts_out) *contacts_out = nh;
 	}
+	report_by_last(sc.stats, sc.host_stats);
 	for (uint64_t t0 = c0; t0 < c1; t0 += kCoopNT) {
 		const uint64_t i = t0 + threadIdx.x;
 		if (!one && i < c1) {
@@ -311,16 +312,22 @@ __global__ void __launch_bounds__(kRankNT) k_np_rank(DevStats *stats, uint64_t p
                                                      float *__restrict__ cpta, float *__restrict__ cptb,
                                                      float *__restrict__ depth, int32_t *__restrict__ bids) {
 	pdl_begin();
+	// the pass's counters, final once the first block has added its own, to the host
+	const auto report = [&] {
+		if (blockIdx.x != 0 || !sc.host_stats) return;
+		__syncthreads();
+		report_stats(stats, sc.host_stats);
+	};
 	constexpr unsigned long long kMiss = 1ull << 63;
 	extern __shared__ unsigned long long rank_keys[];
 	const unsigned long long P = stats->pairs;
 	const bool fits = P <= pair_cap && P <= out_cap, first = blockIdx.x == 0 && threadIdx.x == 0;
-	if (first) stats->np_n = fits ? P : 0ull;
-	if (!fits) return;
-	if (P > room) {
-		if (first) atomicOr(&stats->err, (uint32_t)kErrLongList);
-		return;
+	if (first) {
+		stats->np_n = fits ? P : 0ull;
+		if (fits && P > room) atomicOr(&stats->err, (uint32_t)kErrLongList);
+		__threadfence();
 	}
+	if (!fits || P > room) return report();
 	const uint32_t n = (uint32_t)P, padded = (n + 31u) & ~31u;
 	uint32_t hits = 0;
 	for (uint32_t i0 = threadIdx.x; i0 < padded; i0 += 8 * kRankNT) {  // eight keys a thread in flight
@@ -341,8 +348,12 @@ __global__ void __launch_bounds__(kRankNT) k_np_rank(DevStats *stats, uint64_t p
 	}
 	hits = __reduce_add_sync(0xffffffffu, hits);
 	const uint32_t lane = threadIdx.x & 31;
-	if (blockIdx.x == 0 && lane == 0 && hits) atomicAdd(&stats->contacts, (unsigned long long)hits);
+	if (blockIdx.x == 0 && lane == 0 && hits) {
+		atomicAdd(&stats->contacts, (unsigned long long)hits);
+		__threadfence();
+	}
 	__syncthreads();
+	report();
 	const uint32_t step = gridDim.x * (kRankNT / 32) * kRankRows;
 	for (uint32_t i0 = (blockIdx.x * (kRankNT / 32) + (threadIdx.x >> 5)) * kRankRows; i0 < n; i0 += step) {
 		unsigned long long own[kRankRows];
