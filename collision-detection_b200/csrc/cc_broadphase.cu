@@ -404,7 +404,7 @@ __global__ void __launch_bounds__(kNT, 5) k_pair_test(const DevStats *stats, con
 			const uint64_t end = min((uint64_t)cell_start[c + 1], entry_cap);
 			my_n = (int)(end > e + 1 ? end - e - 1 : 0);
 			if (end - beg > dense_cell) {
-				if (dense) {  // left to k_pair_test_dense
+				if (dense) {  // left to k_dense_test
 					my_n = 0;
 					if (e == beg) {
 						const uint32_t k = (uint32_t)(end - beg), chunks = (k + kNT - 1) / kNT;

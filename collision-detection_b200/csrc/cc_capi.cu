@@ -89,7 +89,7 @@ struct cc_ctx {
 	// descriptor table of cc_perturb_scenes
 	Buf pt_desc;
 	// overlapped narrowphase (cc_set_narrowphase_overlap): the MPR on the
-	// unsorted pairs on np_stream while the main stream sorts them; the
+	// unsorted pairs, beside their sort (in the fast modes on np_stream); the
 	// contact hash (keys, values) sized for 4x the expected pair count
 	bool np_overlap = true;
 	cudaStream_t np_stream = nullptr;
