@@ -209,7 +209,7 @@ __device__ __forceinline__ uint32_t hash_find(const NpScratch &sc, unsigned long
 
 // kSorted: the MPR ran on the unsorted pairs (overlapped with their sort) and each
 // sorted key in `pairs` finds its result through the contact hash; else results
-// and sc.pairs are in pair order. tmp: the sorted keys of chunks of several tiles.
+// and sc.pairs are in pair order. tmp: receives the sorted keys.
 template <bool kSorted>
 __global__ void __launch_bounds__(kCoopNT) k_np_compact(uint64_t P_cap, const unsigned long long *P_dev, NpScratch sc,
                                                    long long *__restrict__ pairs, unsigned long long *__restrict__ tmp,
@@ -231,10 +231,8 @@ __global__ void __launch_bounds__(kCoopNT) k_np_compact(uint64_t P_cap, const un
 		if constexpr (kSorted) {
 			t = hash_find(sc, key);
 			hit = t != kNoHit;
-			if (!one) {
-				tmp[i] = key;
-				sc.order[i] = (uint32_t)t;
-			}
+			tmp[i] = key;  // also where the block does not read it again: a full hash has the sorted list restored from it
+			if (!one) sc.order[i] = (uint32_t)t;
 		} else {
 			hit = sc.flag[i] != 0;
 			t = hit ? i : (uint64_t)kNoHit;
