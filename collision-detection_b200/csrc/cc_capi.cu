@@ -104,6 +104,9 @@ struct cc_ctx {
 	// retained broadphase result (owner buckets not yet scattered)
 	bool retained = false;
 	uint64_t retained_n = 0, retained_P = 0;
+	// the dense cells' part of it: their emission reads these counters, which
+	// another call in between may have cleared (dense_items; mask_words, tmp_pairs)
+	uint64_t retained_dense = 0, retained_split[2] = {0, 0};
 	bool retained_fused = false, retained_direct = false;
 	// this call's pairs are emitted by the fused owner sort (one scene, not
 	// incremental, few owner buckets); set by prepare and the call
@@ -874,6 +877,9 @@ void retain(cc_ctx *c, uint64_t n, uint64_t P) {
 	c->retained = true;
 	c->retained_n = n;
 	c->retained_P = P;
+	c->retained_dense = c->h_stats->dense_items;
+	c->retained_split[0] = c->h_stats->mask_words;
+	c->retained_split[1] = c->h_stats->tmp_pairs;
 	c->retained_fused = c->fused_now;
 	c->retained_direct = c->direct;
 }
@@ -884,6 +890,14 @@ cc_status emit_retained(cc_ctx *c, unsigned long long *out, uint64_t cap, cudaSt
 	DevStats *d = ptr<DevStats>(c->stats);
 	c->h_word[0] = c->retained_P;
 	CC_CUDA(c, cudaMemcpyAsync(&d->pairs, c->h_word, sizeof(unsigned long long), cudaMemcpyHostToDevice, s));
+	if (c->retained_direct) {
+		static_assert(offsetof(DevStats, tmp_pairs) == offsetof(DevStats, mask_words) + 8, "copied together");
+		c->h_word[1] = c->retained_dense;
+		c->h_word[2] = c->retained_split[0];
+		c->h_word[3] = c->retained_split[1];
+		CC_CUDA(c, cudaMemcpyAsync(&d->dense_items, c->h_word + 1, 8, cudaMemcpyHostToDevice, s));
+		CC_CUDA(c, cudaMemcpyAsync(&d->mask_words, c->h_word + 2, 16, cudaMemcpyHostToDevice, s));
+	}
 	CC_CUDA(c, cudaMemsetAsync(&d->big_segments, 0, 3 * sizeof(unsigned long long), s));
 	CC_CUDA(c, cudaMemsetAsync(&d->err, 0, sizeof(uint32_t), s));
 	c->fused_now = c->retained_fused;
