@@ -107,7 +107,7 @@ struct cc_ctx {
 	// the dense cells' part of it: their emission reads these counters, which
 	// another call in between may have cleared (dense_items; mask_words, tmp_pairs)
 	uint64_t retained_dense = 0, retained_split[2] = {0, 0};
-	bool retained_fused = false, retained_direct = false;
+	bool retained_fused = false, retained_direct = false, retained_scan = false;
 	// this call's pairs are emitted by the fused owner sort (one scene, not
 	// incremental, few owner buckets); set by prepare and the call
 	bool fused_now = false;
@@ -460,6 +460,7 @@ uint64_t with_slack(uint64_t used, uint64_t room) { return used + used / 16 <= r
 // ends with a synchronize, so nothing in flight uses a buffer replaced here.
 cc_status prepare(cc_ctx *c, uint64_t n, uint64_t np_cap, uint64_t g_override = 0) {
 	c->report_now = c->report_sort = false;  // (left by a call that failed before its wait)
+	c->rank_now = false;
 	c->gp.g_max = g_override ? (uint32_t)g_override : g_max_for(n);
 	c->dense_skip = c->last_dense == 0;
 	c->chain = chain_enabled() && c->chain_state != cc_ctx::kChainNo && n < ((uint64_t)1 << 31);
@@ -882,6 +883,7 @@ void retain(cc_ctx *c, uint64_t n, uint64_t P) {
 	c->retained_split[1] = c->h_stats->tmp_pairs;
 	c->retained_fused = c->fused_now;
 	c->retained_direct = c->direct;
+	c->retained_scan = c->rank_now && !c->fused_now;  // short lists are ordered without owner offsets
 }
 
 // Writes the retained pair list into `out` (cap >= P checked by the caller).
@@ -902,6 +904,11 @@ cc_status emit_retained(cc_ctx *c, unsigned long long *out, uint64_t cap, cudaSt
 	CC_CUDA(c, cudaMemsetAsync(&d->err, 0, sizeof(uint32_t), s));
 	c->fused_now = c->retained_fused;
 	c->direct = c->retained_direct;
+	if (c->retained_scan) {
+		StageMark m(c, ST_SCAN_OWNER, s);
+		launch_scan_owner(c->retained_n, bp_buffers(c), s);
+		c->launches += 1;
+	}
 	enqueue_emit(c, c->retained_n, out, cap, s);
 	CC_TRY(check_launch(c));
 	CC_TRY(read_stats(c, s));

@@ -1,6 +1,9 @@
 """A pair list retained after CC_ERR_CAPACITY (cc_broadphase_fetch) is the whole
 list, whatever the context computed in between."""
 import ctypes
+import os
+import subprocess
+import sys
 
 import numpy as np
 import pytest
@@ -43,3 +46,41 @@ def test_a_narrowphase_in_between(cb, crowded):
         cb.Narrowphase(ctx).DoNarrowphase(other.T, other.A, other.B, other.C, other.R, other.ID, other.active, other.pos,
                                           other.rot, (q[0] << 32) | q[1])
         assert np.array_equal(fetch(ctx, len(p)), p)
+
+
+def lattice(n, moved):
+    """n unit-spaced spheres; the first `moved` of every second body touch their neighbour."""
+    k = int(np.ceil(n ** (1 / 3)))
+    c = np.stack(np.meshgrid(*[np.arange(k)] * 3, indexing="ij"), -1).reshape(-1, 3)[:n].astype(np.float32)
+    c[0:2 * moved:2] = c[1:2 * moved:2] + np.float32(0.125)
+    B = np.zeros((n, 3), np.float32)
+    B[:, 0] = 0.25
+    return S._one_shape_per_body(np.full(n, S.SPHERE), B, c, S._identity_quats(n), "lattice")
+
+
+def short_list_fetched(cb, n, cap=16, moved=600):
+    """cc_collide on a scene without a pair, then with `moved` of them and no room, then the fetch."""
+    still, touching = lattice(n, 0), lattice(n, moved)
+    _, p = O.broadphase(O.aabb(touching), (32, 32, 32))
+    assert len(p) >= moved
+    ds, ctx = cb.DeviceScene(still), cb.Context()
+    pipe = cb.DevicePipeline(ds, ctx=ctx, pairs_cap=cap)
+    for _ in range(2):
+        ds.pos.copy_(torch.from_numpy(still.pos))
+        assert pipe.run() == (0, 0)
+        ds.pos.copy_(torch.from_numpy(touching.pos))
+        st = _lib.lib.cc_collide(ctx.h, ctypes.byref(pipe.scene), 16, 16, 16, 0.0, ctypes.byref(pipe.res), None)
+        assert st == _lib.CC_ERR_CAPACITY and pipe.res.n_pairs == len(p)
+        assert np.array_equal(fetch(ctx, len(p)), p)
+
+
+@pytest.mark.parametrize("n", [1500, 9000, 300_001])
+def test_short_list(cb, n):
+    # above 262,144 bodies the last call's empty list leaves too many owner buckets for the one-launch sort
+    short_list_fetched(cb, n)
+
+
+def test_short_list_without_the_fused_sort():
+    env = dict(os.environ, CC_FUSED_SORT="0")
+    code = "import conftest, collide_b200 as cb, test_gpu_fetch as t; t.short_list_fetched(cb, 9000); t.short_list_fetched(cb, 1500)"
+    subprocess.run([sys.executable, "-c", code], check=True, env=env, cwd=os.path.dirname(os.path.abspath(__file__)))
