@@ -742,6 +742,14 @@ cc_status overlap_prepare(cc_ctx *c, uint64_t n, uint64_t pairs_cap, bool &ov) {
 	return ensure(c, c->np_hvals, sizeof(uint32_t) * c->np_hslots);
 }
 
+// Without the ranges that no buffer stands behind (a call without room for pairs
+// has no narrowphase scratch).
+ZeroList allocated(ZeroList zero) {
+	for (int r = 0; r < 5; r++)
+		if (!zero.p[r]) zero.words[r] = 0;
+	return zero;
+}
+
 // What a pass's first kernel zeroes: scan control words, class counters, cell
 // counts and, with the narrowphase overlapped, the contact hash.
 ZeroList pass_zero_list(cc_ctx *c, bool ov) {
@@ -758,9 +766,7 @@ ZeroList pass_zero_list(cc_ctx *c, bool ov) {
 		zero.p[4] = ptr<uint32_t>(c->np_hkeys);
 		zero.words[4] = 2 * c->np_hslots;
 	}
-	for (int r = 0; r < 5; r++)
-		if (!zero.p[r]) zero.words[r] = 0;
-	return zero;
+	return allocated(zero);
 }
 
 // After a pass's counters were read: runs the narrowphase again, in order, where
@@ -1212,7 +1218,7 @@ cc_status collide_verlet(cc_ctx *c, const cc_scene &sc, int gx, int gy, int gz, 
 			zero.words[1] = 16;
 			zero.p[2] = ptr<uint32_t>(c->np_classes);
 			zero.words[2] = 2 * kNpClasses + 1;
-			CC_TRY(enqueue_front(s, zero));
+			CC_TRY(enqueue_front(s, allocated(zero)));
 		}
 		c->report_now = pairs_cap != 0;
 		CC_TRY(enqueue_tail(s));
