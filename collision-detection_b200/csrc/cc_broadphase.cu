@@ -227,7 +227,7 @@ __device__ __forceinline__ void load_shifted_tile(uint64_t n, float *__restrict_
 }
 
 template <bool kBatch>
-__global__ void __launch_bounds__(kNT) k_count(uint64_t n, float *__restrict__ aabb, const DevStats *stats,
+__global__ void __launch_bounds__(kNT) k_count(uint64_t n, float *__restrict__ aabb, DevStats *stats,
                                                 uint32_t *__restrict__ cell_count, uint32_t *__restrict__ owner_count,
                                                 SceneMap sm, int oshift, uint32_t *__restrict__ owner_cursor, int shift) {
 	pdl_begin();
@@ -251,6 +251,7 @@ __global__ void __launch_bounds__(kNT) k_count(uint64_t n, float *__restrict__ a
 	const Plan &p = one ? sp : plan_of<kBatch>(sp, sm, i, base);
 	if (kBatch && !p.valid) return;
 	const CellRange r = cell_range(p, mn, mx);
+	if ((uint64_t)(r.c1[0] - r.c0[0] + 1) * (r.c1[1] - r.c0[1] + 1) * (r.c1[2] - r.c0[2] + 1) > kWideCells) stats->wide = 1u;
 	for (int z = r.c0[2]; z <= r.c1[2]; z++)
 		for (int y = r.c0[1]; y <= r.c1[1]; y++)
 			for (int x = r.c0[0]; x <= r.c1[0]; x++) atomicAdd(&cell_count[cell_index(p, base, x, y, z)], 1u);

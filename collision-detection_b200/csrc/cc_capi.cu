@@ -867,14 +867,14 @@ void remember(cc_ctx *c) {
 	c->last_tmp = unsorted_pairs(*c->h_stats, c->direct);
 	c->last_mask = c->h_stats->mask_words;
 	c->last_dense = c->h_stats->dense_items;
-	// chains while no cell is crowded; back to them once sorted cells show none
-	// (which they tell through their dense cells, so a raised threshold makes
-	// them blind) or some calls after a box over too many cells
+	// chains while no cell is crowded and no box over too many cells; back to them
+	// once sorted cells show neither (crowded ones they tell through their dense
+	// cells, so with a raised threshold some calls later)
 	if (c->all_pairs) {  // tells nothing of the cells
 	} else if (c->chain) {
 		c->chain_state = c->last_dense ? cc_ctx::kChainNo : cc_ctx::kChainOk;
 		c->chain_wait = c->gp.dense_cell <= kChainLong ? 0 : kChainWait;
-	} else if (c->last_dense == 0 && --c->chain_wait < 0) {
+	} else if (c->last_dense == 0 && !c->h_stats->wide && --c->chain_wait < 0) {
 		c->chain_state = cc_ctx::kChainUnknown;
 	}
 	for (int d = 0; d < 3; d++) c->last_dim[d] = c->h_stats->plan.dim[d];

@@ -58,6 +58,7 @@ struct DevStats {
 	uint32_t vbad;
 	float vmargin;
 	uint32_t reported;     // blocks of the pass's last kernel that are done with these counters
+	uint32_t wide;         // the sorted search met a box over more than kWideCells cells
 };
 #ifdef __CUDACC__
 // A blocking call's last kernel writes the counters to the host itself: a copy behind
@@ -219,8 +220,16 @@ struct BpBuffers {
 // Cells with more entries make the next call search on sorted cells: above
 // this the tests of a cell are work for whole warps, not a lane's chain.
 constexpr uint32_t kChainLong = 128;
-// A box over more cells than this also turns the search to sorted cells.
-constexpr uint32_t kChainCells = 65535;
+// A box over more cells than this also turns the search to sorted cells: one lane
+// links its entries one after the other, some 0.4 us each, where the sorted search
+// takes two independent atomics for a quarter to a half as many. Steps on chains and
+// on sorted cells, us, with one box of about 128 cells among 5K, 20K, 130K and 1M
+// bodies: 164 and 129, 190 and 152, 146 and 132, 278 and 244; of about 32 cells: 125
+// and 124, 148 and 134, 111 and 108, 208 and 223; with a floor under 130K 5,940 and 2,450.
+constexpr uint32_t kChainCells = 128;
+// A sorted search (cells two to four times as large) that meets a box over more
+// cells than this keeps the next call from trying the chains again.
+constexpr uint32_t kWideCells = kChainCells / 4;
 constexpr uint32_t kScanCoopBlocks = 2048;
 // Owner buckets of n bodies at a shift.
 __host__ __device__ inline uint64_t owner_buckets(uint64_t n, int shift) {
