@@ -333,7 +333,7 @@ __device__ __forceinline__ void write_contact(uint64_t i, double env, D3 org, D3
 	sc.flag[i] = 1u;
 	if (sc.hkeys) {  // overlapped narrowphase: key -> i for the compaction in sorted order
 		const unsigned long long tag = sc.pairs[i] + 1ull;
-		uint64_t h = (tag * 0x9E3779B97F4A7C15ull) >> 20;
+		uint64_t h = contact_slot(tag);
 		bool placed = false;
 		for (uint64_t probe = 0; probe <= sc.hmask && probe < 256; probe++, h++) {
 			const uint64_t slot = h & sc.hmask;

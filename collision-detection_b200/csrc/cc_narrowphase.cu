@@ -198,7 +198,7 @@ constexpr uint32_t kNoHit = 0xffffffffu;
 // Contact hash: the row of a pair's result, kNoHit where it is no contact.
 __device__ __forceinline__ uint32_t hash_find(const NpScratch &sc, unsigned long long key) {
 	const unsigned long long tag = key + 1ull;
-	uint64_t h = (tag * 0x9E3779B97F4A7C15ull) >> 20;
+	uint64_t h = contact_slot(tag);
 	for (uint64_t probe = 0; probe <= sc.hmask && probe < 256; probe++, h++) {
 		const unsigned long long v = __ldcg(&sc.hkeys[h & sc.hmask]);
 		if (v == tag) return __ldcg(&sc.hvals[h & sc.hmask]);

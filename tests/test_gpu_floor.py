@@ -55,3 +55,17 @@ def test_batch(cb):
         owner = b.pairs[:P].cpu().numpy() >> 32
         want = np.histogram(owner, bins=db.shape_offsets.astype(np.int64))[0]
         assert np.array_equal(b.scene_pairs.astype(np.int64), want)
+
+
+def test_no_redo_where_contacts_share_a_body(cb):
+    # the same scene with the floor first and last: as many launches a step (a redo takes two more)
+    n, launches = 7_500, []
+    for last in (False, True):
+        sc = on_floor(n, 5, 2.0, last)
+        pipe = cb.DevicePipeline(cb.DeviceScene(sc), ctx=cb.Context(), pairs_cap=4 * n)
+        for _ in range(4):
+            P, C = pipe.run()
+        floor = n if last else 0
+        assert P > 4096 and 3000 < int((pipe.bids[:C] == floor).any(1).sum()) < 4000
+        launches.append(pipe.ctx.launches())
+    assert launches[0] == launches[1]
