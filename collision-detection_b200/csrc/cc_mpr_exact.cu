@@ -51,7 +51,7 @@ __device__ __noinline__ D3 unit_rare(double x, double y, double z) { return unit
 // unit<double, true> bit for bit where ok stays true.
 __device__ __forceinline__ D3 unit_fast(D3 a, bool &ok) {
 	const InvRoot v = inv_root(dotp(a, a));
-	ok &= v.ok & quot_large(a.x, a.y, a.z);
+	ok &= v.ok & quot_ok(a.x, a.y, a.z);
 	return mk(quot_root(a.x, v), quot_root(a.y, v), quot_root(a.z, v));
 }
 __device__ __forceinline__ D3 unit_x(D3 a) {
@@ -139,17 +139,23 @@ __device__ __forceinline__ double with_sign_of(double b, double x) {  // sgn(x) 
 
 __device__ __noinline__ D3 support_rare(Side s, D3 d) { return support<double, true>(shape_of(s), d); }
 // support<double, true>(s, d) bit for bit where ok stays true; need: the union
-// over the warp. All components of the direction in the shape's frame are
-// nonzero there, so the signs that box and cylinder take are sign bits.
+// over the warp. The signs that box and cylinder take are sign bits; where the
+// direction in the shape's frame has a zero, the sign is zero and they take the
+// product with it.
 __device__ __forceinline__ D3 support_fast(const Side &s, D3 d, uint32_t need, bool &ok) {
 	const bool cyl = s.type == CYLINDER, ell = s.type == ELLIPSOID, box = s.type == BOX;
 	const D3 n = mcol(s.r0, s.r1, s.r2, d);
-	ok &= s.fast & quot_large(n.x, n.y, n.z);
+	const uint32_t nx = size_or_zero(n.x), ny = size_or_zero(n.y), nz = size_or_zero(n.z);
+	ok &= s.fast & quot_ok(nx, ny, nz);
 	D3 u = n, e = n;
 	if (need & kNeedUnit) {  // ellipsoid: n / |n|; cylinder: (n.x, 0, n.z) / |.|
 		const bool uses = cyl | ell;
-		const D3 w = mk(n.x, cyl ? 0.0 : n.y, n.z);
-		const InvRoot v = inv_root(dotp(w, w));
+		D3 w = mk(n.x, cyl ? 0.0 : n.y, n.z);
+		const double s2 = dotp(w, w);
+		const bool axis = cyl & (s2 == 0.0);  // along the cylinder's axis: (0, sgn(n.y) B.y, 0)
+		w.x = axis ? 0.0 : w.x;
+		w.z = axis ? 0.0 : w.z;
+		const InvRoot v = inv_root(axis ? 1.0 : s2);
 		u = pick(uses, mk(quot_root(w.x, v), quot_root(w.y, v), quot_root(w.z, v)), n);
 		ok &= !uses | v.ok;
 	}
@@ -160,10 +166,12 @@ __device__ __forceinline__ D3 support_fast(const Side &s, D3 d, uint32_t need, b
 		ok &= !ell | v.ok;
 	}
 	// sphere: B.x n; box: sgn(n) B; cylinder: (B.x u.x, sgn(n.y) B.y, B.x u.z)
-	const D3 t = mulv(s.Y, u);
-	const D3 l = mk(box ? with_sign_of(s.Y.x, n.x) : (ell ? e.x : t.x),
-	                (box | cyl) ? with_sign_of(s.Y.y, n.y) : (ell ? e.y : t.y),
-	                box ? with_sign_of(s.Y.z, n.z) : (ell ? e.z : t.z));
+	const uint32_t sign = box ? 0x7fffffffu : 0xffffffffu;  // sgn(-0) is +0
+	const auto plain = [&](double x) { return __hiloint2double(__double2hiint(x) & sign, __double2loint(x)); };
+	const D3 t = mulv(s.Y, mk(plain(u.x), plain(u.y), plain(u.z)));
+	const D3 l = mk(box & (nx != kSizeOfZero) ? with_sign_of(s.Y.x, n.x) : (ell ? e.x : t.x),
+	                (box | cyl) & (ny != kSizeOfZero) ? with_sign_of(s.Y.y, n.y) : (ell ? e.y : t.y),
+	                box & (nz != kSizeOfZero) ? with_sign_of(s.Y.z, n.z) : (ell ? e.z : t.z));
 	return add(mrow(s.r0, s.r1, s.r2, l), s.X);
 }
 __device__ __forceinline__ D3 shfl_partner(uint32_t mask, D3 a) {
