@@ -48,6 +48,7 @@ constexpr int kMaxMarks = 64;
 // spheres 22, 20, 19; crowded scenes are bound by the extent floor instead).
 constexpr float kChainCellTarget = 0.25f;
 constexpr int kChainWait = 32;  // calls (cc_ctx::chain_wait)
+constexpr int kMaskWait = 32;   // calls (cc_ctx::mask_wait)
 
 // A CUDA graph of one kind of call, replayed while the call's configuration
 // (its key: everything its launches depend on) repeats.
@@ -125,6 +126,7 @@ struct cc_ctx {
 	bool chain = false, chain_check = false;
 	GridParams call_gp{};  // gp as this call's search uses it (set by prepare)
 	int chain_wait = 0;  // calls on sorted cells left before the chains are tried again
+	int mask_wait = 0;   // calls left before more room for hit masks is asked for again
 	uint64_t last_E = 0, last_P = 0, last_tmp = 0, last_mask = 0;  // last_tmp: pairs that went through pairs_tmp
 	bool sized = false;  // a pass has set these
 	bool all_pairs = false;  // this call tests all pairs of boxes
@@ -434,12 +436,40 @@ bool chain_enabled() {
 	return on;
 }
 
+// Room for the last call's hit masks, up to 16 GB and a quarter of the free memory,
+// which the rest of the program needs too. No call fails for want of it: cells whose
+// masks do not fit are tested twice.
+void mask_prepare(cc_ctx *c) {
+	const uint64_t want = std::min<uint64_t>(sizeof(uint32_t) * (c->last_mask + c->last_mask / 8), (uint64_t)1 << 34);
+	if (want <= c->masks.bytes) return;
+	if (c->mask_wait > 0) {  // refused lately
+		c->mask_wait -= c->dry_run ? 0 : 1;
+		return;
+	}
+	if (c->dry_run) {
+		c->would_grow = true;
+		return;
+	}
+	size_t free_bytes = 0, total = 0;
+	if (cudaMemGetInfo(&free_bytes, &total) != cudaSuccess) free_bytes = 0;
+	const uint64_t get = std::min<uint64_t>(want, c->masks.bytes + free_bytes / 4) & ~(uint64_t)255;
+	if (get > c->masks.bytes) {
+		if (c->masks.p) cudaFree(c->masks.p);
+		c->masks.p = nullptr;
+		c->masks.bytes = cudaMalloc(&c->masks.p, get) == cudaSuccess ? get : 0;
+		if (!c->masks.bytes) c->masks.p = nullptr;
+		c->masks.allocs++;
+		c->buf_gen++;
+	}
+	cudaGetLastError();  // a refused allocation is no error of the call
+	if (c->masks.bytes < want) c->mask_wait = kMaskWait;
+}
+
 // Scratch of the dense-cell test for the entries there is room for.
 cc_status direct_prepare(cc_ctx *c) {
 	CC_TRY(ensure(c, c->sorted, c->entries.bytes));
 	CC_TRY(ensure(c, c->sorted_body, sizeof(uint32_t) * (c->entries.bytes / (2 * sizeof(float4)))));
-	// the last call's mask words, up to 16 GB (what does not fit is tested twice)
-	CC_TRY(ensure(c, c->masks, std::min<uint64_t>(sizeof(uint32_t) * (c->last_mask + c->last_mask / 8), (uint64_t)1 << 34)));
+	mask_prepare(c);
 	return ensure(c, c->row_count, sizeof(uint32_t) * (c->entries.bytes / (2 * sizeof(float4))));
 }
 
