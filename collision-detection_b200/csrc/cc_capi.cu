@@ -485,6 +485,29 @@ constexpr uint64_t kCrowdedFine = (uint64_t)1 << 21;
 // Room to ask for where the last call used `used` and there is room for `room`.
 uint64_t with_slack(uint64_t used, uint64_t room) { return used + used / 16 <= room ? room : used + used / 4; }
 
+// Scratch that only this call's search (c->chain, c->direct) and pair sort
+// (c->fused_now) use, for the entries there is room for. A first call is mostly
+// allocations (130K mixed shapes 2.35 of 2.6 ms), so the other routes' scratch waits
+// until they are taken. First calls with all routes' scratch at once and with this,
+// ms: 130K 2.6 and 2.1, three class calls on 20K spheres 1.46 and 1.16, an incremental
+// step of 500K 10.3 and 7.4 (that also by a search less, prepare's guess).
+cc_status route_prepare(cc_ctx *c, uint64_t n) {
+	const uint64_t cap = c->entries.bytes / (2 * sizeof(float4));
+	if (c->chain) {
+		CC_TRY(ensure(c, c->extra, sizeof(uint32_t) * cap));
+	} else {
+		CC_TRY(ensure(c, c->bp_bsum, sizeof(unsigned long long) * kScanCoopBlocks));
+		CC_TRY(ensure(c, c->cell_cs, sizeof(unsigned long long) * c->gp.g_max));
+		CC_TRY(ensure(c, c->cell_start, sizeof(uint32_t) * (c->gp.g_max + 1)));
+	}
+	if (c->direct) {
+		CC_TRY(ensure(c, c->dense, sizeof(DenseItem) * (cap / kDenseCell + 1024)));
+		CC_TRY(direct_prepare(c));
+	}
+	if (!c->fused_now) CC_TRY(ensure(c, c->big_list, sizeof(uint32_t) * (n + 1024)));
+	return CC_OK;
+}
+
 // Allocates the n-dependent broadphase scratch and, if np_cap > 0, the
 // narrowphase scratch for np_cap pairs. Buffers only grow; every public call
 // ends with a synchronize, so nothing in flight uses a buffer replaced here.
@@ -508,26 +531,22 @@ cc_status prepare(cc_ctx *c, uint64_t n, uint64_t np_cap, uint64_t g_override = 
 	if (c->chain) c->call_gp.k_target *= kChainCellTarget;
 	if (c->direct && !g_override && n <= kCrowdedFine) c->call_gp.k_target *= 0.5f;
 	CC_TRY(ensure(c, c->stats, sizeof(DevStats)));
-	CC_TRY(ensure(c, c->bp_bsum, sizeof(unsigned long long) * kScanCoopBlocks));
-	CC_TRY(ensure(c, c->cell_cs, sizeof(unsigned long long) * c->gp.g_max));
 	CC_TRY(ensure(c, c->cell_count, sizeof(uint32_t) * c->gp.g_max));
-	CC_TRY(ensure(c, c->cell_start, sizeof(uint32_t) * (c->gp.g_max + 1)));
 	CC_TRY(ensure(c, c->owner_count, sizeof(uint32_t) * std::max<uint64_t>(n, 1)));
 	CC_TRY(ensure(c, c->owner_off, sizeof(unsigned long long) * (n + 1)));
-	// Small cells (chained search) hold a body 2.4 to 2.8 times. Room that is there
-	// is enough while a sixteenth of the last call's count is left.
-	const uint64_t e_guess = std::max<uint64_t>(with_slack(c->last_E, c->entries.bytes / (2 * sizeof(float4))), (c->chain ? 3 : 2) * n + 1024);
+	// Small cells (chained search) hold a body 2.4 to 2.8 times, cells at the extent
+	// floor up to 1.5^3 = 3.4 times. Room that is there is enough while a sixteenth of
+	// the last call's count is left.
+	const uint64_t e_guess = std::max<uint64_t>(with_slack(c->last_E, c->entries.bytes / (2 * sizeof(float4))),
+	                                            (c->chain ? n * 7 / 2 : 2 * n) + 1024);
 	CC_TRY(ensure(c, c->entries, 2 * sizeof(float4) * e_guess));
-	if (c->chain) CC_TRY(ensure(c, c->extra, sizeof(uint32_t) * (c->entries.bytes / (2 * sizeof(float4)))));
-	if (c->direct) CC_TRY(direct_prepare(c));
 	const uint64_t p_guess = std::max<uint64_t>(with_slack(c->last_tmp, c->pairs_tmp.bytes / sizeof(unsigned long long)), n / 4 + 1024);
 	CC_TRY(ensure(c, c->pairs_tmp, sizeof(unsigned long long) * p_guess));
 	c->st_words[0] = std::max<uint64_t>(c->st_words[0], status_words_for(c->gp.g_max));
 	c->st_words[1] = std::max<uint64_t>(c->st_words[1], status_words_for(n + 1));
 	CC_TRY(ensure_status(c));
 	CC_TRY(ensure(c, c->ticket, 64));
-	CC_TRY(ensure(c, c->big_list, sizeof(uint32_t) * (n + 1024)));
-	CC_TRY(ensure(c, c->dense, sizeof(DenseItem) * (c->entries.bytes / (2 * sizeof(float4)) / kDenseCell + 1024)));
+	CC_TRY(route_prepare(c, n));
 	if (np_cap) CC_TRY(np_prepare(c, np_cap));
 	return CC_OK;
 }
@@ -690,6 +709,13 @@ void enqueue_np(cc_ctx *c, const NpArgs &a, uint64_t P_cap, const unsigned long 
 	c->launches += 1 + mpr_launches(P_cap, c->np_precision, P_dev ? hint_P(c, a.n) : P_cap);  // MPR, compaction
 }
 
+// The exact MPR's blocks fill the SMs' registers, and the fused sort, a
+// cooperative launch, then waits for the last of them. So the sort goes first,
+// and the MPR starts beside it as its programmatic dependent once all of its
+// blocks are resident (1M mixed shapes: the sort ran after the MPR on the other
+// stream, 197 us a step; beside it 191; 130K bodies 111 and 105).
+bool np_beside(const cc_ctx *c) { return c->fused_now && c->np_precision == CC_NP_EXACT; }
+
 // The step after the pair test with the narrowphase overlapped: a short list
 // (rank_now) is ordered by counting behind the MPR; else
 // the MPR runs on the unsorted pairs on c->np_stream (forked after the pair
@@ -718,12 +744,7 @@ cc_status enqueue_sort_and_np_overlapped(cc_ctx *c, uint64_t n, const NpArgs &a,
 	sc.hkeys = ptr<unsigned long long>(c->np_hkeys);
 	sc.hvals = ptr<uint32_t>(c->np_hvals);
 	sc.hmask = c->np_hslots - 1;
-	// The exact MPR's blocks fill the SMs' registers, and the fused sort, a
-	// cooperative launch, then waits for the last of them. So the sort goes first,
-	// and the MPR starts beside it as its programmatic dependent once all of its
-	// blocks are resident (1M mixed shapes: the sort ran after the MPR on the other
-	// stream, 197 us a step; beside it 191; 130K bodies 111 and 105).
-	const bool beside = c->fused_now && c->np_precision == CC_NP_EXACT;
+	const bool beside = np_beside(c);
 	cudaStream_t t = s;
 	if (!beside) {
 		t = c->np_stream;
@@ -764,9 +785,11 @@ cc_status overlap_prepare(cc_ctx *c, uint64_t n, uint64_t pairs_cap, bool &ov) {
 	ov = c->np_overlap && !c->direct && pairs_cap > 0 && pairs_cap <= ((uint64_t)1 << 24);
 	c->rank_now = ov && hint_P(c, n) <= kRankPairs && n < ((uint64_t)1 << 31);
 	if (!ov || c->rank_now) return CC_OK;
-	if (!c->np_stream) CC_CUDA(c, cudaStreamCreateWithFlags(&c->np_stream, cudaStreamNonBlocking));
-	if (!c->ev_fork) CC_CUDA(c, cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming));
-	if (!c->ev_join) CC_CUDA(c, cudaEventCreateWithFlags(&c->ev_join, cudaEventDisableTiming));
+	if (!np_beside(c)) {
+		if (!c->np_stream) CC_CUDA(c, cudaStreamCreateWithFlags(&c->np_stream, cudaStreamNonBlocking));
+		if (!c->ev_fork) CC_CUDA(c, cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming));
+		if (!c->ev_join) CC_CUDA(c, cudaEventCreateWithFlags(&c->ev_join, cudaEventDisableTiming));
+	}
 	c->np_hslots = pow2ceil(std::max<uint64_t>(4 * std::min<uint64_t>(hint_P(c, n), pairs_cap), 4096));
 	CC_TRY(ensure(c, c->np_hkeys, sizeof(unsigned long long) * c->np_hslots));
 	return ensure(c, c->np_hvals, sizeof(uint32_t) * c->np_hslots);
@@ -833,11 +856,7 @@ cc_status settle(cc_ctx *c, uint64_t n, float *aabb, unsigned long long *out, ui
 		if (E <= b.entry_cap && P <= b.pair_cap && !crowded) return CC_OK;
 		if (E >= 0xffffffffull)
 			return set_err(c, CC_ERR_CAPACITY, "search grid needs %llu entries (>= 2^32)", (unsigned long long)E);
-		if (E > b.entry_cap) {
-			CC_TRY(ensure(c, c->entries, 2 * sizeof(float4) * (E + E / 8)));
-			if (c->chain) CC_TRY(ensure(c, c->extra, sizeof(uint32_t) * (c->entries.bytes / (2 * sizeof(float4)))));
-			CC_TRY(ensure(c, c->dense, sizeof(DenseItem) * ((E + E / 8) / kDenseCell + 1024)));
-		}
+		if (E > b.entry_cap) CC_TRY(ensure(c, c->entries, 2 * sizeof(float4) * (E + E / 8)));
 		if (redone) *redone = true;
 		if (crowded) {
 			c->chain = false;
@@ -851,7 +870,7 @@ cc_status settle(cc_ctx *c, uint64_t n, float *aabb, unsigned long long *out, ui
 				c->key_bits = 32;
 			}
 		}
-		if (c->direct) CC_TRY(direct_prepare(c));
+		CC_TRY(route_prepare(c, n));
 		if (P > b.pair_cap) CC_TRY(ensure(c, c->pairs_tmp, sizeof(unsigned long long) * (P + P / 8)));
 		CC_TRY(reset_pass_counters(c, n, s));
 		c->chain_check = c->chain_check && c->chain;
