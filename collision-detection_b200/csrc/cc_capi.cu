@@ -251,6 +251,21 @@ cc_status ensure(cc_ctx *c, Buf &b, size_t bytes) {
 	return CC_OK;
 }
 
+void drop(cc_ctx *c, Buf &b) {
+	if (!b.p) return;
+	cudaFree(b.p);
+	b.p = nullptr;
+	b.bytes = 0;
+	c->buf_gen++;
+}
+
+// A refused allocation that the call does without is no error of it.
+void refused(cc_ctx *c) {
+	cudaGetLastError();
+	c->cuda_err = cudaSuccess;
+	c->err.clear();
+}
+
 template <class T>
 T *ptr(const Buf &b) { return reinterpret_cast<T *>(b.p); }
 
@@ -461,7 +476,7 @@ void mask_prepare(cc_ctx *c) {
 		c->masks.allocs++;
 		c->buf_gen++;
 	}
-	cudaGetLastError();  // a refused allocation is no error of the call
+	refused(c);
 	if (c->masks.bytes < want) c->mask_wait = kMaskWait;
 }
 
@@ -501,35 +516,32 @@ cc_status route_prepare(cc_ctx *c, uint64_t n) {
 		CC_TRY(ensure(c, c->cell_start, sizeof(uint32_t) * (c->gp.g_max + 1)));
 	}
 	if (c->direct) {
-		CC_TRY(ensure(c, c->dense, sizeof(DenseItem) * (cap / kDenseCell + 1024)));
-		CC_TRY(direct_prepare(c));
+		cc_status st = ensure(c, c->dense, sizeof(DenseItem) * (cap / kDenseCell + 1024));
+		if (st == CC_OK) st = direct_prepare(c);
+		if (st == CC_ERR_OUT_OF_MEMORY) {  // without the dense-cell test
+			refused(c);
+			c->direct = false;
+			c->dense_skip = true;
+			for (Buf *b : {&c->sorted, &c->sorted_body, &c->row_count, &c->masks}) drop(c, *b);
+		} else {
+			CC_TRY(st);
+		}
 	}
 	if (!c->fused_now) CC_TRY(ensure(c, c->big_list, sizeof(uint32_t) * (n + 1024)));
 	return CC_OK;
 }
 
-// Allocates the n-dependent broadphase scratch and, if np_cap > 0, the
-// narrowphase scratch for np_cap pairs. Buffers only grow; every public call
-// ends with a synchronize, so nothing in flight uses a buffer replaced here.
-cc_status prepare(cc_ctx *c, uint64_t n, uint64_t np_cap, uint64_t g_override = 0) {
-	c->report_now = c->report_sort = false;  // (left by a call that failed before its wait)
-	c->rank_now = false;
-	c->gp.g_max = g_override ? (uint32_t)g_override : g_max_for(n);
-	c->dense_skip = c->last_dense == 0;
-	c->chain = chain_enabled() && c->chain_state != cc_ctx::kChainNo && n < ((uint64_t)1 << 31);
-	// (a scene of nearly all pairs is left to the dense cells, which write them in order)
-	c->all_pairs = c->chain && !g_override && n <= kAllPairsBodies && c->last_P <= 32 * n;
-	c->chain_check = c->chain && !c->all_pairs && c->chain_state == cc_ctx::kChainUnknown;
-	c->direct = !c->chain && !c->dense_skip;
+// The n-dependent scratch of the route that prepare chose.
+cc_status size_scratch(cc_ctx *c, uint64_t n, uint64_t np_cap, bool batch) {
 	choose_owner_shift(c, n);
-	if (g_override && c->direct) {  // a batch counts its scenes' pairs by owner if its output is too small
+	if (batch && c->direct) {  // a batch counts its scenes' pairs by owner if its output is too small
 		c->owner_shift = 0;
 		c->key_bits = 32;
 	}
 	c->fused_now = !c->direct && fused_sort_enabled() && fused_sort_fits(owner_buckets(n, c->owner_shift));
 	c->call_gp = c->gp;
 	if (c->chain) c->call_gp.k_target *= kChainCellTarget;
-	if (c->direct && !g_override && n <= kCrowdedFine) c->call_gp.k_target *= 0.5f;
+	if (c->direct && !batch && n <= kCrowdedFine) c->call_gp.k_target *= 0.5f;
 	CC_TRY(ensure(c, c->stats, sizeof(DevStats)));
 	CC_TRY(ensure(c, c->cell_count, sizeof(uint32_t) * c->gp.g_max));
 	CC_TRY(ensure(c, c->owner_count, sizeof(uint32_t) * std::max<uint64_t>(n, 1)));
@@ -549,6 +561,35 @@ cc_status prepare(cc_ctx *c, uint64_t n, uint64_t np_cap, uint64_t g_override = 
 	CC_TRY(route_prepare(c, n));
 	if (np_cap) CC_TRY(np_prepare(c, np_cap));
 	return CC_OK;
+}
+
+// Chooses the call's route, allocates the n-dependent broadphase scratch and, if
+// np_cap > 0, the narrowphase scratch for np_cap pairs. Chained cells take 150 bytes a
+// body, sorted ones 180 and without the dense-cell test's copies 100: where memory is
+// short the call runs on those. Buffers only grow; every public call ends with a
+// synchronize, so nothing in flight uses a buffer replaced here.
+cc_status prepare(cc_ctx *c, uint64_t n, uint64_t np_cap, uint64_t g_override = 0) {
+	c->report_now = c->report_sort = false;  // (left by a call that failed before its wait)
+	c->rank_now = false;
+	c->gp.g_max = g_override ? (uint32_t)g_override : g_max_for(n);
+	c->dense_skip = c->last_dense == 0;
+	c->chain = chain_enabled() && c->chain_state != cc_ctx::kChainNo && n < ((uint64_t)1 << 31);
+	// (a scene of nearly all pairs is left to the dense cells, which write them in order)
+	c->all_pairs = c->chain && !g_override && n <= kAllPairsBodies && c->last_P <= 32 * n;
+	c->chain_check = c->chain && !c->all_pairs && c->chain_state == cc_ctx::kChainUnknown;
+	c->direct = !c->chain && !c->dense_skip;
+	cc_status st = size_scratch(c, n, np_cap, g_override != 0);
+	if (st == CC_ERR_OUT_OF_MEMORY && (c->chain || c->direct)) {
+		refused(c);
+		for (Buf *b : {&c->entries, &c->extra, &c->sorted, &c->sorted_body, &c->row_count, &c->masks}) drop(c, *b);
+		c->chain = c->all_pairs = c->chain_check = c->direct = false;
+		c->dense_skip = true;
+		c->chain_state = cc_ctx::kChainNo;
+		c->chain_wait = kChainWait;
+		c->last_E = std::min<uint64_t>(c->last_E, 2 * n);
+		st = size_scratch(c, n, np_cap, g_override != 0);
+	}
+	return st;
 }
 
 NpScratch np_scratch(cc_ctx *c) {
@@ -791,8 +832,16 @@ cc_status overlap_prepare(cc_ctx *c, uint64_t n, uint64_t pairs_cap, bool &ov) {
 		if (!c->ev_join) CC_CUDA(c, cudaEventCreateWithFlags(&c->ev_join, cudaEventDisableTiming));
 	}
 	c->np_hslots = pow2ceil(std::max<uint64_t>(4 * std::min<uint64_t>(hint_P(c, n), pairs_cap), 4096));
-	CC_TRY(ensure(c, c->np_hkeys, sizeof(unsigned long long) * c->np_hslots));
-	return ensure(c, c->np_hvals, sizeof(uint32_t) * c->np_hslots);
+	cc_status st = ensure(c, c->np_hkeys, sizeof(unsigned long long) * c->np_hslots);
+	if (st == CC_OK) st = ensure(c, c->np_hvals, sizeof(uint32_t) * c->np_hslots);
+	if (st == CC_ERR_OUT_OF_MEMORY) {  // in order then
+		refused(c);
+		drop(c, c->np_hkeys);
+		drop(c, c->np_hvals);
+		ov = false;
+		return CC_OK;
+	}
+	return st;
 }
 
 // Without the ranges that no buffer stands behind (a call without room for pairs
@@ -856,7 +905,14 @@ cc_status settle(cc_ctx *c, uint64_t n, float *aabb, unsigned long long *out, ui
 		if (E <= b.entry_cap && P <= b.pair_cap && !crowded) return CC_OK;
 		if (E >= 0xffffffffull)
 			return set_err(c, CC_ERR_CAPACITY, "search grid needs %llu entries (>= 2^32)", (unsigned long long)E);
-		if (E > b.entry_cap) CC_TRY(ensure(c, c->entries, 2 * sizeof(float4) * (E + E / 8)));
+		if (E > b.entry_cap) {
+			const cc_status st = ensure(c, c->entries, 2 * sizeof(float4) * (E + E / 8));
+			if (st == CC_ERR_OUT_OF_MEMORY && c->chain) {  // the next calls on sorted cells, which hold a body less often
+				c->chain_state = cc_ctx::kChainNo;
+				c->chain_wait = kChainWait;
+			}
+			CC_TRY(st);
+		}
 		if (redone) *redone = true;
 		if (crowded) {
 			c->chain = false;
