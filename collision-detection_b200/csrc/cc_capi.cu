@@ -926,7 +926,15 @@ cc_status settle(cc_ctx *c, uint64_t n, float *aabb, unsigned long long *out, ui
 				c->key_bits = 32;
 			}
 		}
-		CC_TRY(route_prepare(c, n));
+		cc_status st = route_prepare(c, n);
+		if (st == CC_ERR_OUT_OF_MEMORY && crowded) {  // the chains' room is more than this search needs
+			refused(c);
+			drop(c, c->extra);
+			drop(c, c->entries);
+			CC_TRY(ensure(c, c->entries, 2 * sizeof(float4) * (E + E / 8)));
+			st = route_prepare(c, n);
+		}
+		CC_TRY(st);
 		if (P > b.pair_cap) CC_TRY(ensure(c, c->pairs_tmp, sizeof(unsigned long long) * (P + P / 8)));
 		CC_TRY(reset_pass_counters(c, n, s));
 		c->chain_check = c->chain_check && c->chain;
