@@ -37,6 +37,7 @@
 // Compiled with -fmad=false (the shift and the bin scale must round exactly as
 // the reference's host build does).
 #include <algorithm>
+#include <atomic>
 #include <climits>
 #include <cstdlib>
 
@@ -1974,14 +1975,25 @@ void launch_segsort(uint64_t n, unsigned long long *out, const BpBuffers &b, cud
 	           b.big_list, b.big_cap, b.stats, kp);
 }
 
+// Opts two kernels into `bytes` of dynamic shared memory (above 48 KB) on the current
+// device, once for each: the attribute is the device's. done: a bit per device.
+template <class K>
+void opt_in_shared(std::atomic<uint64_t> &done, int bytes, K a, K b) {
+	int dev = 0;
+	if (cudaGetDevice(&dev) != cudaSuccess) return;  // the launch tells
+	const uint64_t bit = dev < 64 ? (uint64_t)1 << dev : 0;
+	if (done.load(std::memory_order_acquire) & bit) return;
+	if (cudaFuncSetAttribute(a, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess &&
+	    cudaFuncSetAttribute(b, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess)
+		done.fetch_or(bit, std::memory_order_release);
+}
+
 void launch_segsort_mid(unsigned long long *out, const BpBuffers &b, cudaStream_t s) {
 	const KeyPack kp{b.owner_shift, b.key_bits};
 	if (b.dense) {  // rows of dense cells arrive as ascending runs
 		constexpr int bytes = 2 * kMergeSeg * (int)sizeof(uint32_t);  // 64 KB: three blocks fit on an SM
-		static const bool attr =
-		    cudaFuncSetAttribute(k_segsort_runs<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess &&
-		    cudaFuncSetAttribute(k_segsort_runs<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess;
-		(void)attr;
+		static std::atomic<uint64_t> done{0};
+		opt_in_shared(done, bytes, k_segsort_runs<true>, k_segsort_runs<false>);
 		launch_pdl(kp.shift ? k_segsort_runs<true> : k_segsort_runs<false>, dim3(kNumSMs * 3), dim3(kNT), bytes, s, b.stats,
 		           b.big_cap, b.big_list, b.owner_off, out, kp);
 	}
@@ -1993,13 +2005,8 @@ void launch_segsort_mid(unsigned long long *out, const BpBuffers &b, cudaStream_
 		           out, kp);
 }
 void launch_segsort_big(unsigned long long *out, const BpBuffers &b, cudaStream_t s) {
-	static const bool attr = [] {
-		return cudaFuncSetAttribute(k_segsort_big<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-		                            kBigSeg * (int)sizeof(uint32_t)) == cudaSuccess &&
-		       cudaFuncSetAttribute(k_segsort_big<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-		                            kBigSeg * (int)sizeof(uint32_t)) == cudaSuccess;
-	}();
-	(void)attr;
+	static std::atomic<uint64_t> done{0};
+	opt_in_shared(done, kBigSeg * (int)sizeof(uint32_t), k_segsort_big<true>, k_segsort_big<false>);
 	// 64 KB of shared memory a block: three blocks fit on an SM
 	const KeyPack kp{b.owner_shift, b.key_bits};
 	if (kp.shift)
