@@ -110,7 +110,7 @@ struct MoveUnits {
 __device__ __forceinline__ void move_bytes(const char *src, char *dst, uint64_t from, uint64_t to) {
 	for (uint64_t b = from; b < to; b++) dst[b] = src[b];
 }
-__global__ void __launch_bounds__(kNT) k_move(MoveList m, const DevStats *stats, uint64_t pair_cap) {
+__global__ void __launch_bounds__(kNT) k_move(MoveList m, const DevStats *stats, PassRoom room) {
 	__shared__ MoveUnits u;
 	if (threadIdx.x == 0) {
 		uint64_t P = 0, nc = 0, end = 0;
@@ -118,7 +118,7 @@ __global__ void __launch_bounds__(kNT) k_move(MoveList m, const DevStats *stats,
 		if (stats) {
 			P = stats->np_n;
 			nc = stats->contacts;
-			ok = stats->err == 0 && P == stats->pairs && P <= pair_cap && nc <= P;
+			ok = complete_pass(*stats, room);  // a result to be redone must not reach the caller's boxes, the redo's input
 		}
 		for (int k = 0; k < m.count; k++) {
 			const uint64_t at = reinterpret_cast<uint64_t>(m.src[k]) | reinterpret_cast<uint64_t>(m.dst[k]);
@@ -292,9 +292,9 @@ void launch_gather_c(uint64_t n, const int32_t *T, const float *src, float *dst,
 	k_gather_c<<<g, kNT, 0, s>>>(n, T, src, dst);
 }
 
-void launch_move(const MoveList &m, uint64_t bytes_hint, const DevStats *stats, uint64_t pair_cap, cudaStream_t s) {
+void launch_move(const MoveList &m, uint64_t bytes_hint, const DevStats *stats, const PassRoom &room, cudaStream_t s) {
 	const unsigned g = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(bytes_hint / (16 * 4 * kNT) + 1, (uint64_t)kNumSMs * 8));
-	k_move<<<g, kNT, 0, s>>>(m, stats, pair_cap);
+	k_move<<<g, kNT, 0, s>>>(m, stats, room);
 }
 
 void launch_batch_pair_counts(uint64_t P, const unsigned long long *pairs, const uint32_t *scene_of,

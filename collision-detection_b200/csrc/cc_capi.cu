@@ -166,8 +166,8 @@ struct cc_ctx {
 		cc_result *res = nullptr;
 		int grid[3] = {0, 0, 0};
 		float env = 0.f;
-		uint64_t cap = 0, entry_cap = 0, pair_cap = 0;
-		bool direct = false;
+		uint64_t cap = 0;
+		PassRoom room{};
 	} hs[2];
 	cudaStream_t hs_copy = nullptr, hs_comp = nullptr, hs_out = nullptr;
 	cudaEvent_t hs_user = nullptr, hs_back = nullptr;
@@ -487,9 +487,6 @@ cc_status direct_prepare(cc_ctx *c) {
 	mask_prepare(c);
 	return ensure(c, c->row_count, sizeof(uint32_t) * (c->entries.bytes / (2 * sizeof(float4))));
 }
-
-// Pairs of a pass that went through the unsorted scratch list.
-uint64_t unsorted_pairs(const DevStats &st, bool direct) { return direct ? st.tmp_pairs : st.pairs; }
 
 // Crowded scenes of up to this many bodies take half the cell target: fewer tests in
 // the dense cells against more entries. Clustered spheres, a pass in us with the
@@ -1364,10 +1361,9 @@ cc_status collide_verlet(cc_ctx *c, const cc_scene &sc, int gx, int gy, int gz, 
 	return set_err(c, CC_ERR_INTERNAL, "incremental step did not settle");
 }
 
-// Whether a pass's counters show a result that needs no redo.
-bool complete_pass(const DevStats &st, uint64_t entry_cap, uint64_t pair_cap, bool direct, uint64_t out_cap) {
-	return st.err == 0 && st.entries <= entry_cap && unsorted_pairs(st, direct) <= pair_cap && st.pairs <= out_cap &&
-	       st.np_n == st.pairs;
+PassRoom pass_room(cc_ctx *c, uint64_t out_cap) {
+	const BpBuffers b = bp_buffers(c);
+	return {b.entry_cap, b.pair_cap, out_cap, c->direct};
 }
 
 // GenerateAABB -> broadphase -> narrowphase on device pointers with one
@@ -1385,16 +1381,16 @@ cc_status collide_dev(cc_ctx *c, const cc_scene &sc, int gx, int gy, int gz, flo
 		                      n_pairs, n_contacts, s);
 	CC_TRY(collide_enqueue(c, sc, gx, gy, gz, envelope, aabb, pairs, pairs_cap, norm, cpta, cptb, depth, bids, s,
 	                       true));
+	const PassRoom room = pass_room(c, pairs_cap);
 	if (push) {
 		StageMark m(c, ST_COPY_OUT, s);
-		launch_move(*push, 24 * sc.n + 56 * hint_P(c, sc.n), ptr<DevStats>(c->stats), pairs_cap, s);
+		launch_move(*push, 24 * sc.n + 56 * hint_P(c, sc.n), ptr<DevStats>(c->stats), room, s);
 		c->launches += 1;
 		CC_TRY(check_launch(c));
 	}
-	const BpBuffers b = bp_buffers(c);
 	CC_TRY(await_stats(c, s));
 	// what went out is the result unless something is redone below
-	if (push) *pushed = complete_pass(*c->h_stats, b.entry_cap, b.pair_cap, c->direct, pairs_cap);
+	if (push) *pushed = complete_pass(*c->h_stats, room);
 	return collide_finish(c, sc, envelope, aabb, pairs, pairs_cap, norm, cpta, cptb, depth, bids, n_pairs, n_contacts, s);
 }
 
@@ -2278,10 +2274,7 @@ cc_status cc_collide_host_submit(cc_ctx *c, const cc_scene *sc, int gx, int gy, 
 		                       ptr<float>(h.norm), ptr<float>(h.pa), ptr<float>(h.pb), ptr<float>(h.depth),
 		                       ptr<int32_t>(h.bids), c->hs_comp, false));
 		CC_CUDA(c, cudaMemcpyAsync(h.h_stats, c->stats.p, sizeof(DevStats), cudaMemcpyDeviceToHost, c->hs_comp));
-		const BpBuffers b = bp_buffers(c);
-		h.entry_cap = b.entry_cap;
-		h.pair_cap = b.pair_cap;
-		h.direct = c->direct;
+		h.room = pass_room(c, cap);
 	} else {
 		memset(h.h_stats, 0, sizeof(DevStats));
 	}
@@ -2311,7 +2304,7 @@ cc_status cc_collide_host_wait(cc_ctx *c, cc_result *res, void *stream) {
 	res->n_pairs = res->n_contacts = 0;
 	if (h.dev.n == 0) return CC_OK;
 	const DevStats &st = *h.h_stats;
-	const bool fast = complete_pass(st, h.entry_cap, h.pair_cap, h.direct, h.cap);
+	const bool fast = complete_pass(st, h.room);
 	uint64_t P = st.pairs, nc = st.contacts;
 	if (fast) {
 		memcpy(c->h_stats, h.h_stats, sizeof(DevStats));
@@ -2389,7 +2382,7 @@ cc_status cc_collide_host(cc_ctx *c, const cc_scene *sc, int gx, int gy, int gz,
 			list.add(mapped_host(sc->body_rot), c->in_rot.p, 16 * nb);
 			list.add(mapped_host(sc->active), c->in_act.p, nb);
 			if (res->aabb) list.add(mapped_host(res->aabb), c->out_aabb.p, 24 * n);
-			launch_move(list, 77 * std::max(n, nb), nullptr, 0, s);
+			launch_move(list, 77 * std::max(n, nb), nullptr, PassRoom(), s);
 			c->launches += 1;
 		} else {
 			if (gather_c) {

@@ -60,6 +60,17 @@ struct DevStats {
 	uint32_t reported;     // blocks of the pass's last kernel that are done with these counters
 	uint32_t wide;         // the sorted search met a box over more than kWideCells cells
 };
+// Scratch and output room of a pass, and whether its counters show a result that
+// needs no redo. direct: the dense cells' pairs do not go through the unsorted list.
+struct PassRoom {
+	uint64_t entries, unsorted, out;
+	bool direct;
+};
+__host__ __device__ inline uint64_t unsorted_pairs(const DevStats &st, bool direct) { return direct ? st.tmp_pairs : st.pairs; }
+__host__ __device__ inline bool complete_pass(const DevStats &st, const PassRoom &r) {
+	return st.err == 0 && st.entries <= r.entries && unsorted_pairs(st, r.direct) <= r.unsorted && st.pairs <= r.out &&
+	       st.np_n == st.pairs && st.contacts <= st.pairs;
+}
 #ifdef __CUDACC__
 // A blocking call's last kernel writes the counters to the host itself: a copy behind
 // it costs 3 to 6 us (16K spheres: 44 us a step with, 38 without; 1M mixed shapes 181 and
@@ -357,7 +368,7 @@ cudaError_t copy_small_h2d(void *dst, const void *src, size_t bytes, cudaStream_
 // (pinned, mapped) host array.
 // Moves whole arrays between mapped host memory and the device in one launch.
 // Array k has fixed + per_pair * np_n + per_contact * contacts bytes (counts of
-// `stats`, whose lists must be complete: else nothing moves; null: fixed only).
+// `stats`, whose pass must be complete in `room`: else nothing moves; null: fixed only).
 // Where array 0 holds the shape types and c_src is set, c_dst also receives C of
 // the CONE and TRIANGLEMESH shapes.
 struct MoveList {
@@ -377,7 +388,7 @@ struct MoveList {
 		per_contact[count++] = contact_bytes;
 	}
 };
-void launch_move(const MoveList &m, uint64_t bytes_hint, const DevStats *stats, uint64_t pair_cap, cudaStream_t s);
+void launch_move(const MoveList &m, uint64_t bytes_hint, const DevStats *stats, const PassRoom &room, cudaStream_t s);
 void launch_gather_c(uint64_t n, const int32_t *T, const float *src, float *dst, cudaStream_t s);
 // The front of a batch pass (cc_aabb.cu): scene_of, global ids, boxes, bounds,
 // plans, cell_base[0..S] and stats->cells; with src the scenes are gathered into
