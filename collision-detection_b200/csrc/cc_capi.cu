@@ -313,6 +313,7 @@ void prof_collect(cc_ctx *c) {
 	c->nmarks = 0;
 }
 
+bool aligned4(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 3) == 0; }
 bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
 cc_status check_launch(cc_ctx *c) {
@@ -2157,7 +2158,7 @@ cc_status upload_shapes(cc_ctx *c, cc_ctx::ShapeCopy &sh, Buf *const dst[6], con
 		same = same && sh.src[k] == src[k] && sh.dst[k] == dst[k]->p && sh.allocs[k] == dst[k]->allocs;
 	if (same) return CC_OK;
 	sh.gen = 0;  // not valid until every copy is enqueued
-	const float *c_mapped = sc->n ? static_cast<const float *>(mapped_host(sc->C)) : nullptr;
+	const float *c_mapped = sc->n && aligned4(sc->C) ? static_cast<const float *>(mapped_host(sc->C)) : nullptr;
 	for (int k = 0; k < 6; k++) {
 		if (k == 3 && c_mapped)
 			*gather_c = c_mapped;
@@ -2366,7 +2367,9 @@ cc_status cc_collide_host(cc_ctx *c, const cc_scene *sc, int gx, int gy, int gz,
 	CC_TRY(ensure(c, c->out_depth, 4 * std::max<uint64_t>(cap, 1)));
 	CC_TRY(ensure(c, c->out_bids, 8 * std::max<uint64_t>(cap, 1)));
 	const void *const in[] = {sc->T, sc->A, sc->B, sc->C, sc->R, sc->ID, sc->body_pos, sc->body_rot, sc->active};
-	const bool pull = 77 * std::max(n, nb) <= kMoveBytes && all_mapped(in) && (!res->aabb || mapped_host(res->aabb));
+	// (types and C off a word boundary: the kernel reads them word by word where C is needed)
+	const bool pull = 77 * std::max(n, nb) <= kMoveBytes && aligned4(sc->T) && aligned4(sc->C) && all_mapped(in) &&
+	                  (!res->aabb || mapped_host(res->aabb));
 	std::unique_ptr<StageMark> cin(new StageMark(c, ST_COPY_IN, s));
 	{
 		Buf *const dst[6] = {&c->in_T, &c->in_A, &c->in_B, &c->in_C, &c->in_R, &c->in_ID};
