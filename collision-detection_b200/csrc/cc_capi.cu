@@ -971,12 +971,8 @@ cc_status sort_fallback(cc_ctx *c, uint64_t n, uint64_t P, unsigned long long *o
 	return CC_OK;
 }
 
-void remember(cc_ctx *c) {
-	c->last_E = c->h_stats->entries;
-	c->last_P = c->h_stats->pairs;
-	c->sized = true;
-	c->last_tmp = unsorted_pairs(*c->h_stats, c->direct);
-	c->last_mask = c->h_stats->mask_words;
+// What a search tells the next one of the route to take.
+void remember_route(cc_ctx *c) {
 	c->last_dense = c->h_stats->dense_items;
 	// chains while no cell is crowded and no box over too many cells; back to them
 	// once sorted cells show neither (crowded ones they tell through their dense
@@ -988,6 +984,15 @@ void remember(cc_ctx *c) {
 	} else if (c->last_dense == 0 && !c->h_stats->wide && --c->chain_wait < 0) {
 		c->chain_state = cc_ctx::kChainUnknown;
 	}
+}
+
+void remember(cc_ctx *c) {
+	c->last_E = c->h_stats->entries;
+	c->last_P = c->h_stats->pairs;
+	c->sized = true;
+	c->last_tmp = unsorted_pairs(*c->h_stats, c->direct);
+	c->last_mask = c->h_stats->mask_words;
+	remember_route(c);
 	for (int d = 0; d < 3; d++) c->last_dim[d] = c->h_stats->plan.dim[d];
 }
 
@@ -1282,6 +1287,7 @@ cc_status collide_verlet(cc_ctx *c, const cc_scene &sc, int gx, int gy, int gz, 
 			CC_TRY(read_stats(c, s));
 			CC_TRY(device_err(c));
 			CC_TRY(settle(c, n, scratch, cand, cap, nullptr, s));
+			remember_route(c);
 			uint64_t nc = c->h_stats->pairs;
 			if (nc > cap) {  // more candidates than the list holds: grow it and emit the retained pairs
 				CC_TRY(ensure(c, c->v_cand, sizeof(unsigned long long) * (nc + nc / 8)));
