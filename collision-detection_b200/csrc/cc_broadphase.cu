@@ -137,6 +137,14 @@ __global__ void __launch_bounds__(kNT) k_bounds(uint64_t n, const float *__restr
 	accumulate_stats_one<kNT>(mn, mx, have, stats, pa);
 }
 
+// The plan again for another search grid (the boxes may be shifted already).
+__global__ void k_replan(DevStats *stats, PlanArgs pa) {
+	pa.gx = stats->plan.grid[0];
+	pa.gy = stats->plan.grid[1];
+	pa.gz = stats->plan.grid[2];
+	store_plan(stats, pa);
+}
+
 // The plan a shape is searched with: the block's staged plan (one scene) or
 // its scene's plan (batch).
 template <bool kBatch>
@@ -1750,6 +1758,13 @@ void launch_bounds(uint64_t n, const float *aabb, DevStats *stats, const GridPar
 	pa.gz = grid[2];
 	pa.n = n;
 	if (n) k_bounds<<<blocks_for(n), kNT, 0, s>>>(n, aabb, stats, pa, zero);
+}
+
+void launch_replan(uint64_t n, const BpBuffers &b, const GridParams &gp, cudaStream_t s) {
+	PlanArgs pa;
+	pa.gp = gp;
+	pa.n = n;
+	k_replan<<<1, 1, 0, s>>>(b.stats, pa);
 }
 
 void launch_count(uint64_t n, float *aabb, const BpBuffers &b, cudaStream_t s, bool shift) {

@@ -495,6 +495,14 @@ cc_status direct_prepare(cc_ctx *c) {
 // and 1270, 1.5M 2257 and 2222; 2.5M 4800 and 4848, 4.2M 10360 and 10803.
 constexpr uint64_t kCrowdedFine = (uint64_t)1 << 21;
 
+// The search grid of the call's route.
+GridParams route_grid(const cc_ctx *c, uint64_t n, bool batch) {
+	GridParams gp = c->gp;
+	if (c->chain) gp.k_target *= kChainCellTarget;
+	if (c->direct && !batch && n <= kCrowdedFine) gp.k_target *= 0.5f;
+	return gp;
+}
+
 // Room to ask for where the last call used `used` and there is room for `room`.
 uint64_t with_slack(uint64_t used, uint64_t room) { return used + used / 16 <= room ? room : used + used / 4; }
 
@@ -537,9 +545,7 @@ cc_status size_scratch(cc_ctx *c, uint64_t n, uint64_t np_cap, bool batch) {
 		c->key_bits = 32;
 	}
 	c->fused_now = !c->direct && fused_sort_enabled() && fused_sort_fits(owner_buckets(n, c->owner_shift));
-	c->call_gp = c->gp;
-	if (c->chain) c->call_gp.k_target *= kChainCellTarget;
-	if (c->direct && !batch && n <= kCrowdedFine) c->call_gp.k_target *= 0.5f;
+	c->call_gp = route_grid(c, n, batch);
 	CC_TRY(ensure(c, c->stats, sizeof(DevStats)));
 	CC_TRY(ensure(c, c->cell_count, sizeof(uint32_t) * c->gp.g_max));
 	CC_TRY(ensure(c, c->owner_count, sizeof(uint32_t) * std::max<uint64_t>(n, 1)));
@@ -916,12 +922,15 @@ cc_status settle(cc_ctx *c, uint64_t n, float *aabb, unsigned long long *out, ui
 			c->chain = false;
 			c->chain_state = cc_ctx::kChainNo;
 			c->chain_wait = c->h_stats->dense_items && c->gp.dense_cell <= kChainLong ? 0 : kChainWait;
-			c->dense_skip = false;
-			c->direct = true;
-			c->fused_now = false;
-			if (c->sm.plans) {
-				c->owner_shift = 0;
-				c->key_bits = 32;
+			// where no cell was crowded, only a box too wide, the plain sorted search will do
+			c->dense_skip = c->chain_check && c->h_stats->dense_items == 0;
+			c->direct = !c->dense_skip;
+			if (c->direct) {
+				c->fused_now = false;
+				if (c->sm.plans) {
+					c->owner_shift = 0;
+					c->key_bits = 32;
+				}
 			}
 		}
 		cc_status st = route_prepare(c, n);
@@ -936,6 +945,14 @@ cc_status settle(cc_ctx *c, uint64_t n, float *aabb, unsigned long long *out, ui
 		if (P > b.pair_cap) CC_TRY(ensure(c, c->pairs_tmp, sizeof(unsigned long long) * (P + P / 8)));
 		CC_TRY(reset_pass_counters(c, n, s));
 		c->chain_check = c->chain_check && c->chain;
+		// A crowded or wide scene is searched again on the sorted cells' own, larger grid. First
+		// calls over a floor, on the chains' grid with the dense-cell test and so, ms: 3K bodies,
+		// three class calls, 1.96 and 1.20; 60K, the same, 12.4 and 7.5, a step 14.1 and 9.4.
+		if (crowded && !c->sm.plans) {
+			c->call_gp = route_grid(c, n, false);
+			launch_replan(n, bp_buffers(c), c->call_gp, s);
+			c->launches += 1;
+		}
 		enqueue_pairs(c, n, aabb, E, s, false);
 		if (!c->fused_now) {
 			launch_scan_owner(n, bp_buffers(c), s);

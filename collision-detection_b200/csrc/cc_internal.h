@@ -250,6 +250,8 @@ __host__ __device__ inline uint64_t owner_buckets(uint64_t n, int shift) {
 // Bounds pass over caller AABBs; its last block writes stats->plan.
 void launch_bounds(uint64_t n, const float *aabb, DevStats *stats, const GridParams &gp, const int grid[3],
                    cudaStream_t s, const ZeroList &zero = ZeroList());
+// The pass's plan for another search grid, from its bounds (one scene).
+void launch_replan(uint64_t n, const BpBuffers &b, const GridParams &gp, cudaStream_t s);
 // In-place shift + per-cell counts on the plan's search grid.
 // (shift false: the boxes are shifted already).
 void launch_count(uint64_t n, float *aabb, const BpBuffers &b, cudaStream_t s, bool shift = true);

@@ -68,6 +68,21 @@ struct PlanArgs {
 	uint64_t n;
 };
 
+// The plan from the complete reduction (one thread).
+__device__ inline void store_plan(DevStats *stats, const PlanArgs &pa) {
+	uint32_t bmin_inv[3], bmax[3];
+	double ext_mean[3];
+	const unsigned long long cnt = __ldcg(&stats->ext_count);
+	for (int d = 0; d < 3; d++) {
+		bmin_inv[d] = __ldcg(&stats->bmin_inv[d]);
+		bmax[d] = __ldcg(&stats->bmax[d]);
+		ext_mean[d] = __ldcg(&stats->ext_sum[d]) / (double)(cnt ? cnt : 1);
+	}
+	const Plan p = make_plan(bmin_inv, bmax, __ldcg(&stats->err), ext_mean, pa.gp, pa.gx, pa.gy, pa.gz, pa.n);
+	stats->plan = p;
+	stats->cells = p.G;
+}
+
 // Every thread of the block calls this once with the bounds of the boxes it
 // saw (mn/mx; `have` false if none), its error bits, and the sum of those
 // boxes' extents (esum) over ecnt boxes for the grid tuner's mean extent.
@@ -141,18 +156,7 @@ __device__ __forceinline__ void accumulate_stats(float3 mn, float3 mx, bool have
 	__syncthreads();
 	if (s_last && threadIdx.x == 0) {
 		__threadfence();
-		uint32_t bmin_inv[3], bmax[3];
-		double ext_mean[3];
-		const unsigned long long cnt = __ldcg(&stats->ext_count);
-		for (int d = 0; d < 3; d++) {
-			bmin_inv[d] = __ldcg(&stats->bmin_inv[d]);
-			bmax[d] = __ldcg(&stats->bmax[d]);
-			ext_mean[d] = __ldcg(&stats->ext_sum[d]) / (double)(cnt ? cnt : 1);
-		}
-		const uint32_t err = __ldcg(&stats->err);
-		Plan p = make_plan(bmin_inv, bmax, err, ext_mean, pa.gp, pa.gx, pa.gy, pa.gz, pa.n);
-		stats->plan = p;
-		stats->cells = p.G;
+		store_plan(stats, pa);
 	}
 }
 
