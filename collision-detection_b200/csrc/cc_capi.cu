@@ -77,7 +77,7 @@ struct cc_ctx {
 	// device scratch
 	Buf stats, cell_count, cell_start, entries, owner_count, owner_off, pairs_tmp, status, ticket, big_list, dense;
 	Buf ref_cnt, ref_off, ref_keys, ref_tmp, ref_flags, ref_runpos, rx_hist, rx_hoff;
-	Buf np_norm, np_pa, np_pb, np_depth, np_ids, np_pairs, np_flag, np_pos, np_order, np_classes, np_bsum;
+	Buf np_norm, np_pa, np_pb, np_depth, np_ids, np_pairs, np_flag, np_order, np_classes, np_bsum;
 	Buf bp_bsum;  // block sums of the cooperative cell scan
 	Buf cell_cs;  // packed (start, cursor) words of the cells
 	Buf sorted, sorted_body, row_count, masks;  // entries of dense cells in body order, their pairs as rows, hit masks
@@ -174,7 +174,7 @@ struct cc_ctx {
 	int hs_next = 0, hs_oldest = 0, hs_inflight = 0;
 	// look-back status regions (words) of the cell, owner and contact-flag
 	// scans, laid out back to back in `status`
-	uint64_t st_words[3] = {0, 0, 0};
+	uint64_t st_words[2] = {0, 0};
 	// incremental broadphase (cc_set_incremental, cc_verlet.cu): the sorted
 	// candidate pairs of the boxes inflated by inc_margin mean extents, the
 	// rebuild's unshifted boxes, a copy of the current step's unshifted boxes,
@@ -419,7 +419,7 @@ void choose_owner_shift(cc_ctx *c, uint64_t n) {
 // 256 bytes).
 size_t status_words_for(uint64_t n) { return (scan_tiles(n) + 8 + 31) & ~size_t(31); }
 cc_status ensure_status(cc_ctx *c) {
-	return ensure(c, c->status, sizeof(uint64_t) * (c->st_words[0] + c->st_words[1] + c->st_words[2]));
+	return ensure(c, c->status, sizeof(uint64_t) * (c->st_words[0] + c->st_words[1]));
 }
 
 // Narrowphase scratch for up to P pairs.
@@ -432,13 +432,10 @@ cc_status np_prepare(cc_ctx *c, uint64_t P) {
 	CC_TRY(ensure(c, c->np_ids, 8 * P));
 	CC_TRY(ensure(c, c->np_pairs, 8 * P));
 	CC_TRY(ensure(c, c->np_flag, 4 * P));
-	CC_TRY(ensure(c, c->np_pos, 8 * (P + 1)));
 	CC_TRY(ensure(c, c->np_order, 4 * P));
 	CC_TRY(ensure(c, c->np_classes, (2 * kNpClasses + 32) * sizeof(uint32_t)));
 	CC_TRY(ensure(c, c->np_bsum, kNpCoopBlocks * sizeof(unsigned long long)));
 	CC_TRY(ensure(c, c->stats, sizeof(DevStats)));
-	c->st_words[2] = std::max<uint64_t>(c->st_words[2], status_words_for(P + 1));
-	CC_TRY(ensure_status(c));
 	CC_TRY(ensure(c, c->ticket, 64));
 	return CC_OK;
 }
@@ -605,9 +602,6 @@ NpScratch np_scratch(cc_ctx *c) {
 	sc.ids = ptr<int32_t>(c->np_ids);
 	sc.pairs = ptr<unsigned long long>(c->np_pairs);
 	sc.flag = ptr<uint32_t>(c->np_flag);
-	sc.pos = ptr<unsigned long long>(c->np_pos);
-	sc.status = ptr<uint64_t>(c->status) + c->st_words[0] + c->st_words[1];
-	sc.ticket = ptr<uint32_t>(c->ticket) + 8;
 	sc.bar_classes = ptr<DevStats>(c->stats)->bar_np;
 	sc.bar_compact = ptr<DevStats>(c->stats)->bar_compact;
 	sc.block_sums = ptr<unsigned long long>(c->np_bsum);
@@ -861,7 +855,7 @@ ZeroList allocated(ZeroList zero) {
 ZeroList pass_zero_list(cc_ctx *c, bool ov) {
 	ZeroList zero;
 	zero.p[0] = ptr<uint32_t>(c->status);
-	zero.words[0] = 2 * (c->st_words[0] + c->st_words[1] + c->st_words[2]);
+	zero.words[0] = 2 * (c->st_words[0] + c->st_words[1]);
 	zero.p[1] = ptr<uint32_t>(c->ticket);
 	zero.words[1] = 16;
 	zero.p[2] = ptr<uint32_t>(c->np_classes);
@@ -1176,7 +1170,7 @@ cc_status collide_enqueue(cc_ctx *c, const cc_scene &sc, int gx, int gy, int gz,
 	}
 	// everything the captured launches depend on
 	struct {
-		uint64_t n, nb, pairs_cap, hE, hP, gen, st[3];
+		uint64_t n, nb, pairs_cap, hE, hP, gen, st[2];
 		const void *p[18];
 		int dims[3], prec, oshift, kbits, ov, fused, dense_skip, chain;
 		float env;
@@ -1185,7 +1179,7 @@ cc_status collide_enqueue(cc_ctx *c, const cc_scene &sc, int gx, int gy, int gz,
 	} k;
 	memset(&k, 0, sizeof(k));
 	k.n = n; k.nb = sc.nb; k.pairs_cap = pairs_cap; k.hE = hint_E(c, n); k.hP = hint_P(c, n); k.gen = c->buf_gen;
-	for (int r = 0; r < 3; r++) k.st[r] = c->st_words[r];
+	for (int r = 0; r < 2; r++) k.st[r] = c->st_words[r];
 	const void *ps[18] = {sc.T, sc.A, sc.B, sc.C, sc.R, sc.ID, sc.active, sc.body_pos, sc.body_rot, aabb,
 	                      pairs, norm, cpta, cptb, depth, bids, nullptr, nullptr};
 	memcpy(k.p, ps, sizeof(ps));
@@ -1454,7 +1448,7 @@ void cc_ctx_destroy(cc_ctx *c) {
 	               &c->ref_off,
 	               &c->ref_keys, &c->ref_tmp,    &c->ref_flags,  &c->ref_runpos, &c->rx_hist,   &c->rx_hoff,
 	               &c->np_norm,  &c->np_pa,      &c->np_pb,      &c->np_depth, &c->np_ids,      &c->np_pairs,
-	               &c->np_flag,  &c->np_pos,     &c->np_order, &c->np_classes, &c->in_T,       &c->in_A,     &c->in_B,        &c->in_C,
+	               &c->np_flag,  &c->np_order, &c->np_classes, &c->in_T,       &c->in_A,     &c->in_B,        &c->in_C,
 	               &c->in_R,     &c->in_ID,      &c->in_pos,     &c->in_rot,   &c->in_act,      &c->out_aabb,
 	               &c->out_pairs, &c->out_norm,  &c->out_pa,     &c->out_pb,   &c->out_depth,   &c->out_bids,
 	               &c->b_off,    &c->b_scene_of, &c->b_gid,      &c->b_sst,    &c->b_plans,
@@ -1935,7 +1929,7 @@ cc_status batch_impl(cc_ctx *c, const cc_batch *bt, int gx, int gy, int gz, floa
 	// everything the pass's launches depend on (the offsets' contents are
 	// copied in before every pass, outside the graph)
 	struct {
-		uint64_t n, nb, S, pairs_cap, hE, hP, gen, st[3];
+		uint64_t n, nb, S, pairs_cap, hE, hP, gen, st[2];
 		const void *p[18];
 		int dims[3], prec, want, chain, oshift, kbits, ov, fused, dense_skip;
 		float env;
@@ -1945,7 +1939,7 @@ cc_status batch_impl(cc_ctx *c, const cc_batch *bt, int gx, int gy, int gz, floa
 	memset(&k, 0, sizeof(k));
 	k.n = n; k.nb = sc.nb; k.S = S; k.pairs_cap = pairs_cap; k.hE = hint_E(c, n); k.hP = hint_P(c, n);
 	k.gen = c->buf_gen;
-	for (int r = 0; r < 3; r++) k.st[r] = c->st_words[r];
+	for (int r = 0; r < 2; r++) k.st[r] = c->st_words[r];
 	const void *ps[18] = {sc.T, sc.A, sc.B, sc.C, sc.R, sc.ID, sc.active, sc.body_pos, sc.body_rot, res->aabb,
 	                      res->pairs, res->norm, res->cpta, res->cptb, res->depth, res->bids, src, d_off};
 	memcpy(k.p, ps, sizeof(ps));

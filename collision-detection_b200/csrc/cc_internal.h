@@ -426,16 +426,13 @@ struct NpScratch {
 	int32_t *ids;           // 2 * P
 	unsigned long long *pairs;  // P (copy of the input keys)
 	uint32_t *flag;         // P
-	unsigned long long *pos;  // P + 1
-	uint64_t *status;       // look-back tiles of the flag scan
-	uint32_t *ticket;
 	uint32_t *err;
 	uint32_t *order;        // P: pair indices grouped by (type A, type B); null for the MPR: not grouped
 	uint32_t *classes;      // 2 * kNpClasses counters + the work-queue counter (zeroed per call)
 	uint32_t *queue;        // the exact MPR's work queue (zeroed per call)
 	DevStats *stats = nullptr;       // with host_stats (mapped host memory, may be null): the last
 	uint32_t *host_stats = nullptr;  // kernel reports the pass's counters there
-	bool pre_zeroed = false;  // classes, queue, status and ticket already zeroed for this pass
+	bool pre_zeroed = false;  // classes and queue already zeroed for this pass
 	void *bar_classes = nullptr;  // grid barriers (GridBarrier) of the cooperative class sort and compaction,
 	void *bar_compact = nullptr;  // zeroed at the start of the call
 	unsigned long long *block_sums = nullptr;  // per-block flag counts of the compaction (>= its grid)

@@ -306,10 +306,6 @@ __device__ __forceinline__ D3 vd(vec<S> pb, vec<S> pa) { return sub(cvt<double>(
 template <class S>
 __device__ __forceinline__ D3 dd(vec<S> a) { return cvt<double>(a); }
 
-struct Outputs {
-	const NpScratch *sc;
-};
-
 __device__ __forceinline__ void st3(float *p, uint64_t i, D3 v) {
 	p[3 * i] = (float)v.x;
 	p[3 * i + 1] = (float)v.y;

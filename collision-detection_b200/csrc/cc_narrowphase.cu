@@ -252,10 +252,7 @@ __global__ void __launch_bounds__(kCoopNT) k_np_compact(uint64_t P_cap, const un
 		if (b < blockIdx.x) run += v;
 	}
 	block_sum2(run, nh, sm);
-	if (blockIdx.x == 0 && threadIdx.x == 0) {
-		if (!kSorted) sc.pos[P] = nh;
-		if (contacts_out) *contacts_out = nh;
-	}
+	if (blockIdx.x == 0 && threadIdx.x == 0 && contacts_out) *contacts_out = nh;
 	report_by_last(sc.stats, sc.host_stats);
 	for (uint64_t t0 = c0; t0 < c1; t0 += kCoopNT) {
 		const uint64_t i = t0 + threadIdx.x;
@@ -275,7 +272,6 @@ __global__ void __launch_bounds__(kCoopNT) k_np_compact(uint64_t P_cap, const un
 		const uint32_t r = block_rank(i < c1 && hit, reinterpret_cast<uint32_t *>(sm), tile_total);
 		if (i < c1) {
 			const uint64_t j = run + r;
-			if (!kSorted) sc.pos[i] = j;
 			if (hit) {
 				pairs[j] = (long long)key;
 #pragma unroll
@@ -487,7 +483,6 @@ void launch_np_compact(uint64_t P_cap, const unsigned long long *P_dev, const Np
                        float *norm, float *cpta, float *cptb, float *depth, int32_t *bids,
                        unsigned long long *contacts_out, uint64_t P_hint, cudaStream_t s) {
 	if (!P_cap) {
-		cudaMemsetAsync(sc.pos, 0, sizeof(unsigned long long), s);
 		if (contacts_out) cudaMemsetAsync(contacts_out, 0, sizeof(unsigned long long), s);
 		return;
 	}
