@@ -172,8 +172,8 @@ struct cc_ctx {
 	cudaStream_t hs_copy = nullptr, hs_comp = nullptr, hs_out = nullptr;
 	cudaEvent_t hs_user = nullptr, hs_back = nullptr;
 	int hs_next = 0, hs_oldest = 0, hs_inflight = 0;
-	// look-back status regions (words) of the cell, owner and contact-flag
-	// scans, laid out back to back in `status`
+	// look-back status regions (words) of the cell and owner scans, laid out
+	// back to back in `status`
 	uint64_t st_words[2] = {0, 0};
 	// incremental broadphase (cc_set_incremental, cc_verlet.cu): the sorted
 	// candidate pairs of the boxes inflated by inc_margin mean extents, the
@@ -2142,8 +2142,6 @@ cc_status host_copy_out(cc_ctx *c, cc_ctx::HostSlot &h, cc_result *res, uint64_t
 	return CC_OK;
 }
 
-// The six shape arrays of a host step (T, A, B, C, R, ID) into dst, unless
-// static shapes are on and dst already holds these host arrays' contents.
 // The device address of a pinned, mapped host array; null for pageable memory.
 const void *mapped_host(const void *p) {
 	static const bool off = [] {
@@ -2159,11 +2157,13 @@ const void *mapped_host(const void *p) {
 	return a.type == cudaMemoryTypeHost ? a.devicePointer : nullptr;
 }
 
-// The six shape arrays to the device. C is read only for CONE and
-// TRIANGLEMESH shapes, so from a pinned host array it is not copied whole:
-// *gather_c receives its device mapping and the caller gathers those shapes'
-// C with launch_gather_c once T is on the device, on its compute stream (a
-// kernel on the copy stream would hold the later copies until the SMs are free).
+// The six shape arrays of a host step (T, A, B, C, R, ID) into dst, unless
+// static shapes are on and dst already holds these host arrays' contents. C is
+// read only for CONE and TRIANGLEMESH shapes, so from a pinned host array it is
+// not copied whole: *gather_c receives its device mapping and the caller gathers
+// those shapes' C with launch_gather_c once T is on the device, on its compute
+// stream (a kernel on the copy stream would hold the later copies until the SMs
+// are free).
 // list: the other arrays are mapped too and join it instead of being copied.
 cc_status upload_shapes(cc_ctx *c, cc_ctx::ShapeCopy &sh, Buf *const dst[6], const cc_scene *sc, cudaStream_t t,
                         const float **gather_c, MoveList *list = nullptr) {

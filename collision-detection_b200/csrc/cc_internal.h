@@ -206,7 +206,7 @@ struct BpBuffers {
 	// ceil(n / 2^owner_shift) buckets. Inside a bucket the sort keys are packed to
 	// 32 bits as ((a mod 2^owner_shift) << key_bits) | b, with key_bits the bits of
 	// n - 1 (owner_shift + key_bits <= 32). owner_shift 0: one bucket per body, keys
-	// are the partner halves b (batches, incremental steps, the clustered scenes).
+	// are the partner halves b (scenes of many pairs a body; crowded batches).
 	int owner_shift = 0;
 	int key_bits = 32;
 	// launch shape of the sparse pair test: entries staged per warp (64, 96 or
@@ -258,18 +258,18 @@ void launch_count(uint64_t n, float *aabb, const BpBuffers &b, cudaStream_t s, b
 void launch_scan_cells(const BpBuffers &b, uint32_t g_max, cudaStream_t s);
 void launch_scatter(uint64_t n, const float *aabb, const BpBuffers &b, cudaStream_t s, bool packed = false);
 void launch_pair_test(uint64_t n, const BpBuffers &b, uint64_t entries_hint, cudaStream_t s);
-// The chained search, for scenes without crowded cells: in-place shift (shift
-// false: done already), entries and the cells' chains in one pass; the pair
-// test along the chains in a second. Entries past entry_cap are counted and
-// dropped (stats->entries tells). check: a pass in between that looks for
-// chains above kChainLong and makes the walk return at once if there are any;
-// without it the walk itself notes them, and gives up (kErrLongChain) only on
-// chains many times as long.
 // Small scenes: the in-place shift alone (with the owner counts zeroed), then
 // every box against every later one.
 constexpr uint64_t kAllPairsBodies = 2048;
 void launch_shift(uint64_t n, float *aabb, const BpBuffers &b, cudaStream_t s, bool shift);
 void launch_all_pairs(uint64_t n, const float *aabb, const BpBuffers &b, cudaStream_t s);
+// The chained search, for scenes without crowded cells: in-place shift (shift
+// false: done already), entries and the cells' chains in one pass; the pair
+// test along the chains in a second. Entries past entry_cap are counted and
+// dropped (stats->entries tells). launch_chain_check: a pass in between that looks
+// for chains above kChainLong and makes the walk return at once if there are any;
+// without it the walk itself notes them, and gives up (kErrLongChain) only on
+// chains many times as long.
 void launch_link(uint64_t n, float *aabb, const BpBuffers &b, cudaStream_t s, bool shift = true);
 void launch_chain_check(const BpBuffers &b, uint32_t g_max, cudaStream_t s);
 void launch_walk(uint64_t n, const BpBuffers &b, uint64_t entries_hint, cudaStream_t s);
@@ -365,9 +365,6 @@ void launch_perturb_scenes(uint32_t count, uint64_t total, const PerturbScene *d
 constexpr size_t kParamChunkBytes = 8192;
 constexpr size_t kParamCopyMax = 64 * 1024;
 cudaError_t copy_small_h2d(void *dst, const void *src, size_t bytes, cudaStream_t s);
-// dst[i] = src[i] (3 floats) for the shapes of type CONE or TRIANGLEMESH, the
-// only ones whose C is read; T is on the device, src a device-accessible
-// (pinned, mapped) host array.
 // Moves whole arrays between mapped host memory and the device in one launch.
 // Array k has fixed + per_pair * np_n + per_contact * contacts bytes (counts of
 // `stats`, whose pass must be complete in `room`: else nothing moves; null: fixed only).
@@ -391,6 +388,9 @@ struct MoveList {
 	}
 };
 void launch_move(const MoveList &m, uint64_t bytes_hint, const DevStats *stats, const PassRoom &room, cudaStream_t s);
+// dst[i] = src[i] (3 floats) for the shapes of type CONE or TRIANGLEMESH, the
+// only ones whose C is read; T is on the device, src a device-accessible
+// (pinned, mapped) host array.
 void launch_gather_c(uint64_t n, const int32_t *T, const float *src, float *dst, cudaStream_t s);
 // The front of a batch pass (cc_aabb.cu): scene_of, global ids, boxes, bounds,
 // plans, cell_base[0..S] and stats->cells; with src the scenes are gathered into
