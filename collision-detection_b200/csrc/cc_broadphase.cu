@@ -1571,7 +1571,7 @@ __global__ void __launch_bounds__(512) k_segsort_big(const DevStats *stats, uint
 // their room.
 constexpr int kFusedNT = 256;
 constexpr int kFusedSeg = 4096;
-constexpr uint32_t kFusedBuckets = 8191;  // offsets + block-tier keys fit the default 48 KB of shared memory
+constexpr uint32_t kFusedBuckets = 8191;  // offsets + block-tier keys are 48 KB; with the static words the launch opts in
 
 template <bool kPack>
 __global__ void __launch_bounds__(kFusedNT, 4) k_owner_sort_fused(DevStats *stats, uint64_t pair_cap, uint64_t out_cap,
@@ -2045,15 +2045,12 @@ void launch_owner_sort_fused(uint64_t n, uint64_t out_cap, unsigned long long *o
                              uint32_t *host_stats, cudaStream_t s) {
 	const uint32_t nbk = (uint32_t)owner_buckets(n, b.owner_shift);
 	const size_t smem = sizeof(uint32_t) * ((size_t)nbk + 1 + kFusedSeg);
-	static const int per_sm = [] {
-		int v = 0;
-		const int most = (int)(sizeof(uint32_t) * ((size_t)kFusedBuckets + 1 + kFusedSeg));
-		if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, k_owner_sort_fused<true>, kFusedNT, most) != cudaSuccess || v < 1)
-			v = 1;
-		return v;
-	}();
+	static std::atomic<uint64_t> done{0};
+	opt_in_shared(done, (int)(sizeof(uint32_t) * ((size_t)kFusedBuckets + 1 + kFusedSeg)), k_owner_sort_fused<true>,
+	              k_owner_sort_fused<false>);
+	// one block an SM at most: every block scans all bucket counts, and the MPR's blocks run beside these
 	const uint64_t want = (std::max<uint64_t>(P_hint, nbk) + kFusedNT - 1) / kFusedNT;
-	unsigned grid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(want, (uint64_t)per_sm * kNumSMs));
+	const unsigned grid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(want, kNumSMs));
 	uint64_t pair_cap = b.pair_cap;
 	const unsigned long long *tmp = b.pairs_tmp;
 	const uint32_t *cnt = b.owner_count;
